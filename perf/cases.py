@@ -67,7 +67,7 @@ def draw(rng):
     # voxel-volumes of the map: up to half of the largest listed case's for a forward, a fifth of that where each
     # costs several times as much or goes through host memory
     units = math.exp(rng.uniform(math.log(1e6), math.log(1.6e9 if kind == "forward" else 2.5e8)))
-    c["T"] = log_int(40, 120) if kind == "batches" else log_int(4, 120)
+    c["T"] = log_int(40, 120) if kind == "batches" else log_int(6, 120)
     if kind == "legacy":
         mag, units = (rng.choice([2, 3, 4, 5]),) * 3, min(units, 4e7)
     side = (units / c["T"] / (mag[0] * mag[1] * mag[2])) ** (1 / 3)
