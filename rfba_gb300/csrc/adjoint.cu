@@ -729,9 +729,9 @@ __global__ void __launch_bounds__(kAdjThreads, 2) radiality_adjoint_kernel(const
         const TileDesc td = p.tiles[tile_i];
         const BlockDev& B = p.blocks[td.block];
         const int bw = B.size[0], bh = B.size[1], bd = B.size[2];
-        const int X0 = B.lo[0] + td.tx * kTileX;
-        const int Y0 = B.lo[1] + td.ty * kAdjRows;
-        const int Z0 = B.zbase + td.tz * FZ;
+        const int X0 = B.lo[0] + td.t[0] * kTileX;
+        const int Y0 = B.lo[1] + td.t[1] * kAdjRows;
+        const int Z0 = B.zbase + td.t[2] * FZ;
         const int cx0 = floordiv(X0, mx) - 2;
         const int cy0 = floordiv(Y0, my) - 2;
         const int cz0 = Z0 / MZ - 2;

@@ -127,6 +127,15 @@ static int ensure_plan(rfba_ctx* ctx, const rfba_srrf_config& cfg, cudaStream_t 
         set_error("ring has no (0, 0) pair");
         return RFBA_ERR_UNSUPPORTED;
     }
+    if (!build_forward_plan(cfg, &P.fwd, &err)) {
+        set_error(err);
+        return RFBA_ERR_UNSUPPORTED;
+    }
+    while (P.words.size() % 4) P.words.push_back(0.f);
+    P.fwd_lane = P.words.size();
+    P.words.insert(P.words.end(), P.fwd.lane.begin(), P.fwd.lane.end());
+    P.fwd_utab = P.words.size();
+    P.words.insert(P.words.end(), P.fwd.utab.begin(), P.fwd.utab.end());
     const int rc = ctx->tables.ensure(P.words.size() * 4, "tables");
     if (rc) return rc;
     RFBA_CUDA(cudaMemcpyAsync(ctx->tables.p, P.words.data(), P.words.size() * 4, cudaMemcpyHostToDevice, st),
@@ -137,8 +146,6 @@ static int ensure_plan(rfba_ctx* ctx, const rfba_srrf_config& cfg, cudaStream_t 
     P.valid = true;
     return RFBA_OK;
 }
-
-static int fz_for(int mz) { return mz * cz_for_mag(mz); }
 
 // Order this call's work after the previous call's when the streams differ.
 int order_streams(rfba_ctx* ctx, cudaStream_t st) {
@@ -157,7 +164,12 @@ static int make_blocks(rfba_ctx* ctx, const rfba_srrf_config& cfg, const int dim
                        int nblocks, std::vector<BlockDev>* outb, int ty = 0, int tb = 0, int fields = 0) {
     const RingPlan& rp = ctx->plan.ring;
     const int T = dims[3];
-    const int FZ = fz_for(cfg.mag[2]);
+    // z slabs are whole tiles deep
+    const FwdPlan& fp = ctx->plan.fwd;
+    std::vector<std::array<int, 2>> depth;
+    for (int i = 0; i < nblocks; ++i) depth.push_back({blocks[i].lo[fp.ax2], blocks[i].hi[fp.ax2]});
+    const int cz = forward_depth(fp, depth);
+    const int FZ = fp.ax2 == 2 ? fp.mag[2] * cz : (ty > 0 ? ty : kTileRows);
     outb->clear();
     // bytes per subvoxel: the stacks of the volumes held at once plus the
     // carried temporal state when the series runs in time batches
@@ -185,6 +197,7 @@ static int make_blocks(rfba_ctx* ctx, const rfba_srrf_config& cfg, const int dim
             fine_window_int(cfg.mag[a], b.size[a], &d.int_lo[a], &d.int_hi[a]);
         }
         if (b.hi[0] <= b.lo[0] || b.hi[1] <= b.lo[1] || b.hi[2] <= b.lo[2]) continue;
+        d.cz = cz;
         d.out_offset = b.out_offset;
         for (int a = 0; a < 3; ++a) d.out_stride[a] = b.out_stride[a];
         // z slabs under the budget
@@ -198,10 +211,7 @@ static int make_blocks(rfba_ctx* ctx, const rfba_srrf_config& cfg, const int dim
             s.out_offset = d.out_offset + (long long)(z0 - b.lo[2]) * d.out_stride[2];
             for (int a = 0; a < 3; ++a) s.nreg[a] = s.hi[a] - s.lo[a];
             s.zbase = (s.lo[2] / cfg.mag[2]) * cfg.mag[2];
-            const int TY = ty > 0 ? ty : tile_rows_for_mag(cfg.mag[1]);
-            s.ntile[0] = (s.nreg[0] + kTileX - 1) / kTileX;
-            s.ntile[1] = (s.nreg[1] + TY - 1) / TY;
-            s.ntile[2] = (s.hi[2] - s.zbase + FZ - 1) / FZ;
+            forward_tiles(fp, ty, &s);
             s.vox = (long long)s.nreg[0] * s.nreg[1] * s.nreg[2];
             outb->push_back(s);
         }
@@ -211,10 +221,20 @@ static int make_blocks(rfba_ctx* ctx, const rfba_srrf_config& cfg, const int dim
 
 static size_t elem_size(rfba_dtype dt) { return dt == RFBA_U16 ? 2 : 4; }
 
-// Kernel parameters common to the forward and adjoint radiality kernels
-// (everything but the block / tile lists and the schedule).
+// Forward kernel parameters: everything but the block / tile lists and the schedule.
+static FwdParams fill_fwd_params(rfba_ctx* ctx, const rfba_srrf_config& cfg, const void* in_dev, rfba_dtype dtype,
+                                 const int dims[4], int ty, int cz) {
+    const PlanCache& P = ctx->plan;
+    FwdParams p = forward_params(P.fwd, cfg, in_dev, dtype == RFBA_U16, dims, ty, cz);
+    const float* t = static_cast<const float*>(ctx->tables.p);
+    p.lane = t + P.fwd_lane;
+    p.utab = reinterpret_cast<const float4*>(t + P.fwd_utab);
+    return p;
+}
+
+// Adjoint kernel parameters (everything but the block / tile lists and the schedule).
 static RadParams fill_rad_params(rfba_ctx* ctx, const rfba_srrf_config& cfg, const void* in_dev, const int dims[4],
-                                 int CZ, int ty = 0) {
+                                 int CZ) {
     const PlanCache& P = ctx->plan;
     const int T = dims[3];
     RadParams rp;
@@ -248,7 +268,7 @@ static RadParams fill_rad_params(rfba_ctx* ctx, const rfba_srrf_config& cfg, con
         rp.grad_mode = 2;
     else
         rp.grad_mode = 0;
-    rp.TY = ty > 0 ? ty : tile_rows_for_mag(cfg.mag[1]);
+    rp.TY = kAdjRows;
     rp.NU = (kTileX - 1) / cfg.mag[0] + 2 + 4;
     rp.NV = (rp.TY - 1) / cfg.mag[1] + 2 + 4;
     rp.NW = CZ + 4;
@@ -278,16 +298,16 @@ static int plan_passes(rfba_ctx* ctx, const rfba_srrf_config& cfg, rfba_dtype dt
     ps->passes.clear();
     ps->max_stack = 0;
     ps->max_vox = 0;
-    ps->ty = tune.ty > 0 ? tune.ty : tile_rows_for_mag(cfg.mag[1]);
-    RadParams rp = fill_rad_params(ctx, cfg, nullptr, dims, cz_for_mag(cfg.mag[2]), ps->ty);
-    rp.tma_bx = radiality_tma_box_x(rp, dtype == RFBA_U16);
+    ps->ty = tune.ty > 0 ? tune.ty : kTileRows;
+    ps->cz = all.empty() ? 4 : all[0].cz;
+    const FwdParams rp = fill_fwd_params(ctx, cfg, nullptr, dtype, dims, ps->ty, ps->cz);
     const size_t smem = radiality_smem_bytes(rp);
     if (smem > 227 * 1024) {
         set_error("shared memory tile too large for this configuration");
         return RFBA_ERR_UNSUPPORTED;
     }
     int per_sm = 0;
-    int ce = radiality_max_ctas_per_sm(rp, dtype == RFBA_U16, &per_sm);
+    int ce = radiality_max_ctas_per_sm(rp, &per_sm);
     if (ce != 0) return cuda_fail((cudaError_t)ce, "occupancy");
     if (per_sm < 1) {
         set_error("radiality kernel does not fit on an SM");
@@ -398,8 +418,7 @@ static int enqueue_passes(rfba_ctx* ctx, const rfba_srrf_config& cfg, const void
     for (size_t i = 0; i < ps.passes.size(); ++i) {
         const PassPlan& pp = ps.passes[i];
         unsigned int* counter = dcounters + 64 * i;
-        RadParams rp = fill_rad_params(ctx, cfg, in_dev, dims, cz_for_mag(cfg.mag[2]), ps.ty);
-        rp.tma_bx = radiality_tma_box_x(rp, dtype == RFBA_U16);
+        FwdParams rp = fill_fwd_params(ctx, cfg, in_dev, dtype, dims, ps.ty, ps.cz);
         rp.err = static_cast<unsigned long long*>(ctx->errw.p);
         rp.test_skip_copy = test_tma_stall();
         rp.blocks = dblocks + pp.b0;
@@ -453,7 +472,7 @@ static int enqueue_passes(rfba_ctx* ctx, const rfba_srrf_config& cfg, const void
         const bool windows = win && ps.tb == 0 && ps.passes.size() == 1;
         const int nlaunch = windows ? win->n : ps.nbatch;
         for (int b = 0; b < nlaunch; ++b) {
-            RadParams rb = rp;
+            FwdParams rb = rp;
             if (windows) {
                 rb.t_lo = win->t[b];
                 rb.t_hi = win->t[b + 1];
@@ -467,7 +486,7 @@ static int enqueue_passes(rfba_ctx* ctx, const rfba_srrf_config& cfg, const void
             rb.nitems = (long long)rb.ntiles * rb.nchunks;
             const int grid = (int)std::max<long long>(1, std::min<long long>(pp.grid, rb.nitems));
             RFBA_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned int), st), "counter reset");
-            int le = launch_radiality(rb, grid, pp.smem, dtype == RFBA_U16, st);
+            int le = launch_radiality(rb, ctx->plan.fwd, grid, pp.smem, st);
             if (le != 0) return cuda_fail((cudaError_t)le, "radiality launch");
             if (ps.tb > 0) {
                 const bool last = b == ps.nbatch - 1;
@@ -644,18 +663,13 @@ static std::string sched_key(const rfba_srrf_config& cfg, rfba_dtype dtype, cons
     return k;
 }
 
-// Autotuner: time every candidate schedule (tile rows valid for mag_y, and for
+// Autotuner: time every candidate schedule (tile rows, and for
 // block lists the two tile orders) on the first few volumes of this call's
 // own input, keep the fastest.
 static int autotune(rfba_ctx* ctx, const rfba_srrf_config& cfg, const void* in_dev, rfba_dtype dtype,
                     const int dims[4], const rfba_block* blocks, int nblocks, float* out_dev, cudaStream_t st,
                     Tuning* best) {
-    const int my = cfg.mag[1];
-    std::vector<int> tys;
-    for (int ty : {8, 12, 16, 24})
-        if (ty % (2 * my) == 0 && ty * (kTileX / 2) <= kMaxThreads) tys.push_back(ty);
-    const int dty = tile_rows_for_mag(my);
-    if (std::find(tys.begin(), tys.end(), dty) == tys.end()) tys.push_back(dty);
+    const std::vector<int> tys = {kTileRows, 2 * kTileRows};
     std::vector<int> orders = {0};
     if (nblocks > 1) orders.push_back(1);
     const int sd[4] = {dims[0], dims[1], dims[2], std::min(dims[3], 3)};
@@ -754,7 +768,7 @@ static int forward_blocks_locked(rfba_ctx* ctx, const rfba_srrf_config* cfg, con
         work += b.vox * dims[3];
     }
     const size_t in_bytes = (size_t)dims[0] * dims[1] * dims[2] * dims[3] * elem_size(dtype);
-    ctx->last_ty = tile_rows_for_mag(cfg->mag[1]);
+    ctx->last_ty = kTileRows;
     ctx->last_order = 0;
     ctx->last_graph = 0;
     ctx->last_tuned = 0;
@@ -782,11 +796,11 @@ static int forward_blocks_locked(rfba_ctx* ctx, const rfba_srrf_config* cfg, con
             ctx->tunes[tkey] = std::make_pair(tune.ty, tune.order);
             ctx->last_tuned = 1;
         }
-        if (tune.ty > 0 && tune.ty != tile_rows_for_mag(cfg->mag[1]) &&
+        if (tune.ty > 0 && tune.ty != kTileRows &&
             (s = make_blocks(ctx, *cfg, dims, blocks, nblocks, &all, tune.ty, tb, tfields)))
             return s;
         tune.tb = tb;
-        ctx->last_ty = tune.ty > 0 ? tune.ty : tile_rows_for_mag(cfg->mag[1]);
+        ctx->last_ty = tune.ty > 0 ? tune.ty : kTileRows;
         ctx->last_order = tune.order;
         // replay: the whole call as one CUDA graph (device pointers, or pinned host buffers)
         const bool graphable = flags == RFBA_DEVICE_PTRS || (host_pinned(in) && host_pinned(out));
@@ -1190,9 +1204,6 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
         if (e) return cuda_fail((cudaError_t)e, "temporal adjoint launch");
     }
     RadParams rp = fill_rad_params(ctx, *cfg, iprime, dims, cza_for_mag(cfg->mag[2]));
-    rp.TY = kAdjRows;
-    rp.NV = (kAdjRows - 1) / cfg->mag[1] + 2 + 4;
-    rp.NIY = rp.NV + 2 * rp.R;
     rp.blocks = dblk;
     rp.tiles = static_cast<const TileDesc*>(ctx->atiles.p);
     rp.ntiles = (int)tiles.size();
@@ -1299,8 +1310,7 @@ static int backward_batched(rfba_ctx* ctx, const rfba_srrf_config* cfg, const fl
         RFBA_CUDA(cudaMemcpyAsync(ctx->tiles.p, ps.tiles.data(), ps.tiles.size() * sizeof(TileDesc),
                                   cudaMemcpyHostToDevice, st), "tiles upload");
         const BlockDev* dblk = static_cast<const BlockDev*>(ctx->blocks.p);
-        RadParams rp = fill_rad_params(ctx, scfg, ip, dims, cz_for_mag(scfg.mag[2]), ps.ty);
-        rp.tma_bx = radiality_tma_box_x(rp, 0);
+        FwdParams rp = fill_fwd_params(ctx, scfg, ip, RFBA_F32, dims, ps.ty, ps.cz);
         rp.err = err;
         rp.blocks = dblk;
         rp.tiles = static_cast<const TileDesc*>(ctx->tiles.p);
@@ -1313,7 +1323,7 @@ static int backward_batched(rfba_ctx* ctx, const rfba_srrf_config* cfg, const fl
         blk.stack_off = 0;
         for (int t_lo = 0; t_lo < T; t_lo += tb) {
             const int t_hi = std::min(T, t_lo + tb);
-            RadParams rb = rp;
+            FwdParams rb = rp;
             rb.t_lo = std::max(0, t_lo - h);
             rb.t_hi = std::min(T, t_hi + h);
             rb.stack_t0 = rb.t_lo;
@@ -1321,7 +1331,7 @@ static int backward_batched(rfba_ctx* ctx, const rfba_srrf_config* cfg, const fl
             rb.nitems = (long long)rb.ntiles * rb.nchunks;
             const int grid = (int)std::max<long long>(1, std::min<long long>(pp.grid, rb.nitems));
             RFBA_CUDA(cudaMemsetAsync(ctx->counter.p, 0, sizeof(unsigned int), st), "counter reset");
-            int e = launch_radiality(rb, grid, pp.smem, 0, st);
+            int e = launch_radiality(rb, ctx->plan.fwd, grid, pp.smem, st);
             if (e) return cuda_fail((cudaError_t)e, "radiality launch");
             StreamAdjParams ap;
             std::memset(&ap, 0, sizeof ap);

@@ -48,6 +48,8 @@ struct PlanCache {
     std::vector<float> words;
     TableLayout tl;
     int zero_pair = -1;
+    FwdPlan fwd;
+    size_t fwd_lane = 0, fwd_utab = 0;  // word offsets of the forward tables in the uploaded buffer
 };
 
 // Schedule choices of the forward: tile rows (tile shape) and tile order
@@ -76,7 +78,7 @@ struct PassSet {
     std::vector<PassPlan> passes;
     long long max_stack = 0;
     long long max_vox = 0;
-    int ty = 0;
+    int ty = 0, cz = 4;  // tile rows and innermost cells
     // time batches: the stacks hold tb volumes and the temporal reduction is
     // carried across batches in `fields` floats per subvoxel (tb 0: the whole
     // series at once)

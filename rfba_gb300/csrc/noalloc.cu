@@ -109,9 +109,9 @@ __global__ void static_setup_kernel(const SetupArgs a, BlockDev* blk, TileDesc* 
     for (int i = i0; i < a.ntiles; i += gridDim.x * blockDim.x) {
         TileDesc d;
         d.block = 0;
-        d.tx = i % a.ntile[0];
-        d.ty = (i / a.ntile[0]) % a.ntile[1];
-        d.tz = i / (a.ntile[0] * a.ntile[1]);
+        d.t[0] = i % a.ntile[0];
+        d.t[1] = (i / a.ntile[0]) % a.ntile[1];
+        d.t[2] = i / (a.ntile[0] * a.ntile[1]);
         tiles[i] = d;
     }
 }
@@ -171,14 +171,14 @@ extern "C" int rfba_srrf_forward_static_scratch(const rfba_srrf_config* cfg, con
     TableLayout tl;
     if (!build_ring_plan(*cfg, &ring, &err) || !build_tables(*cfg, ring, &words, &tl, &err))
         return fail(RFBA_ERR_UNSUPPORTED, err);
-    const int zero_pair = ring_zero_pair(ring);
-    if (zero_pair < 0) return fail(RFBA_ERR_UNSUPPORTED, "ring has no (0, 0) pair");
+    if (ring_zero_pair(ring) < 0) return fail(RFBA_ERR_UNSUPPORTED, "ring has no (0, 0) pair");
+    FwdPlan plan;
+    if (!build_forward_plan(*cfg, &plan, &err)) return fail(RFBA_ERR_UNSUPPORTED, err);
+    words = plan.lane;  // lane tables, then the uniform ones
+    words.insert(words.end(), plan.utab.begin(), plan.utab.end());
 
     // the whole volume as one block
     const int T = dims[3];
-    const int mz = cfg->mag[2];
-    const int FZ = mz * cz_for_mag(mz);
-    const int TY = tile_rows_for_mag(cfg->mag[1]);
     BlockDev b;
     std::memset(&b, 0, sizeof b);
     for (int a = 0; a < 3; ++a) {
@@ -191,9 +191,8 @@ extern "C" int rfba_srrf_forward_static_scratch(const rfba_srrf_config* cfg, con
         fine_window_int(cfg->mag[a], dims[a], &b.int_lo[a], &b.int_hi[a]);
     }
     b.zbase = 0;
-    b.ntile[0] = (b.nreg[0] + kTileX - 1) / kTileX;
-    b.ntile[1] = (b.nreg[1] + TY - 1) / TY;
-    b.ntile[2] = (b.hi[2] + FZ - 1) / FZ;
+    b.cz = forward_depth(plan, {{b.lo[plan.ax2], b.hi[plan.ax2]}});
+    forward_tiles(plan, 0, &b);
     b.vox = (long long)b.nreg[0] * b.nreg[1] * b.nreg[2];
     b.stack_off = 0;
     b.out_offset = 0;
@@ -255,46 +254,10 @@ extern "C" int rfba_srrf_forward_static_scratch(const rfba_srrf_config* cfg, con
         if ((s = cuda_ok(cudaGetLastError(), "descriptor set-up"))) return s;
     }
 
-    RadParams rp;
-    std::memset(&rp, 0, sizeof rp);
-    rp.in = in;
-    rp.W = dims[0];
-    rp.H = dims[1];
-    rp.D = dims[2];
-    rp.T = T;
-    for (int a = 0; a < 3; ++a) rp.mag[a] = cfg->mag[a];
-    rp.nxv = (int)ring.xv.size();
-    rp.nyv = (int)ring.yv.size();
-    rp.nzv = (int)ring.zv.size();
-    rp.ngroups = (int)ring.grp_xval.size();
-    rp.npairs = (int)ring.pair_yval.size();
-    rp.npoints = (int)ring.pt_zval.size();
-    rp.zero_pair = zero_pair;
-    if (cfg->gradient_smooth == 0) {
-        rp.gr[0] = 1;
-        rp.gr[1] = rp.gr[2] = rp.gr[3] = 0;
-    } else {
-        rp.gr[0] = cfg->main_range;
-        rp.gr[1] = cfg->x_range;
-        rp.gr[2] = cfg->y_range;
-        rp.gr[3] = cfg->z_range;
-    }
-    rp.R = std::max(std::max(rp.gr[0], rp.gr[1]), std::max(rp.gr[2], rp.gr[3]));
-    rp.grad_mode = (rp.gr[0] == 1 && rp.gr[1] == 1 && rp.gr[2] == 1 && rp.gr[3] == 1)   ? 1
-                   : (rp.gr[0] == 1 && rp.gr[1] == 0 && rp.gr[2] == 0 && rp.gr[3] == 0) ? 2
-                                                                                       : 0;
-    rp.TY = TY;
-    rp.NU = (kTileX - 1) / cfg->mag[0] + 2 + 4;
-    rp.NV = (TY - 1) / cfg->mag[1] + 2 + 4;
-    rp.NW = cz_for_mag(mz) + 4;
-    rp.NIX = rp.NU + 2 * rp.R;
-    rp.NIY = rp.NV + 2 * rp.R;
-    rp.NIZ = rp.NW + 2 * rp.R;
-    rp.renorm = cfg->renormalize == 1;
-    rp.poscon = cfg->remove_con == 1;
-    rp.tables = reinterpret_cast<const float*>(sc + o_tab);
-    rp.tl = tl;
-    rp.smem_table_words = tl.words;
+    FwdParams rp = forward_params(plan, *cfg, in, dtype == RFBA_U16, dims, 0, b.cz);
+    rp.tma_bx = 0;  // plain loads
+    rp.lane = reinterpret_cast<const float*>(sc + o_tab);
+    rp.utab = reinterpret_cast<const float4*>(sc + o_tab) + plan.lane.size() / 4;
     rp.blocks = reinterpret_cast<const BlockDev*>(sc + o_blk);
     rp.tiles = reinterpret_cast<const TileDesc*>(sc + o_til);
     rp.ntiles = (int)ntiles64;
@@ -304,7 +267,7 @@ extern "C" int rfba_srrf_forward_static_scratch(const rfba_srrf_config* cfg, con
     const size_t smem = radiality_smem_bytes(rp);
     if (smem > 227 * 1024) return fail(RFBA_ERR_UNSUPPORTED, "shared memory tile too large for this configuration");
     int per_sm = 0, dev = 0, sms = 0;
-    if ((s = cuda_ok((cudaError_t)radiality_max_ctas_per_sm(rp, dtype == RFBA_U16, &per_sm), "occupancy"))) return s;
+    if ((s = cuda_ok((cudaError_t)radiality_max_ctas_per_sm(rp, &per_sm), "occupancy"))) return s;
     if ((s = cuda_ok(cudaGetDevice(&dev), "cudaGetDevice"))) return s;
     if ((s = cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count"))) return s;
     if (per_sm < 1) return fail(RFBA_ERR_UNSUPPORTED, "radiality kernel does not fit on an SM");
@@ -331,7 +294,7 @@ extern "C" int rfba_srrf_forward_static_scratch(const rfba_srrf_config* cfg, con
     tp.int_stack = rp.int_stack;
     tp.out = out;
 
-    if ((s = cuda_ok((cudaError_t)launch_radiality(rp, grid, smem, dtype == RFBA_U16, st), "radiality launch")))
+    if ((s = cuda_ok((cudaError_t)launch_radiality(rp, plan, grid, smem, st), "radiality launch")))
         return s;
     if ((s = cuda_ok((cudaError_t)launch_temporal(tp, st), "temporal launch"))) return s;
     return RFBA_OK;

@@ -180,33 +180,41 @@ static int value_index(std::vector<float>& vals, float v, float tol) {
     return (int)vals.size() - 1;
 }
 
+// Distinct points of the ring and their multiplicities. Points that coincide up
+// to float rounding of sin/cos (|d| <= 1e-6 r) are one point; coordinates within
+// 1e-6 r of 0 are 0.
+static void distinct_points(float r, const std::vector<float>& rx, const std::vector<float>& ry,
+                            const std::vector<float>& rz, std::vector<std::array<float, 3>>* reps,
+                            std::vector<int>* mult) {
+    const float tol = 1e-6f * r;
+    auto snap = [&](float v) { return std::fabs(v) <= tol ? 0.f : v; };
+    for (size_t i = 0; i < rx.size(); ++i) {
+        const float px = snap(rx[i]), py = snap(ry[i]), pz = snap(rz[i]);
+        int found = -1;
+        for (size_t k = 0; k < reps->size(); ++k)
+            if (std::fabs((*reps)[k][0] - px) <= tol && std::fabs((*reps)[k][1] - py) <= tol &&
+                std::fabs((*reps)[k][2] - pz) <= tol) {
+                found = (int)k;
+                break;
+            }
+        if (found < 0) {
+            reps->push_back({px, py, pz});
+            mult->push_back(1);
+        } else
+            (*mult)[found]++;
+    }
+}
+
 bool build_ring_plan(const rfba_srrf_config& c, RingPlan* rp, std::string* err) {
     const int n = 2 * c.axes_in_ring;
     const float r = c.ring_radius;
     rp->n = n;
     raw_ring(r, n, rp->rx, rp->ry, rp->rz);
     rp->npoints_raw = n * n;
-    // Points that coincide up to float rounding of sin/cos (|d| <= 1e-6 r) are
-    // one point with a multiplicity; coordinates within 1e-6 r of 0 are 0.
     const float tol = 1e-6f * r;
-    auto snap = [&](float v) { return std::fabs(v) <= tol ? 0.f : v; };
     std::vector<std::array<float, 3>> reps;
     std::vector<int> mult;
-    for (int i = 0; i < n * n; ++i) {
-        const float px = snap(rp->rx[i]), py = snap(rp->ry[i]), pz = snap(rp->rz[i]);
-        int found = -1;
-        for (size_t k = 0; k < reps.size(); ++k)
-            if (std::fabs(reps[k][0] - px) <= tol && std::fabs(reps[k][1] - py) <= tol &&
-                std::fabs(reps[k][2] - pz) <= tol) {
-                found = (int)k;
-                break;
-            }
-        if (found < 0) {
-            reps.push_back({px, py, pz});
-            mult.push_back(1);
-        } else
-            mult[found]++;
-    }
+    distinct_points(r, rp->rx, rp->ry, rp->rz, &reps, &mult);
     // distinct axis values, sorted
     std::vector<float> xv, yv, zv;
     for (auto& p : reps) {
@@ -410,6 +418,298 @@ bool build_tables(const rfba_srrf_config& c, const RingPlan& rp, std::vector<flo
     align4();
     tl->words = (int)W.size();
     return true;
+}
+
+// ---------------------------------------------------------------------------
+// Forward plan
+
+bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err) {
+    const int n = 2 * c.axes_in_ring;
+    const float r = c.ring_radius, tol = 1e-6f * r;
+    std::vector<float> raw[3];
+    raw_ring(r, n, raw[0], raw[1], raw[2]);
+    std::vector<std::array<float, 3>> reps;
+    std::vector<int> mult;
+    distinct_points(r, raw[0], raw[1], raw[2], &reps, &mult);
+    struct P {
+        int a, b, c, m;
+        double u[3];
+    };
+    // one order of the axes: distinct values, points grouped by mid and then x
+    // value, and the pairs' start indices
+    struct Order {
+        std::vector<float> val[3];
+        std::vector<P> pts;
+        std::vector<int> pair0;
+    };
+    auto arrange = [&](int a1, int a2) {
+        Order o;
+        const int ax[3] = {0, a1, a2};
+        for (int k = 0; k < 3; ++k) {
+            for (auto& p : reps) value_index(o.val[k], p[ax[k]], tol);
+            value_index(o.val[k], 0.f, tol);  // the intensity's sample
+            std::sort(o.val[k].begin(), o.val[k].end());
+        }
+        for (size_t i = 0; i < reps.size(); ++i) {
+            P p;
+            p.a = value_index(o.val[0], reps[i][0], tol);
+            p.b = value_index(o.val[1], reps[i][a1], tol);
+            p.c = value_index(o.val[2], reps[i][a2], tol);
+            p.m = mult[i];
+            for (int k = 0; k < 3; ++k) p.u[k] = (double)reps[i][ax[k]] / r;
+            o.pts.push_back(p);
+        }
+        // nearest the centre first, +v and -v next to each other: samples on opposite
+        // sides mostly cancel, so the running sum stays small (in value order its
+        // rounding made the map's error against 64 bits a fifth larger)
+        std::vector<int> rank[2];
+        for (int k = 0; k < 2; ++k) {
+            std::vector<float> mag;
+            for (float v : o.val[k]) value_index(mag, std::fabs(v), tol);
+            std::sort(mag.begin(), mag.end());
+            for (float v : o.val[k]) rank[k].push_back(value_index(mag, std::fabs(v), tol));
+        }
+        std::sort(o.pts.begin(), o.pts.end(), [&](const P& u, const P& v) {
+            return std::make_tuple(rank[1][u.b], u.b, rank[0][u.a], u.a, u.c) <
+                   std::make_tuple(rank[1][v.b], v.b, rank[0][v.a], v.a, v.c);
+        });
+        for (size_t i = 0; i < o.pts.size(); ++i) {
+            const P& p = o.pts[i];
+            const bool axis = p.u[0] == 0 && p.u[1] == 0;
+            if (i == 0 || axis || p.a != o.pts[i - 1].a || p.b != o.pts[i - 1].b) o.pair0.push_back((int)i);
+        }
+        return o;
+    };
+    // clocks per subvoxel up to a common factor: 22 a pair's second pass, 7 a
+    // group's first (as in forward_depth)
+    auto cost = [&](const Order& o, int a2) {
+        int groups = 0;
+        for (size_t i = 0; i < o.pts.size(); ++i) groups += i == 0 || o.pts[i].b != o.pts[i - 1].b;
+        return (22.0 * o.pair0.size() + 7.0 * groups) / c.mag[a2];
+    };
+    Order o = arrange(1, 2);
+    fp->ax1 = 1;
+    fp->ax2 = 2;
+    {
+        Order alt = arrange(2, 1);
+        if (cost(alt, 1) < cost(o, 2)) {
+            o = std::move(alt);
+            fp->ax1 = 2;
+            fp->ax2 = 1;
+        }
+    }
+    const int ax[3] = {0, fp->ax1, fp->ax2};
+    for (int k = 0; k < 3; ++k) fp->mag[k] = c.mag[ax[k]];
+
+    // lane tables
+    std::vector<float>& L = fp->lane;
+    L.clear();
+    auto bits = [](int v) {
+        float f;
+        std::memcpy(&f, &v, 4);
+        return f;
+    };
+    static const char* const names = "xyz";
+    auto too_large = [&](int axis) {
+        *err = std::string("ring radius too large for the ") + names[axis] +
+               " magnification (needs ring_radius < (1 + mag)/2)";
+        return false;
+    };
+    // taps of one value at every phase; the offsets as a mask
+    auto taps = [&](int k, float v, std::vector<std::array<float, 4>>* w, std::vector<int>* off) {
+        for (int ph = 0; ph < fp->mag[k]; ++ph) {
+            std::array<float, 4> t;
+            int of;
+            if (!tap4(ph, v, fp->mag[k], t.data(), &of)) return too_large(ax[k]);
+            w->push_back(t);
+            off->push_back(of);
+        }
+        return true;
+    };
+    int* wpos[2] = {&fp->l_wx, &fp->l_wm};
+    int* opos[2] = {&fp->l_offx, &fp->l_offm};
+    std::vector<std::array<float, 4>> w;
+    std::vector<int> off;
+    for (int k = 0; k < 2; ++k) {
+        w.clear();
+        off.clear();
+        for (float v : o.val[k])
+            if (!taps(k, v, &w, &off)) return false;
+        *wpos[k] = (int)L.size();
+        for (auto& t : w) L.insert(L.end(), t.begin(), t.end());
+        *opos[k] = (int)L.size();
+        for (int of : off) L.push_back(bits(of));
+        while (L.size() % 4) L.push_back(0.f);
+    }
+    fp->zero_x = value_index(o.val[0], 0.f, tol);
+    fp->zero_m = value_index(o.val[1], 0.f, tol);
+
+    // uniform tables
+    const int mz = fp->mag[2];
+    const int npairs = (int)o.pair0.size(), npts = (int)o.pts.size(), nzv = (int)o.val[2].size();
+    std::vector<std::array<int, 3>> groups;
+    for (int i = 0; i < npairs; ++i) {
+        const int b = o.pts[o.pair0[i]].b;
+        if (groups.empty() || groups.back()[0] != b) groups.push_back({b, i, i});
+        groups.back()[2] = i + 1;
+    }
+    fp->ngroups = (int)groups.size();
+    fp->npairs = npairs;
+    fp->npoints = npts;
+    fp->u_grp = 0;
+    fp->u_pair = fp->ngroups;
+    fp->u_pt = fp->u_pair + 4 * npairs;
+    fp->u_wz = fp->u_pt + 3 * npts;
+    fp->u_wi = fp->u_wz + 2 * nzv * mz;
+    std::vector<float>& U = fp->utab;
+    U.clear();
+    auto put = [&](double a, double b, double cc, double d) {
+        for (double v : {a, b, cc, d}) U.push_back((float)v);
+    };
+    auto put_bits = [&](int a, int b, int cc, int d) {
+        for (int v : {a, b, cc, d}) U.push_back(bits(v));
+    };
+    for (auto& g : groups) put_bits(g[0], g[1], g[2], 0);
+    // the commonest multiplicity carries the weight 1
+    std::map<int, int> count;
+    for (auto& p : o.pts) count[p.m]++;
+    int common = o.pts[0].m;
+    for (auto& e : count)
+        if (e.second > count[common]) common = e.first;
+    fp->neg_weight = -((float)common / (float)n);  // kernel.cu:244 divides by n, not n^2
+    std::vector<double> kappa(npts, 0.0);
+    for (int i = 0; i < npairs; ++i) {
+        const int q0 = o.pair0[i], q1 = i + 1 < npairs ? o.pair0[i + 1] : npts;
+        const P& f = o.pts[q0];
+        const double ux = f.u[0], um = f.u[1];
+        double pa = 1, pb = 0, ea = 0, eb = 1;
+        int plane[3] = {2, 1, 0};
+        if (ux == 0 && um == 0) {
+            pa = f.u[2] < 0 ? -1 : 1;
+        } else {
+            plane[0] = 0;
+            plane[2] = 2;
+            const double h = std::sqrt(ux * ux + um * um);
+            double mean = 0;
+            for (int q = q0; q < q1; ++q) {
+                kappa[q] = o.pts[q].u[2] / h;
+                mean += std::fabs(kappa[q]) / (q1 - q0);
+            }
+            const double scale = std::sqrt(1 + mean * mean);
+            pa = ux / h;
+            pb = um / h;
+            ea = -scale * um / h;
+            eb = scale * ux / h;
+        }
+        put(pa, pa, pb, pb);
+        put(ea, ea, eb, eb);
+        put_bits(plane[0], plane[1], plane[2], f.a);
+        put_bits(q0, q1, 0, 0);
+    }
+    w.clear();
+    off.clear();
+    for (float v : o.val[2])
+        if (!taps(2, v, &w, &off)) return false;
+    for (int q = 0; q < npts; ++q) {
+        const P& p = o.pts[q];
+        const double un = std::sqrt(p.u[0] * p.u[0] + p.u[1] * p.u[1] + p.u[2] * p.u[2]);
+        const double rho = std::sqrt((double)p.m / common);
+        int mask = 0;
+        for (int ph = 0; ph < mz; ++ph) mask |= off[p.c * mz + ph] << ph;
+        put(kappa[q], kappa[q], -kappa[q], -kappa[q]);
+        put(-rho * un, -rho * un, rho, rho);
+        put_bits(p.c * mz, mask, 0, 0);
+    }
+    for (auto& t : w) {
+        put(t[0], t[0], t[1], t[1]);
+        put(t[2], t[2], t[3], t[3]);
+    }
+    for (int ph = 0; ph < mz; ++ph) {
+        float t[5];
+        tap5(ph, 0.0, mz, t);
+        const int m0 = 2 * ph + 1 >= mz ? 1 : 0;
+        put(t[m0], t[m0 + 1], t[m0 + 2], t[m0 + 3]);
+    }
+    return true;
+}
+
+FwdParams forward_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, int in_u16, const int dims[4],
+                         int ty, int cz) {
+    FwdParams p;
+    std::memset(&p, 0, sizeof p);
+    p.in = in;
+    p.in_u16 = in_u16;
+    p.W = dims[0];
+    p.H = dims[1];
+    p.D = dims[2];
+    p.T = dims[3];
+    for (int a = 0; a < 3; ++a) p.mag[a] = fp.mag[a];
+    p.ax1 = fp.ax1;
+    p.ax2 = fp.ax2;
+    const int lat[3] = {c.x_range, c.y_range, c.z_range};
+    p.gr[0] = c.gradient_smooth == 0 ? 1 : c.main_range;
+    p.gr[1] = c.gradient_smooth == 0 ? 0 : lat[0];
+    p.gr[2] = c.gradient_smooth == 0 ? 0 : lat[fp.ax1];
+    p.gr[3] = c.gradient_smooth == 0 ? 0 : lat[fp.ax2];
+    p.R = std::max(std::max(p.gr[0], p.gr[1]), std::max(p.gr[2], p.gr[3]));
+    const auto ranges = [&](int a, int b) { return p.gr[0] == a && p.gr[1] == b && p.gr[2] == b && p.gr[3] == b; };
+    p.grad_mode = ranges(1, 1) ? 1 : ranges(1, 0) ? 2 : 0;
+    p.TY = ty > 0 ? ty : kTileRows;
+    p.cz = cz;
+    p.NU = (kTileX - 1) / fp.mag[0] + 2 + 4;
+    p.NV = (p.TY - 1) / fp.mag[1] + 2 + 4;
+    p.NIX = p.NU + 2 * p.R;
+    p.NIY = p.NV + 2 * p.R;
+    p.NIZ = cz + 4 + 2 * p.R;
+    p.u_region = radiality_u_region(p);
+    p.renorm = c.renormalize == 1;
+    p.poscon = c.remove_con == 1;
+    p.lane_words = (int)fp.lane.size();
+    p.l_wx = fp.l_wx;
+    p.l_offx = fp.l_offx;
+    p.l_wm = fp.l_wm;
+    p.l_offm = fp.l_offm;
+    p.u_count = (int)(fp.utab.size() / 4);
+    p.u_grp = fp.u_grp;
+    p.u_pair = fp.u_pair;
+    p.u_pt = fp.u_pt;
+    p.u_wz = fp.u_wz;
+    p.u_wi = fp.u_wi;
+    p.ngroups = fp.ngroups;
+    p.zero_x = fp.zero_x;
+    p.zero_m = fp.zero_m;
+    p.neg_weight = fp.neg_weight;
+    p.tma_bx = radiality_tma_box_x(p);
+    return p;
+}
+
+int forward_depth(const FwdPlan& fp, const std::vector<std::array<int, 2>>& lo_hi) {
+    // records too many for the kernel parameters run on the shallow kernel only, and
+    // so do depths whose sums would not fit the registers beside the columns
+    if (fp.utab.size() / 4 > (size_t)kUTabMax || fp.mag[2] > 5) return 4;
+    // time per tile column in clocks (one SM, as measured): a point at one subvoxel
+    // 29, a pair's second pass at one cell 22, a group's first pass at one cell 7
+    double best = 0;
+    int cz = 4;
+    for (int c : {8, 4}) {
+        const int mz = fp.mag[2], fz = mz * c;
+        double tiles = 0;
+        for (auto& r : lo_hi) tiles += (r[1] - (r[0] / mz) * mz + fz - 1) / fz;
+        const double t = tiles * (fz * 29.0 * fp.npoints + (c + 4) * (22.0 * fp.npairs + 7.0 * fp.ngroups));
+        if (c == 8 || t < best) {
+            best = t;
+            cz = c;
+        }
+    }
+    return cz;
+}
+
+void forward_tiles(const FwdPlan& fp, int ty, BlockDev* b) {
+    const int rows = ty > 0 ? ty : kTileRows;
+    const int mz = fp.mag[2], fz = mz * b->cz;
+    b->ntile[0] = (b->nreg[0] + kTileX - 1) / kTileX;
+    b->ntile[fp.ax1] = (b->nreg[fp.ax1] + rows - 1) / rows;
+    b->ntile[fp.ax2] = (b->hi[fp.ax2] - (b->lo[fp.ax2] / mz) * mz + fz - 1) / fz;
 }
 
 // ---------------------------------------------------------------------------

@@ -10,32 +10,45 @@
 //      copy (requested one time point ahead) and converted to float with the
 //      reference's block-edge clamp (its fminf/fmaxf clamps); inputs whose rows
 //      a tensor map cannot address are read with plain loads instead;
-//   2. the smoothed gradient G = (Gx, Gy, Gz) and the intensity I of every
-//      coarse cell the tile's taps reach is formed in shared memory (float4);
+//   2. the smoothed gradient of every coarse cell the tile's taps reach is formed
+//      in shared memory, one plane per component, four cells of the tile's
+//      innermost axis to a float4;
 //   3. the ring's n^2 samples are reduced to their distinct points (62 for
-//      n = 12) and factorised per axis. Catmull-Rom interpolation is separable,
-//      and a sample's x taps and weights depend only on the subvoxel's x phase
-//      (X mod mag_x) and the ring point's x coordinate, so for each distinct ring
-//      x value the x-filtered field U is formed once in shared memory;
-//   4. each thread owns two subvoxel columns (X, Y) and (X, Y + mag_y): same y
-//      phase, adjacent coarse rows, so the y pass reads 5 rows of U for both.
-//      For each distinct (x, y) ring pair it y-filters U into a register column
-//      T[w] over coarse z (one float2 per w: the two columns), and for each ring
-//      point of that pair it z-filters T (4 taps; the tap offset per z phase is
-//      uniform over the warp, so both offsets are unrolled with static register
-//      indices) for its FZ subvoxels per column and accumulates the radiality
-//      term. The per-point work runs on packed f32x2 FMAs (two columns per
-//      instruction);
+//      n = 12) and factorised per axis: Catmull-Rom interpolation is separable,
+//      and a sample's taps along an axis depend only on the subvoxel's phase
+//      there and the ring point's coordinate. For each distinct value along the
+//      tile's mid axis the filtered planes U are formed once in shared memory;
+//   4. each thread owns one column of subvoxels along the innermost axis, its
+//      lower and upper half packed in register pairs. For each (mid, x) pair of
+//      ring values it filters U along x into a column and turns it into the
+//      pair's frame; for each ring point of the pair it filters the column along
+//      the innermost axis (the tap offset per phase is uniform over the warp, so
+//      both offsets are unrolled with static register indices) and accumulates
+//      the radiality term, on packed f32x2 FMAs (two subvoxels per instruction);
 //   5. radiality and interpolated intensity per subvoxel and time point are
 //      written to the stack that the temporal kernel reduces.
 //
+// What bounds it: the point loop's 20 packed FMAs and 4 MUFUs per point and two
+// subvoxels (of 28 warp instructions), 5 of 7.5 ms for four volumes of 128 x
+// 128 x 64 at 4 x 4 x 2 (134 M subvoxels x 62 points), where the FMA pipe is 71 %
+// busy; in isolation that loop takes 58 clocks per warp and two subvoxels on one
+// SM partition against 41 for its FMAs alone, 51 without the MUFUs. The register
+// file is what is in the way: it serves two operands per lane and clock, so an
+// FMA whose three operands are different vector registers runs at two thirds of
+// the rate (80 against 112 to 118 lanes per clock and SM, measured). Hence the
+// uniform tables below, the frame that needs no products for the projection, and
+// sqrt(weight) folded into 1 - Dk/r so that the square is the accumulating FMA.
+// With (x, y) pairs, y columns and 22 packed FMAs per point the same four volumes
+// took 10.8 ms.
+//
 // The radiality term of a sample with interpolated gradient g and ring offset
-// rho (kernel.cu:224-240), with u = rho / r, is evaluated in a rotated frame:
-// (x, y) is turned about z so that u lies in the x'z plane, u = |u| (h x' + c z).
-// Then g.u / |u| = h g_x' + c g_z, the part of g perpendicular to u has the
-// components g_y' and h g_z - c g_x', and
+// rho (kernel.cu:224-240), with u = rho / r: the pair's frame turns (x, mid) so that
+// u lies in its P-Z plane, and scales every component alike (FwdPlan in
+// srrf_internal.h). Then with kappa the tangent of u's elevation dot = P + kappa Z is
+// g.u, cp = Z - kappa P and E are the part of g perpendicular to u, up to the scale,
 //   Dk / r = |u| sin(angle(g, u)) = |u| sqrt(|g_perp|^2 / |g|^2),
-//   D = (1 - Dk/r)^2,   S -= D if g.u > 0, S += D otherwise.
+//   D = (1 - Dk/r)^2,   S -= D if g.u > 0, S += D otherwise
+// (at g.u = 0 the sample is perpendicular to g and D vanishes, whatever the sign).
 // The perpendicular part is formed directly, so Dk has full relative accuracy
 // even when g is almost parallel to u; g = 0 gives 0 * inf = NaN exactly as the
 // reference's 0/0 does. Coordinates are local (phase + ring offset), so no
@@ -45,6 +58,7 @@
 // valid box.
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -127,26 +141,15 @@ template <int V>
 struct IntC {
     static constexpr int value = V;
 };
-// copysign(w, -d) for w >= 0: -w when d > 0 (diverging), +w when d < 0. At
-// d = 0 the sample is perpendicular to g, s = |u| and D vanishes, so the sign
-// taken there does not matter.
-__device__ __forceinline__ float sign_weight(float w, float d) {
-    return __int_as_float(__float_as_int(w) | (~__float_as_int(d) & 0x80000000));
-}
 
 __device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-
-template <typename Tin>
-__device__ __forceinline__ float load_in(const Tin* p, long long i);
-template <>
-__device__ __forceinline__ float load_in<float>(const float* p, long long i) {
-    return __ldg(p + i);
-}
-template <>
-__device__ __forceinline__ float load_in<uint16_t>(const uint16_t* p, long long i) {
-    return (float)__ldg(p + i);
+__device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
+// v with its sign flipped where d < 0
+__device__ __forceinline__ float flip_sign(float v, float d) {
+    return __int_as_float(__float_as_int(v) ^ (__float_as_int(d) & 0x80000000));
 }
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
@@ -156,69 +159,141 @@ __device__ __forceinline__ int floordiv(int a, int b) {  // b > 0
     return (a % b != 0 && a < 0) ? q - 1 : q;
 }
 
-// gradKernel's smoothed gradient (kernel.cu:73-124) at one coarse cell from the
-// clamped input tile: Gx = sum over i in [1, mR], j in [-yR, yR], k in
-// [-zR, zR] of I(+i, j, k) - I(-i, j, k), and likewise for y and z; with
-// smoothing off the reference's central difference is the case mR = 1 and all
-// lateral ranges 0. The .w component carries I at the cell. Fixed ranges are
-// fully unrolled; integer inputs make the sums exact in float whatever the order.
-template <int MR, int XR, int YR, int ZR>
-__device__ __forceinline__ float4 gradient_fixed(const float* base, int NIX, int NIY) {
-    auto I = [&](int dx, int dy, int dz) { return base[(dz * NIY + dy) * NIX + dx]; };
-    float gx = 0.f, gy = 0.f, gz = 0.f;
-#pragma unroll
-    for (int i = 1; i <= MR; ++i)
-#pragma unroll
-        for (int j = -YR; j <= YR; ++j)
-#pragma unroll
-            for (int k = -ZR; k <= ZR; ++k) gx += I(i, j, k) - I(-i, j, k);
-#pragma unroll
-    for (int j = 1; j <= MR; ++j)
-#pragma unroll
-        for (int i = -XR; i <= XR; ++i)
-#pragma unroll
-            for (int k = -ZR; k <= ZR; ++k) gy += I(i, j, k) - I(i, -j, k);
-#pragma unroll
-    for (int k = 1; k <= MR; ++k)
-#pragma unroll
-        for (int i = -XR; i <= XR; ++i)
-#pragma unroll
-            for (int j = -YR; j <= YR; ++j) gz += I(i, j, k) - I(i, j, -k);
-    return make_float4(gx, gy, gz, I(0, 0, 0));
+// Division of 0 <= c < 65536 by d >= 2 with one multiply-high.
+struct FastDiv {
+    unsigned m;
+    __device__ explicit FastDiv(int d) : m(0xffffffffu / (unsigned)d + 1u) {}
+    __device__ int operator()(int c) const { return (int)__umulhi((unsigned)c, m); }
+};
+
+// The warp-uniform tables of a launch. They travel in the kernel's parameters
+// when they fit (UN > 1): the compiler then keeps the tap weights and point
+// constants in uniform registers, which a packed FMA takes as one operand
+// without using a vector register read port. The ports are what bounds the
+// point loop: FMAs with three different vector register operands run at 80
+// lanes per clock and SM here, with a uniform operand at 112 of 128 (measured
+// side by side). Rings too large for the parameters (AxesinRing above 8 or so)
+// read the same records from global memory.
+template <int UN>
+struct UTab {
+    float4 q[UN];
+};
+template <int UN>
+__device__ __forceinline__ float4 uget(const UTab<UN>& ut, const float4* g, int i) {
+    if constexpr (UN > 1)
+        return ut.q[i];
+    else
+        return __ldg(g + i);
 }
 
-__device__ __forceinline__ float4 gradient_generic(const float* base, int NIX, int NIY, const int gr[4]) {
-    auto I = [&](int dx, int dy, int dz) { return base[(dz * NIY + dy) * NIX + dx]; };
-    const int mR = gr[0], xR = gr[1], yR = gr[2], zR = gr[3];
-    float gx = 0.f, gy = 0.f, gz = 0.f;
-    for (int i = 1; i <= mR; ++i)
-        for (int j = -yR; j <= yR; ++j)
-            for (int k = -zR; k <= zR; ++k) gx += I(i, j, k) - I(-i, j, k);
-    for (int j = 1; j <= mR; ++j)
-        for (int i = -xR; i <= xR; ++i)
-            for (int k = -zR; k <= zR; ++k) gy += I(i, j, k) - I(i, -j, k);
-    for (int k = 1; k <= mR; ++k)
-        for (int i = -xR; i <= xR; ++i)
-            for (int j = -yR; j <= yR; ++j) gz += I(i, j, k) - I(i, j, -k);
-    return make_float4(gx, gy, gz, I(0, 0, 0));
+// gradKernel's smoothed gradient (kernel.cu:73-124) at four coarse cells that
+// follow each other along the innermost axis, from the clamped input tile
+// (base: the first cell's voxel; x stride 1, mid stride sv, inner rows at
+// row(k)): Gx = sum over i in [1, mR], j in [-yR, yR], k in [-zR, zR] of
+// I(+i, j, k) - I(-i, j, k), and likewise for the other axes, in tile axis
+// order. Ranges (1, 1, 1, 1) share their 6 x 9 loads between the four cells;
+// with smoothing off the reference's central difference is the case mR = 1 and
+// all lateral ranges 0. Integer inputs make the sums exact in float whatever
+// the order.
+template <class Row>
+__device__ __forceinline__ void gradient4(int mode, const int gr[4], Row&& row, int sv, float (&g)[3][4]) {
+    if (mode == 1) {
+        float v[6][3][3];  // [w - 1 .. w + 4][mid][x]
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            const float* r = row(k - 1);
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int i = 0; i < 3; ++i) v[k][j][i] = r[(j - 1) * sv + (i - 1)];
+        }
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            float gx = 0.f, gm = 0.f, gn = 0.f;
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    gx += v[w + b][a][2] - v[w + b][a][0];
+                    gm += v[w + b][2][a] - v[w + b][0][a];
+                    gn += v[w + 2][a][b] - v[w][a][b];
+                }
+            g[0][w] = gx;
+            g[1][w] = gm;
+            g[2][w] = gn;
+        }
+    } else if (mode == 2) {
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const float* r = row(w);
+            g[0][w] = r[1] - r[-1];
+            g[1][w] = r[sv] - r[-sv];
+            g[2][w] = row(w + 1)[0] - row(w - 1)[0];
+        }
+    } else {
+        const int mR = gr[0], xR = gr[1], yR = gr[2], zR = gr[3];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            float gx = 0.f, gm = 0.f, gn = 0.f;
+            auto I = [&](int dx, int dm, int dn) { return row(w + dn)[dm * sv + dx]; };
+            for (int i = 1; i <= mR; ++i)
+                for (int j = -yR; j <= yR; ++j)
+                    for (int k = -zR; k <= zR; ++k) gx += I(i, j, k) - I(-i, j, k);
+            for (int j = 1; j <= mR; ++j)
+                for (int i = -xR; i <= xR; ++i)
+                    for (int k = -zR; k <= zR; ++k) gm += I(i, j, k) - I(i, -j, k);
+            for (int k = 1; k <= mR; ++k)
+                for (int i = -xR; i <= xR; ++i)
+                    for (int j = -yR; j <= yR; ++j) gn += I(i, j, k) - I(i, j, -k);
+            g[0][w] = gx;
+            g[1][w] = gm;
+            g[2][w] = gn;
+        }
+    }
 }
 
-template <int MZ, int CZ, typename Tin, bool WIDE>
-__global__ void __launch_bounds__(WIDE ? kMaxThreads : 128, WIDE ? 2 : RFBA_FWD_CTAS)
-    radiality_kernel(const RadParams p, const __grid_constant__ CUtensorMap tmap) {
+// Four taps along x (src, src + 1, ..) at four cells of the innermost axis.
+__device__ __forceinline__ void filter4(float4 w, const float4* src, float (&r)[4]) {
+    const float4 u0 = src[0], u1 = src[1], u2 = src[2], u3 = src[3];
+    r[0] = fmaf(w.w, u3.x, fmaf(w.z, u2.x, fmaf(w.y, u1.x, w.x * u0.x)));
+    r[1] = fmaf(w.w, u3.y, fmaf(w.z, u2.y, fmaf(w.y, u1.y, w.x * u0.y)));
+    r[2] = fmaf(w.w, u3.z, fmaf(w.z, u2.z, fmaf(w.y, u1.z, w.x * u0.z)));
+    r[3] = fmaf(w.w, u3.w, fmaf(w.z, u2.w, fmaf(w.y, u1.w, w.x * u0.w)));
+}
+// Cell w of a column into the packed halves (compile-time w).
+template <int CH, int NH>
+__device__ __forceinline__ void put_half(float2 (&T)[NH], int w, float v) {
+    if (w < NH) T[w].x = v;
+    if (w >= CH) T[w - CH].y = v;
+}
+
+template <int MZ, int CZ, int UN>
+__global__ void __maxnreg__(fwd_regs(MZ, CZ))
+    radiality_kernel(const __grid_constant__ FwdParams p, const __grid_constant__ CUtensorMap tmap,
+                     const __grid_constant__ UTab<UN> ut) {
+    // the tile's two halves along its innermost axis share one register pair: cell
+    // w of the lower half and cell w + CH of the upper one
+    constexpr int CH = CZ / 2;
+    constexpr int HZ = MZ * CH;
     constexpr int FZ = MZ * CZ;
+    constexpr int NH = CH + 4;
     constexpr int NW = CZ + 4;
+    constexpr int NQ = NW / 4;
+    static_assert(CZ % 4 == 0, "whole quads");
     extern __shared__ float4 smem4[];
 
-    // Shared layout: [G tile float4][U tile float4][input tile][tables][TMA staging, 128-byte aligned]
+    // Shared layout: [G planes][U planes, the input tile from plane 1 on][lane tables][TMA staging, 128-byte aligned].
+    // Planes are [NQ][NV or TY][NU] float4 over four cells of the innermost axis.
     const int NU = p.NU, NV = p.NV;
-    float4* gt = smem4;                           // [NW][NV][NU]
-    float4* ut = gt + NU * NV * NW;               // [NW][NV][16]
-    float* inp = reinterpret_cast<float*>(ut + kTileX * NV * NW);  // [NIZ][NIY][NIX]
-    float* tab = inp + ((p.NIX * p.NIY * p.NIZ + 3) & ~3);         // 16-byte aligned (float4 reads)
-    Tin* stage = reinterpret_cast<Tin*>((reinterpret_cast<uintptr_t>(tab + p.smem_table_words) + 127) &
-                                        ~(uintptr_t)127);           // [NIZ][NIY][tma_bx]
+    const int uplane = NQ * p.TY * NU;
+    float4* gt = smem4;
+    float4* ut4 = gt + 3 * NQ * NV * NU;
+    float* inp = reinterpret_cast<float*>(ut4 + uplane);  // [NIZ][NIY][NIX], dead once G and the intensity's plane are built
+    float* tab = reinterpret_cast<float*>(ut4 + p.u_region);
+    unsigned char* stage = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(tab + p.lane_words) + 127) & ~(uintptr_t)127);  // [box z][box y][tma_bx]
     __shared__ unsigned int s_item;
+    __shared__ int2 s_row[kMaxThreads / kTileX];
     __shared__ alignas(8) uint64_t s_bar;
     const bool use_tma = p.use_tma != 0;
     unsigned phase = 0;
@@ -230,31 +305,22 @@ __global__ void __launch_bounds__(WIDE ? kMaxThreads : 128, WIDE ? 2 : RFBA_FWD_
     const int nthr = blockDim.x;
     const int tid = threadIdx.x;
     const int mx = p.mag[0], my = p.mag[1];
-    // column pair of this thread: (X, Ya) and (X, Ya + my)
+    const int a1 = p.ax1, a2 = p.ax2;  // volume axes of the tile's mid and innermost axis
+    // one column (X, Y) per thread
     const int xf = tid & (kTileX - 1);
-    const int q = tid / kTileX;                   // 0 .. TY/2 - 1
-    const int yfa = (q / my) * (2 * my) + (q % my);
+    const int q = tid / kTileX;                   // 0 .. TY - 1
+    const int TY = p.TY;
 
-    for (int i = tid; i < p.smem_table_words; i += nthr) tab[i] = p.tables[i];
-    const float* wx = tab + p.tl.wx;
-    const int* offx = reinterpret_cast<const int*>(tab + p.tl.offx);
-    const float* wy = tab + p.tl.wy;
-    const int* offy = reinterpret_cast<const int*>(tab + p.tl.offy);
-    const float* wz = tab + p.tl.wz;
-    const int* offz = reinterpret_cast<const int*>(tab + p.tl.offz);
-    const float* wzi = tab + p.tl.wzi;
-    const int* grp_xval = reinterpret_cast<const int*>(tab + p.tl.grp_xval);
-    const int* grp = reinterpret_cast<const int*>(tab + p.tl.grp);
-    const int* pair_yval = reinterpret_cast<const int*>(tab + p.tl.pair_yval);
-    const int* pair_pt = reinterpret_cast<const int*>(tab + p.tl.pair_pt);
-    const int* pt_zval = reinterpret_cast<const int*>(tab + p.tl.pt_zval);
-    const float4* pt_vec = reinterpret_cast<const float4*>(tab + p.tl.pt_vec);
-    const float2* pair_rot = reinterpret_cast<const float2*>(tab + p.tl.pair_rot);
+    for (int i = tid; i < p.lane_words; i += nthr) tab[i] = p.lane[i];
+    const float* wx = tab + p.l_wx;
+    const int* offx = reinterpret_cast<const int*>(tab + p.l_offx);
+    const float* wy = tab + p.l_wm;
+    const int* offy = reinterpret_cast<const int*>(tab + p.l_offm);
 
-    const Tin* in = static_cast<const Tin*>(p.in);
     const int NIX = p.NIX, NIY = p.NIY, NIZ = p.NIZ, R = p.R;
-    const int ncell = NU * NV * NW;
-    const int nut = kTileX * NV * NW;
+    const FastDiv div_nu(NU), div_nv(NV), div_ty(TY);
+    const int es = p.in_u16 ? 2 : 4;
+    const int box1 = a1 == 1 ? NIY : NIZ;  // rows of the staged box along the volume's y
 
     for (;;) {
         __syncthreads();
@@ -266,46 +332,45 @@ __global__ void __launch_bounds__(WIDE ? kMaxThreads : 128, WIDE ? 2 : RFBA_FWD_
         const int chunk = (int)(item / p.ntiles);
         const TileDesc td = p.tiles[tile_i];
         const BlockDev& B = p.blocks[td.block];
-        const int bw = B.size[0], bh = B.size[1], bd = B.size[2];
+        const int bw = B.size[0], bh = B.size[a1], bd = B.size[a2];
 
-        // Tile geometry (block-local fine and coarse coordinates).
-        const int X0 = B.lo[0] + td.tx * kTileX;
-        const int Y0 = B.lo[1] + td.ty * p.TY;
-        const int Z0 = B.zbase + td.tz * FZ;
+        // Tile geometry (block-local fine and coarse coordinates; y is the tile's
+        // mid axis and z its innermost axis).
+        const int X0 = B.lo[0] + td.t[0] * kTileX;
+        const int Y0 = B.lo[a1] + td.t[a1] * p.TY;
+        const int Z0 = (B.lo[a2] / MZ) * MZ + td.t[a2] * FZ;
         const int cx0 = floordiv(X0, mx) - 2;
         const int cy0 = floordiv(Y0, my) - 2;
         const int cz0 = Z0 / MZ - 2;
         const int X = X0 + xf;
-        const int Ya = Y0 + yfa, Yb = Ya + my;
+        const int Y = Y0 + q;
         const int xi = floordiv(X, mx), xr = X - xi * mx;
-        const int yi = floordiv(Ya, my), yr = Ya - yi * my;  // Yb: yi + 1, same phase
-        const bool xin = X < B.hi[0];
-        const bool ina = xin && Ya < B.hi[1];
-        const bool inb = xin && Yb < B.hi[1];
-        const bool xrad = X >= B.rad_lo[0] && X <= B.rad_hi[0];
-        const bool xint = X >= B.int_lo[0] && X <= B.int_hi[0];
-        const bool rada = xrad && Ya >= B.rad_lo[1] && Ya <= B.rad_hi[1];
-        const bool radb = xrad && Yb >= B.rad_lo[1] && Yb <= B.rad_hi[1];
-        const bool inta = xint && Ya >= B.int_lo[1] && Ya <= B.int_hi[1];
-        const bool intb = xint && Yb >= B.int_lo[1] && Yb <= B.int_hi[1];
+        if (xf == 0) {
+            const int yi = floordiv(Y, my);
+            s_row[q] = make_int2(yi - cy0 - 2, Y - yi * my);  // first tap row at offset 0, phase
+        }
+        const bool in = X < B.hi[0] && Y < B.hi[a1];
         const long long V = B.vox;
-        const long long va = ((long long)(Ya - B.lo[1])) * B.nreg[0] + (X - B.lo[0]);
-        const long long vb = ((long long)(Yb - B.lo[1])) * B.nreg[0] + (X - B.lo[0]);
-        const long long zstride = (long long)B.nreg[0] * B.nreg[1];
+        const long long ystride = a1 == 1 ? B.nreg[0] : (long long)B.nreg[0] * B.nreg[1];
+        const long long zstride = a1 == 1 ? (long long)B.nreg[0] * B.nreg[1] : B.nreg[0];
+        const int zlo = B.lo[a2], zhi = B.hi[a2];
+        const long long v0 = (long long)(Y - B.lo[a1]) * ystride + (X - B.lo[0]) + (Z0 - zlo) * zstride;
+        const bool rad = X >= B.rad_lo[0] && X <= B.rad_hi[0] && Y >= B.rad_lo[a1] && Y <= B.rad_hi[a1];
+        // rows without a valid sample only take part in the shared work
+        const bool work = __any_sync(0xffffffffu, in && rad);
 
         const int t0 = p.t_lo + chunk * p.t_chunk;
         const int t1 = min(p.t_hi > 0 ? p.t_hi : p.T, t0 + p.t_chunk);
         // TMA box origin: x rounded down to a 16-byte boundary; the offset back
         // (0 .. 16 bytes / element size - 1) is where the tile starts in a staged row
-        constexpr int kAl = 16 / (int)sizeof(Tin);
-        auto box_ox = [&]() {
-            const int gx0 = B.origin[0] + cx0 - R;
-            return ((gx0 % kAl) + kAl) % kAl;
-        };
+        const int kal = 16 / es;
+        const int gx0 = B.origin[0] + cx0 - R;
+        const int box_ox = ((gx0 % kal) + kal) % kal;
         auto issue = [&](int tt) {
-            const int gx0 = B.origin[0] + cx0 - R;
-            tma_load_box(stage, &tmap, &s_bar, (unsigned)(p.tma_bx * NIY * NIZ * (int)sizeof(Tin)), gx0 - box_ox(),
-                         B.origin[1] + cy0 - R, B.origin[2] + cz0 - R, tt);
+            int c[3];
+            c[a1] = B.origin[a1] + cy0 - R;
+            c[a2] = B.origin[a2] + cz0 - R;
+            tma_load_box(stage, &tmap, &s_bar, (unsigned)(p.tma_bx * NIY * NIZ * es), gx0 - box_ox, c[1], c[2], tt);
         };
         if (use_tma && tid == 0) {
             fence_proxy_async();  // the previous item's generic reads of the staging area come first
@@ -317,7 +382,6 @@ __global__ void __launch_bounds__(WIDE ? kMaxThreads : 128, WIDE ? 2 : RFBA_FWD_
             const long long sbase = B.stack_off + (long long)(t - p.stack_t0) * V;
             // 1. input tile with block-edge clamp; 16 lanes per row, one division
             //    per row
-            const long long tbase = (long long)t * p.D * p.H * p.W;
             if (use_tma) {
                 const bool ok = mbar_wait_bounded(&s_bar, phase);
                 if (__syncthreads_or(!ok)) {
@@ -330,216 +394,252 @@ __global__ void __launch_bounds__(WIDE ? kMaxThreads : 128, WIDE ? 2 : RFBA_FWD_
                     return;
                 }
                 phase ^= 1u;
-                for (int r = tid / kTileX; r < NIY * NIZ; r += nthr / kTileX) {
-                    const int iy = r % NIY, iz = r / NIY;
-                    const int sy = clampi(cy0 - R + iy, 0, bh - 1) - (cy0 - R);
-                    const int sz = clampi(cz0 - R + iz, 0, bd - 1) - (cz0 - R);
-                    const Tin* srow = stage + (sz * NIY + sy) * p.tma_bx + box_ox();
-                    float* rows = inp + r * NIX;
-                    for (int ix = xf; ix < NIX; ix += kTileX)
-                        rows[ix] = (float)srow[clampi(cx0 - R + ix, 0, bw - 1) - (cx0 - R)];
-                }
+                auto unpack = [&](auto* st) {
+                    for (int r = q, iy = q, iz = 0; r < NIY * NIZ; r += TY, iy += TY) {
+                        while (iy >= NIY) {
+                            iy -= NIY;
+                            ++iz;
+                        }
+                        const int sy = clampi(cy0 - R + iy, 0, bh - 1) - (cy0 - R);
+                        const int sz = clampi(cz0 - R + iz, 0, bd - 1) - (cz0 - R);
+                        const auto* srow = st + (a1 == 1 ? sz * box1 + sy : sy * box1 + sz) * p.tma_bx + box_ox;
+                        float* rows = inp + r * NIX;
+                        for (int ix = xf; ix < NIX; ix += kTileX)
+                            rows[ix] = (float)srow[clampi(cx0 - R + ix, 0, bw - 1) - (cx0 - R)];
+                    }
+                };
+                if (p.in_u16)
+                    unpack(reinterpret_cast<const uint16_t*>(stage));
+                else
+                    unpack(reinterpret_cast<const float*>(stage));
                 __syncthreads();
                 if (tid == 0 && t + 1 < t1) {
                     fence_proxy_async();  // the staging area's generic reads before the next async write
                     issue(t + 1);
                 }
             } else {
-                for (int r = tid / kTileX; r < NIY * NIZ; r += nthr / kTileX) {
-                    const int iy = r % NIY, iz = r / NIY;
-                    const int by = clampi(cy0 - R + iy, 0, bh - 1);
-                    const int bz = clampi(cz0 - R + iz, 0, bd - 1);
-                    const long long rowg = tbase + ((long long)(B.origin[2] + bz) * p.H + (B.origin[1] + by)) * p.W +
-                                           B.origin[0];
+                const long long tbase = (long long)t * p.D * p.H * p.W;
+                __syncthreads();  // the tile shares the U planes, read until here by the previous time point
+                for (int r = q, iy = q, iz = 0; r < NIY * NIZ; r += TY, iy += TY) {
+                    while (iy >= NIY) {
+                        iy -= NIY;
+                        ++iz;
+                    }
+                    const int by = B.origin[a1] + clampi(cy0 - R + iy, 0, bh - 1);
+                    const int bz = B.origin[a2] + clampi(cz0 - R + iz, 0, bd - 1);
+                    const long long rowg =
+                        tbase + (a1 == 1 ? (long long)bz * p.H + by : (long long)by * p.H + bz) * p.W + B.origin[0];
                     float* rows = inp + r * NIX;
-                    for (int ix = xf; ix < NIX; ix += kTileX)
-                        rows[ix] = load_in<Tin>(in, rowg + clampi(cx0 - R + ix, 0, bw - 1));
+                    for (int ix = xf; ix < NIX; ix += kTileX) {
+                        const long long gi = rowg + clampi(cx0 - R + ix, 0, bw - 1);
+                        rows[ix] = p.in_u16 ? (float)__ldg(static_cast<const uint16_t*>(p.in) + gi)
+                                            : __ldg(static_cast<const float*>(p.in) + gi);
+                    }
                 }
                 __syncthreads();
             }
-            // 2. gradient + intensity per coarse cell
-            for (int c = tid; c < ncell; c += nthr) {
-                const int u = c % NU;
-                const int v = (c / NU) % NV;
-                const int w = c / (NU * NV);
-                const int cu = cx0 + u, cv = cy0 + v, cw = cz0 + w;
-                float4 g4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (cu >= 0 && cu < bw && cv >= 0 && cv < bh && cw >= 0 && cw < bd) {
-                    const float* base = inp + ((w + R) * NIY + (v + R)) * NIX + (u + R);
-                    if (p.grad_mode == 1)
-                        g4 = gradient_fixed<1, 1, 1, 1>(base, NIX, NIY);
-                    else if (p.grad_mode == 2)
-                        g4 = gradient_fixed<1, 0, 0, 0>(base, NIX, NIY);
-                    else
-                        g4 = gradient_generic(base, NIX, NIY, p.gr);
+            // 2. gradient planes, and the intensity filtered along the mid axis (ring
+            //    value 0) in U plane 0. Cells outside the block are 0.
+            for (int c = tid; c < NQ * NV * NU; c += nthr) {
+                const int row = div_nu(c), u = c - row * NU;
+                const int wq = div_nv(row), v = row - wq * NV, w0 = wq * 4;
+                const int cu = cx0 + u, cv = cy0 + v, cw = cz0 + w0;
+                float g[3][4];
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) g[k][w] = 0.f;
+                if (cu >= 0 && cu < bw && cv >= 0 && cv < bh && cw + 3 >= 0 && cw < bd) {
+                    const float* base = inp + (v + R) * NIX + (u + R);
+                    auto row = [&](int k) { return base + (w0 + R + k) * (NIY * NIX); };
+                    gradient4(p.grad_mode, p.gr, row, NIX, g);
+#pragma unroll
+                    for (int w = 0; w < 4; ++w)
+                        if (cw + w < 0 || cw + w >= bd) g[0][w] = g[1][w] = g[2][w] = 0.f;
                 }
-                gt[c] = g4;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) gt[k * (NQ * NV * NU) + c] = make_float4(g[k][0], g[k][1], g[k][2], g[k][3]);
+            }
+            for (int c = tid; c < uplane; c += nthr) {
+                const int r = div_nu(c), u = c - r * NU;
+                const int wq = div_ty(r), y = r - wq * TY, w0 = wq * 4;
+                const int2 ri = s_row[y];
+                const float4 wv = *reinterpret_cast<const float4*>(wy + (p.zero_m * my + ri.y) * 4);
+                const int v = ri.x + offy[p.zero_m * my + ri.y];
+                const bool uin = cx0 + u >= 0 && cx0 + u < bw;
+                const float wk[4] = {wv.x, wv.y, wv.z, wv.w};
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const bool vin = uin && cy0 + v + k >= 0 && cy0 + v + k < bh;
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) {
+                        const int cw = cz0 + w0 + w;
+                        const float x = inp[((w0 + w + R) * NIY + (v + k + R)) * NIX + u + R];
+                        acc[w] = fmaf(wk[k], vin && cw >= 0 && cw < bd ? x : 0.f, acc[w]);
+                    }
+                }
+                ut4[c] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+            }
+            __syncthreads();
+            // intensity at the subvoxel centre (interpolateIntensity)
+            {
+                const float4 wv = *reinterpret_cast<const float4*>(wx + (p.zero_x * mx + xr) * 4);
+                const float4* src = ut4 + q * NU + xi - cx0 - 2 + offx[p.zero_x * mx + xr];
+                float2 Tw[NH];
+#pragma unroll
+                for (int wq = 0; wq < NQ; ++wq) {
+                    float u[4];
+                    filter4(wv, src + wq * TY * NU, u);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) put_half<CH>(Tw, wq * 4 + k, u[k]);
+                }
+                const bool okc = X >= B.int_lo[0] && X <= B.int_hi[0] && Y >= B.int_lo[a1] && Y <= B.int_hi[a1];
+                const int ilo = B.int_lo[a2], ihi = B.int_hi[a2];
+                float* dst = p.int_stack + sbase + v0;
+#pragma unroll
+                for (int zr = 0; zr < MZ; ++zr) {
+                    // exactly the reference's 4 taps (kernel.cu:268-283), so a
+                    // non-finite voxel reaches the same subvoxels: they start one
+                    // coarse cell later when floor((zr + 0.5) / mz - 0.5) = 0,
+                    // i.e. when 2 zr + 1 >= mz
+                    const int m0 = (2 * zr + 1 >= MZ) ? 1 : 0;
+                    const float4 qz = uget(ut, p.utab, p.u_wi + zr);
+#pragma unroll
+                    for (int zi = 0; zi < CH; ++zi) {
+                        float2 acc = mul2(dup(qz.x), Tw[zi + m0]);
+                        acc = fma2(dup(qz.y), Tw[zi + m0 + 1], acc);
+                        acc = fma2(dup(qz.z), Tw[zi + m0 + 2], acc);
+                        acc = fma2(dup(qz.w), Tw[zi + m0 + 3], acc);
+                        const int z = zi * MZ + zr, Z = Z0 + z;
+                        if (in && Z >= zlo && Z < zhi)
+                            dst[z * zstride] = okc && Z >= ilo && Z <= ihi ? fmaxf(acc.x, 0.f) : 0.f;
+                        if (in && Z + HZ >= zlo && Z + HZ < zhi)
+                            dst[(z + HZ) * zstride] = okc && Z + HZ >= ilo && Z + HZ <= ihi ? fmaxf(acc.y, 0.f) : 0.f;
+                    }
+                }
             }
 
-            float2 S[FZ];
+            float2 S[HZ];
 #pragma unroll
-            for (int z = 0; z < FZ; ++z) S[z] = make_float2(0.f, 0.f);
+            for (int z = 0; z < HZ; ++z) S[z] = make_float2(0.f, 0.f);
 
             for (int gi = 0; gi < p.ngroups; ++gi) {
+                const float4 grp = uget(ut, p.utab, p.u_grp + gi);
                 __syncthreads();  // gt ready / previous U consumed
-                // 3. x-filter for ring x value a
-                const int a = grp_xval[gi];
+                // 3. the gradient planes filtered along the mid axis for this group's
+                //    ring value
                 {
-                    const int o = offx[a * mx + xr];
-                    const float4 wv = *reinterpret_cast<const float4*>(wx + (a * mx + xr) * 4);
-                    const int ub = xi - cx0 - 2 + o;
-                    for (int e = tid; e < nut; e += nthr) {
-                        const int vw = e / kTileX;  // (w * NV + v)
-                        const float4* src = gt + vw * NU + ub;
-                        const float4 g0 = src[0], g1 = src[1], g2 = src[2], g3 = src[3];
-                        float4 r;
-                        r.x = fmaf(wv.w, g3.x, fmaf(wv.z, g2.x, fmaf(wv.y, g1.x, wv.x * g0.x)));
-                        r.y = fmaf(wv.w, g3.y, fmaf(wv.z, g2.y, fmaf(wv.y, g1.y, wv.x * g0.y)));
-                        r.z = fmaf(wv.w, g3.z, fmaf(wv.z, g2.z, fmaf(wv.y, g1.z, wv.x * g0.z)));
-                        r.w = fmaf(wv.w, g3.w, fmaf(wv.z, g2.w, fmaf(wv.y, g1.w, wv.x * g0.w)));
-                        ut[e] = r;
+                    const int b0 = __float_as_int(grp.x) * my;
+                    for (int c = tid; c < 3 * uplane; c += nthr) {
+                        const int r = div_nu(c), u = c - r * NU;
+                        const int pw = div_ty(r), y = r - pw * TY;
+                        const int2 ri = s_row[y];
+                        const float4 wv = *reinterpret_cast<const float4*>(wy + (b0 + ri.y) * 4);
+                        const float4* src = gt + (pw * NV + ri.x + offy[b0 + ri.y]) * NU + u;
+                        const float4 c0 = src[0], c1 = src[NU], c2 = src[2 * NU], c3 = src[3 * NU];
+                        const float2 w0 = dup(wv.x), w1 = dup(wv.y), w2 = dup(wv.z), w3 = dup(wv.w);
+                        const float2 l = fma2(w3, lo2(c3), fma2(w2, lo2(c2), fma2(w1, lo2(c1), mul2(w0, lo2(c0)))));
+                        const float2 h = fma2(w3, hi2(c3), fma2(w2, hi2(c2), fma2(w1, hi2(c1), mul2(w0, hi2(c0)))));
+                        ut4[c] = make_float4(l.x, l.y, h.x, h.y);
                     }
                 }
                 __syncthreads();
-                // 4. pairs of this x value
-                for (int pi = grp[gi]; pi < grp[gi + 1]; ++pi) {
-                    const int b = pair_yval[pi];
-                    const int o = offy[b * my + yr];
-                    const float4 wv = *reinterpret_cast<const float4*>(wy + (b * my + yr) * 4);
-                    const int vbase = yi - cy0 - 2 + o;  // column a rows vbase..+3, column b rows vbase+1..+4
-                    if (pi == p.zero_pair) {
-                        // intensity at the subvoxel centre (interpolateIntensity): the
-                        // (0, 0) pair's x/y passes are the intensity's; z pass with rho_z = 0
-                        float2 Tw[NW];
+                // 4. pairs of this mid value
+                if (!work) continue;
+                for (int pi = __float_as_int(grp.y); pi < __float_as_int(grp.z); ++pi) {
+                    const float4 r0 = uget(ut, p.utab, p.u_pair + 4 * pi);
+                    const float4 r1 = uget(ut, p.utab, p.u_pair + 4 * pi + 1);
+                    const float4 r2 = uget(ut, p.utab, p.u_pair + 4 * pi + 2);
+                    const float4 r3 = uget(ut, p.utab, p.u_pair + 4 * pi + 3);
+                    const int a = __float_as_int(r2.w) * mx + xr;
+                    const float4 wv = *reinterpret_cast<const float4*>(wx + a * 4);
+                    const float4* ubase = ut4 + q * NU + xi - cx0 - 2 + offx[a];
+                    const float4* pa = ubase + __float_as_int(r2.x) * uplane;
+                    const float4* pb = ubase + __float_as_int(r2.y) * uplane;
+                    const float4* pc = ubase + __float_as_int(r2.z) * uplane;
+                    // x pass of the three planes, in the pair's plane order, then into the
+                    // pair's frame on both halves at once (on single cells, before the
+                    // halves are packed, the same products took 8.4 instead of 7.5 ms on
+                    // four volumes of 128 x 128 x 64 at 4 x 4 x 2)
+                    float2 TP[NH], TE[NH], TZ[NH];
 #pragma unroll
-                        for (int w = 0; w < NW; ++w) {
-                            const float4* src = ut + (w * NV + vbase) * kTileX + xf;
-                            const float u0 = src[0].w, u1 = src[kTileX].w, u2 = src[2 * kTileX].w,
-                                        u3 = src[3 * kTileX].w, u4 = src[4 * kTileX].w;
-                            Tw[w].x = fmaf(wv.w, u3, fmaf(wv.z, u2, fmaf(wv.y, u1, wv.x * u0)));
-                            Tw[w].y = fmaf(wv.w, u4, fmaf(wv.z, u3, fmaf(wv.y, u2, wv.x * u1)));
-                        }
+                    for (int wq = 0; wq < NQ; ++wq) {
+                        float A[4], Bv[4], Cv[4];
+                        filter4(wv, pa + wq * TY * NU, A);
+                        filter4(wv, pb + wq * TY * NU, Bv);
+                        filter4(wv, pc + wq * TY * NU, Cv);
 #pragma unroll
-                        for (int z = 0; z < FZ; ++z) {
-                            const int zr = z % MZ, zi = z / MZ;
-                            const float* qz = wzi + zr * 5;
-                            // exactly the reference's 4 taps (kernel.cu:268-283), so a
-                            // non-finite voxel reaches the same subvoxels: they start one
-                            // coarse cell later when floor((zr + 0.5) / mz - 0.5) = 0,
-                            // i.e. when 2 zr + 1 >= mz (the fifth weight is 0)
-                            const int m0 = (2 * zr + 1 >= MZ) ? 1 : 0;
-                            float2 acc = mul2(dup(qz[m0]), Tw[zi + m0]);
-#pragma unroll
-                            for (int m = m0 + 1; m < m0 + 4; ++m) acc = fma2(dup(qz[m]), Tw[zi + m], acc);
-                            const int Z = Z0 + z;
-                            if (Z >= B.lo[2] && Z < B.hi[2]) {
-                                const bool zint = Z >= B.int_lo[2] && Z <= B.int_hi[2];
-                                const long long zo = sbase + (long long)(Z - B.lo[2]) * zstride;
-                                if (ina) p.int_stack[zo + va] = (inta && zint) ? fmaxf(acc.x, 0.f) : 0.f;
-                                if (inb) p.int_stack[zo + vb] = (intb && zint) ? fmaxf(acc.y, 0.f) : 0.f;
-                            }
+                        for (int k = 0; k < 4; ++k) {
+                            put_half<CH>(TP, wq * 4 + k, A[k]);
+                            put_half<CH>(TE, wq * 4 + k, Bv[k]);
+                            put_half<CH>(TZ, wq * 4 + k, Cv[k]);
                         }
                     }
-                    float2 Tx[NW], Ty[NW], Tz[NW];
 #pragma unroll
-                    for (int w = 0; w < NW; ++w) {
-                        const float4* src = ut + (w * NV + vbase) * kTileX + xf;
-                        const float4 u0 = src[0], u1 = src[kTileX], u2 = src[2 * kTileX], u3 = src[3 * kTileX],
-                                     u4 = src[4 * kTileX];
-                        Tx[w].x = fmaf(wv.w, u3.x, fmaf(wv.z, u2.x, fmaf(wv.y, u1.x, wv.x * u0.x)));
-                        Ty[w].x = fmaf(wv.w, u3.y, fmaf(wv.z, u2.y, fmaf(wv.y, u1.y, wv.x * u0.y)));
-                        Tz[w].x = fmaf(wv.w, u3.z, fmaf(wv.z, u2.z, fmaf(wv.y, u1.z, wv.x * u0.z)));
-                        Tx[w].y = fmaf(wv.w, u4.x, fmaf(wv.z, u3.x, fmaf(wv.y, u2.x, wv.x * u1.x)));
-                        Ty[w].y = fmaf(wv.w, u4.y, fmaf(wv.z, u3.y, fmaf(wv.y, u2.y, wv.x * u1.y)));
-                        Tz[w].y = fmaf(wv.w, u4.z, fmaf(wv.z, u3.z, fmaf(wv.y, u2.z, wv.x * u1.z)));
+                    for (int w = 0; w < NH; ++w) {
+                        const float2 A = TP[w], Bv = TE[w];
+                        TP[w] = fma2(hi2(r0), Bv, mul2(lo2(r0), A));
+                        TE[w] = fma2(hi2(r1), Bv, mul2(lo2(r1), A));
                     }
-                    // rotate (x, y) about z so that the pair's ring direction lies in the
-                    // x'z plane: P = g.x', E = g.y' (x' = (ux, uy)/h, y' = z x x')
-                    {
-                        const float2 rot = pair_rot[pi];
-                        const float2 ca = dup(rot.x), sb = dup(rot.y), nsb = dup(-rot.y);
-#pragma unroll
-                        for (int w = 0; w < NW; ++w) {
-                            const float2 gx = Tx[w], gy = Ty[w];
-                            Tx[w] = fma2(gy, sb, mul2(gx, ca));
-                            Ty[w] = fma2(gy, ca, mul2(gx, nsb));
-                        }
-                    }
-                    for (int qi = pair_pt[pi]; qi < pair_pt[pi + 1]; ++qi) {
-                        // point u = |u| (h x' + c z): dot = g.u/|u| = h P + c Z, the
-                        // perpendicular part of g is (E, h Z - c P), and Dk/r = |u| sin(angle)
-                        const float4 pv = pt_vec[qi];
-                        const float2 hh = dup(pv.x), cc = dup(pv.y), ncc = dup(-pv.y);
-                        const float wgt = pv.z;
-                        const float2 nun = dup(pv.w);  // -|u|
-                        const int zc = pt_zval[qi];
-                        const float* wzc = wz + zc * (MZ * 4);
-                        const int offmask = offz[zc];
-                        auto zpass = [&](auto OFF, int zr, const float2 (&w4)[4]) {
+                    for (int qi = __float_as_int(r3.x); qi < __float_as_int(r3.y); ++qi) {
+                        const float4 c0 = uget(ut, p.utab, p.u_pt + 3 * qi);
+                        const float4 c1 = uget(ut, p.utab, p.u_pt + 3 * qi + 1);
+                        const float4 c2i = uget(ut, p.utab, p.u_pt + 3 * qi + 2);
+                        const int offmask = __float_as_int(c2i.y);
+                        // in a vector register: an FMA takes one uniform operand, a second
+                        // one would be copied in front of every use
+                        float root = c1.z;
+                        asm volatile("" : "+f"(root));
+                        auto zpass = [&](auto OFF, int zr, float2 w0, float2 w1, float2 w2, float2 w3) {
                             constexpr int o = decltype(OFF)::value;
 #pragma unroll
-                            for (int zi = 0; zi < CZ; ++zi) {
+                            for (int zi = 0; zi < CH; ++zi) {
                                 const int z = zi * MZ + zr;
-                                float2 gx = mul2(w4[0], Tx[zi + o]);
-                                float2 gy = mul2(w4[0], Ty[zi + o]);
-                                float2 gz = mul2(w4[0], Tz[zi + o]);
-#pragma unroll
-                                for (int m = 1; m < 4; ++m) {
-                                    gx = fma2(w4[m], Tx[zi + o + m], gx);
-                                    gy = fma2(w4[m], Ty[zi + o + m], gy);
-                                    gz = fma2(w4[m], Tz[zi + o + m], gz);
-                                }
-                                // gx = P, gy = E, gz = Z after the pair rotation
-                                const float2 dot = fma2(cc, gz, mul2(hh, gx));
-                                const float2 cp = fma2(hh, gz, mul2(ncc, gx));
-                                const float2 c2 = fma2(cp, cp, mul2(gy, gy));  // |g_perp|^2
-                                const float2 g2 = fma2(dot, dot, c2);          // |g|^2
+                                const float2 P = fma2(w3, TP[zi + o + 3], fma2(w2, TP[zi + o + 2], fma2(w1, TP[zi + o + 1], mul2(w0, TP[zi + o]))));
+                                const float2 E = fma2(w3, TE[zi + o + 3], fma2(w2, TE[zi + o + 2], fma2(w1, TE[zi + o + 1], mul2(w0, TE[zi + o]))));
+                                const float2 Zc = fma2(w3, TZ[zi + o + 3], fma2(w2, TZ[zi + o + 2], fma2(w1, TZ[zi + o + 1], mul2(w0, TZ[zi + o]))));
+                                const float2 dot = fma2(lo2(c0), Zc, P);         // along the ring direction
+                                const float2 cp = fma2(hi2(c0), P, Zc);          // across it
+                                const float2 c2 = fma2(cp, cp, mul2(E, E));      // |g_perp|^2
+                                const float2 g2 = fma2(dot, dot, c2);            // |g|^2
                                 // sin = sqrt(c2) / sqrt(g2): g parallel to u gives 0, g = 0
                                 // gives 0 * inf = NaN (the reference's 0/0).
                                 const float2 sn = mul2(make_float2(sqrt_approx(c2.x), sqrt_approx(c2.y)),
                                                        make_float2(rsqrt_approx(g2.x), rsqrt_approx(g2.y)));
-                                const float2 om = fma2(sn, nun, dup(1.0f));     // 1 - Dk/r
-                                const float2 D = mul2(om, om);
-                                const float2 sw = make_float2(sign_weight(wgt, dot.x), sign_weight(wgt, dot.y));
-                                S[z] = fma2(D, sw, S[z]);
+                                const float2 om = fma2(sn, lo2(c1), dup(root));  // sqrt(weight) (1 - Dk/r)
+                                S[z] = fma2(om, make_float2(flip_sign(om.x, dot.x), flip_sign(om.y, dot.y)), S[z]);
                             }
                         };
 #pragma unroll
                         for (int zr = 0; zr < MZ; ++zr) {
-                            // weights of one phase at a time keep register pressure low;
-                            // the tap offset is uniform over the warp
-                            float2 w4[4];
-#pragma unroll
-                            for (int m = 0; m < 4; ++m) w4[m] = dup(wzc[zr * 4 + m]);
+                            const float4 wa = uget(ut, p.utab, p.u_wz + 2 * (__float_as_int(c2i.x) + zr));
+                            const float4 wb = uget(ut, p.utab, p.u_wz + 2 * (__float_as_int(c2i.x) + zr) + 1);
                             if ((offmask >> zr) & 1)
-                                zpass(IntC<1>{}, zr, w4);
+                                zpass(IntC<1>{}, zr, lo2(wa), hi2(wa), lo2(wb), hi2(wb));
                             else
-                                zpass(IntC<0>{}, zr, w4);
+                                zpass(IntC<0>{}, zr, lo2(wa), hi2(wa), lo2(wb), hi2(wb));
                         }
                     }
                 }
             }
 
-            // 5. finalize and store radiality
+            // 5. finalize and store radiality (S holds the sum with the sign of the
+            //    projection; converging samples count positive)
+            const int rlo = B.rad_lo[a2], rhi = B.rad_hi[a2];
+            float* dst = p.rad_stack + sbase + v0;
 #pragma unroll
-            for (int z = 0; z < FZ; ++z) {
-                const int Z = Z0 + z;
-                if (Z < B.lo[2] || Z >= B.hi[2]) continue;
-                const bool zok = Z >= B.rad_lo[2] && Z <= B.rad_hi[2];
-                const long long zo = sbase + (long long)(Z - B.lo[2]) * zstride;
-                float ra = (rada && zok) ? S[z].x : __int_as_float(0x7fc00000);
-                float rb = (radb && zok) ? S[z].y : __int_as_float(0x7fc00000);
-                if (p.renorm) {
-                    ra = 0.5f + ra * 0.5f;
-                    rb = 0.5f + rb * 0.5f;
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int z = 0; z < HZ; ++z) {
+                    const int Z = Z0 + h * HZ + z;
+                    if (!in || Z < zlo || Z >= zhi) continue;
+                    float r = rad && Z >= rlo && Z <= rhi ? (h ? S[z].y : S[z].x) * p.neg_weight
+                                                          : __int_as_float(0x7fc00000);
+                    if (p.renorm) r = 0.5f + r * 0.5f;
+                    if (p.poscon) r = fmaxf(r, 0.f);
+                    dst[(h * HZ + z) * zstride] = r;
                 }
-                if (p.poscon) {
-                    ra = fmaxf(ra, 0.f);
-                    rb = fmaxf(rb, 0.f);
-                }
-                if (ina) p.rad_stack[zo + va] = ra;
-                if (inb) p.rad_stack[zo + vb] = rb;
-            }
         }
     }
 }
@@ -565,8 +665,9 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 // 4D tensor map (x, y, z, t) of the input with the tile's staging box; false
 // (plain loads) when TMA staging is off for this launch or the input cannot be
 // described (base or row pitch not 16-byte aligned).
-bool encode_input_map(const RadParams& p, int es, CUtensorMap* map) {
+bool encode_input_map(const FwdParams& p, CUtensorMap* map) {
     std::memset(map, 0, sizeof *map);
+    const int es = p.in_u16 ? 2 : 4;
     if (p.tma_bx <= 0) return false;
     if ((reinterpret_cast<uintptr_t>(p.in) & 15) != 0 || ((long long)p.W * es) % 16 != 0) return false;
     if (p.tma_bx > 256 || p.NIY > 256 || p.NIZ > 256 || (p.tma_bx * es) % 16 != 0) return false;
@@ -574,7 +675,9 @@ bool encode_input_map(const RadParams& p, int es, CUtensorMap* map) {
     if (!fn) return false;
     const cuuint64_t dim[4] = {(cuuint64_t)p.W, (cuuint64_t)p.H, (cuuint64_t)p.D, (cuuint64_t)p.T};
     const cuuint64_t stride[3] = {(cuuint64_t)p.W * es, (cuuint64_t)p.W * p.H * es, (cuuint64_t)p.W * p.H * p.D * es};
-    const cuuint32_t box[4] = {(cuuint32_t)p.tma_bx, (cuuint32_t)p.NIY, (cuuint32_t)p.NIZ, 1u};
+    const bool zin = p.ax2 == 2;
+    const cuuint32_t box[4] = {(cuuint32_t)p.tma_bx, (cuuint32_t)(zin ? p.NIY : p.NIZ),
+                               (cuuint32_t)(zin ? p.NIZ : p.NIY), 1u};
     const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
     const CUresult r = fn(map, es == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
                           const_cast<void*>(p.in), dim, stride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -583,84 +686,51 @@ bool encode_input_map(const RadParams& p, int es, CUtensorMap* map) {
     return r == CUDA_SUCCESS;
 }
 
-template <int MZ, typename Tin>
-int launch_mz(const RadParams& p, int grid, size_t smem, cudaStream_t st) {
-    constexpr int CZ = cz_for_mag(MZ);
-    auto k = p.TY > 16 ? radiality_kernel<MZ, CZ, Tin, true> : radiality_kernel<MZ, CZ, Tin, false>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    RadParams q = p;
-    CUtensorMap map;
-    q.use_tma = encode_input_map(p, (int)sizeof(Tin), &map) ? 1 : 0;
-    k<<<grid, p.TY * (kTileX / 2), smem, st>>>(q, map);
-    return (int)cudaGetLastError();
+size_t g4_words(const FwdParams& p) {  // float4s of the G planes
+    const int nq = p.cz / 4 + 1;
+    return (size_t)3 * nq * p.NV * p.NU;
 }
 
-template <int MZ, typename Tin>
-int occ_mz(int threads, size_t smem, int* out) {
-    constexpr int CZ = cz_for_mag(MZ);
-    auto k = threads > 128 ? radiality_kernel<MZ, CZ, Tin, true> : radiality_kernel<MZ, CZ, Tin, false>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k, threads, smem);
-}
-
-template <typename Tin>
-int dispatch(const RadParams& p, int grid, size_t smem, cudaStream_t st) {
+// f(kernel, table size) for the launch's z magnification and table form
+template <class F>
+int with_kernel(const FwdParams& p, F&& f) {
+    auto go = [&](auto mz) -> int {
+        constexpr int MZ = decltype(mz)::value;
+        if (p.u_count > kUTabMax) return f(radiality_kernel<MZ, 4, 1>, IntC<1>{});
+        if (p.cz == 8) return f(radiality_kernel<MZ, 8, kUTabMax>, IntC<kUTabMax>{});
+        return f(radiality_kernel<MZ, 4, kUTabMax>, IntC<kUTabMax>{});
+    };
     switch (p.mag[2]) {
-        case 1: return launch_mz<1, Tin>(p, grid, smem, st);
-        case 2: return launch_mz<2, Tin>(p, grid, smem, st);
-        case 3: return launch_mz<3, Tin>(p, grid, smem, st);
-        case 4: return launch_mz<4, Tin>(p, grid, smem, st);
-        case 5: return launch_mz<5, Tin>(p, grid, smem, st);
-        case 6: return launch_mz<6, Tin>(p, grid, smem, st);
-        case 7: return launch_mz<7, Tin>(p, grid, smem, st);
-        case 8: return launch_mz<8, Tin>(p, grid, smem, st);
-    }
-    return (int)cudaErrorInvalidValue;
-}
-
-template <typename Tin>
-int occ_dispatch(int mz, int threads, size_t smem, int* out) {
-    switch (mz) {
-        case 1: return occ_mz<1, Tin>(threads, smem, out);
-        case 2: return occ_mz<2, Tin>(threads, smem, out);
-        case 3: return occ_mz<3, Tin>(threads, smem, out);
-        case 4: return occ_mz<4, Tin>(threads, smem, out);
-        case 5: return occ_mz<5, Tin>(threads, smem, out);
-        case 6: return occ_mz<6, Tin>(threads, smem, out);
-        case 7: return occ_mz<7, Tin>(threads, smem, out);
-        case 8: return occ_mz<8, Tin>(threads, smem, out);
+        case 1: return go(IntC<1>{});
+        case 2: return go(IntC<2>{});
+        case 3: return go(IntC<3>{});
+        case 4: return go(IntC<4>{});
+        case 5: return go(IntC<5>{});
+        case 6: return go(IntC<6>{});
+        case 7: return go(IntC<7>{});
+        case 8: return go(IntC<8>{});
     }
     return (int)cudaErrorInvalidValue;
 }
 
 }  // namespace
 
-// Tile height (subvoxel rows) for a y magnification: a multiple of 2*my (each
-// thread pairs row y with y + my) and of 4 (whole warps of 16 x 2 threads).
-int tile_rows_for_mag(int my) {
-    switch (my) {
-        case 1: case 2: case 4: case 8: return 16;
-        case 3: case 6: return 12;
-        case 5: return 20;
-        default: return 28;  // 7
-    }
+// float4s of the U planes, which also hold the input tile (from plane 1 on)
+// while the gradient is formed
+int radiality_u_region(const FwdParams& p) {
+    const int nq = p.cz / 4 + 1;
+    const int plane = nq * p.TY * p.NU;
+    return std::max(3 * plane, plane + (p.NIX * p.NIY * p.NIZ + 3) / 4);
 }
 
-size_t radiality_smem_bytes(const RadParams& p) {
-    const int NW = cz_for_mag(p.mag[2]) + 4;
-    size_t b = sizeof(float4) * ((size_t)p.NU * p.NV * NW + (size_t)kTileX * p.NV * NW);
-    b += sizeof(float) * ((((size_t)p.NIX * p.NIY * p.NIZ + 3) & ~(size_t)3) + p.smem_table_words);
-    if (p.tma_bx > 0) {
-        // staging box (element size 4 covers both input types), 128-byte aligned start
-        b += 128 + (size_t)p.tma_bx * p.NIY * p.NIZ * 4;
-    }
+size_t radiality_smem_bytes(const FwdParams& p) {
+    size_t b = sizeof(float4) * (g4_words(p) + (size_t)p.u_region) + sizeof(float) * (size_t)p.lane_words;
+    if (p.tma_bx > 0) b += 128 + (size_t)p.tma_bx * p.NIY * p.NIZ * (p.in_u16 ? 2 : 4);  // 128-byte aligned start
     return (b + 15) & ~(size_t)15;
 }
 
-int radiality_tma_box_x(const RadParams& p, int in_u16) {
-    const int es = in_u16 ? 2 : 4;
+int radiality_tma_box_x(const FwdParams& p) {
+    const int es = p.in_u16 ? 2 : 4;
     const int al = 16 / es;
     if (((long long)p.W * es) % 16 != 0) return 0;
     const char* e = std::getenv("RFBA_TMA");
@@ -669,16 +739,35 @@ int radiality_tma_box_x(const RadParams& p, int in_u16) {
     return bx <= 256 ? bx : 0;
 }
 
-int launch_radiality(const RadParams& p, int grid, size_t smem, int in_u16, void* stream) {
+int launch_radiality(const FwdParams& p, const FwdPlan& plan, int grid, size_t smem, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    return in_u16 ? dispatch<uint16_t>(p, grid, smem, st) : dispatch<float>(p, grid, smem, st);
+    return with_kernel(p, [&](auto k, auto n) -> int {
+        constexpr int UN = decltype(n)::value;
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        FwdParams q = p;
+        CUtensorMap map;
+        q.use_tma = encode_input_map(p, &map) ? 1 : 0;
+        UTab<UN> tab;
+        if (UN > 1) {
+            std::memcpy(tab.q, plan.utab.data(), plan.utab.size() * sizeof(float));
+            std::memset(reinterpret_cast<char*>(tab.q) + plan.utab.size() * sizeof(float), 0,
+                        sizeof tab.q - plan.utab.size() * sizeof(float));
+        } else {
+            std::memset(&tab, 0, sizeof tab);
+        }
+        k<<<grid, p.TY * kTileX, smem, st>>>(q, map, tab);
+        return (int)cudaGetLastError();
+    });
 }
 
-int radiality_max_ctas_per_sm(const RadParams& p, int in_u16, int* out) {
+int radiality_max_ctas_per_sm(const FwdParams& p, int* out) {
     const size_t smem = radiality_smem_bytes(p);
-    const int threads = p.TY * (kTileX / 2);
-    return in_u16 ? occ_dispatch<uint16_t>(p.mag[2], threads, smem, out)
-                  : occ_dispatch<float>(p.mag[2], threads, smem, out);
+    return with_kernel(p, [&](auto k, auto) -> int {
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k, p.TY * kTileX, smem);
+    });
 }
 
 }  // namespace rfba

@@ -3,6 +3,7 @@
 #pragma once
 #include <vector_types.h>
 
+#include <array>
 #include <cstdint>
 #include <cstddef>
 #include <string>
@@ -12,29 +13,20 @@
 
 namespace rfba {
 
-// Output tile of the radiality kernel: 16 x TY subvoxel columns (two per
-// thread, TY from tile_rows_for_mag) and FZ = MZ * CZ subvoxels deep along z,
-// held in registers.
+// Output tile of the radiality kernel: 16 x TY subvoxel columns (one per thread,
+// TY = kTileRows unless tuned) and FZ = MZ * CZ subvoxels deep along its innermost axis, held in registers.
 constexpr int kTileX = 16;
-constexpr int kMaxThreads = 224;  // 16 x 14 threads for the 28-row tile (mag_y 7)
+constexpr int kTileRows = 8;
+constexpr int kMaxThreads = 256;  // 16 x 16 threads for the 32-row tile (mid magnification 8)
 constexpr int kMaxMag = 8;
 constexpr int kMaxGradRange = 3;
 // Adjoint tile: 16 x 16 subvoxel columns (two consecutive rows per thread).
 constexpr int kAdjRows = 16;
 constexpr int kAdjThreads = kTileX * kAdjRows / 2;
 
-// Coarse z cells per tile for a given z magnification (FZ = MZ * CZ), and the
-// forward kernel's resident CTAs per SM (launch bound; 128-thread tiles).
-// Compile-time tuning knobs: -DRFBA_CZ_MZ2=n / -DRFBA_FWD_CTAS=n.
-#ifndef RFBA_CZ_MZ2
-#define RFBA_CZ_MZ2 8
-#endif
-#ifndef RFBA_FWD_CTAS
-#define RFBA_FWD_CTAS 3
-#endif
-constexpr int cz_for_mag(int mz) {
-    return mz == 1 ? 8 : mz == 2 ? RFBA_CZ_MZ2 : mz == 3 ? 5 : mz == 4 ? 4 : mz == 5 ? 3 : 2;
-}
+// The forward kernel's register limit for MZ x CZ tiles: MZ CZ for the sums and
+// 6 (CZ / 2 + 4) for the y-filtered columns are live through the point loop.
+constexpr int fwd_regs(int mz, int cz) { return mz * cz + 6 * (cz / 2 + 4) <= 88 ? 128 : 168; }
 
 // Coarse z cells per tile of the adjoint kernel (it holds twice the register
 // columns of the forward).
@@ -53,16 +45,16 @@ struct BlockDev {
     int zbase;       // first fine z of the tile grid (multiple of mz, <= lo[2])
     int ntile[3];    // tiles along x, y, z
     int nreg[3];     // region extent hi - lo
-    int pad;
+    int cz;          // coarse cells per forward tile along its innermost axis (4 or 8)
     long long vox;        // region voxels
     long long stack_off;  // element offset of this block's [t][v] stack slice
     long long out_offset;
     long long out_stride[3];
 };
 
-// Tile work unit: block index and tile coordinates.
+// Tile work unit: block index and tile coordinates along x, y, z.
 struct TileDesc {
-    int block, tx, ty, tz;
+    int block, t[3];
 };
 
 // Deduplicated ring and its factorisation per axis. The n^2 ring samples of
@@ -88,13 +80,98 @@ struct RingPlan {
     std::vector<float> rx, ry, rz;
 };
 
+// Largest uniform table (float4s) that travels in the forward kernel's parameters.
+constexpr int kUTabMax = 768;
+
+// The forward kernel's plan of a configuration. Its tiles run over (x, mid,
+// innermost) = (x, y, z) or (x, z, y). The first pass filters along mid, once for
+// each of its distinct ring values; the second along x, once for each (mid, x) pair
+// and cell of the innermost axis, (CZ + 4) / (MZ CZ) per subvoxel, so less the larger
+// the innermost magnification MZ; the third along the innermost axis for each point.
+// The ring has fewer distinct z than y values (7 against 13 at 6 axes), so z is the
+// mid axis unless its magnification is the larger one (arrange() in plan.cpp
+// compares the two orders' costs).
+//
+// A ring point u = (x, m, n)/r belongs to the pair of its (m, x) values. The pair's
+// columns are turned into a frame where u lies in the P-Z plane (P along (x, m), E
+// across it) with every component scaled by 1 / cos of u's elevation, so that most
+// products drop out: with kappa = tan of the elevation dot = P + kappa Z and cp = Z -
+// kappa P are the same positive multiple of g.u/|u| and of the part of g across u
+// in that plane, and E carries the scale itself. On the axis (x = m = 0) P is the
+// innermost component, one pair per direction.
+//
+// utab, records of float4 (words as int bits where marked *):
+//   groups [ngroups]     {mid value*, first pair*, end pair*, 0}
+//   pairs  [npairs][4]   P = r0.x A + r0.z B: {r0.x, r0.x, r0.z, r0.z}, E likewise,
+//                        {plane of A*, B*, Z*, x value*}, {first point*, end point*, 0, 0}
+//   points [npoints][3]  {kappa, kappa, -kappa, -kappa}, {-sqrt(rho)|u| x 2, sqrt(rho) x 2},
+//                        {first record of the n value's weights*, offset mask*, 0, 0}
+//   wz     [nzv][mz][2]  {w0, w0, w1, w1}, {w2, w2, w3, w3}
+//   wi     [mz]          the intensity's four weights
+// Offset masks: bit ph says that phase ph's taps start one coarse cell later. rho is
+// the point's multiplicity over the commonest one, whose weight is neg_weight. lane:
+// per x and per mid value and phase the 4 tap weights and their offset, looked up by
+// lane and row in shared memory.
+struct FwdPlan {
+    int mag[3] = {0, 0, 0};  // tile axis order
+    int ax1 = 1, ax2 = 2;    // volume axes of the mid and innermost tile axis
+    std::vector<float> utab, lane;
+    int u_grp = 0, u_pair = 0, u_pt = 0, u_wz = 0, u_wi = 0;
+    int l_wx = 0, l_offx = 0, l_wm = 0, l_offm = 0;
+    int ngroups = 0, npairs = 0, npoints = 0, zero_x = 0, zero_m = 0;
+    float neg_weight = 0.f;
+};
+
+// Everything the forward radiality kernel needs; passed by value.
+struct FwdParams {
+    const void* in;       // input volume [t][z][y][x]
+    int W, H, D, T;       // full input dims
+    int in_u16;
+    int mag[3];           // tile axis order (x, mid, innermost), as gr
+    int ax1, ax2;
+    int gr[4];            // gradient ranges: main, x, mid, innermost (smooth=0 => 1,0,0,0)
+    int grad_mode;        // 1: ranges (1,1,1,1), 2: (1,0,0,0), 0: generic loops
+    int R;                // gradient halo
+    int TY, cz;           // subvoxel rows (threads = 16 * TY) and innermost cells per tile
+    int NU, NV;           // coarse G tile extents
+    int NIX, NIY, NIZ;    // input tile extents (G tile + halo)
+    int u_region;         // float4s of the U planes / input tile
+    int renorm, poscon;
+    int t_chunk, nchunks;
+    int ntiles;
+    long long nitems;
+    const float* lane;    // lane tables
+    int lane_words, l_wx, l_offx, l_wm, l_offm;
+    const float4* utab;   // uniform tables in global memory (read when they do not fit the parameters)
+    int u_count, u_grp, u_pair, u_pt, u_wz, u_wi;
+    int ngroups, zero_x, zero_m;
+    float neg_weight;     // minus the commonest point's weight
+    const BlockDev* blocks;
+    const TileDesc* tiles;
+    float* rad_stack;     // [block slice][t][v]
+    float* int_stack;
+    unsigned int* work_counter;
+    // TMA staging of the input tile: box width in elements (0 = no staging area)
+    // and whether this launch uses it
+    int tma_bx;
+    int use_tma;
+    unsigned long long* err;  // bounded-wait failures (may be null)
+    // failure-detection test (RFBA_TEST_TMA_STALL): the first copy request of
+    // every work item is left out, so the bounded staging wait gives up
+    int test_skip_copy;
+    // time window of this launch: volumes [t_lo, t_hi) (t_hi 0: up to T), and
+    // the volume held by the first [t] row of the stacks (0 when they hold the
+    // whole series, t_lo when they hold one batch)
+    int t_lo, t_hi, stack_t0;
+};
+
 // Device-side tables (one contiguous buffer), offsets in 4-byte words.
 struct TableLayout {
     int wx, offx, wy, offy, wz, offz, wzi, grp_xval, grp, pair_yval, pair_pt, pt_zval, pt_vec, pair_rot;
     int words;
 };
 
-// Everything the radiality kernel needs; passed by value.
+// Everything the radiality adjoint kernel needs; passed by value.
 struct RadParams {
     const void* in;       // input volume [t][z][y][x]
     int W, H, D, T;       // full input dims
@@ -116,21 +193,10 @@ struct RadParams {
     TableLayout tl;
     const BlockDev* blocks;
     const TileDesc* tiles;
-    float* rad_stack;     // [block slice][t][v]
-    float* int_stack;
     unsigned int* work_counter;
     int smem_table_words;
-    // TMA staging of the input tile (forward only): box width in elements
-    // (0 = no staging area) and whether this launch uses it
-    int tma_bx;
-    int use_tma;
-    unsigned long long* err;  // bounded-wait failures (may be null)
-    // failure-detection test (RFBA_TEST_TMA_STALL): the first copy request of
-    // every work item is left out, so the bounded staging wait gives up
-    int test_skip_copy;
-    // time window of this launch: volumes [t_lo, t_hi) (t_hi 0: up to T), and
-    // the volume held by the first [t] row of the stacks (0 when they hold the
-    // whole series, t_lo when they hold one batch)
+    // volumes [t_lo, t_hi) of this launch (t_hi 0: up to T) and the volume of the
+    // adjoint stacks' first row
     int t_lo, t_hi, stack_t0;
 };
 
@@ -210,13 +276,13 @@ int launch_drift3d(const float* src, float* dst, const float* g, int W, int H, i
 int launch_drift_dot(const float* g, const float* dv, long long nv, int T, int axis, double* out,
                      unsigned long long* err, void* stream);
 int launch_double_to_float(const double* src, float* dst, int n, void* stream);
-int launch_radiality(const RadParams& p, int grid, size_t smem, int in_u16, void* stream);
+int launch_radiality(const FwdParams& p, const FwdPlan& plan, int grid, size_t smem, void* stream);
 // Box width (elements) of the TMA input staging for this tile, 0 when the input
 // rows cannot be addressed by a tensor map (row pitch not a multiple of 16 B).
-int radiality_tma_box_x(const RadParams& p, int in_u16);
-size_t radiality_smem_bytes(const RadParams& p);
-int tile_rows_for_mag(int my);
-int radiality_max_ctas_per_sm(const RadParams& p, int in_u16, int* out);
+int radiality_tma_box_x(const FwdParams& p);
+int radiality_u_region(const FwdParams& p);
+size_t radiality_smem_bytes(const FwdParams& p);
+int radiality_max_ctas_per_sm(const FwdParams& p, int* out);
 int launch_temporal(const TemporalParams& p, void* stream);
 int launch_temporal_stream(const StreamParams& p, void* stream);
 int launch_temporal_stream_adjoint(const StreamAdjParams& p, long long vox, void* stream);
@@ -234,6 +300,15 @@ int launch_seed_spots(const float* map, const int map_dims[3], int mag, const in
 bool build_ring_plan(const rfba_srrf_config& c, RingPlan* rp, std::string* err);
 bool build_tables(const rfba_srrf_config& c, const RingPlan& rp, std::vector<float>* words, TableLayout* tl,
                   std::string* err);
+bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err);
+// Parameters of a forward launch that follow from the plan and configuration
+// (not the block and tile lists, stacks and schedule). ty: tile rows, 0 = default.
+FwdParams forward_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, int in_u16, const int dims[4],
+                         int ty, int cz);
+// Tiles of a block's region [lo, hi) in the plan's tile axes (b->cz set).
+void forward_tiles(const FwdPlan& fp, int ty, BlockDev* b);
+// Tile depth (innermost cells, 4 or 8) for regions of these innermost extents.
+int forward_depth(const FwdPlan& fp, const std::vector<std::array<int, 2>>& lo_hi);
 bool window_range(float ring_radius_dummy, const std::vector<float>& rcoord, int mag, int dim, int* lo, int* hi);
 int fine_window_int(int mag, int dim, int* lo, int* hi);
 
