@@ -370,10 +370,12 @@ static int plan_passes(rfba_ctx* ctx, const rfba_srrf_config& cfg, rfba_dtype dt
         pp.vox = vox;
         ps->max_vox = std::max(ps->max_vox, vox);
         const long long nt = (long long)(pp.t1 - pp.t0);
-        // time chunk: enough work items for ~8 per CTA slot
+        // time chunk: enough work items for 64 per CTA slot, so that the last round
+        // of items leaves the chip idle for at most 1 / 64 of the launch (an item
+        // costs a few microseconds beyond its volumes' 100 and more each)
         int chunk = ctx->chunk_override;
         if (chunk <= 0) {
-            const long long want = 8LL * slots;
+            const long long want = 64LL * slots;
             long long nch = (want + nt - 1) / nt;
             nch = std::max<long long>(1, std::min<long long>(nch, stack_t));
             chunk = (int)((stack_t + nch - 1) / nch);
@@ -1221,7 +1223,7 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
         return RFBA_ERR_UNSUPPORTED;
     }
     const int slots = per_sm * ctx->sm_count;
-    long long nch = (8LL * slots + rp.ntiles - 1) / rp.ntiles;
+    long long nch = (64LL * slots + rp.ntiles - 1) / rp.ntiles;
     nch = std::max<long long>(1, std::min<long long>(nch, TW));
     rp.t_chunk = (int)((TW + nch - 1) / nch);
     rp.nchunks = (TW + rp.t_chunk - 1) / rp.t_chunk;

@@ -272,7 +272,7 @@ extern "C" int rfba_srrf_forward_static_scratch(const rfba_srrf_config* cfg, con
     if ((s = cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count"))) return s;
     if (per_sm < 1) return fail(RFBA_ERR_UNSUPPORTED, "radiality kernel does not fit on an SM");
     const int slots = per_sm * sms;
-    long long nch = (8LL * slots + rp.ntiles - 1) / rp.ntiles;
+    long long nch = (64LL * slots + rp.ntiles - 1) / rp.ntiles;
     nch = std::max<long long>(1, std::min<long long>(nch, T));
     rp.t_chunk = (int)((T + nch - 1) / nch);
     rp.nchunks = (T + rp.t_chunk - 1) / rp.t_chunk;
