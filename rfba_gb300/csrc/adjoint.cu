@@ -13,42 +13,21 @@
 //      dL/dmap and the stored radiality/intensity stacks;
 //   2. radiality adjoint, persistent over (tile, time) like the forward: the
 //      interpolated gradient at every ring sample is recomputed (not stored),
-//      the derivative of the radiality term is pushed back through the z pass
-//      (registers), the frame rotation, the y pass (shared-memory atomics), the
-//      x pass (shared-memory atomics) and the gradient stencil (gather), and the
-//      tile's contribution to dL/dI' is added to global memory;
+//      the derivative of the radiality term is pushed back through the transposed
+//      passes, and the tile's contribution to dL/dI' is added to global memory;
 //   3. the drift operator's transpose gives dL/dI, and dL/dd_t is the sum over
 //      the volume of dL/dI'_t times the resampling with derivative weights on
 //      one axis.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
+#include <cstring>
 
+#include "radiality_common.cuh"
 #include "srrf_internal.h"
 
 namespace rfba {
 namespace {
-
-__device__ __forceinline__ float rsqrt_approx(float x) {
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ float sign_weight(float w, float d) {
-    return __int_as_float(__float_as_int(w) | (~__float_as_int(d) & 0x80000000));
-}
-__device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
-__device__ __forceinline__ int floordiv(int a, int b) {
-    int q = a / b;
-    return (a % b != 0 && a < 0) ? q - 1 : q;
-}
-template <int V>
-struct IntC {
-    static constexpr int value = V;
-};
 
 // Bounds check of a computed global index: out of range records the first
 // offence (site in the top byte, index below) and the access is skipped.
@@ -587,136 +566,82 @@ __global__ void temporal_adjoint_kernel(const BlockDev* __restrict__ blocks, con
 }
 
 // ---------------------------------------------------------------------------
-// Radiality adjoint.
-template <int MR, int XR, int YR, int ZR>
-__device__ __forceinline__ float4 gradient_fixed(const float* base, int NIX, int NIY) {
-    auto I = [&](int dx, int dy, int dz) { return base[(dz * NIY + dy) * NIX + dx]; };
-    float gx = 0.f, gy = 0.f, gz = 0.f;
-#pragma unroll
-    for (int i = 1; i <= MR; ++i)
-#pragma unroll
-        for (int j = -YR; j <= YR; ++j)
-#pragma unroll
-            for (int k = -ZR; k <= ZR; ++k) gx += I(i, j, k) - I(-i, j, k);
-#pragma unroll
-    for (int j = 1; j <= MR; ++j)
-#pragma unroll
-        for (int i = -XR; i <= XR; ++i)
-#pragma unroll
-            for (int k = -ZR; k <= ZR; ++k) gy += I(i, j, k) - I(i, -j, k);
-#pragma unroll
-    for (int k = 1; k <= MR; ++k)
-#pragma unroll
-        for (int i = -XR; i <= XR; ++i)
-#pragma unroll
-            for (int j = -YR; j <= YR; ++j) gz += I(i, j, k) - I(i, j, -k);
-    return make_float4(gx, gy, gz, I(0, 0, 0));
-}
-
-__device__ __forceinline__ float4 gradient_generic(const float* base, int NIX, int NIY, const int gr[4]) {
-    auto I = [&](int dx, int dy, int dz) { return base[(dz * NIY + dy) * NIX + dx]; };
-    const int mR = gr[0], xR = gr[1], yR = gr[2], zR = gr[3];
-    float gx = 0.f, gy = 0.f, gz = 0.f;
-    for (int i = 1; i <= mR; ++i)
-        for (int j = -yR; j <= yR; ++j)
-            for (int k = -zR; k <= zR; ++k) gx += I(i, j, k) - I(-i, j, k);
-    for (int j = 1; j <= mR; ++j)
-        for (int i = -xR; i <= xR; ++i)
-            for (int k = -zR; k <= zR; ++k) gy += I(i, j, k) - I(i, -j, k);
-    for (int k = 1; k <= mR; ++k)
-        for (int i = -xR; i <= xR; ++i)
-            for (int j = -yR; j <= yR; ++j) gz += I(i, j, k) - I(i, j, -k);
-    return make_float4(gx, gy, gz, I(0, 0, 0));
-}
-
-// Adjoint tile: 16 fine x columns x kAdjRows fine y rows x FZ fine z rows,
-// kAdjThreads threads. Warp k owns x columns 4k..4k+3; lane l of a warp takes
-// column 4k + (l >> 3) and the fine rows 2 (l & 7), 2 (l & 7) + 1. All
-// threads that touch an x column's U-stage entries sit in one warp, so the
-// y-pass transpose needs no shared-memory atomics: the lanes of one column
-// whose 5-row windows start on the same row (possible when my > 2) add in
-// separate phases, and __syncwarp orders the row updates of lanes whose
-// windows overlap. The x pass and its transpose run one (z, y) row of cells
-// per thread with a sliding 4-cell window, so every cell has one writer.
+// Radiality adjoint, on the forward's plan and tiles (16 x kTileRows columns, one
+// per thread, two halves of a column in a register pair; see radiality.cu). Every
+// (tile, time point) recomputes the interpolated gradient at each ring sample and
+// pushes the derivative back through the passes, transposed and in reverse order:
 //
-// Shared-memory row strides are odd in float4 units (17 for the U stage, NU
-// rounded up to odd for the cell grid). A 16-byte access is served a quarter
-// warp (8 lanes) at a time; 8 lanes walking 8 consecutive rows at one column
-// (the row windows of one x column, or one cell row per thread) then hit 8
-// different bank groups.
-constexpr int kURow = kTileX + 1;
-
-__host__ __device__ __forceinline__ int adj_nup(int NU) { return NU | 1; }
-__host__ __device__ __forceinline__ int adj_u_region_f4(int NV, int NW, int NIX, int NIY, int NIZ) {
-    const int ustage = 2 * kURow * (NV + 1) * NW;
-    const int inp = (NIX * NIY * NIZ + 3) / 4;
-    return ustage > inp ? ustage : inp;
-}
-
-// Division of 0 <= c < 65536 by d >= 2 with one multiply-high.
-struct FastDiv {
-    unsigned m;
-    __device__ explicit FastDiv(int d) : m(0xffffffffu / (unsigned)d + 1u) {}
-    __device__ int operator()(int c) const { return (int)__umulhi((unsigned)c, m); }
-};
-
+//   point   with the forward's scaled frame values (dot, cp, E, c2 = cp^2 + E^2, g2 =
+//           dot^2 + c2, s = sqrt(c2 / g2)) and K = dL/ds,
+//             ds = ((1 - s^2) (cp dcp + E dE) - s^2 dot ddot) / sqrt(c2 g2),
+//           so with k = K / sqrt(c2 g2), b = s^2 k, m = k - b:
+//             dE = m E, dZ = m cp - kappa b dot, -dP = kappa m cp + b dot;
+//   third   transposed along the innermost axis in registers, over the points of a
+//           pair;
+//   second  transposed along x: the lanes of a row exchange their columns through
+//           shared memory, plane by plane, sorted by x phase. Lane u then
+//           gathers coarse cell u: for each phase and tap one shift of the row, so the
+//           weights are uniform and no two lanes add to the same place;
+//   first   transposed along the mid axis as a gather over the tile's rows, once per
+//           ring value of that axis;
+//   stencil transposed as a gather over the cells' 3^3 neighbourhood, and one global
+//           atomic add per input voxel of the tile.
+//
+// Where two lanes of a warp updated the same shared-memory rows in turn (the second
+// pass along y, two phases for magnifications above 2), short-scoreboard and barrier
+// waits kept the FMA pipe at 43 %.
 __device__ __forceinline__ float4 f4fma(float s, float4 a, float4 c) {
     return make_float4(fmaf(s, a.x, c.x), fmaf(s, a.y, c.y), fmaf(s, a.z, c.z), fmaf(s, a.w, c.w));
 }
-__device__ __forceinline__ float4 f4add(float4 a, float4 b) {
-    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
-}
 
-template <int MZ, int CZ>
-__global__ void __launch_bounds__(kAdjThreads, 2) radiality_adjoint_kernel(const RadParams p, const AdjParams a) {
+template <int MZ, int CZ, int UN>
+__global__ void __maxnreg__(adj_regs(MZ, CZ))
+    radiality_adjoint_kernel(const __grid_constant__ FwdParams p, const __grid_constant__ AdjParams a,
+                             const __grid_constant__ UTab<UN> ut) {
+    constexpr int CH = CZ / 2;
+    constexpr int HZ = MZ * CH;
     constexpr int FZ = MZ * CZ;
+    constexpr int NH = CH + 4;
     constexpr int NW = CZ + 4;
+    constexpr int NQ = NW / 4;
     extern __shared__ float4 smem4[];
-    const int NU = p.NU, NV = p.NV, NVA = p.NV + 1, NUP = adj_nup(p.NU);
-    const int ncell = NUP * NV * NW;
-    const int nut = kURow * NVA * NW;
-    float4* gt = smem4;                    // forward G + I   [NW][NV][NUP]
-    float4* ggt = gt + ncell;              // dL/d(G, I)      [NW][NV][NUP]
-    float4* ut = ggt + ncell;              // forward U       [NW][NVA][kURow]; row NV is zero
-    float4* gut = ut + nut;                // dL/dU           [NW][NVA][kURow]
-    float* inp = reinterpret_cast<float*>(ut);  // input tile, dead once gt is built
-    float4* xw4 = ut + adj_u_region_f4(NV, NW, p.NIX, p.NIY, p.NIZ);  // x weights of the group [16]
-    int* xub = reinterpret_cast<int*>(xw4 + kTileX);                 // first tap cell of each x column [16]
-    float* tab = reinterpret_cast<float*>(xub + kTileX);
-    __shared__ unsigned int s_item;
 
-    const int nthr = blockDim.x;
-    const int tid = threadIdx.x;
+    const int NU = p.NU, NV = p.NV, TY = p.TY;
+    const int gplane = NQ * NV * NU, uplane = NQ * TY * NU;
+    // Shared layout: [G][dL/dG][U, sharing its place with the input tile and the
+    // intensity's cells][dL/dU][exchange rows][lane tables]
+    float4* gt = smem4;
+    float4* gg = gt + 3 * gplane;
+    float4* ut4 = gg + 3 * gplane;
+    float4* gu = ut4 + p.u_region;
+    float4* ex = gu + 3 * uplane;
+    float* inp = reinterpret_cast<float*>(ut4);
+    float4* icell = ut4;
     const int mx = p.mag[0], my = p.mag[1];
-    const int lane = tid & 31;
-    const int xf = (tid >> 5) * 4 + (lane >> 3);
-    const int tr = lane & 7;
-    // lanes tr, tr' of one column with tr = tr' mod nph have rows >= my apart,
-    // hence different window starts
-    const int nph = (my + 1) >> 1;
-    const int myph = tr % nph;
-    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int a1 = p.ax1, a2 = p.ax2;
+    // exchange row: four zeros, then per x phase the tile's coarse cells and four zeros
+    const int nxc = adj_cells(mx), exw = 4 + mx * nxc;
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    const int warp = tid >> 5, half = (tid >> 4) & 1;
+    float4* ex_warp = ex + warp * (2 * NQ * exw);  // [quad][row of the warp][exw]
+    float* tab = reinterpret_cast<float*>(ex + (nthr >> 5) * (2 * NQ * exw));
+    __shared__ unsigned int s_item;
+    __shared__ int2 s_row[kMaxThreads / kTileX];
+    __shared__ int s_base[kMaxThreads / kTileX];
+    __shared__ alignas(16) float s_weight[kMaxThreads / kTileX * 4];
 
-    for (int i = tid; i < p.smem_table_words; i += nthr) tab[i] = p.tables[i];
-    const float* wx = tab + p.tl.wx;
-    const int* offx = reinterpret_cast<const int*>(tab + p.tl.offx);
-    const float* wy = tab + p.tl.wy;
-    const int* offy = reinterpret_cast<const int*>(tab + p.tl.offy);
-    const float* wz = tab + p.tl.wz;
-    const int* offz = reinterpret_cast<const int*>(tab + p.tl.offz);
-    const float* wzi = tab + p.tl.wzi;
-    const int* grp_xval = reinterpret_cast<const int*>(tab + p.tl.grp_xval);
-    const int* grp = reinterpret_cast<const int*>(tab + p.tl.grp);
-    const int* pair_yval = reinterpret_cast<const int*>(tab + p.tl.pair_yval);
-    const int* pair_pt = reinterpret_cast<const int*>(tab + p.tl.pair_pt);
-    const int* pt_zval = reinterpret_cast<const int*>(tab + p.tl.pt_zval);
-    const float4* pt_vec = reinterpret_cast<const float4*>(tab + p.tl.pt_vec);
-    const float2* pair_rot = reinterpret_cast<const float2*>(tab + p.tl.pair_rot);
-
-    const float* in = static_cast<const float*>(p.in);
+    const int xf = tid & (kTileX - 1);
+    const int q = tid / kTileX;
+    for (int i = tid; i < p.lane_words; i += nthr) tab[i] = p.lane[i];
+    const float* wx = tab + p.l_wx;
+    const int* offx = reinterpret_cast<const int*>(tab + p.l_offx);
+    const float* wy = tab + p.l_wm;
+    const int* offy = reinterpret_cast<const int*>(tab + p.l_offm);
     const int NIX = p.NIX, NIY = p.NIY, NIZ = p.NIZ, R = p.R;
     const int nin = NIX * NIY * NIZ;
-    const FastDiv div_nup(NUP), div_nv(NV), div_nva(NVA), div_nix(NIX), div_niy(NIY), div_nixy(NIX * NIY);
+    const FastDiv div_nu(NU), div_nv(NV), div_ty(TY), div_nix(NIX), div_nixy(NIX * NIY);
+    const float* in = static_cast<const float*>(p.in);
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
 
     for (;;) {
         __syncthreads();
@@ -728,461 +653,438 @@ __global__ void __launch_bounds__(kAdjThreads, 2) radiality_adjoint_kernel(const
         const int chunk = (int)(item / p.ntiles);
         const TileDesc td = p.tiles[tile_i];
         const BlockDev& B = p.blocks[td.block];
-        const int bw = B.size[0], bh = B.size[1], bd = B.size[2];
+        const int bw = B.size[0], bh = B.size[a1], bd = B.size[a2];
         const int X0 = B.lo[0] + td.t[0] * kTileX;
-        const int Y0 = B.lo[1] + td.t[1] * kAdjRows;
-        const int Z0 = B.zbase + td.t[2] * FZ;
+        const int Y0 = B.lo[a1] + td.t[a1] * TY;
+        const int Z0 = (B.lo[a2] / MZ) * MZ + td.t[a2] * FZ;
         const int cx0 = floordiv(X0, mx) - 2;
         const int cy0 = floordiv(Y0, my) - 2;
         const int cz0 = Z0 / MZ - 2;
-        const int X = X0 + xf;
-        const int Ya = Y0 + 2 * tr, Yb = Ya + 1;
-        const int yia = floordiv(Ya, my), yra = Ya - yia * my;
-        const int yib = floordiv(Yb, my), yrb = Yb - yib * my;
-        const bool xin = X < B.hi[0];
-        const bool ina = xin && Ya < B.hi[1];
-        const bool inb = xin && Yb < B.hi[1];
+        const int X = X0 + xf, Y = Y0 + q;
+        const int xi = floordiv(X, mx), xr = X - xi * mx;
+        if (xf == 0) {
+            const int yi = floordiv(Y, my);
+            s_row[q] = make_int2(yi - cy0 - 2, Y - yi * my);  // first tap row at offset 0, phase
+        }
+        // exchange slots that no lane of this tile fills read as zero
+        for (int i = tid & 31; i < 2 * NQ * exw; i += 32) ex_warp[i] = zero4;
+        const int ex_put = half * exw + xr * nxc + (xi - cx0 - 2) + 4;
+        const bool in_tile = X < B.hi[0] && Y < B.hi[a1];
         const long long V = B.vox;
-        const long long va = ((long long)(Ya - B.lo[1])) * B.nreg[0] + (X - B.lo[0]);
-        const long long vb = va + B.nreg[0];
-        const long long zstride = (long long)B.nreg[0] * B.nreg[1];
-        // volumes [t_lo, t_hi) of this launch (t_hi 0: up to T); dL/dS and dL/dI
-        // hold rows from volume stack_t0 on
+        const long long ystride = a1 == 1 ? B.nreg[0] : (long long)B.nreg[0] * B.nreg[1];
+        const long long zstride = a1 == 1 ? (long long)B.nreg[0] * B.nreg[1] : B.nreg[0];
+        const int zlo = B.lo[a2], zhi = B.hi[a2];
+        const long long v0 = (long long)(Y - B.lo[a1]) * ystride + (X - B.lo[0]) + (Z0 - zlo) * zstride;
+
         const int t0 = p.t_lo + chunk * p.t_chunk;
         const int t1 = min(p.t_hi > 0 ? p.t_hi : p.T, t0 + p.t_chunk);
         for (int t = t0; t < t1; ++t) {
-            const long long sbase = B.stack_off + (long long)(t - p.stack_t0) * V;
+            const long long sbase = B.stack_off + (long long)(t - p.stack_t0) * V + v0;
             const long long tbase = (long long)t * p.D * p.H * p.W;
-            // forward: input tile, gradient cells; clear the adjoint cells
-            for (int r = tid / kTileX; r < NIY * NIZ; r += nthr / kTileX) {
-                const int iz = div_niy(r), iy = r - iz * NIY;
-                const int by = clampi(cy0 - R + iy, 0, bh - 1);
-                const int bz = clampi(cz0 - R + iz, 0, bd - 1);
-                const long long rowg = tbase + ((long long)(B.origin[2] + bz) * p.H + (B.origin[1] + by)) * p.W +
-                                       B.origin[0];
-                for (int ix = tid % kTileX; ix < NIX; ix += kTileX) {
+            // dL/dS or dL/dI of this thread's subvoxels
+            auto stack_value = [&](const float* st, int z) -> float {
+                const int Z = Z0 + z;
+                const long long i = sbase + z * zstride;
+                return in_tile && Z >= zlo && Z < zhi && in_range(i, a.n_stack, a.err, 9) ? st[i] : 0.f;
+            };
+            auto global_row = [&](int iy, int iz) -> long long {
+                const int by = B.origin[a1] + clampi(cy0 - R + iy, 0, bh - 1);
+                const int bz = B.origin[a2] + clampi(cz0 - R + iz, 0, bd - 1);
+                return tbase + (a1 == 1 ? (long long)bz * p.H + by : (long long)by * p.H + bz) * p.W + B.origin[0];
+            };
+            __syncthreads();  // the previous time point is done with the input tile's place
+            for (int r = q, iy = q, iz = 0; r < NIY * NIZ; r += TY, iy += TY) {
+                while (iy >= NIY) {
+                    iy -= NIY;
+                    ++iz;
+                }
+                const long long rowg = global_row(iy, iz);
+                for (int ix = xf; ix < NIX; ix += kTileX) {
                     const long long gi = rowg + clampi(cx0 - R + ix, 0, bw - 1);
                     inp[r * NIX + ix] = in_range(gi, a.n_in, a.err, 8) ? __ldg(in + gi) : 0.f;
                 }
             }
             __syncthreads();
-            for (int c = tid; c < ncell; c += nthr) {
-                const int row = div_nup(c);
-                const int u = c - row * NUP;
-                const int w = div_nv(row), v = row - w * NV;
-                const int cu = cx0 + u, cv = cy0 + v, cw = cz0 + w;
-                float4 g4 = zero4;
-                if (u < NU && cu >= 0 && cu < bw && cv >= 0 && cv < bh && cw >= 0 && cw < bd) {
-                    const float* base = inp + ((w + R) * NIY + (v + R)) * NIX + (u + R);
-                    if (p.grad_mode == 1)
-                        g4 = gradient_fixed<1, 1, 1, 1>(base, NIX, NIY);
-                    else if (p.grad_mode == 2)
-                        g4 = gradient_fixed<1, 0, 0, 0>(base, NIX, NIY);
-                    else
-                        g4 = gradient_generic(base, NIX, NIY, p.gr);
-                }
-                gt[c] = g4;
-                ggt[c] = zero4;
-            }
-            // dL/dS of this thread's subvoxels (dL/dI is read in the (0, 0) pair)
-            float2 gS[FZ];
+            for (int c = tid; c < gplane; c += nthr) {
+                const int row = div_nu(c), u = c - row * NU;
+                const int wq = div_nv(row), v = row - wq * NV, w0 = wq * 4;
+                const int cu = cx0 + u, cv = cy0 + v, cw = cz0 + w0;
+                float g[3][4];
 #pragma unroll
-            for (int z = 0; z < FZ; ++z) {
-                const int Z = Z0 + z;
-                const bool zin = Z >= B.lo[2] && Z < B.hi[2];
-                const long long zo = sbase + (long long)(Z - B.lo[2]) * zstride;
-                const bool oka = zin && ina && in_range(zo + va, a.n_stack, a.err, 9);
-                const bool okb = zin && inb && in_range(zo + vb, a.n_stack, a.err, 9);
-                gS[z].x = oka ? a.gS[zo + va] : 0.f;
-                gS[z].y = okb ? a.gS[zo + vb] : 0.f;
+                for (int k = 0; k < 3; ++k)
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) g[k][w] = 0.f;
+                if (cu >= 0 && cu < bw && cv >= 0 && cv < bh && cw + 3 >= 0 && cw < bd) {
+                    const float* base = inp + (v + R) * NIX + (u + R);
+                    gradient4(p.grad_mode, p.gr, [&](int k) { return base + (w0 + R + k) * (NIY * NIX); }, NIX, g);
+#pragma unroll
+                    for (int w = 0; w < 4; ++w)
+                        if (cw + w < 0 || cw + w >= bd) g[0][w] = g[1][w] = g[2][w] = 0.f;
+                }
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    gt[k * gplane + c] = make_float4(g[k][0], g[k][1], g[k][2], g[k][3]);
+                    gg[k * gplane + c] = zero4;
+                }
             }
+            float2 gS[HZ];
+#pragma unroll
+            for (int z = 0; z < HZ; ++z) gS[z] = make_float2(stack_value(a.gS, z), stack_value(a.gS, z + HZ));
 
-            for (int gi_ = 0; gi_ < p.ngroups; ++gi_) {
-                __syncthreads();  // gt built / previous group's x transpose done with gut and the x tables
-                const int av = grp_xval[gi_];
-                if (tid < kTileX) {
-                    const int Xc = X0 + tid;
-                    const int xic = floordiv(Xc, mx), xrc = Xc - xic * mx;
-                    xub[tid] = xic - cx0 - 2 + offx[av * mx + xrc];
-                    xw4[tid] = *reinterpret_cast<const float4*>(wx + (av * mx + xrc) * 4);
-                }
-                for (int e = tid; e < nut; e += nthr) gut[e] = zero4;
-                __syncthreads();
-                // x pass, one (w, v) row per thread: U[xf] = sum_k wx_xf[k] G[ub(xf) + k];
-                // ub steps by 0 or 1 from one column to the next
-                for (int row = tid; row < NVA * NW; row += nthr) {
-                    const int w = div_nva(row), v = row - w * NVA;
-                    float4* dst = ut + row * kURow;
-                    if (v >= NV) {
+            // x pass transposed of one plane: every lane lays down its column, then lane u
+            // gathers cell u of its row (and a second one where a row has more than 16
+            // cells) and adds it to, or stores it in, dst
+            auto x_transpose = [&](const float2(&g)[NH], int xval, int mask, float4* dst, bool add) {
+                __syncwarp();  // the row's previous readers
 #pragma unroll
-                        for (int x = 0; x < kTileX; ++x) dst[x] = zero4;
-                        continue;
-                    }
-                    const float4* src = gt + (w * NV + v) * NUP;
-                    int ub = xub[0];
-                    float4 c0 = src[ub], c1 = src[ub + 1], c2 = src[ub + 2], c3 = src[ub + 3];
+                for (int wq = 0; wq < NQ; ++wq)
+                    ex_warp[ex_put + wq * (2 * exw)] =
+                        make_float4(get_halves<CH>(g, wq * 4), get_halves<CH>(g, wq * 4 + 1),
+                                    get_halves<CH>(g, wq * 4 + 2), get_halves<CH>(g, wq * 4 + 3));
+                __syncwarp();
+                for (int u0 = 0; u0 < NU; u0 += kTileX) {
+                    const float4* from = ex_warp + half * exw + 4 + min(u0 + xf, NU - 1);
+                    float2 lo[NQ], hi[NQ];
 #pragma unroll
-                    for (int x = 0; x < kTileX; ++x) {
-                        if (x > 0) {
-                            const int nb = xub[x];
-                            if (nb != ub) {
-                                ub = nb;
-                                c0 = c1;
-                                c1 = c2;
-                                c2 = c3;
-                                c3 = src[ub + 3];
-                            }
+                    for (int wq = 0; wq < NQ; ++wq) lo[wq] = hi[wq] = make_float2(0.f, 0.f);
+                    for (int r = 0; r < mx; ++r) {
+                        const float4 wa = uget(ut, p.utab, p.u_wx + 2 * (xval * mx + r));
+                        const float4 wb = uget(ut, p.utab, p.u_wx + 2 * (xval * mx + r) + 1);
+                        const float4* src = from + r * nxc - ((mask >> r) & 1);
+#pragma unroll
+                        for (int wq = 0; wq < NQ; ++wq) {
+                            const float4* sw = src + wq * (2 * exw);
+                            const float4 g0 = sw[0], g1 = sw[-1], g2 = sw[-2], g3 = sw[-3];
+                            lo[wq] = fma2(hi2(wb), lo2(g3), fma2(lo2(wb), lo2(g2), fma2(hi2(wa), lo2(g1), fma2(lo2(wa), lo2(g0), lo[wq]))));
+                            hi[wq] = fma2(hi2(wb), hi2(g3), fma2(lo2(wb), hi2(g2), fma2(hi2(wa), hi2(g1), fma2(lo2(wa), hi2(g0), hi[wq]))));
                         }
-                        const float4 wk = xw4[x];
-                        float4 r;
-                        r.x = fmaf(wk.w, c3.x, fmaf(wk.z, c2.x, fmaf(wk.y, c1.x, wk.x * c0.x)));
-                        r.y = fmaf(wk.w, c3.y, fmaf(wk.z, c2.y, fmaf(wk.y, c1.y, wk.x * c0.y)));
-                        r.z = fmaf(wk.w, c3.z, fmaf(wk.z, c2.z, fmaf(wk.y, c1.z, wk.x * c0.z)));
-                        r.w = 0.f;
-                        dst[x] = r;
+                    }
+                    if (u0 + xf < NU) {
+                        float4* d = dst + q * NU + u0 + xf;
+#pragma unroll
+                        for (int wq = 0; wq < NQ; ++wq) {
+                            const float4 o4 = add ? d[wq * (TY * NU)] : zero4;
+                            d[wq * (TY * NU)] = make_float4(o4.x + lo[wq].x, o4.y + lo[wq].y, o4.z + hi[wq].x, o4.w + hi[wq].y);
+                        }
                     }
                 }
+            };
+            // first pass transposed: dL/dU planes [y][u] into cells [v][u]
+            auto mid_transpose = [&](const float4* src, float4* dst, int planes, bool add) {
+                for (int c = tid; c < planes * gplane; c += nthr) {
+                    const int r = div_nu(c), u = c - r * NU;
+                    const int pw = div_nv(r), v = r - pw * NV;
+                    const float4 o4 = add ? dst[c] : zero4;
+                    float2 lo = lo2(o4), hi = hi2(o4);
+                    const float4* col = src + pw * TY * NU + u;
+#pragma unroll 4
+                    for (int y = 0; y < TY; ++y) {
+                        const int k = v - s_base[y];
+                        if ((unsigned)k < 4u) {
+                            const float2 wk = dup(s_weight[y * 4 + k]);
+                            const float4 g = col[y * NU];
+                            lo = fma2(wk, lo2(g), lo);
+                            hi = fma2(wk, hi2(g), hi);
+                        }
+                    }
+                    dst[c] = make_float4(lo.x, lo.y, hi.x, hi.y);
+                }
+            };
+            // the tile rows' first tap cell and weights for a ring value of the mid axis
+            auto row_table = [&](int mval) {
+                if (xf < 4) {
+                    const int i = mval * my + s_row[q].y;
+                    if (xf == 0) s_base[q] = s_row[q].x + offy[i];
+                    s_weight[q * 4 + xf] = wy[i * 4 + xf];
+                }
+            };
+
+            for (int gi = 0; gi < p.ngroups; ++gi) {
+                const float4 grp = uget(ut, p.utab, p.u_grp + gi);
+                __syncthreads();  // gt built / the previous group's dL/dU folded into the cells
+                row_table(__float_as_int(grp.x));
                 __syncthreads();
-                for (int pi = grp[gi_]; pi < grp[gi_ + 1]; ++pi) {
-                    const int b = pair_yval[pi];
-                    const int sa = yia - cy0 - 2 + offy[b * my + yra];
-                    const int sb = yib - cy0 - 2 + offy[b * my + yrb];
-                    const bool sh = sb != sa;  // column b's taps start one row later
-                    const float4 wa = *reinterpret_cast<const float4*>(wy + (b * my + yra) * 4);
-                    const float4 wb = *reinterpret_cast<const float4*>(wy + (b * my + yrb) * 4);
-                    // (column a, column b) weights of rows sa .. sa + 4
-                    float2 w2[5];
-                    w2[0] = make_float2(wa.x, sh ? 0.f : wb.x);
-                    w2[1] = make_float2(wa.y, sh ? wb.x : wb.y);
-                    w2[2] = make_float2(wa.z, sh ? wb.y : wb.z);
-                    w2[3] = make_float2(wa.w, sh ? wb.z : wb.w);
-                    w2[4] = make_float2(0.f, sh ? wb.w : 0.f);
-                    const int r0 = sa * kURow + xf;
-                    float2 Tx[NW], Ty[NW], Tz[NW];
+                for (int c = tid; c < 3 * uplane; c += nthr) {
+                    const int r = div_nu(c), u = c - r * NU;
+                    const int pw = div_ty(r), y = r - pw * TY;
+                    ut4[c] = filter_rows(*reinterpret_cast<const float4*>(s_weight + y * 4),
+                                         gt + (pw * NV + s_base[y]) * NU + u, NU);
+                    gu[c] = zero4;
+                }
+                __syncthreads();
+                for (int pi = __float_as_int(grp.y); pi < __float_as_int(grp.z); ++pi) {
+                    const float4 r0 = uget(ut, p.utab, p.u_pair + 4 * pi);
+                    const float4 r1 = uget(ut, p.utab, p.u_pair + 4 * pi + 1);
+                    const float4 r2 = uget(ut, p.utab, p.u_pair + 4 * pi + 2);
+                    const float4 r3 = uget(ut, p.utab, p.u_pair + 4 * pi + 3);
+                    const int xv = __float_as_int(r2.w), ax = xv * mx + xr;
+                    const float4 wv = *reinterpret_cast<const float4*>(wx + ax * 4);
+                    const float4* ubase = ut4 + q * NU + xi - cx0 - 2 + offx[ax];
+                    const int pa = __float_as_int(r2.x), pb = __float_as_int(r2.y), pc = __float_as_int(r2.z);
+                    float2 TP[NH], TE[NH], TZ[NH];
 #pragma unroll
-                    for (int w = 0; w < NW; ++w) {
-                        const float4* src = ut + w * NVA * kURow + r0;
-                        const float4 u0 = src[0], u1 = src[kURow], u2 = src[2 * kURow], u3 = src[3 * kURow],
-                                     u4 = src[4 * kURow];
-                        Tx[w].x = fmaf(wa.w, u3.x, fmaf(wa.z, u2.x, fmaf(wa.y, u1.x, wa.x * u0.x)));
-                        Ty[w].x = fmaf(wa.w, u3.y, fmaf(wa.z, u2.y, fmaf(wa.y, u1.y, wa.x * u0.y)));
-                        Tz[w].x = fmaf(wa.w, u3.z, fmaf(wa.z, u2.z, fmaf(wa.y, u1.z, wa.x * u0.z)));
-                        Tx[w].y = fmaf(w2[4].y, u4.x, fmaf(w2[3].y, u3.x, fmaf(w2[2].y, u2.x, fmaf(w2[1].y, u1.x, w2[0].y * u0.x))));
-                        Ty[w].y = fmaf(w2[4].y, u4.y, fmaf(w2[3].y, u3.y, fmaf(w2[2].y, u2.y, fmaf(w2[1].y, u1.y, w2[0].y * u0.y))));
-                        Tz[w].y = fmaf(w2[4].y, u4.z, fmaf(w2[3].y, u3.z, fmaf(w2[2].y, u2.z, fmaf(w2[1].y, u1.z, w2[0].y * u0.z))));
+                    for (int wq = 0; wq < NQ; ++wq) {
+                        float A[4], Bv[4], Cv[4];
+                        filter4(wv, ubase + pa * uplane + wq * TY * NU, A);
+                        filter4(wv, ubase + pb * uplane + wq * TY * NU, Bv);
+                        filter4(wv, ubase + pc * uplane + wq * TY * NU, Cv);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            put_half<CH>(TP, wq * 4 + k, A[k]);
+                            put_half<CH>(TE, wq * 4 + k, Bv[k]);
+                            put_half<CH>(TZ, wq * 4 + k, Cv[k]);
+                        }
                     }
-                    const float2 rot = pair_rot[pi];
-                    const float2 ca = dup(rot.x), sb2 = dup(rot.y), nsb = dup(-rot.y);
 #pragma unroll
-                    for (int w = 0; w < NW; ++w) {
-                        const float2 gx = Tx[w], gy = Ty[w];
-                        Tx[w] = fma2(gy, sb2, mul2(gx, ca));   // P
-                        Ty[w] = fma2(gy, ca, mul2(gx, nsb));   // E
+                    for (int w = 0; w < NH; ++w) {
+                        const float2 A = TP[w], Bv = TE[w];
+                        TP[w] = fma2(hi2(r0), Bv, mul2(lo2(r0), A));
+                        TE[w] = fma2(hi2(r1), Bv, mul2(lo2(r1), A));
                     }
-                    float2 gP[NW], gE[NW], gZ[NW];
+                    float2 gP[NH], gE[NH], gZ[NH];  // gP with the sign turned
 #pragma unroll
-                    for (int w = 0; w < NW; ++w) gP[w] = gE[w] = gZ[w] = make_float2(0.f, 0.f);
-                    for (int qi = pair_pt[pi]; qi < pair_pt[pi + 1]; ++qi) {
-                        const float4 pv = pt_vec[qi];
-                        const float2 hh = dup(pv.x), cc = dup(pv.y), ncc = dup(-pv.y), nhh = dup(-pv.x);
-                        const float wgt2 = pv.z * (-2.0f * pv.w);  // multiplicity / n times 2|u|
-                        const float2 nun = dup(pv.w);              // -|u|
-                        const int zc = pt_zval[qi];
-                        const float* wzc = wz + zc * (MZ * 4);
-                        const int offmask = offz[zc];
-                        auto zpass = [&](auto OFF, int zr, const float2 (&w4)[4]) {
+                    for (int w = 0; w < NH; ++w) gP[w] = gE[w] = gZ[w] = make_float2(0.f, 0.f);
+                    for (int qi = __float_as_int(r3.x); qi < __float_as_int(r3.y); ++qi) {
+                        const float4 c0 = uget(ut, p.utab, p.u_pt + 3 * qi);
+                        const float4 c1 = uget(ut, p.utab, p.u_pt + 3 * qi + 1);
+                        const float4 c2i = uget(ut, p.utab, p.u_pt + 3 * qi + 2);
+                        const int offmask = __float_as_int(c2i.y);
+                        float wun = c1.z;  // 2 weight |u|, in a vector register (see radiality.cu)
+                        asm volatile("" : "+f"(wun));
+                        auto zpass = [&](auto OFF, int zr, float2 w0, float2 w1, float2 w2, float2 w3) {
                             constexpr int o = decltype(OFF)::value;
 #pragma unroll
-                            for (int zi = 0; zi < CZ; ++zi) {
-                                const int z = zi * MZ + zr;
-                                float2 gx = mul2(w4[0], Tx[zi + o]);
-                                float2 gy = mul2(w4[0], Ty[zi + o]);
-                                float2 gz = mul2(w4[0], Tz[zi + o]);
-#pragma unroll
-                                for (int m = 1; m < 4; ++m) {
-                                    gx = fma2(w4[m], Tx[zi + o + m], gx);
-                                    gy = fma2(w4[m], Ty[zi + o + m], gy);
-                                    gz = fma2(w4[m], Tz[zi + o + m], gz);
-                                }
-                                // forward quantities (P = gx, E = gy, Z = gz)
-                                const float2 dot = fma2(cc, gz, mul2(hh, gx));
-                                const float2 cp = fma2(hh, gz, mul2(ncc, gx));
-                                const float2 c2 = fma2(cp, cp, mul2(gy, gy));
+                            for (int zi = 0; zi < CH; ++zi) {
+                                const float2 P = fma2(w3, TP[zi + o + 3], fma2(w2, TP[zi + o + 2], fma2(w1, TP[zi + o + 1], mul2(w0, TP[zi + o]))));
+                                const float2 E = fma2(w3, TE[zi + o + 3], fma2(w2, TE[zi + o + 2], fma2(w1, TE[zi + o + 1], mul2(w0, TE[zi + o]))));
+                                const float2 Zc = fma2(w3, TZ[zi + o + 3], fma2(w2, TZ[zi + o + 2], fma2(w1, TZ[zi + o + 1], mul2(w0, TZ[zi + o]))));
+                                const float2 dot = fma2(lo2(c0), Zc, P);
+                                const float2 cp = fma2(hi2(c0), P, Zc);
+                                const float2 c2 = fma2(cp, cp, mul2(E, E));
                                 const float2 g2 = fma2(dot, dot, c2);
                                 const float2 xx = mul2(c2, g2);
-                                // inv = 1/(|g| |g_perp|); where g is parallel to u (c2 = 0) every
-                                // product below carries a factor c2, cp or E and vanishes
+                                // 1 / sqrt(c2 g2); where g is parallel to u (c2 = 0) every product
+                                // below carries a factor c2, cp or E and vanishes
                                 const float2 inv = make_float2(rsqrt_approx(fmaxf(xx.x, 1e-30f)),
                                                                rsqrt_approx(fmaxf(xx.y, 1e-30f)));
-                                const float2 sn = mul2(c2, inv);                          // sin
-                                const float2 om = fma2(sn, nun, dup(1.0f));               // 1 - Dk/r
-                                // -dL/dsin = (dL/dS) (+-w) 2 om |u| (signed weight and 2|u|
-                                // folded into one table value)
-                                const float2 sw = make_float2(sign_weight(wgt2, dot.x), sign_weight(wgt2, dot.y));
-                                const float2 coef = mul2(mul2(sw, om), gS[z]);
-                                // d sin / d(P, E, Z) = g_perp/(|g||g_perp|) - sin g/|g|^2 with
-                                // g_perp = (-c cp, E, h cp) and 1/(|g||g_perp|) = inv, sin/|g|^2
-                                // = sin^2 inv; times dL/dsin = -coef:
-                                //   dP = k (sin^2 P + c cp), dZ = k (sin^2 Z - h cp),
-                                //   dE = k (sin^2 - 1) E,   k = coef inv
-                                const float2 k = mul2(coef, inv);
-                                const float2 s2 = mul2(sn, sn);
-                                const float2 dP = mul2(k, fma2(s2, gx, mul2(cc, cp)));
-                                const float2 dZ = mul2(k, fma2(s2, gz, mul2(nhh, cp)));
-                                const float2 dE = mul2(fma2(s2, k, make_float2(-k.x, -k.y)), gy);
-#pragma unroll
-                                for (int m = 0; m < 4; ++m) {
-                                    gP[zi + o + m] = fma2(w4[m], dP, gP[zi + o + m]);
-                                    gE[zi + o + m] = fma2(w4[m], dE, gE[zi + o + m]);
-                                    gZ[zi + o + m] = fma2(w4[m], dZ, gZ[zi + o + m]);
-                                }
+                                const float2 sn = mul2(c2, inv);
+                                // K = dL/ds = dL/dS sign(dot) 2 weight |u| (1 - |u| s)
+                                const float2 om = mul2(fma2(sn, lo2(c1), dup(wun)), gS[zi * MZ + zr]);
+                                const float2 k = mul2(make_float2(flip_sign(om.x, dot.x), flip_sign(om.y, dot.y)), inv);
+                                const float2 b = mul2(mul2(sn, sn), k);
+                                const float2 m = fma2(b, dup(-1.0f), k);
+                                const float2 mc = mul2(m, cp), bd2 = mul2(b, dot), dE = mul2(m, E);
+                                const float2 dP = fma2(lo2(c0), mc, bd2);   // -dL/dP
+                                const float2 dZ = fma2(hi2(c0), bd2, mc);
+                                gP[zi + o] = fma2(w0, dP, gP[zi + o]);
+                                gE[zi + o] = fma2(w0, dE, gE[zi + o]);
+                                gZ[zi + o] = fma2(w0, dZ, gZ[zi + o]);
+                                gP[zi + o + 1] = fma2(w1, dP, gP[zi + o + 1]);
+                                gE[zi + o + 1] = fma2(w1, dE, gE[zi + o + 1]);
+                                gZ[zi + o + 1] = fma2(w1, dZ, gZ[zi + o + 1]);
+                                gP[zi + o + 2] = fma2(w2, dP, gP[zi + o + 2]);
+                                gE[zi + o + 2] = fma2(w2, dE, gE[zi + o + 2]);
+                                gZ[zi + o + 2] = fma2(w2, dZ, gZ[zi + o + 2]);
+                                gP[zi + o + 3] = fma2(w3, dP, gP[zi + o + 3]);
+                                gE[zi + o + 3] = fma2(w3, dE, gE[zi + o + 3]);
+                                gZ[zi + o + 3] = fma2(w3, dZ, gZ[zi + o + 3]);
                             }
                         };
 #pragma unroll
                         for (int zr = 0; zr < MZ; ++zr) {
-                            float2 w4[4];
-#pragma unroll
-                            for (int m = 0; m < 4; ++m) w4[m] = dup(wzc[zr * 4 + m]);
+                            const float4 wa = uget(ut, p.utab, p.u_wz + 2 * (__float_as_int(c2i.x) + zr));
+                            const float4 wb = uget(ut, p.utab, p.u_wz + 2 * (__float_as_int(c2i.x) + zr) + 1);
                             if ((offmask >> zr) & 1)
-                                zpass(IntC<1>{}, zr, w4);
+                                zpass(IntC<1>{}, zr, lo2(wa), hi2(wa), lo2(wb), hi2(wb));
                             else
-                                zpass(IntC<0>{}, zr, w4);
+                                zpass(IntC<0>{}, zr, lo2(wa), hi2(wa), lo2(wb), hi2(wb));
                         }
                     }
-                    // back to (x, y): X = ca P - sb E, Y = sb P + ca E
+                    // out of the pair's frame (transposed)
+                    {
+                        const float2 na = make_float2(-r0.x, -r0.y), nb = make_float2(-r0.z, -r0.w);
 #pragma unroll
-                    for (int w = 0; w < NW; ++w) {
-                        const float2 P = gP[w], E = gE[w];
-                        gP[w] = fma2(E, nsb, mul2(P, ca));
-                        gE[w] = fma2(E, ca, mul2(P, sb2));
-                    }
-                    // intensity at the subvoxel centre rides on the (0, 0) pair: z pass
-                    // transpose with rho_z = 0 (5 taps) of dL/dI
-                    float2 gW[NW];
-#pragma unroll
-                    for (int w = 0; w < NW; ++w) gW[w] = make_float2(0.f, 0.f);
-                    if (pi == p.zero_pair) {
-#pragma unroll
-                        for (int z = 0; z < FZ; ++z) {
-                            const int Z = Z0 + z;
-                            const bool zin = Z >= B.lo[2] && Z < B.hi[2];
-                            const long long zo = sbase + (long long)(Z - B.lo[2]) * zstride;
-                            const bool oka = zin && ina && in_range(zo + va, a.n_stack, a.err, 9);
-                            const bool okb = zin && inb && in_range(zo + vb, a.n_stack, a.err, 9);
-                            const float2 gi = make_float2(oka ? a.gI[zo + va] : 0.f, okb ? a.gI[zo + vb] : 0.f);
-                            const int zr = z % MZ, zi = z / MZ;
-                            const float* qz = wzi + zr * 5;
-#pragma unroll
-                            for (int m = 0; m < 5; ++m)
-                                if (zi + m < NW) gW[zi + m] = fma2(dup(qz[m]), gi, gW[zi + m]);
+                        for (int w = 0; w < NH; ++w) {
+                            const float2 P = gP[w], E = gE[w];
+                            gP[w] = fma2(lo2(r1), E, mul2(na, P));
+                            gE[w] = fma2(hi2(r1), E, mul2(nb, P));
                         }
                     }
-                    // y pass transpose: row sa + m of every z cell gets w2[m] . (column a, column b)
-                    for (int ph = 0; ph < nph; ++ph) {
-                        const bool act = myph == ph;
-#pragma unroll
-                        for (int w = 0; w < NW; ++w) {
-                            float4* dst = gut + w * NVA * kURow + r0;
-                            const float2 xya = make_float2(gP[w].x, gE[w].x), xyb = make_float2(gP[w].y, gE[w].y);
-                            const float2 zwa = make_float2(gZ[w].x, gW[w].x), zwb = make_float2(gZ[w].y, gW[w].y);
-#pragma unroll
-                            for (int m = 0; m < 5; ++m) {
-                                if (act) {
-                                    float4* d = dst + m * kURow;
-                                    const float4 o4 = *d;
-                                    float2 xy = make_float2(o4.x, o4.y), zw = make_float2(o4.z, o4.w);
-                                    xy = fma2(dup(w2[m].x), xya, xy);
-                                    xy = fma2(dup(w2[m].y), xyb, xy);
-                                    zw = fma2(dup(w2[m].x), zwa, zw);
-                                    zw = fma2(dup(w2[m].y), zwb, zw);
-                                    *d = make_float4(xy.x, xy.y, zw.x, zw.y);
-                                }
-                                if (m < 4) __syncwarp();
-                            }
-                        }
-                        if (nph > 1) __syncwarp();
-                    }
+                    const int mask = __float_as_int(r3.z);
+                    x_transpose(gP, xv, mask, gu + pa * uplane, true);
+                    x_transpose(gE, xv, mask, gu + pb * uplane, true);
+                    x_transpose(gZ, xv, mask, gu + pc * uplane, true);
                 }
                 __syncthreads();
-                // x pass transpose, one (w, v) row of cells per thread: a 4-cell window
-                // slides with ub; a cell leaving the window is final for this group
-                for (int row = tid; row < NV * NW; row += nthr) {
-                    const int w = div_nv(row), v = row - w * NV;
-                    const float4* src = gut + (w * NVA + v) * kURow;
-                    float4* dst = ggt + row * NUP;
-                    int ub = xub[0];
-                    float4 a0 = zero4, a1 = zero4, a2 = zero4, a3 = zero4;
+                mid_transpose(gu, gg, 3, true);
+            }
+            // intensity at the subvoxel centre: the same passes with ring value 0
+            {
+                float2 gW[NH];
 #pragma unroll
-                    for (int x = 0; x < kTileX; ++x) {
-                        if (x > 0) {
-                            const int nb = xub[x];
-                            if (nb != ub) {
-                                dst[ub] = f4add(dst[ub], a0);
-                                a0 = a1;
-                                a1 = a2;
-                                a2 = a3;
-                                a3 = zero4;
-                                ub = nb;
-                            }
-                        }
-                        const float4 g = src[x];
-                        const float4 wk = xw4[x];
-                        a0 = f4fma(wk.x, g, a0);
-                        a1 = f4fma(wk.y, g, a1);
-                        a2 = f4fma(wk.z, g, a2);
-                        a3 = f4fma(wk.w, g, a3);
+                for (int w = 0; w < NH; ++w) gW[w] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int zr = 0; zr < MZ; ++zr) {
+                    const int m0 = (2 * zr + 1 >= MZ) ? 1 : 0;
+                    const float4 qz = uget(ut, p.utab, p.u_wi + zr);
+#pragma unroll
+                    for (int zi = 0; zi < CH; ++zi) {
+                        const int z = zi * MZ + zr;
+                        const float2 gi = make_float2(stack_value(a.gI, z), stack_value(a.gI, z + HZ));
+                        gW[zi + m0] = fma2(dup(qz.x), gi, gW[zi + m0]);
+                        gW[zi + m0 + 1] = fma2(dup(qz.y), gi, gW[zi + m0 + 1]);
+                        gW[zi + m0 + 2] = fma2(dup(qz.z), gi, gW[zi + m0 + 2]);
+                        gW[zi + m0 + 3] = fma2(dup(qz.w), gi, gW[zi + m0 + 3]);
                     }
-                    dst[ub] = f4add(dst[ub], a0);
-                    dst[ub + 1] = f4add(dst[ub + 1], a1);
-                    dst[ub + 2] = f4add(dst[ub + 2], a2);
-                    dst[ub + 3] = f4add(dst[ub + 3], a3);
                 }
+                __syncthreads();  // the last group's dL/dU is folded into the cells
+                row_table(p.zero_m);
+                x_transpose(gW, p.zero_x, p.zero_xoff, gu, false);
+                __syncthreads();
+                mid_transpose(gu, icell, 1, false);
             }
             __syncthreads();
             // stencil transpose onto the input tile positions, then into dL/dI'. Cells
-            // outside the tile grid or the block do not depend on the input.
+            // outside the tile grid or the block do not depend on the input. With ranges
+            // (1, 1, 1, 1) the cell at offset d adds -(dx Gx + dm Gm + dn Gn), so per position
+            // of the x-mid plane sA = sum of -(dx Gx + dm Gm) and sB = sum of Gn over its nine
+            // neighbours are formed first, four cells of the innermost axis at a time
+            // (straight from the cells the scattered single-word reads took a seventh of
+            // the kernel's shared-memory cycles).
+            float4 *sA = gt, *sB = gu;  // [quad][NIY][NIX]
+            if (p.grad_mode == 1) {
+                for (int i = tid; i < NQ * NIY * NIX; i += nthr) {
+                    const int wq = div_nixy(i);
+                    const int rem = i - wq * (NIX * NIY);
+                    const int iy = div_nix(rem), ix = rem - iy * NIX;
+                    float4 A = zero4, Bs = zero4;
+#pragma unroll
+                    for (int dm = 0; dm < 3; ++dm)
+#pragma unroll
+                        for (int dx = 0; dx < 3; ++dx) {
+                            const int uu = ix - R + dx - 1, vv = iy - R + dm - 1;
+                            if (uu < 0 || uu >= NU || cx0 + uu < 0 || cx0 + uu >= bw || vv < 0 || vv >= NV ||
+                                cy0 + vv < 0 || cy0 + vv >= bh)
+                                continue;
+                            const float4* c = gg + (wq * NV + vv) * NU + uu;
+                            if (dx != 1) A = f4fma(dx == 0 ? 1.f : -1.f, c[0], A);
+                            if (dm != 1) A = f4fma(dm == 0 ? 1.f : -1.f, c[gplane], A);
+                            Bs = f4fma(1.f, c[2 * gplane], Bs);
+                        }
+                    sA[i] = A;
+                    sB[i] = Bs;
+                }
+                __syncthreads();
+            }
+            const float* gf = reinterpret_cast<const float*>(gg);
+            const float* icf = reinterpret_cast<const float*>(icell);
             for (int i = tid; i < nin; i += nthr) {
                 const int iz = div_nixy(i);
                 const int rem = i - iz * (NIX * NIY);
                 const int iy = div_nix(rem), ix = rem - iy * NIX;
                 const int u = ix - R, v = iy - R, w = iz - R;  // cell with the same position
                 float acc = 0.f;
-                if (p.grad_mode == 1 || p.grad_mode == 2) {
-                    // 3 x 3 x 3 neighbourhood with clamped indices and 0/1 masks
-                    int cu[3], cv[3], cw[3];
-                    float mu[3], mv[3], mw[3];
+                auto inside = [&](int uu, int vv, int ww) {
+                    return uu >= 0 && uu < NU && vv >= 0 && vv < NV && ww >= 0 && ww < NW && cx0 + uu >= 0 &&
+                           cx0 + uu < bw && cy0 + vv >= 0 && cy0 + vv < bh && cz0 + ww >= 0 && cz0 + ww < bd;
+                };
+                if (inside(u, v, w)) acc = icf[((w >> 2) * NV + v) * (4 * NU) + u * 4 + (w & 3)];
+                if (p.grad_mode == 1) {
+                    const float* fa = reinterpret_cast<const float*>(sA) + 4 * rem;
+                    const float* fb = reinterpret_cast<const float*>(sB) + 4 * rem;
 #pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        const int uu = u + d - 1, vv = v + d - 1, ww = w + d - 1;
-                        mu[d] = (uu >= 0 && uu < NU && cx0 + uu >= 0 && cx0 + uu < bw) ? 1.f : 0.f;
-                        mv[d] = (vv >= 0 && vv < NV && cy0 + vv >= 0 && cy0 + vv < bh) ? 1.f : 0.f;
-                        mw[d] = (ww >= 0 && ww < NW && cz0 + ww >= 0 && cz0 + ww < bd) ? 1.f : 0.f;
-                        cu[d] = clampi(uu, 0, NU - 1);
-                        cv[d] = clampi(vv, 0, NV - 1) * NUP;
-                        cw[d] = clampi(ww, 0, NW - 1) * (NV * NUP);
-                    }
-                    auto G = [&](int dx, int dy, int dz) -> float4 { return ggt[cw[dz + 1] + cv[dy + 1] + cu[dx + 1]]; };
-                    if (p.grad_mode == 1) {
-                        // neighbour d adds -(dx Gx + dy Gy + dz Gz) (ranges 1, 1, 1, 1)
-#pragma unroll
-                        for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-                            for (int dy = -1; dy <= 1; ++dy) {
-                                const float myz = mv[dy + 1] * mw[dz + 1];
-#pragma unroll
-                                for (int dx = -1; dx <= 1; ++dx) {
-                                    const float4 g = G(dx, dy, dz);
-                                    float s = 0.f;
-                                    if (dx) s = dx < 0 ? s + g.x : s - g.x;
-                                    if (dy) s = dy < 0 ? s + g.y : s - g.y;
-                                    if (dz) s = dz < 0 ? s + g.z : s - g.z;
-                                    if (!dx && !dy && !dz) s = g.w;
-                                    acc = fmaf(myz * mu[dx + 1], s, acc);
-                                }
-                            }
-                    } else {
-                        // ranges 1, 0, 0, 0: axis neighbours only
-                        acc = mu[1] * mv[1] * mw[1] * G(0, 0, 0).w;
-                        acc = fmaf(mu[0] * mv[1] * mw[1], G(-1, 0, 0).x, acc);
-                        acc = fmaf(-mu[2] * mv[1] * mw[1], G(1, 0, 0).x, acc);
-                        acc = fmaf(mu[1] * mv[0] * mw[1], G(0, -1, 0).y, acc);
-                        acc = fmaf(-mu[1] * mv[2] * mw[1], G(0, 1, 0).y, acc);
-                        acc = fmaf(mu[1] * mv[1] * mw[0], G(0, 0, -1).z, acc);
-                        acc = fmaf(-mu[1] * mv[1] * mw[2], G(0, 0, 1).z, acc);
+                    for (int dn = 0; dn < 3; ++dn) {
+                        const int ww = w + dn - 1;
+                        if (ww < 0 || ww >= NW || cz0 + ww < 0 || cz0 + ww >= bd) continue;
+                        const int at = (ww >> 2) * (4 * NIX * NIY) + (ww & 3);
+                        acc += fa[at];
+                        if (dn != 1) acc += dn == 0 ? fb[at] : -fb[at];
                     }
                 } else {
                     const int mR = p.gr[0], xR = p.gr[1], yR = p.gr[2], zR = p.gr[3];
-                    auto G = [&](int du, int dv, int dw) -> float4 {
+                    auto G = [&](int plane, int du, int dv, int dw) -> float {
                         const int uu = u + du, vv = v + dv, ww = w + dw;
-                        if (uu < 0 || uu >= NU || vv < 0 || vv >= NV || ww < 0 || ww >= NW) return zero4;
-                        if (cx0 + uu < 0 || cx0 + uu >= bw || cy0 + vv < 0 || cy0 + vv >= bh || cz0 + ww < 0 ||
-                            cz0 + ww >= bd)
-                            return zero4;
-                        return ggt[(ww * NV + vv) * NUP + uu];
+                        return inside(uu, vv, ww) ? gf[plane * 4 * gplane + ((ww >> 2) * NV + vv) * (4 * NU) + uu * 4 + (ww & 3)]
+                                                  : 0.f;
                     };
-                    acc = G(0, 0, 0).w;
                     // Gx(c) = sum_{i>0, j, k} I(c + (i, j, k)) - I(c + (-i, j, k))
                     for (int ii = 1; ii <= mR; ++ii)
                         for (int j = -yR; j <= yR; ++j)
-                            for (int k = -zR; k <= zR; ++k) acc += G(-ii, -j, -k).x - G(ii, -j, -k).x;
+                            for (int k = -zR; k <= zR; ++k) acc += G(0, -ii, -j, -k) - G(0, ii, -j, -k);
                     for (int jj = 1; jj <= mR; ++jj)
                         for (int ii = -xR; ii <= xR; ++ii)
-                            for (int k = -zR; k <= zR; ++k) acc += G(-ii, -jj, -k).y - G(-ii, jj, -k).y;
+                            for (int k = -zR; k <= zR; ++k) acc += G(1, -ii, -jj, -k) - G(1, -ii, jj, -k);
                     for (int kk = 1; kk <= mR; ++kk)
                         for (int ii = -xR; ii <= xR; ++ii)
-                            for (int j = -yR; j <= yR; ++j) acc += G(-ii, -j, -kk).z - G(-ii, -j, kk).z;
+                            for (int j = -yR; j <= yR; ++j) acc += G(2, -ii, -j, -kk) - G(2, -ii, -j, kk);
                 }
                 if (acc != 0.f) {
-                    const int bx = clampi(cx0 - R + ix, 0, bw - 1);
-                    const int by = clampi(cy0 - R + iy, 0, bh - 1);
-                    const int bz = clampi(cz0 - R + iz, 0, bd - 1);
-                    const long long gidx = tbase + ((long long)(B.origin[2] + bz) * p.H + (B.origin[1] + by)) * p.W +
-                                           (B.origin[0] + bx);
+                    const long long gidx = global_row(iy, iz) + clampi(cx0 - R + ix, 0, bw - 1);
                     if (in_range(gidx, a.n_in, a.err, 10)) atomicAdd(a.gin + gidx, acc);
                 }
             }
         }
     }
 }
-template <int MZ>
-int launch_adj_mz(const RadParams& p, const AdjParams& a, int grid, size_t smem, cudaStream_t st) {
-    constexpr int CZ = cza_for_mag(MZ);
-    auto k = radiality_adjoint_kernel<MZ, CZ>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    k<<<grid, kAdjThreads, smem, st>>>(p, a);
-    return (int)cudaGetLastError();
-}
 
-template <int MZ>
-int occ_adj_mz(int threads, size_t smem, int* out) {
-    constexpr int CZ = cza_for_mag(MZ);
-    auto k = radiality_adjoint_kernel<MZ, CZ>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k, threads, smem);
+template <class F>
+int with_adj_kernel(const FwdParams& p, F&& f) {
+    auto go = [&](auto mz) -> int {
+        constexpr int MZ = decltype(mz)::value;
+        constexpr int CZ = adj_cz(MZ);
+        return p.u_count <= kUAdjMax ? f(radiality_adjoint_kernel<MZ, CZ, kUAdjMax>, IntC<kUAdjMax>{})
+                                     : f(radiality_adjoint_kernel<MZ, CZ, 1>, IntC<1>{});
+    };
+    switch (p.mag[2]) {
+        case 1: return go(IntC<1>{});
+        case 2: return go(IntC<2>{});
+        case 3: return go(IntC<3>{});
+        case 4: return go(IntC<4>{});
+        case 5: return go(IntC<5>{});
+        case 6: return go(IntC<6>{});
+        case 7: return go(IntC<7>{});
+        case 8: return go(IntC<8>{});
+    }
+    return (int)cudaErrorInvalidValue;
 }
 
 }  // namespace
 
-size_t radiality_adjoint_smem_bytes(const RadParams& p) {
-    const int NW = cza_for_mag(p.mag[2]) + 4;
-    size_t b = sizeof(float4) * (2 * (size_t)adj_nup(p.NU) * p.NV * NW +
-                                 (size_t)adj_u_region_f4(p.NV, NW, p.NIX, p.NIY, p.NIZ));
-    b += sizeof(float4) * kTileX + sizeof(int) * kTileX;  // x weights and first tap cell of each column
-    b += sizeof(float) * p.smem_table_words;
-    return (b + 15) & ~(size_t)15;
+// float4s of the place that U, the input tile and the intensity's cells share
+int radiality_adjoint_u_region(const FwdParams& p) {
+    const int nq = p.cz / 4 + 1;
+    return std::max(std::max(3 * nq * p.TY * p.NU, (p.NIX * p.NIY * p.NIZ + 3) / 4), nq * p.NV * p.NU);
 }
 
-int launch_radiality_adjoint(const RadParams& p, const AdjParams& a, int grid, size_t smem, void* stream) {
+size_t radiality_adjoint_smem_bytes(const FwdParams& p) {
+    const int nq = p.cz / 4 + 1, warps = p.TY * kTileX / 32;
+    const size_t f4 = (size_t)6 * nq * p.NV * p.NU + p.u_region + (size_t)3 * nq * p.TY * p.NU +
+                      (size_t)warps * 2 * nq * (4 + p.mag[0] * adj_cells(p.mag[0]));
+    return (f4 * sizeof(float4) + (size_t)p.lane_words * sizeof(float) + 15) & ~(size_t)15;
+}
+
+int launch_radiality_adjoint(const FwdParams& p, const FwdPlan& plan, const AdjParams& a, int grid, size_t smem,
+                             void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    switch (p.mag[2]) {
-        case 1: return launch_adj_mz<1>(p, a, grid, smem, st);
-        case 2: return launch_adj_mz<2>(p, a, grid, smem, st);
-        case 3: return launch_adj_mz<3>(p, a, grid, smem, st);
-        case 4: return launch_adj_mz<4>(p, a, grid, smem, st);
-        case 5: return launch_adj_mz<5>(p, a, grid, smem, st);
-        case 6: return launch_adj_mz<6>(p, a, grid, smem, st);
-        case 7: return launch_adj_mz<7>(p, a, grid, smem, st);
-        case 8: return launch_adj_mz<8>(p, a, grid, smem, st);
-    }
-    return (int)cudaErrorInvalidValue;
+    return with_adj_kernel(p, [&](auto k, auto n) -> int {
+        constexpr int UN = decltype(n)::value;
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        UTab<UN> tab;
+        std::memset(&tab, 0, sizeof tab);
+        if (UN > 1) std::memcpy(tab.q, plan.adj_utab.data(), plan.adj_utab.size() * sizeof(float));
+        k<<<grid, p.TY * kTileX, smem, st>>>(p, a, tab);
+        return (int)cudaGetLastError();
+    });
 }
 
-int radiality_adjoint_max_ctas_per_sm(const RadParams& p, int* out) {
+int radiality_adjoint_max_ctas_per_sm(const FwdParams& p, int* out) {
     const size_t smem = radiality_adjoint_smem_bytes(p);
-    const int threads = kAdjThreads;
-    switch (p.mag[2]) {
-        case 1: return occ_adj_mz<1>(threads, smem, out);
-        case 2: return occ_adj_mz<2>(threads, smem, out);
-        case 3: return occ_adj_mz<3>(threads, smem, out);
-        case 4: return occ_adj_mz<4>(threads, smem, out);
-        case 5: return occ_adj_mz<5>(threads, smem, out);
-        case 6: return occ_adj_mz<6>(threads, smem, out);
-        case 7: return occ_adj_mz<7>(threads, smem, out);
-        case 8: return occ_adj_mz<8>(threads, smem, out);
-    }
-    return (int)cudaErrorInvalidValue;
+    return with_adj_kernel(p, [&](auto k, auto) -> int {
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k, p.TY * kTileX, smem);
+    });
 }
 
 int launch_temporal_adjoint(const BlockDev* blocks, long long vox, const float* rad, const float* inten,

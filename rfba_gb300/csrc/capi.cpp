@@ -118,24 +118,19 @@ static int ensure_plan(rfba_ctx* ctx, const rfba_srrf_config& cfg, cudaStream_t 
         return RFBA_OK;
     std::string err;
     P.valid = false;
-    if (!build_ring_plan(cfg, &P.ring, &err) || !build_tables(cfg, P.ring, &P.words, &P.tl, &err)) {
+    if (!build_ring_plan(cfg, &P.ring, &err) || !build_forward_plan(cfg, &P.fwd, &err)) {
         set_error(err);
         return RFBA_ERR_UNSUPPORTED;
     }
-    P.zero_pair = ring_zero_pair(P.ring);
-    if (P.zero_pair < 0) {
+    if (ring_zero_pair(P.ring) < 0) {
         set_error("ring has no (0, 0) pair");
         return RFBA_ERR_UNSUPPORTED;
     }
-    if (!build_forward_plan(cfg, &P.fwd, &err)) {
-        set_error(err);
-        return RFBA_ERR_UNSUPPORTED;
-    }
-    while (P.words.size() % 4) P.words.push_back(0.f);
-    P.fwd_lane = P.words.size();
-    P.words.insert(P.words.end(), P.fwd.lane.begin(), P.fwd.lane.end());
+    P.words = P.fwd.lane;
     P.fwd_utab = P.words.size();
     P.words.insert(P.words.end(), P.fwd.utab.begin(), P.fwd.utab.end());
+    P.adj_utab = P.words.size();
+    P.words.insert(P.words.end(), P.fwd.adj_utab.begin(), P.fwd.adj_utab.end());
     const int rc = ctx->tables.ensure(P.words.size() * 4, "tables");
     if (rc) return rc;
     RFBA_CUDA(cudaMemcpyAsync(ctx->tables.p, P.words.data(), P.words.size() * 4, cudaMemcpyHostToDevice, st),
@@ -227,60 +222,9 @@ static FwdParams fill_fwd_params(rfba_ctx* ctx, const rfba_srrf_config& cfg, con
     const PlanCache& P = ctx->plan;
     FwdParams p = forward_params(P.fwd, cfg, in_dev, dtype == RFBA_U16, dims, ty, cz);
     const float* t = static_cast<const float*>(ctx->tables.p);
-    p.lane = t + P.fwd_lane;
+    p.lane = t;
     p.utab = reinterpret_cast<const float4*>(t + P.fwd_utab);
     return p;
-}
-
-// Adjoint kernel parameters (everything but the block / tile lists and the schedule).
-static RadParams fill_rad_params(rfba_ctx* ctx, const rfba_srrf_config& cfg, const void* in_dev, const int dims[4],
-                                 int CZ) {
-    const PlanCache& P = ctx->plan;
-    const int T = dims[3];
-    RadParams rp;
-    std::memset(&rp, 0, sizeof rp);
-    rp.in = in_dev;
-    rp.W = dims[0];
-    rp.H = dims[1];
-    rp.D = dims[2];
-    rp.T = T;
-    for (int a = 0; a < 3; ++a) rp.mag[a] = cfg.mag[a];
-    rp.nxv = (int)P.ring.xv.size();
-    rp.nyv = (int)P.ring.yv.size();
-    rp.nzv = (int)P.ring.zv.size();
-    rp.ngroups = (int)P.ring.grp_xval.size();
-    rp.npairs = (int)P.ring.pair_yval.size();
-    rp.npoints = (int)P.ring.pt_zval.size();
-    rp.zero_pair = P.zero_pair;
-    if (cfg.gradient_smooth == 0) {
-        rp.gr[0] = 1;
-        rp.gr[1] = rp.gr[2] = rp.gr[3] = 0;
-    } else {
-        rp.gr[0] = cfg.main_range;
-        rp.gr[1] = cfg.x_range;
-        rp.gr[2] = cfg.y_range;
-        rp.gr[3] = cfg.z_range;
-    }
-    rp.R = std::max(std::max(rp.gr[0], rp.gr[1]), std::max(rp.gr[2], rp.gr[3]));
-    if (rp.gr[0] == 1 && rp.gr[1] == 1 && rp.gr[2] == 1 && rp.gr[3] == 1)
-        rp.grad_mode = 1;
-    else if (rp.gr[0] == 1 && rp.gr[1] == 0 && rp.gr[2] == 0 && rp.gr[3] == 0)
-        rp.grad_mode = 2;
-    else
-        rp.grad_mode = 0;
-    rp.TY = kAdjRows;
-    rp.NU = (kTileX - 1) / cfg.mag[0] + 2 + 4;
-    rp.NV = (rp.TY - 1) / cfg.mag[1] + 2 + 4;
-    rp.NW = CZ + 4;
-    rp.NIX = rp.NU + 2 * rp.R;
-    rp.NIY = rp.NV + 2 * rp.R;
-    rp.NIZ = rp.NW + 2 * rp.R;
-    rp.renorm = cfg.renormalize == 1;
-    rp.poscon = cfg.remove_con == 1;
-    rp.tables = static_cast<const float*>(ctx->tables.p);
-    rp.tl = P.tl;
-    rp.smem_table_words = P.tl.words;
-    return rp;
 }
 
 static int plan_passes(rfba_ctx* ctx, const rfba_srrf_config& cfg, rfba_dtype dtype, const int dims[4],
@@ -1177,9 +1121,9 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
     const size_t nin = (size_t)dims[0] * dims[1] * dims[2] * T;
     const long long V = blk.vox;
     blk.stack_off = 0;
-    const int FZ = cfg->mag[2] * cza_for_mag(cfg->mag[2]);
-    blk.ntile[1] = (blk.hi[1] - blk.lo[1] + kAdjRows - 1) / kAdjRows;
-    blk.ntile[2] = (blk.hi[2] - blk.zbase + FZ - 1) / FZ;
+    const FwdPlan& fp = ctx->plan.fwd;
+    blk.cz = adj_cz(fp.mag[2]);
+    forward_tiles(fp, 0, &blk);
     std::vector<TileDesc> tiles;
     for (int tz = 0; tz < blk.ntile[2]; ++tz)
         for (int ty = 0; ty < blk.ntile[1]; ++ty)
@@ -1205,7 +1149,9 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
                                     gS, gI, ngmap, err, st);
         if (e) return cuda_fail((cudaError_t)e, "temporal adjoint launch");
     }
-    RadParams rp = fill_rad_params(ctx, *cfg, iprime, dims, cza_for_mag(cfg->mag[2]));
+    FwdParams rp = adjoint_params(fp, *cfg, iprime, dims);
+    rp.lane = static_cast<const float*>(ctx->tables.p);
+    rp.utab = reinterpret_cast<const float4*>(rp.lane + ctx->plan.adj_utab);
     rp.blocks = dblk;
     rp.tiles = static_cast<const TileDesc*>(ctx->atiles.p);
     rp.ntiles = (int)tiles.size();
@@ -1233,7 +1179,7 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
     rp.stack_t0 = rp.t_lo;
     const int grid = (int)std::max<long long>(1, std::min<long long>(slots, rp.nitems));
     AdjParams ap{gS, gI, static_cast<float*>(ctx->gin.p), (long long)nin, (long long)V * TW, err};
-    e = launch_radiality_adjoint(rp, ap, grid, smem, st);
+    e = launch_radiality_adjoint(rp, fp, ap, grid, smem, st);
     if (e) return cuda_fail((cudaError_t)e, "radiality adjoint launch");
     ctx->launches += window ? 1 : 2;
     return RFBA_OK;

@@ -45,11 +45,9 @@ struct PlanCache {
     float ring_radius = 0.f;
     int axes = 0, mag[3] = {0, 0, 0};
     RingPlan ring;
-    std::vector<float> words;
-    TableLayout tl;
-    int zero_pair = -1;
     FwdPlan fwd;
-    size_t fwd_lane = 0, fwd_utab = 0;  // word offsets of the forward tables in the uploaded buffer
+    std::vector<float> words;  // the uploaded tables: lane tables, uniform tables, the adjoint's uniform tables
+    size_t fwd_utab = 0, adj_utab = 0;  // word offsets in them
 };
 
 // Schedule choices of the forward: tile rows (tile shape) and tile order

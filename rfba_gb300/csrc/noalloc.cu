@@ -167,14 +167,11 @@ extern "C" int rfba_srrf_forward_static_scratch(const rfba_srrf_config* cfg, con
 
     // ring plan and tables
     RingPlan ring;
-    std::vector<float> words;
-    TableLayout tl;
-    if (!build_ring_plan(*cfg, &ring, &err) || !build_tables(*cfg, ring, &words, &tl, &err))
+    FwdPlan plan;
+    if (!build_ring_plan(*cfg, &ring, &err) || !build_forward_plan(*cfg, &plan, &err))
         return fail(RFBA_ERR_UNSUPPORTED, err);
     if (ring_zero_pair(ring) < 0) return fail(RFBA_ERR_UNSUPPORTED, "ring has no (0, 0) pair");
-    FwdPlan plan;
-    if (!build_forward_plan(*cfg, &plan, &err)) return fail(RFBA_ERR_UNSUPPORTED, err);
-    words = plan.lane;  // lane tables, then the uniform ones
+    std::vector<float> words = plan.lane;  // lane tables, then the uniform ones
     words.insert(words.end(), plan.utab.begin(), plan.utab.end());
 
     // the whole volume as one block

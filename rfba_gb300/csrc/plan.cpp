@@ -303,7 +303,7 @@ int ring_zero_pair(const RingPlan& rp) {
 }
 
 // ---------------------------------------------------------------------------
-// Weight tables
+// Tap weights
 
 // Catmull-Rom kernel, a = 0.5 (kernel.cu:128-138), evaluated in double.
 static double cubic(double xx) {
@@ -331,92 +331,6 @@ static bool tap5(int ph, double rho, int mag, float w[5]) {
     const double f = (ph + 0.5 + rho) / mag;
     if (!(f >= -0.5 && f < 1.5)) return false;
     for (int m = 0; m < 5; ++m) w[m] = (float)cubic(f - ((m - 2) + 0.5));
-    return true;
-}
-
-bool build_tables(const rfba_srrf_config& c, const RingPlan& rp, std::vector<float>* words, TableLayout* tl,
-                  std::string* err) {
-    const int mx = c.mag[0], my = c.mag[1], mz = c.mag[2];
-    const int na = (int)rp.xv.size(), nb = (int)rp.yv.size(), nc = (int)rp.zv.size();
-    std::vector<float>& W = *words;
-    W.clear();
-    auto align4 = [&]() {
-        while (W.size() % 4) W.push_back(0.f);
-    };
-    auto push_int = [&](int v) {
-        float f;
-        std::memcpy(&f, &v, 4);
-        W.push_back(f);
-    };
-    align4();
-    tl->wx = (int)W.size();
-    std::vector<int> ox(na * mx), oy(nb * my);
-    for (int a = 0; a < na; ++a)
-        for (int ph = 0; ph < mx; ++ph) {
-            float w[4];
-            int off;
-            if (!tap4(ph, rp.xv[a], mx, w, &off)) {
-                *err = "ring radius too large for the x magnification (needs ring_radius < (1 + mag)/2)";
-                return false;
-            }
-            for (int k = 0; k < 4; ++k) W.push_back(w[k]);
-            ox[a * mx + ph] = off;
-        }
-    tl->offx = (int)W.size();
-    for (int v : ox) push_int(v);
-    align4();
-    tl->wy = (int)W.size();
-    for (int b = 0; b < nb; ++b)
-        for (int ph = 0; ph < my; ++ph) {
-            float w[4];
-            int off;
-            if (!tap4(ph, rp.yv[b], my, w, &off)) {
-                *err = "ring radius too large for the y magnification (needs ring_radius < (1 + mag)/2)";
-                return false;
-            }
-            for (int k = 0; k < 4; ++k) W.push_back(w[k]);
-            oy[b * my + ph] = off;
-        }
-    tl->offy = (int)W.size();
-    for (int v : oy) push_int(v);
-    tl->wz = (int)W.size();
-    std::vector<int> oz(nc, 0);
-    for (int cc = 0; cc < nc; ++cc)
-        for (int ph = 0; ph < mz; ++ph) {
-            float w[4];
-            int off;
-            if (!tap4(ph, rp.zv[cc], mz, w, &off)) {
-                *err = "ring radius too large for the z magnification (needs ring_radius < (1 + mag)/2)";
-                return false;
-            }
-            for (int m = 0; m < 4; ++m) W.push_back(w[m]);
-            oz[cc] |= off << ph;  // bit ph: taps start one coarse cell later
-        }
-    tl->offz = (int)W.size();
-    for (int v : oz) push_int(v);
-    tl->wzi = (int)W.size();
-    for (int ph = 0; ph < mz; ++ph) {
-        float w[5];
-        tap5(ph, 0.0, mz, w);
-        for (int m = 0; m < 5; ++m) W.push_back(w[m]);
-    }
-    tl->grp_xval = (int)W.size();
-    for (int v : rp.grp_xval) push_int(v);
-    tl->grp = (int)W.size();
-    for (int v : rp.grp) push_int(v);
-    tl->pair_yval = (int)W.size();
-    for (int v : rp.pair_yval) push_int(v);
-    tl->pair_pt = (int)W.size();
-    for (int v : rp.pair_pt) push_int(v);
-    tl->pt_zval = (int)W.size();
-    for (int v : rp.pt_zval) push_int(v);
-    align4();
-    tl->pt_vec = (int)W.size();
-    for (float v : rp.pt_vec) W.push_back(v);
-    tl->pair_rot = (int)W.size();
-    for (float v : rp.pair_rot) W.push_back(v);
-    align4();
-    tl->words = (int)W.size();
     return true;
 }
 
@@ -528,8 +442,8 @@ bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err
     };
     int* wpos[2] = {&fp->l_wx, &fp->l_wm};
     int* opos[2] = {&fp->l_offx, &fp->l_offm};
-    std::vector<std::array<float, 4>> w;
-    std::vector<int> off;
+    std::vector<std::array<float, 4>> w, w_x;
+    std::vector<int> off, x_mask;
     for (int k = 0; k < 2; ++k) {
         w.clear();
         off.clear();
@@ -537,12 +451,20 @@ bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err
             if (!taps(k, v, &w, &off)) return false;
         *wpos[k] = (int)L.size();
         for (auto& t : w) L.insert(L.end(), t.begin(), t.end());
+        if (k == 0) {
+            w_x = w;
+            for (size_t i = 0; i < off.size(); ++i) {
+                if (i % fp->mag[0] == 0) x_mask.push_back(0);
+                x_mask.back() |= off[i] << (i % fp->mag[0]);
+            }
+        }
         *opos[k] = (int)L.size();
         for (int of : off) L.push_back(bits(of));
         while (L.size() % 4) L.push_back(0.f);
     }
     fp->zero_x = value_index(o.val[0], 0.f, tol);
     fp->zero_m = value_index(o.val[1], 0.f, tol);
+    fp->zero_xoff = x_mask[fp->zero_x];
 
     // uniform tables
     const int mz = fp->mag[2];
@@ -604,7 +526,7 @@ bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err
         put(pa, pa, pb, pb);
         put(ea, ea, eb, eb);
         put_bits(plane[0], plane[1], plane[2], f.a);
-        put_bits(q0, q1, 0, 0);
+        put_bits(q0, q1, x_mask[f.a], 0);
     }
     w.clear();
     off.clear();
@@ -630,6 +552,18 @@ bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err
         const int m0 = 2 * ph + 1 >= mz ? 1 : 0;
         put(t[m0], t[m0 + 1], t[m0 + 2], t[m0 + 3]);
     }
+    fp->adj_utab = U;
+    for (int q = 0; q < npts; ++q) {
+        const P& p = o.pts[q];
+        const double un = std::sqrt(p.u[0] * p.u[0] + p.u[1] * p.u[1] + p.u[2] * p.u[2]);
+        const double f = 2.0 * p.m / n * un;
+        float* r = &fp->adj_utab[4 * (fp->u_pt + 3 * q + 1)];
+        r[0] = r[1] = (float)(-f * un);
+        r[2] = r[3] = (float)f;
+    }
+    fp->u_wx = (int)(fp->adj_utab.size() / 4);
+    for (auto& t : w_x)
+        for (int k : {0, 0, 1, 1, 2, 2, 3, 3}) fp->adj_utab.push_back(t[k]);
     return true;
 }
 
@@ -678,8 +612,18 @@ FwdParams forward_params(const FwdPlan& fp, const rfba_srrf_config& c, const voi
     p.ngroups = fp.ngroups;
     p.zero_x = fp.zero_x;
     p.zero_m = fp.zero_m;
+    p.zero_xoff = fp.zero_xoff;
+    p.u_wx = fp.u_wx;
     p.neg_weight = fp.neg_weight;
     p.tma_bx = radiality_tma_box_x(p);
+    return p;
+}
+
+FwdParams adjoint_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, const int dims[4]) {
+    FwdParams p = forward_params(fp, c, in, 0, dims, 0, adj_cz(fp.mag[2]));
+    p.tma_bx = 0;
+    p.u_region = radiality_adjoint_u_region(p);
+    p.u_count = (int)(fp.adj_utab.size() / 4);
     return p;
 }
 

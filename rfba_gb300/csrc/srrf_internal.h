@@ -20,17 +20,19 @@ constexpr int kTileRows = 8;
 constexpr int kMaxThreads = 256;  // 16 x 16 threads for the 32-row tile (mid magnification 8)
 constexpr int kMaxMag = 8;
 constexpr int kMaxGradRange = 3;
-// Adjoint tile: 16 x 16 subvoxel columns (two consecutive rows per thread).
-constexpr int kAdjRows = 16;
-constexpr int kAdjThreads = kTileX * kAdjRows / 2;
-
 // The forward kernel's register limit for MZ x CZ tiles: MZ CZ for the sums and
 // 6 (CZ / 2 + 4) for the y-filtered columns are live through the point loop.
 constexpr int fwd_regs(int mz, int cz) { return mz * cz + 6 * (cz / 2 + 4) <= 88 ? 128 : 168; }
 
-// Coarse z cells per tile of the adjoint kernel (it holds twice the register
-// columns of the forward).
-constexpr int cza_for_mag(int mz) { return mz <= 2 ? 4 : (mz <= 4 ? 2 : 1); }
+// The adjoint's tile depth (it holds two sets of columns), its register limit (12
+// (CZ / 2 + 4) for the columns, MZ CZ for dL/dS) and the width of an exchange row
+// per x phase (the tile's coarse cells and four zeros).
+constexpr int adj_cz(int mz) { return mz <= 4 ? 8 : 4; }
+constexpr int adj_regs(int mz, int cz) { return mz * cz + 12 * (cz / 2 + 4) <= 88 ? 128 : 168; }
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr int adj_cells(int mx) { return 15 / mx + 2 + 4; }
 
 // One independent block of the input with the fine region it computes.
 struct BlockDev {
@@ -82,6 +84,8 @@ struct RingPlan {
 
 // Largest uniform table (float4s) that travels in the forward kernel's parameters.
 constexpr int kUTabMax = 768;
+// The same for the adjoint's, which holds the x weights too.
+constexpr int kUAdjMax = 1024;
 
 // The forward kernel's plan of a configuration. Its tiles run over (x, mid,
 // innermost) = (x, y, z) or (x, z, y). The first pass filters along mid, once for
@@ -103,7 +107,7 @@ constexpr int kUTabMax = 768;
 // utab, records of float4 (words as int bits where marked *):
 //   groups [ngroups]     {mid value*, first pair*, end pair*, 0}
 //   pairs  [npairs][4]   P = r0.x A + r0.z B: {r0.x, r0.x, r0.z, r0.z}, E likewise,
-//                        {plane of A*, B*, Z*, x value*}, {first point*, end point*, 0, 0}
+//                        {plane of A*, B*, Z*, x value*}, {first point*, end point*, offset mask of the x value*, 0}
 //   points [npoints][3]  {kappa, kappa, -kappa, -kappa}, {-sqrt(rho)|u| x 2, sqrt(rho) x 2},
 //                        {first record of the n value's weights*, offset mask*, 0, 0}
 //   wz     [nzv][mz][2]  {w0, w0, w1, w1}, {w2, w2, w3, w3}
@@ -116,13 +120,18 @@ struct FwdPlan {
     int mag[3] = {0, 0, 0};  // tile axis order
     int ax1 = 1, ax2 = 2;    // volume axes of the mid and innermost tile axis
     std::vector<float> utab, lane;
+    // the adjoint's uniform table: utab with {-2 weight |u|^2 x 2, 2 weight |u| x 2} as the
+    // points' second record, and wx [nxv][mx][2] {w0, w0, w1, w1}, {w2, w2, w3, w3} at u_wx
+    std::vector<float> adj_utab;
+    int u_wx = 0;
     int u_grp = 0, u_pair = 0, u_pt = 0, u_wz = 0, u_wi = 0;
     int l_wx = 0, l_offx = 0, l_wm = 0, l_offm = 0;
-    int ngroups = 0, npairs = 0, npoints = 0, zero_x = 0, zero_m = 0;
+    int ngroups = 0, npairs = 0, npoints = 0, zero_x = 0, zero_xoff = 0, zero_m = 0;
     float neg_weight = 0.f;
 };
 
-// Everything the forward radiality kernel needs; passed by value.
+// Everything the radiality kernel and its adjoint need; passed by value (the
+// adjoint reads float input without TMA staging and writes no stacks).
 struct FwdParams {
     const void* in;       // input volume [t][z][y][x]
     int W, H, D, T;       // full input dims
@@ -143,8 +152,8 @@ struct FwdParams {
     const float* lane;    // lane tables
     int lane_words, l_wx, l_offx, l_wm, l_offm;
     const float4* utab;   // uniform tables in global memory (read when they do not fit the parameters)
-    int u_count, u_grp, u_pair, u_pt, u_wz, u_wi;
-    int ngroups, zero_x, zero_m;
+    int u_count, u_grp, u_pair, u_pt, u_wz, u_wi, u_wx;
+    int ngroups, zero_x, zero_xoff, zero_m;
     float neg_weight;     // minus the commonest point's weight
     const BlockDev* blocks;
     const TileDesc* tiles;
@@ -162,41 +171,6 @@ struct FwdParams {
     // time window of this launch: volumes [t_lo, t_hi) (t_hi 0: up to T), and
     // the volume held by the first [t] row of the stacks (0 when they hold the
     // whole series, t_lo when they hold one batch)
-    int t_lo, t_hi, stack_t0;
-};
-
-// Device-side tables (one contiguous buffer), offsets in 4-byte words.
-struct TableLayout {
-    int wx, offx, wy, offy, wz, offz, wzi, grp_xval, grp, pair_yval, pair_pt, pt_zval, pt_vec, pair_rot;
-    int words;
-};
-
-// Everything the radiality adjoint kernel needs; passed by value.
-struct RadParams {
-    const void* in;       // input volume [t][z][y][x]
-    int W, H, D, T;       // full input dims
-    int mag[3];
-    int nxv, nyv, nzv;    // distinct ring values per axis
-    int ngroups, npairs, npoints;
-    int zero_pair;        // pair index of (x=0, y=0), carries the intensity
-    int gr[4];            // gradient ranges: main, x, y, z (smooth=0 => 1,0,0,0)
-    int grad_mode;        // 1: ranges (1,1,1,1), 2: (1,0,0,0), 0: generic loops
-    int R;                // gradient halo
-    int TY;               // subvoxel rows per tile (threads = 8 * TY)
-    int NU, NV, NW;       // coarse G tile extents
-    int NIX, NIY, NIZ;    // input tile extents (G tile + halo)
-    int renorm, poscon;
-    int t_chunk, nchunks;
-    int ntiles;
-    long long nitems;
-    const float* tables;  // TableLayout words
-    TableLayout tl;
-    const BlockDev* blocks;
-    const TileDesc* tiles;
-    unsigned int* work_counter;
-    int smem_table_words;
-    // volumes [t_lo, t_hi) of this launch (t_hi 0: up to T) and the volume of the
-    // adjoint stacks' first row
     int t_lo, t_hi, stack_t0;
 };
 
@@ -261,9 +235,11 @@ struct AdjParams {
 };
 
 // Launchers (radiality.cu / temporal.cu / adjoint.cu). Return a cudaError_t as int.
-int launch_radiality_adjoint(const RadParams& p, const AdjParams& a, int grid, size_t smem, void* stream);
-size_t radiality_adjoint_smem_bytes(const RadParams& p);
-int radiality_adjoint_max_ctas_per_sm(const RadParams& p, int* out);
+int launch_radiality_adjoint(const FwdParams& p, const FwdPlan& plan, const AdjParams& a, int grid, size_t smem,
+                             void* stream);
+int radiality_adjoint_u_region(const FwdParams& p);
+size_t radiality_adjoint_smem_bytes(const FwdParams& p);
+int radiality_adjoint_max_ctas_per_sm(const FwdParams& p, int* out);
 int launch_temporal_adjoint(const BlockDev* blocks, long long vox, const float* rad, const float* inten,
                             const float* gmap, int T, int method, int itc, int order, int iw, int renorm, int poscon,
                             float* gS, float* gI, long long nmap, unsigned long long* err, void* stream);
@@ -298,13 +274,13 @@ int launch_seed_spots(const float* map, const int map_dims[3], int mag, const in
 
 // Host planning (plan.cpp).
 bool build_ring_plan(const rfba_srrf_config& c, RingPlan* rp, std::string* err);
-bool build_tables(const rfba_srrf_config& c, const RingPlan& rp, std::vector<float>* words, TableLayout* tl,
-                  std::string* err);
 bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err);
 // Parameters of a forward launch that follow from the plan and configuration
 // (not the block and tile lists, stacks and schedule). ty: tile rows, 0 = default.
 FwdParams forward_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, int in_u16, const int dims[4],
                          int ty, int cz);
+// The same for the adjoint kernel.
+FwdParams adjoint_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, const int dims[4]);
 // Tiles of a block's region [lo, hi) in the plan's tile axes (b->cz set).
 void forward_tiles(const FwdPlan& fp, int ty, BlockDev* b);
 // Tile depth (innermost cells, 4 or 8) for regions of these innermost extents.

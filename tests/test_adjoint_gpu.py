@@ -254,3 +254,29 @@ def test_random_adjoint_matches_fp64_adjoint(ctx, oracle_mod, i):
     msg = f"[adjoint] random {i} {kw} {shape}: dL/dI {e_in:.2e}, dL/dshift {e_sh:.2e}"
     assert e_in < 2e-4 and e_sh < 2e-4, msg
     print(msg)
+
+
+PLANS = [
+    # (mag x, y, z), axes, (T, D, H, W)
+    ((1, 2, 2), 6, (5, 8, 8, 19)),   # more than 16 cells of x to a row
+    ((2, 2, 2), 6, (5, 9, 8, 9)),    # one subvoxel row or more past a tile on every axis
+    ((2, 4, 2), 6, (5, 8, 7, 9)),    # y innermost
+    ((8, 2, 3), 6, (5, 7, 8, 7)),    # z innermost, eight x phases
+    ((5, 5, 5), 5, (5, 7, 7, 7)),    # shallow tiles; nothing at a quarter turn of the ring
+    ((2, 2, 2), 12, (5, 8, 8, 8)),   # tables in global memory
+]
+
+
+@pytest.mark.parametrize("mag,axes,shape", PLANS)
+def test_adjoint_plan_choice_matches_fp64_adjoint(ctx, oracle_mod, mag, axes, shape):
+    """The adjoint kernel's tile axis orders, depths, exchange rows and table forms,
+    to the bounds of the cases above."""
+    from rfba_gb300 import srrf
+    O = oracle_mod
+    kw = dict(mag=mag, method=3, itc=0, trac_order=2, axes_in_ring=axes, **SHIPPED)
+    x, sh = _case(70 + axes, *shape, drift=0.25)
+    m, din, dsh = _gpu(ctx, srrf.Config.make(**kw), x, sh)
+    mo = O.forward_shifted(x, O.make_conf(**kw), sh)
+    assert_parity(m, mo, 1e-4, f"{mag} forward")
+    _, din_o, dsh_o = O.adjoint(x, O.make_conf(**kw), _gmap(mo), sh)
+    assert rel_linf(din, din_o) < 2e-4 and rel_linf(dsh, dsh_o) < 2e-4
