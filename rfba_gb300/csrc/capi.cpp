@@ -164,9 +164,16 @@ static int make_blocks(rfba_ctx* ctx, const rfba_srrf_config& cfg, const int dim
     const int T = dims[3];
     // z slabs are whole tiles deep
     const FwdPlan& fp = ctx->plan.fwd;
-    std::vector<std::array<int, 2>> depth;
-    for (int i = 0; i < nblocks; ++i) depth.push_back({blocks[i].lo[fp.ax2], blocks[i].hi[fp.ax2]});
-    const int cz = forward_depth(fp, depth);
+    std::vector<FwdRegion> regions;
+    for (int i = 0; i < nblocks; ++i) {
+        FwdRegion r;
+        for (int a = 0; a < 3; ++a) {
+            r.lo[a] = blocks[i].lo[a];
+            r.hi[a] = std::max(blocks[i].hi[a], blocks[i].lo[a]);
+        }
+        regions.push_back(r);
+    }
+    const int cz = forward_depth(fp, regions, T, ctx->sm_count);
     const int FZ = fp.ax2 == 2 ? fp.mag[2] * cz : (ty > 0 ? ty : kTileRows);
     outb->clear();
     // bytes per subvoxel: the stacks of the volumes held at once plus the
@@ -765,6 +772,8 @@ static int forward_blocks_locked(rfba_ctx* ctx, const rfba_srrf_config* cfg, con
             key_put(&gkey, &tb, 1);
             const int overlap = env_on("RFBA_OVERLAP", true) ? 1 : 0;
             key_put(&gkey, &overlap, 1);
+            const int timed = ctx->timing ? 1 : 0;  // event-record nodes only where they are read
+            key_put(&gkey, &timed, 1);
             key_put(&gkey, blocks, (size_t)nblocks);
             const bool host = flags == RFBA_HOST_PTRS;
             auto deps_now = [&]() {
@@ -807,7 +816,7 @@ static int forward_blocks_locked(rfba_ctx* ctx, const rfba_srrf_config* cfg, con
                 if ((s = g->blocks.ensure(ps.blocks.size() * sizeof(BlockDev), "blocks")) ||
                     (s = g->tiles.ensure(ps.tiles.size() * sizeof(TileDesc), "tiles")) ||
                     (s = g->prefix.ensure(ps.prefix.size() * sizeof(long long), "prefix")) ||
-                    (s = g->counters.ensure(np * 256, "counters")) || (s = ensure_events(&g->evs, 3 * np)))
+                    (s = g->counters.ensure(np * 256, "counters")) || (timed && (s = ensure_events(&g->evs, 3 * np))))
                     return s;
                 RFBA_CUDA(cudaMemcpy(g->blocks.p, ps.blocks.data(), ps.blocks.size() * sizeof(BlockDev),
                                      cudaMemcpyHostToDevice), "blocks upload");
@@ -859,8 +868,8 @@ static int forward_blocks_locked(rfba_ctx* ctx, const rfba_srrf_config* cfg, con
                     cs = enqueue_passes(ctx, *cfg, gin, dtype, dims, ps, static_cast<const BlockDev*>(g->blocks.p),
                                         static_cast<const TileDesc*>(g->tiles.p),
                                         static_cast<const long long*>(g->prefix.p),
-                                        static_cast<unsigned int*>(g->counters.p), gout, ctx->cap, g->evs.data(),
-                                        true, windowed ? &win : nullptr);
+                                        static_cast<unsigned int*>(g->counters.p), gout, ctx->cap,
+                                        timed ? g->evs.data() : nullptr, true, windowed ? &win : nullptr);
                 if (ce == cudaSuccess && cs == RFBA_OK && host)
                     ce = cudaMemcpyAsync(out, gout, (size_t)out_elems * 4, cudaMemcpyDeviceToHost, ctx->cap);
                 cudaGraph_t graph = nullptr;

@@ -188,7 +188,7 @@ extern "C" int rfba_srrf_forward_static_scratch(const rfba_srrf_config* cfg, con
         fine_window_int(cfg->mag[a], dims[a], &b.int_lo[a], &b.int_hi[a]);
     }
     b.zbase = 0;
-    b.cz = forward_depth(plan, {{b.lo[plan.ax2], b.hi[plan.ax2]}});
+    b.cz = forward_depth(plan, {{{0, 0, 0}, {b.hi[0], b.hi[1], b.hi[2]}}}, T, 0);
     forward_tiles(plan, 0, &b);
     b.vox = (long long)b.nreg[0] * b.nreg[1] * b.nreg[2];
     b.stack_off = 0;

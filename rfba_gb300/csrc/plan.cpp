@@ -646,25 +646,32 @@ FwdParams adjoint_params(const FwdPlan& fp, const rfba_srrf_config& c, const voi
     return p;
 }
 
-int forward_depth(const FwdPlan& fp, const std::vector<std::array<int, 2>>& lo_hi) {
+int forward_depth(const FwdPlan& fp, const std::vector<FwdRegion>& regions, int T, int sms) {
     // records too many for the kernel parameters run on the shallow kernel only, and
     // so do depths whose sums would not fit the registers beside the columns
     if (fp.utab.size() / 4 > (size_t)kUTabMax || fp.mag[2] > 5) return 4;
     // time per tile column in clocks (one SM, as measured): a point at one subvoxel
     // 29, a pair's second pass at one cell 22, a group's first pass at one cell 7
-    double best = 0;
-    int cz = 4;
-    for (int c : {8, 4}) {
-        const int mz = fp.mag[2], fz = mz * c;
+    double time[2] = {0, 0};
+    long long items = 0;  // (tile, volume) pairs of the deep tiles
+    for (int i = 0; i < 2; ++i) {
+        const int mz = fp.mag[2], cz = i ? 4 : 8, fz = mz * cz;
         double tiles = 0;
-        for (auto& r : lo_hi) tiles += (r[1] - (r[0] / mz) * mz + fz - 1) / fz;
-        const double t = tiles * (fz * 29.0 * fp.npoints + (c + 4) * (22.0 * fp.npairs + 7.0 * fp.ngroups));
-        if (c == 8 || t < best) {
-            best = t;
-            cz = c;
+        for (auto& r : regions) {
+            const int lo = r.lo[fp.ax2], hi = r.hi[fp.ax2];
+            const int n = (hi - (lo / mz) * mz + fz - 1) / fz;
+            tiles += n;
+            if (i == 0)
+                items += (long long)n * ((r.hi[fp.ax0] - r.lo[fp.ax0] + kTileX - 1) / kTileX) *
+                         ((r.hi[fp.ax1] - r.lo[fp.ax1] + kTileRows - 1) / kTileRows) * T;
         }
+        time[i] = tiles * (fz * 29.0 * fp.npoints + (cz + 4) * (22.0 * fp.npairs + 7.0 * fp.ngroups));
     }
-    return cz;
+    // Two deep items or fewer to an SM: a launch lasts as long as one item, and a
+    // shallow one ends sooner (5 x 10x12x12 at mag 2, the whole call: 63.6 us with
+    // deep tiles, 57 with shallow ones).
+    if (items <= 2LL * sms) return 4;
+    return time[1] < time[0] ? 4 : 8;
 }
 
 void forward_tiles(const FwdPlan& fp, int ty, BlockDev* b) {

@@ -290,8 +290,11 @@ FwdParams forward_params(const FwdPlan& fp, const rfba_srrf_config& c, const voi
 FwdParams adjoint_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, const int dims[4]);
 // Tiles of a block's region [lo, hi) in the plan's tile axes (b->cz set).
 void forward_tiles(const FwdPlan& fp, int ty, BlockDev* b);
-// Tile depth (innermost cells, 4 or 8) for regions of these innermost extents.
-int forward_depth(const FwdPlan& fp, const std::vector<std::array<int, 2>>& lo_hi);
+// Tile depth (innermost cells, 4 or 8) for these regions of T volumes on sms SMs.
+struct FwdRegion {
+    int lo[3], hi[3];
+};
+int forward_depth(const FwdPlan& fp, const std::vector<FwdRegion>& regions, int T, int sms);
 bool window_range(float ring_radius_dummy, const std::vector<float>& rcoord, int mag, int dim, int* lo, int* hi);
 int fine_window_int(int mag, int dim, int* lo, int* hi);
 
