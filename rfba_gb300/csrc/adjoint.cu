@@ -566,25 +566,24 @@ __global__ void temporal_adjoint_kernel(const BlockDev* __restrict__ blocks, con
 }
 
 // ---------------------------------------------------------------------------
-// Radiality adjoint, on tiles and packed columns like the forward's (radiality.cu)
-// with y along the lanes, x as the mid and z as the innermost axis (16 x kTileRows
-// columns, one per thread, two halves of a column in a register pair). Every
+// Radiality adjoint, on the forward's plan and tiles (16 x kTileRows columns, one
+// per thread, two halves of a column in a register pair; see radiality.cu). Every
 // (tile, time point) recomputes the interpolated gradient at each ring sample and
 // pushes the derivative back through the passes, transposed and in reverse order:
 //
-//   point   with u = |u| (h P + c Z), dot = h P + c Z, cp = h Z - c P, c2 = cp^2 + E^2,
-//           g2 = dot^2 + c2, s = sqrt(c2 / g2) and K = dL/ds,
+//   point   with the forward's scaled frame values (dot, cp, E, c2 = cp^2 + E^2, g2 =
+//           dot^2 + c2, s = sqrt(c2 / g2)) and K = dL/ds,
 //             ds = ((1 - s^2) (cp dcp + E dE) - s^2 dot ddot) / sqrt(c2 g2),
 //           so with k = K / sqrt(c2 g2), b = s^2 k, m = k - b:
-//             dE = m E, dZ = h m cp - c b dot, -dP = c m cp + h b dot;
+//             dE = m E, dZ = m cp - kappa b dot, -dP = kappa m cp + b dot;
 //   third   transposed along the innermost axis in registers, over the points of a
 //           pair;
-//   second  transposed along y: the lanes of a row exchange their columns through
-//           shared memory, plane by plane, sorted by y phase. Lane u then
+//   second  transposed along x: the lanes of a row exchange their columns through
+//           shared memory, plane by plane, sorted by x phase. Lane u then
 //           gathers coarse cell u: for each phase and tap one shift of the row, so the
 //           weights are uniform and no two lanes add to the same place;
-//   first   transposed along x as a gather over the tile's rows, once per ring value
-//           of x;
+//   first   transposed along the mid axis as a gather over the tile's rows, once per
+//           ring value of that axis;
 //   stencil transposed as a gather over the cells' 3^3 neighbourhood, and one global
 //           atomic add per input voxel of the tile.
 //
@@ -618,8 +617,8 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
     float4* ex = gu + 3 * uplane;
     float* inp = reinterpret_cast<float*>(ut4);
     float4* icell = ut4;
-    const int mx = p.mag[0], my = p.mag[1];  // along the lanes and the mid axis
-    constexpr int a0 = 1, a1 = 0, a2 = 2;    // volume axes of the tile's lane, mid and innermost axis
+    const int mx = p.mag[0], my = p.mag[1];
+    const int a1 = p.ax1, a2 = p.ax2;
     // exchange row: four zeros, then per x phase the tile's coarse cells and four zeros
     const int nxc = adj_cells(mx), exw = 4 + mx * nxc;
     const int tid = threadIdx.x, nthr = blockDim.x;
@@ -640,7 +639,7 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
     const int* offy = reinterpret_cast<const int*>(tab + p.l_offm);
     const int NIX = p.NIX, NIY = p.NIY, NIZ = p.NIZ, R = p.R;
     const int nin = NIX * NIY * NIZ;
-    const FastDiv div_nu(NU), div_nv(NV), div_ty(TY), div_niy(NIY), div_nixy(NIX * NIY);
+    const FastDiv div_nu(NU), div_nv(NV), div_ty(TY), div_nix(NIX), div_nixy(NIX * NIY);
     const float* in = static_cast<const float*>(p.in);
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
 
@@ -654,8 +653,8 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
         const int chunk = (int)(item / p.ntiles);
         const TileDesc td = p.tiles[tile_i];
         const BlockDev& B = p.blocks[td.block];
-        const int bw = B.size[a0], bh = B.size[a1], bd = B.size[a2];
-        const int X0 = B.lo[a0] + td.t[a0] * kTileX;
+        const int bw = B.size[0], bh = B.size[a1], bd = B.size[a2];
+        const int X0 = B.lo[0] + td.t[0] * kTileX;
         const int Y0 = B.lo[a1] + td.t[a1] * TY;
         const int Z0 = (B.lo[a2] / MZ) * MZ + td.t[a2] * FZ;
         const int cx0 = floordiv(X0, mx) - 2;
@@ -670,11 +669,12 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
         // exchange slots that no lane of this tile fills read as zero
         for (int i = tid & 31; i < 2 * NQ * exw; i += 32) ex_warp[i] = zero4;
         const int ex_put = half * exw + xr * nxc + (xi - cx0 - 2) + 4;
-        const bool in_tile = X < B.hi[a0] && Y < B.hi[a1];
+        const bool in_tile = X < B.hi[0] && Y < B.hi[a1];
         const long long V = B.vox;
-        const long long zstride = (long long)B.nreg[0] * B.nreg[1];
+        const long long ystride = a1 == 1 ? B.nreg[0] : (long long)B.nreg[0] * B.nreg[1];
+        const long long zstride = a1 == 1 ? (long long)B.nreg[0] * B.nreg[1] : B.nreg[0];
         const int zlo = B.lo[a2], zhi = B.hi[a2];
-        const long long v0 = (long long)(X - B.lo[a0]) * B.nreg[0] + (Y - B.lo[a1]) + (Z0 - zlo) * zstride;
+        const long long v0 = (long long)(Y - B.lo[a1]) * ystride + (X - B.lo[0]) + (Z0 - zlo) * zstride;
 
         const int t0 = p.t_lo + chunk * p.t_chunk;
         const int t1 = min(p.t_hi > 0 ? p.t_hi : p.T, t0 + p.t_chunk);
@@ -687,22 +687,21 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                 const long long i = sbase + z * zstride;
                 return in_tile && Z >= zlo && Z < zhi && in_range(i, a.n_stack, a.err, 9) ? st[i] : 0.f;
             };
-            // the input voxel of a tile position, clamped to the block
-            auto global_index = [&](int ix, int iy, int iz) -> long long {
-                const int by = B.origin[a0] + clampi(cx0 - R + ix, 0, bw - 1);
-                const int bx = B.origin[a1] + clampi(cy0 - R + iy, 0, bh - 1);
+            auto global_row = [&](int iy, int iz) -> long long {
+                const int by = B.origin[a1] + clampi(cy0 - R + iy, 0, bh - 1);
                 const int bz = B.origin[a2] + clampi(cz0 - R + iz, 0, bd - 1);
-                return tbase + ((long long)bz * p.H + by) * p.W + bx;
+                return tbase + (a1 == 1 ? (long long)bz * p.H + by : (long long)by * p.H + bz) * p.W + B.origin[0];
             };
             __syncthreads();  // the previous time point is done with the input tile's place
-            for (int r = q, ix = q, iz = 0; r < NIX * NIZ; r += TY, ix += TY) {
-                while (ix >= NIX) {
-                    ix -= NIX;
+            for (int r = q, iy = q, iz = 0; r < NIY * NIZ; r += TY, iy += TY) {
+                while (iy >= NIY) {
+                    iy -= NIY;
                     ++iz;
                 }
-                for (int iy = xf; iy < NIY; iy += kTileX) {
-                    const long long gi = global_index(ix, iy, iz);
-                    inp[(iz * NIY + iy) * NIX + ix] = in_range(gi, a.n_in, a.err, 8) ? __ldg(in + gi) : 0.f;
+                const long long rowg = global_row(iy, iz);
+                for (int ix = xf; ix < NIX; ix += kTileX) {
+                    const long long gi = rowg + clampi(cx0 - R + ix, 0, bw - 1);
+                    inp[r * NIX + ix] = in_range(gi, a.n_in, a.err, 8) ? __ldg(in + gi) : 0.f;
                 }
             }
             __syncthreads();
@@ -850,7 +849,6 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                         const float4 c1 = uget(ut, p.utab, p.u_pt + 3 * qi + 1);
                         const float4 c2i = uget(ut, p.utab, p.u_pt + 3 * qi + 2);
                         const int offmask = __float_as_int(c2i.y);
-                        const float2 nc = hi2(c2i);
                         float wun = c1.z;  // 2 weight |u|, in a vector register (see radiality.cu)
                         asm volatile("" : "+f"(wun));
                         auto zpass = [&](auto OFF, int zr, float2 w0, float2 w1, float2 w2, float2 w3) {
@@ -860,8 +858,8 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                                 const float2 P = fma2(w3, TP[zi + o + 3], fma2(w2, TP[zi + o + 2], fma2(w1, TP[zi + o + 1], mul2(w0, TP[zi + o]))));
                                 const float2 E = fma2(w3, TE[zi + o + 3], fma2(w2, TE[zi + o + 2], fma2(w1, TE[zi + o + 1], mul2(w0, TE[zi + o]))));
                                 const float2 Zc = fma2(w3, TZ[zi + o + 3], fma2(w2, TZ[zi + o + 2], fma2(w1, TZ[zi + o + 1], mul2(w0, TZ[zi + o]))));
-                                const float2 dot = fma2(hi2(c0), Zc, mul2(lo2(c0), P));
-                                const float2 cp = fma2(lo2(c0), Zc, mul2(nc, P));
+                                const float2 dot = fma2(lo2(c0), Zc, P);
+                                const float2 cp = fma2(hi2(c0), P, Zc);
                                 const float2 c2 = fma2(cp, cp, mul2(E, E));
                                 const float2 g2 = fma2(dot, dot, c2);
                                 const float2 xx = mul2(c2, g2);
@@ -876,8 +874,8 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                                 const float2 b = mul2(mul2(sn, sn), k);
                                 const float2 m = fma2(b, dup(-1.0f), k);
                                 const float2 mc = mul2(m, cp), bd2 = mul2(b, dot), dE = mul2(m, E);
-                                const float2 dP = fma2(hi2(c0), mc, mul2(lo2(c0), bd2));  // -dL/dP
-                                const float2 dZ = fma2(lo2(c0), mc, mul2(nc, bd2));
+                                const float2 dP = fma2(lo2(c0), mc, bd2);   // -dL/dP
+                                const float2 dZ = fma2(hi2(c0), bd2, mc);
                                 gP[zi + o] = fma2(w0, dP, gP[zi + o]);
                                 gE[zi + o] = fma2(w0, dE, gE[zi + o]);
                                 gZ[zi + o] = fma2(w0, dZ, gZ[zi + o]);
@@ -953,12 +951,12 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
             // neighbours are formed first, four cells of the innermost axis at a time
             // (straight from the cells the scattered single-word reads took a seventh of
             // the kernel's shared-memory cycles).
-            float4 *sA = gt, *sB = gu;  // [quad][NIX][NIY]: x fastest, as the voxels lie
+            float4 *sA = gt, *sB = gu;  // [quad][NIY][NIX]
             if (p.grad_mode == 1) {
                 for (int i = tid; i < NQ * NIY * NIX; i += nthr) {
                     const int wq = div_nixy(i);
                     const int rem = i - wq * (NIX * NIY);
-                    const int ix = div_niy(rem), iy = rem - ix * NIY;
+                    const int iy = div_nix(rem), ix = rem - iy * NIX;
                     float4 A = zero4, Bs = zero4;
 #pragma unroll
                     for (int dm = 0; dm < 3; ++dm)
@@ -983,7 +981,7 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
             for (int i = tid; i < nin; i += nthr) {
                 const int iz = div_nixy(i);
                 const int rem = i - iz * (NIX * NIY);
-                const int ix = div_niy(rem), iy = rem - ix * NIY;
+                const int iy = div_nix(rem), ix = rem - iy * NIX;
                 const int u = ix - R, v = iy - R, w = iz - R;  // cell with the same position
                 float acc = 0.f;
                 auto inside = [&](int uu, int vv, int ww) {
@@ -1021,7 +1019,7 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                             for (int j = -yR; j <= yR; ++j) acc += G(2, -ii, -j, -kk) - G(2, -ii, -j, kk);
                 }
                 if (acc != 0.f) {
-                    const long long gidx = global_index(ix, iy, iz);
+                    const long long gidx = global_row(iy, iz) + clampi(cx0 - R + ix, 0, bw - 1);
                     if (in_range(gidx, a.n_in, a.err, 10)) atomicAdd(a.gin + gidx, acc);
                 }
             }
@@ -1074,7 +1072,7 @@ int launch_radiality_adjoint(const FwdParams& p, const FwdPlan& plan, const AdjP
         if (e != cudaSuccess) return (int)e;
         UTab<UN> tab;
         std::memset(&tab, 0, sizeof tab);
-        if (UN > 1) std::memcpy(tab.q, plan.utab.data(), plan.utab.size() * sizeof(float));
+        if (UN > 1) std::memcpy(tab.q, plan.adj_utab.data(), plan.adj_utab.size() * sizeof(float));
         k<<<grid, p.TY * kTileX, smem, st>>>(p, a, tab);
         return (int)cudaGetLastError();
     });

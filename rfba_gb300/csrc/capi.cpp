@@ -118,8 +118,7 @@ static int ensure_plan(rfba_ctx* ctx, const rfba_srrf_config& cfg, cudaStream_t 
         return RFBA_OK;
     std::string err;
     P.valid = false;
-    if (!build_ring_plan(cfg, &P.ring, &err) || !build_forward_plan(cfg, &P.fwd, &err) ||
-        !build_adjoint_plan(cfg, &P.adj, &err)) {
+    if (!build_ring_plan(cfg, &P.ring, &err) || !build_forward_plan(cfg, &P.fwd, &err)) {
         set_error(err);
         return RFBA_ERR_UNSUPPORTED;
     }
@@ -130,10 +129,8 @@ static int ensure_plan(rfba_ctx* ctx, const rfba_srrf_config& cfg, cudaStream_t 
     P.words = P.fwd.lane;
     P.fwd_utab = P.words.size();
     P.words.insert(P.words.end(), P.fwd.utab.begin(), P.fwd.utab.end());
-    P.adj_lane = P.words.size();
-    P.words.insert(P.words.end(), P.adj.lane.begin(), P.adj.lane.end());
     P.adj_utab = P.words.size();
-    P.words.insert(P.words.end(), P.adj.utab.begin(), P.adj.utab.end());
+    P.words.insert(P.words.end(), P.fwd.adj_utab.begin(), P.fwd.adj_utab.end());
     const int rc = ctx->tables.ensure(P.words.size() * 4, "tables");
     if (rc) return rc;
     RFBA_CUDA(cudaMemcpyAsync(ctx->tables.p, P.words.data(), P.words.size() * 4, cudaMemcpyHostToDevice, st),
@@ -1133,7 +1130,7 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
     const size_t nin = (size_t)dims[0] * dims[1] * dims[2] * T;
     const long long V = blk.vox;
     blk.stack_off = 0;
-    const FwdPlan& fp = ctx->plan.adj;
+    const FwdPlan& fp = ctx->plan.fwd;
     blk.cz = adj_cz(fp.mag[2]);
     forward_tiles(fp, 0, &blk);
     std::vector<TileDesc> tiles;
@@ -1162,9 +1159,8 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
         if (e) return cuda_fail((cudaError_t)e, "temporal adjoint launch");
     }
     FwdParams rp = adjoint_params(fp, *cfg, iprime, dims);
-    const float* tables = static_cast<const float*>(ctx->tables.p);
-    rp.lane = tables + ctx->plan.adj_lane;
-    rp.utab = reinterpret_cast<const float4*>(tables + ctx->plan.adj_utab);
+    rp.lane = static_cast<const float*>(ctx->tables.p);
+    rp.utab = reinterpret_cast<const float4*>(rp.lane + ctx->plan.adj_utab);
     rp.blocks = dblk;
     rp.tiles = static_cast<const TileDesc*>(ctx->atiles.p);
     rp.ntiles = (int)tiles.size();

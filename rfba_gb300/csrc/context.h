@@ -45,9 +45,9 @@ struct PlanCache {
     float ring_radius = 0.f;
     int axes = 0, mag[3] = {0, 0, 0};
     RingPlan ring;
-    FwdPlan fwd, adj;
-    std::vector<float> words;  // the uploaded tables: lane and uniform tables of both plans
-    size_t fwd_utab = 0, adj_lane = 0, adj_utab = 0;  // word offsets in them
+    FwdPlan fwd;
+    std::vector<float> words;  // the uploaded tables: lane tables, uniform tables, the adjoint's uniform tables
+    size_t fwd_utab = 0, adj_utab = 0;  // word offsets in them
 };
 
 // Schedule choices of the forward: tile rows (tile shape) and tile order

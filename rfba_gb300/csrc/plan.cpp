@@ -337,10 +337,7 @@ static bool tap5(int ph, double rho, int mag, float w[5]) {
 // ---------------------------------------------------------------------------
 // Forward plan
 
-// The plan with the cheapest of the given tile axis orders {lane, mid, innermost};
-// adjoint: the pairs' and points' records in the adjoint's form.
-static bool build_plan(const rfba_srrf_config& c, const std::vector<std::array<int, 3>>& orders, bool adjoint,
-                       FwdPlan* fp, std::string* err) {
+bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err) {
     const int n = 2 * c.axes_in_ring;
     const float r = c.ring_radius, tol = 1e-6f * r;
     std::vector<float> raw[3];
@@ -352,17 +349,16 @@ static bool build_plan(const rfba_srrf_config& c, const std::vector<std::array<i
         int a, b, c, m;
         double u[3];
     };
-    // one order of the axes: distinct values, points grouped by mid and then lane
+    // one order of the axes: distinct values, points grouped by mid and then x
     // value, and the pairs' start indices
     struct Order {
-        std::array<int, 3> ax;
         std::vector<float> val[3];
         std::vector<P> pts;
         std::vector<int> pair0;
     };
-    auto arrange = [&](const std::array<int, 3>& ax) {
+    auto arrange = [&](int a1, int a2) {
         Order o;
-        o.ax = ax;
+        const int ax[3] = {0, a1, a2};
         for (int k = 0; k < 3; ++k) {
             for (auto& p : reps) value_index(o.val[k], p[ax[k]], tol);
             value_index(o.val[k], 0.f, tol);  // the intensity's sample
@@ -370,9 +366,9 @@ static bool build_plan(const rfba_srrf_config& c, const std::vector<std::array<i
         }
         for (size_t i = 0; i < reps.size(); ++i) {
             P p;
-            p.a = value_index(o.val[0], reps[i][ax[0]], tol);
-            p.b = value_index(o.val[1], reps[i][ax[1]], tol);
-            p.c = value_index(o.val[2], reps[i][ax[2]], tol);
+            p.a = value_index(o.val[0], reps[i][0], tol);
+            p.b = value_index(o.val[1], reps[i][a1], tol);
+            p.c = value_index(o.val[2], reps[i][a2], tol);
             p.m = mult[i];
             for (int k = 0; k < 3; ++k) p.u[k] = (double)reps[i][ax[k]] / r;
             o.pts.push_back(p);
@@ -393,27 +389,30 @@ static bool build_plan(const rfba_srrf_config& c, const std::vector<std::array<i
         });
         for (size_t i = 0; i < o.pts.size(); ++i) {
             const P& p = o.pts[i];
-            const bool axis = !adjoint && p.u[0] == 0 && p.u[1] == 0;  // one pair per direction
+            const bool axis = p.u[0] == 0 && p.u[1] == 0;
             if (i == 0 || axis || p.a != o.pts[i - 1].a || p.b != o.pts[i - 1].b) o.pair0.push_back((int)i);
         }
         return o;
     };
     // clocks per subvoxel up to a common factor: 22 a pair's second pass, 7 a
     // group's first (as in forward_depth)
-    auto cost = [&](const Order& o) {
+    auto cost = [&](const Order& o, int a2) {
         int groups = 0;
         for (size_t i = 0; i < o.pts.size(); ++i) groups += i == 0 || o.pts[i].b != o.pts[i - 1].b;
-        return (22.0 * o.pair0.size() + 7.0 * groups) / c.mag[o.ax[2]];
+        return (22.0 * o.pair0.size() + 7.0 * groups) / c.mag[a2];
     };
-    Order o = arrange(orders[0]);
-    for (size_t k = 1; k < orders.size(); ++k) {
-        Order alt = arrange(orders[k]);
-        if (cost(alt) < cost(o)) o = std::move(alt);
+    Order o = arrange(1, 2);
+    fp->ax1 = 1;
+    fp->ax2 = 2;
+    {
+        Order alt = arrange(2, 1);
+        if (cost(alt, 1) < cost(o, 2)) {
+            o = std::move(alt);
+            fp->ax1 = 2;
+            fp->ax2 = 1;
+        }
     }
-    const std::array<int, 3> ax = o.ax;
-    fp->ax0 = ax[0];
-    fp->ax1 = ax[1];
-    fp->ax2 = ax[2];
+    const int ax[3] = {0, fp->ax1, fp->ax2};
     for (int k = 0; k < 3; ++k) fp->mag[k] = c.mag[ax[k]];
 
     // lane tables
@@ -507,16 +506,7 @@ static bool build_plan(const rfba_srrf_config& c, const std::vector<std::array<i
         const double ux = f.u[0], um = f.u[1];
         double pa = 1, pb = 0, ea = 0, eb = 1;
         int plane[3] = {2, 1, 0};
-        if (adjoint) {
-            // A = Gx (the mid axis), B = Gy, turned about z
-            const double h = std::sqrt(um * um + ux * ux);
-            pa = eb = h > 0 ? um / h : 1;
-            pb = h > 0 ? ux / h : 0;
-            ea = -pb;
-            plane[0] = 1;
-            plane[1] = 0;
-            plane[2] = 2;
-        } else if (ux == 0 && um == 0) {
+        if (ux == 0 && um == 0) {
             pa = f.u[2] < 0 ? -1 : 1;
         } else {
             plane[0] = 0;
@@ -544,22 +534,13 @@ static bool build_plan(const rfba_srrf_config& c, const std::vector<std::array<i
         if (!taps(2, v, &w, &off)) return false;
     for (int q = 0; q < npts; ++q) {
         const P& p = o.pts[q];
-        const double un = std::sqrt(p.u[1] * p.u[1] + p.u[0] * p.u[0] + p.u[2] * p.u[2]);
+        const double un = std::sqrt(p.u[0] * p.u[0] + p.u[1] * p.u[1] + p.u[2] * p.u[2]);
         const double rho = std::sqrt((double)p.m / common);
         int mask = 0;
         for (int ph = 0; ph < mz; ++ph) mask |= off[p.c * mz + ph] << ph;
-        if (adjoint) {
-            const double h = std::sqrt(p.u[1] * p.u[1] + p.u[0] * p.u[0]) / un, e = p.u[2] / un;
-            const double f = 2.0 * p.m / n * un;
-            put(h, h, e, e);
-            put(-f * un, -f * un, f, f);
-            put_bits(p.c * mz, mask, 0, 0);
-            U[U.size() - 2] = U[U.size() - 1] = (float)-e;
-        } else {
-            put(kappa[q], kappa[q], -kappa[q], -kappa[q]);
-            put(-rho * un, -rho * un, rho, rho);
-            put_bits(p.c * mz, mask, 0, 0);
-        }
+        put(kappa[q], kappa[q], -kappa[q], -kappa[q]);
+        put(-rho * un, -rho * un, rho, rho);
+        put_bits(p.c * mz, mask, 0, 0);
     }
     for (auto& t : w) {
         put(t[0], t[0], t[1], t[1]);
@@ -571,20 +552,19 @@ static bool build_plan(const rfba_srrf_config& c, const std::vector<std::array<i
         const int m0 = 2 * ph + 1 >= mz ? 1 : 0;
         put(t[m0], t[m0 + 1], t[m0 + 2], t[m0 + 3]);
     }
-    if (adjoint) {
-        fp->u_wx = (int)(U.size() / 4);
-        for (auto& t : w_x)
-            for (int k : {0, 0, 1, 1, 2, 2, 3, 3}) U.push_back(t[k]);
+    fp->adj_utab = U;
+    for (int q = 0; q < npts; ++q) {
+        const P& p = o.pts[q];
+        const double un = std::sqrt(p.u[0] * p.u[0] + p.u[1] * p.u[1] + p.u[2] * p.u[2]);
+        const double f = 2.0 * p.m / n * un;
+        float* r = &fp->adj_utab[4 * (fp->u_pt + 3 * q + 1)];
+        r[0] = r[1] = (float)(-f * un);
+        r[2] = r[3] = (float)f;
     }
+    fp->u_wx = (int)(fp->adj_utab.size() / 4);
+    for (auto& t : w_x)
+        for (int k : {0, 0, 1, 1, 2, 2, 3, 3}) fp->adj_utab.push_back(t[k]);
     return true;
-}
-
-bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err) {
-    return build_plan(c, {{0, 1, 2}, {0, 2, 1}}, false, fp, err);
-}
-
-bool build_adjoint_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err) {
-    return build_plan(c, {{1, 0, 2}}, true, fp, err);
 }
 
 FwdParams forward_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, int in_u16, const int dims[4],
@@ -602,7 +582,7 @@ FwdParams forward_params(const FwdPlan& fp, const rfba_srrf_config& c, const voi
     p.ax2 = fp.ax2;
     const int lat[3] = {c.x_range, c.y_range, c.z_range};
     p.gr[0] = c.gradient_smooth == 0 ? 1 : c.main_range;
-    p.gr[1] = c.gradient_smooth == 0 ? 0 : lat[fp.ax0];
+    p.gr[1] = c.gradient_smooth == 0 ? 0 : lat[0];
     p.gr[2] = c.gradient_smooth == 0 ? 0 : lat[fp.ax1];
     p.gr[3] = c.gradient_smooth == 0 ? 0 : lat[fp.ax2];
     p.R = std::max(std::max(p.gr[0], p.gr[1]), std::max(p.gr[2], p.gr[3]));
@@ -643,6 +623,7 @@ FwdParams adjoint_params(const FwdPlan& fp, const rfba_srrf_config& c, const voi
     FwdParams p = forward_params(fp, c, in, 0, dims, 0, adj_cz(fp.mag[2]));
     p.tma_bx = 0;
     p.u_region = radiality_adjoint_u_region(p);
+    p.u_count = (int)(fp.adj_utab.size() / 4);
     return p;
 }
 
@@ -677,7 +658,7 @@ int forward_depth(const FwdPlan& fp, const std::vector<FwdRegion>& regions, int 
 void forward_tiles(const FwdPlan& fp, int ty, BlockDev* b) {
     const int rows = ty > 0 ? ty : kTileRows;
     const int mz = fp.mag[2], fz = mz * b->cz;
-    b->ntile[fp.ax0] = (b->nreg[fp.ax0] + kTileX - 1) / kTileX;
+    b->ntile[0] = (b->nreg[0] + kTileX - 1) / kTileX;
     b->ntile[fp.ax1] = (b->nreg[fp.ax1] + rows - 1) / rows;
     b->ntile[fp.ax2] = (b->hi[fp.ax2] - (b->lo[fp.ax2] / mz) * mz + fz - 1) / fz;
 }

@@ -128,8 +128,8 @@ __device__ __forceinline__ void gradient4(int mode, const int gr[4], Row&& row, 
                 for (int i = -xR; i <= xR; ++i)
                     for (int k = -zR; k <= zR; ++k) gm += I(i, j, k) - I(i, -j, k);
             for (int k = 1; k <= mR; ++k)
-                for (int j = -yR; j <= yR; ++j)
-                    for (int i = -xR; i <= xR; ++i) gn += I(i, j, k) - I(i, j, -k);
+                for (int i = -xR; i <= xR; ++i)
+                    for (int j = -yR; j <= yR; ++j) gn += I(i, j, k) - I(i, j, -k);
             g[0][w] = gx;
             g[1][w] = gm;
             g[2][w] = gn;

@@ -116,20 +116,14 @@ constexpr int kUAdjMax = 1024;
 // the point's multiplicity over the commonest one, whose weight is neg_weight. lane:
 // per x and per mid value and phase the 4 tap weights and their offset, looked up by
 // lane and row in shared memory.
-//
-// The adjoint's plan takes the axes in the order (y, x, z): its passes run along x,
-// then y, then z, in the rounding of the forms it is compared with. Where the
-// interpolated gradient nearly vanishes, or nearly follows the ring direction, its
-// rounding is amplified into the derivative, so another order of the passes moves
-// single voxels of dL/dI by 1e-3 and more of their size. Pairs hold the plain rotation
-// P = r0.x Gx + r0.z Gy and E likewise, points {h, h, c, c}, {-2 weight |u|^2 x 2, 2
-// weight |u| x 2}, {first record of the z value's weights*, offset mask*, -c, -c} with
-// u = |u| (h P + c Z), and wx [nyv][my][2] {w0, w0, w1, w1}, {w2, w2, w3, w3} follows.
 struct FwdPlan {
     int mag[3] = {0, 0, 0};  // tile axis order
-    int ax0 = 0, ax1 = 1, ax2 = 2;  // volume axes of the tile's lane, mid and innermost axis
+    int ax1 = 1, ax2 = 2;    // volume axes of the mid and innermost tile axis
     std::vector<float> utab, lane;
-    int u_wx = 0;  // adjoint only
+    // the adjoint's uniform table: utab with {-2 weight |u|^2 x 2, 2 weight |u| x 2} as the
+    // points' second record, and wx [nxv][mx][2] {w0, w0, w1, w1}, {w2, w2, w3, w3} at u_wx
+    std::vector<float> adj_utab;
+    int u_wx = 0;
     int u_grp = 0, u_pair = 0, u_pt = 0, u_wz = 0, u_wi = 0;
     int l_wx = 0, l_offx = 0, l_wm = 0, l_offm = 0;
     int ngroups = 0, npairs = 0, npoints = 0, zero_x = 0, zero_xoff = 0, zero_m = 0;
@@ -281,7 +275,6 @@ int launch_seed_spots(const float* map, const int map_dims[3], int mag, const in
 // Host planning (plan.cpp).
 bool build_ring_plan(const rfba_srrf_config& c, RingPlan* rp, std::string* err);
 bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err);
-bool build_adjoint_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err);
 // Parameters of a forward launch that follow from the plan and configuration
 // (not the block and tile lists, stacks and schedule). ty: tile rows, 0 = default.
 FwdParams forward_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, int in_u16, const int dims[4],
