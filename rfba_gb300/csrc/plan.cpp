@@ -643,7 +643,7 @@ int forward_depth(const FwdPlan& fp, const std::vector<FwdRegion>& regions, int 
             const int n = (hi - (lo / mz) * mz + fz - 1) / fz;
             tiles += n;
             if (i == 0)
-                items += (long long)n * ((r.hi[fp.ax0] - r.lo[fp.ax0] + kTileX - 1) / kTileX) *
+                items += (long long)n * ((r.hi[0] - r.lo[0] + kTileX - 1) / kTileX) *
                          ((r.hi[fp.ax1] - r.lo[fp.ax1] + kTileRows - 1) / kTileRows) * T;
         }
         time[i] = tiles * (fz * 29.0 * fp.npoints + (cz + 4) * (22.0 * fp.npairs + 7.0 * fp.ngroups));
