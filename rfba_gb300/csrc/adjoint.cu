@@ -594,6 +594,37 @@ __device__ __forceinline__ float4 f4fma(float s, float4 a, float4 c) {
     return make_float4(fmaf(s, a.x, c.x), fmaf(s, a.y, c.y), fmaf(s, a.z, c.z), fmaf(s, a.w, c.w));
 }
 
+// Ring samples whose gradient nearly vanishes or nearly follows the ring direction
+// amplify the rounding of the interpolated gradient into the derivative, by |g|^2 of
+// the column over |g| |g_perp| of the sample. Below a bound on c2 g2 (this factor
+// times the square of the sum of |g|^2 over four cells of the column) the kernel
+// takes the derivative at the bound, which needs no operation more than the guard
+// against 0 that was there, and lists the sample; adjoint_samples_kernel then adds
+// the difference to the derivative as it comes out in the rounding of passes along x,
+// then y, then z, whatever order this kernel's passes take. About one sample in a
+// million is listed; once kAdjSamplesOpen are, pairs begun later take no bound (the
+// list has room for all that may be under way then). Without that, single voxels of dL/dI differed between the two
+// orders by up to 5e-3 of their size on one of four drift series.
+constexpr float kSampleBound = 6e-9f;
+
+// The derivative of one sample's sine term with respect to (-P, E, Z), times K.
+struct Derivative {
+    float P, E, Z;
+};
+__device__ __forceinline__ Derivative sample_derivative(float P, float E, float Z, float h, float c, float wun, float un,
+                                                        float gS, float inv) {
+    const float dot = fmaf(c, Z, __fmul_rn(h, P)), cp = fmaf(h, Z, __fmul_rn(-c, P));
+    const float c2 = fmaf(cp, cp, __fmul_rn(E, E)), sn = c2 * inv;
+    const float k = flip_sign(wun * fmaf(sn, -un, 1.f), dot) * gS * inv;
+    const float b = sn * sn * k, m = k - b;
+    return Derivative{fmaf(c, m * cp, h * (b * dot)), m * E, fmaf(h, m * cp, -c * (b * dot))};
+}
+
+__device__ __forceinline__ void list_sample(const AdjParams& a, long long index, int point, float bound) {
+    const unsigned int i = atomicAdd(a.nsamples, 1u);
+    if (i < kAdjSamples) a.samples[i] = AdjSample{index, point, bound};
+}
+
 template <int MZ, int CZ, int UN>
 __global__ void __maxnreg__(adj_regs(MZ, CZ))
     radiality_adjoint_kernel(const __grid_constant__ FwdParams p, const __grid_constant__ AdjParams a,
@@ -821,6 +852,7 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                     const float4 wv = *reinterpret_cast<const float4*>(wx + ax * 4);
                     const float4* ubase = ut4 + q * NU + xi - cx0 - 2 + offx[ax];
                     const int pa = __float_as_int(r2.x), pb = __float_as_int(r2.y), pc = __float_as_int(r2.z);
+                    const unsigned int listed = *static_cast<volatile unsigned int*>(a.nsamples);
                     float2 TP[NH], TE[NH], TZ[NH];
 #pragma unroll
                     for (int wq = 0; wq < NQ; ++wq) {
@@ -841,6 +873,13 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                         TP[w] = fma2(hi2(r0), Bv, mul2(lo2(r0), A));
                         TE[w] = fma2(hi2(r1), Bv, mul2(lo2(r1), A));
                     }
+                    float bound = 1e-30f;
+                    if (listed < kAdjSamplesOpen) {
+                        constexpr int w = NH / 2;
+                        const float2 lo = fma2(TZ[w - 1], TZ[w - 1], fma2(TE[w - 1], TE[w - 1], mul2(TP[w - 1], TP[w - 1])));
+                        const float2 g = fma2(TZ[w], TZ[w], fma2(TE[w], TE[w], fma2(TP[w], TP[w], lo)));
+                        bound = fmaxf((g.x + g.y) * (g.x + g.y) * kSampleBound, 1e-30f);
+                    }
                     float2 gP[NH], gE[NH], gZ[NH];  // gP with the sign turned
 #pragma unroll
                     for (int w = 0; w < NH; ++w) gP[w] = gE[w] = gZ[w] = make_float2(0.f, 0.f);
@@ -853,6 +892,7 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                         asm volatile("" : "+f"(wun));
                         auto zpass = [&](auto OFF, int zr, float2 w0, float2 w1, float2 w2, float2 w3) {
                             constexpr int o = decltype(OFF)::value;
+                            float lowest = 1e30f;  // c2 g2 over these samples
 #pragma unroll
                             for (int zi = 0; zi < CH; ++zi) {
                                 const float2 P = fma2(w3, TP[zi + o + 3], fma2(w2, TP[zi + o + 2], fma2(w1, TP[zi + o + 1], mul2(w0, TP[zi + o]))));
@@ -863,10 +903,12 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                                 const float2 c2 = fma2(cp, cp, mul2(E, E));
                                 const float2 g2 = fma2(dot, dot, c2);
                                 const float2 xx = mul2(c2, g2);
-                                // 1 / sqrt(c2 g2); where g is parallel to u (c2 = 0) every product
-                                // below carries a factor c2, cp or E and vanishes
-                                const float2 inv = make_float2(rsqrt_approx(fmaxf(xx.x, 1e-30f)),
-                                                               rsqrt_approx(fmaxf(xx.y, 1e-30f)));
+                                lowest = fminf(lowest, fminf(xx.x, xx.y));
+                                // 1 / sqrt(c2 g2), at most that at the bound; where g is parallel to
+                                // u (c2 = 0) every product below carries a factor c2, cp or E and
+                                // vanishes
+                                const float2 inv = make_float2(rsqrt_approx(fmaxf(xx.x, bound)),
+                                                               rsqrt_approx(fmaxf(xx.y, bound)));
                                 const float2 sn = mul2(c2, inv);
                                 // K = dL/ds = dL/dS sign(dot) 2 weight |u| (1 - |u| s)
                                 const float2 om = mul2(fma2(sn, lo2(c1), dup(wun)), gS[zi * MZ + zr]);
@@ -888,6 +930,21 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                                 gP[zi + o + 3] = fma2(w3, dP, gP[zi + o + 3]);
                                 gE[zi + o + 3] = fma2(w3, dE, gE[zi + o + 3]);
                                 gZ[zi + o + 3] = fma2(w3, dZ, gZ[zi + o + 3]);
+                            }
+                            if (lowest < bound) {
+#pragma unroll
+                                for (int zi = 0; zi < CH; ++zi) {
+                                    const float2 P = fma2(w3, TP[zi + o + 3], fma2(w2, TP[zi + o + 2], fma2(w1, TP[zi + o + 1], mul2(w0, TP[zi + o]))));
+                                    const float2 E = fma2(w3, TE[zi + o + 3], fma2(w2, TE[zi + o + 2], fma2(w1, TE[zi + o + 1], mul2(w0, TE[zi + o]))));
+                                    const float2 Zc = fma2(w3, TZ[zi + o + 3], fma2(w2, TZ[zi + o + 2], fma2(w1, TZ[zi + o + 1], mul2(w0, TZ[zi + o]))));
+                                    const float2 dot = fma2(lo2(c0), Zc, P);
+                                    const float2 cp = fma2(hi2(c0), P, Zc);
+                                    const float2 c2 = fma2(cp, cp, mul2(E, E));
+                                    const float2 xx = mul2(c2, fma2(dot, dot, c2));
+                                    const int z = zi * MZ + zr;
+                                    if (xx.x < bound && gS[z].x != 0.f) list_sample(a, sbase + z * zstride, qi, bound);
+                                    if (xx.y < bound && gS[z].y != 0.f) list_sample(a, sbase + (z + HZ) * zstride, qi, bound);
+                                }
                             }
                         };
 #pragma unroll
@@ -1027,6 +1084,138 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
     }
 }
 
+// The samples that the kernel above listed, one warp to a sample: the gradient at the
+// 4 x 4 x 4 cells its taps reach, interpolated along x, then y, then z, the derivative
+// of the radiality term in the plain rotated frame less the one at the bound, and
+// its transpose onto the input voxels (the taps and the stencil are products over
+// the axes). 8 volumes of 64^3 take 0.1 ms beside the kernel's 4.5.
+__global__ void __launch_bounds__(128) adjoint_samples_kernel(const __grid_constant__ FwdParams p, const AdjParams a,
+                                                              const AdjFixTables f) {
+    const unsigned int n = min(*a.nsamples, kAdjSamples);
+    const int lane = threadIdx.x & 31;
+    const BlockDev& B = p.blocks[0];
+    const float* in = static_cast<const float*>(p.in);
+    const bool zin = p.ax2 == 2;
+    const int mag[3] = {p.mag[0], zin ? p.mag[1] : p.mag[2], zin ? p.mag[2] : p.mag[1]};
+    const int range[3] = {p.gr[1], zin ? p.gr[2] : p.gr[3], zin ? p.gr[3] : p.gr[2]};
+    const int mR = p.gr[0];
+    for (unsigned int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s < n;
+         s += gridDim.x * (blockDim.x >> 5)) {
+        const AdjSample e = a.samples[s];
+        const long long rel = e.index - B.stack_off, row = rel / B.vox;
+        const int t = p.stack_t0 + (int)row, v0 = (int)(rel - row * B.vox);
+        const int at[3] = {B.lo[0] + v0 % B.nreg[0], B.lo[1] + v0 / B.nreg[0] % B.nreg[1],
+                           B.lo[2] + v0 / B.nreg[0] / B.nreg[1]};
+        const int4 vi = f.idx[e.point];
+        const int val[3] = {vi.x, vi.y, vi.z};
+        float w[3][4];
+        int c0[3];  // first tap cell
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int xi = floordiv(at[k], mag[k]), i = val[k] * mag[k] + at[k] - xi * mag[k];
+            const float4 v = f.w[k][i];
+            w[k][0] = v.x, w[k][1] = v.y, w[k][2] = v.z, w[k][3] = v.w;
+            c0[k] = xi - 2 + f.off[k][i];
+        }
+        const long long tbase = (long long)t * p.D * p.H * p.W;
+        auto index = [&](int x, int y, int z) -> long long {
+            return tbase + ((long long)(B.origin[2] + clampi(z, 0, B.size[2] - 1)) * p.H +
+                            (B.origin[1] + clampi(y, 0, B.size[1] - 1))) * p.W + (B.origin[0] + clampi(x, 0, B.size[0] - 1));
+        };
+        // cells 4 (j + 4 k) + i: this lane's and the one 32 further on
+        float g[2][3];
+        for (int h = 0; h < 2; ++h) {
+            const int c = lane + 32 * h;
+            const int cx = c0[0] + (c & 3), cy = c0[1] + ((c >> 2) & 3), cz = c0[2] + (c >> 4);
+            float gx = 0.f, gy = 0.f, gz = 0.f;
+            if (cx >= 0 && cx < B.size[0] && cy >= 0 && cy < B.size[1] && cz >= 0 && cz < B.size[2]) {
+                auto I = [&](int dx, int dy, int dz) -> float {
+                    const long long i = index(cx + dx, cy + dy, cz + dz);
+                    return in_range(i, a.n_in, a.err, 11) ? __ldg(in + i) : 0.f;
+                };
+                for (int i = 1; i <= mR; ++i)
+                    for (int j = -range[1]; j <= range[1]; ++j)
+                        for (int k = -range[2]; k <= range[2]; ++k) gx += I(i, j, k) - I(-i, j, k);
+                for (int j = 1; j <= mR; ++j)
+                    for (int i = -range[0]; i <= range[0]; ++i)
+                        for (int k = -range[2]; k <= range[2]; ++k) gy += I(i, j, k) - I(i, -j, k);
+                for (int k = 1; k <= mR; ++k)
+                    for (int i = -range[0]; i <= range[0]; ++i)
+                        for (int j = -range[1]; j <= range[1]; ++j) gz += I(i, j, k) - I(i, j, -k);
+            }
+            g[h][0] = gx, g[h][1] = gy, g[h][2] = gz;
+        }
+        // x: lanes 0 .. 15 hold (j, k) = (lane & 3, lane >> 2); y: lanes 0 .. 3 hold k; z
+        float v[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            float acc = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float lo = __shfl_sync(0xffffffffu, g[0][d], (4 * lane + i) & 31);
+                const float hi = __shfl_sync(0xffffffffu, g[1][d], (4 * lane + i) & 31);
+                const float u = lane < 8 ? lo : hi;
+                acc = i ? fmaf(w[0][i], u, acc) : w[0][0] * u;
+            }
+            v[d] = acc;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float u = __shfl_sync(0xffffffffu, v[d], (4 * lane + i) & 31);
+                acc = i ? fmaf(w[1][i], u, acc) : w[1][0] * u;
+            }
+            v[d] = acc;
+        }
+        const float4 fr = f.frame[e.point];
+        float pez[3] = {fmaf(v[1], fr.y, __fmul_rn(v[0], fr.x)), fmaf(v[1], fr.x, __fmul_rn(v[0], -fr.y)), v[2]};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            float acc = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float u = __shfl_sync(0xffffffffu, pez[d], i);
+                acc = i ? fmaf(w[2][i], u, acc) : w[2][0] * u;
+            }
+            v[d] = acc;
+        }
+        const float P = v[0], E = v[1], Z = v[2], hh = fr.z, cc = fr.w;
+        const float dot = fmaf(cc, Z, __fmul_rn(hh, P)), cp = fmaf(hh, Z, __fmul_rn(-cc, P));
+        const float c2 = fmaf(cp, cp, __fmul_rn(E, E)), xx = c2 * fmaf(dot, dot, c2);
+        // the kernel above scales this frame by 1 / h (by 1 on the z axis of its plan)
+        const float scale = f.scale[e.point], s4 = scale * scale * scale * scale;
+        const float2 wt = f.weight[e.point];
+        const float gS = in_range(e.index, a.n_stack, a.err, 9) ? a.gS[e.index] : 0.f;
+        const Derivative r = sample_derivative(P, E, Z, hh, cc, wt.x, wt.y, gS, rsqrt_approx(fmaxf(xx, 1e-30f)));
+        const Derivative q0 = sample_derivative(P, E, Z, hh, cc, wt.x, wt.y, gS,
+                                                scale * scale * rsqrt_approx(fmaxf(xx * s4, e.bound)));
+        const float dP = q0.P - r.P, dE = r.E - q0.E, dZ = r.Z - q0.Z;
+        const float dG[3] = {fmaf(dE, -fr.y, dP * fr.x), fmaf(dE, fr.x, dP * fr.y), dZ};
+        // transposed: taps, then the stencil, per axis along the gradient's component (der)
+        // and across it (box); cells outside the block hold no gradient
+        const int nx = 4 + 2 * p.R;
+        for (int q = lane; q < nx * nx * nx; q += 32) {
+            const int pos[3] = {q % nx - p.R, q / nx % nx - p.R, q / (nx * nx) - p.R};
+            float der[3], box[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                der[d] = box[d] = 0.f;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (c0[d] + i < 0 || c0[d] + i >= B.size[d]) continue;
+                    const int o = pos[d] - i;
+                    if (o != 0 && abs(o) <= mR) der[d] += o > 0 ? w[d][i] : -w[d][i];
+                    if (abs(o) <= range[d]) box[d] += w[d][i];
+                }
+            }
+            const float acc = dG[0] * der[0] * box[1] * box[2] + dG[1] * box[0] * der[1] * box[2] +
+                              dG[2] * box[0] * box[1] * der[2];
+            if (acc != 0.f) {
+                const long long i = index(c0[0] + pos[0], c0[1] + pos[1], c0[2] + pos[2]);
+                if (in_range(i, a.n_in, a.err, 11)) atomicAdd(a.gin + i, acc);
+            }
+        }
+    }
+}
+
 template <class F>
 int with_adj_kernel(const FwdParams& p, F&& f) {
     auto go = [&](auto mz) -> int {
@@ -1076,6 +1265,11 @@ int launch_radiality_adjoint(const FwdParams& p, const FwdPlan& plan, const AdjP
         k<<<grid, p.TY * kTileX, smem, st>>>(p, a, tab);
         return (int)cudaGetLastError();
     });
+}
+
+int launch_adjoint_samples(const FwdParams& p, const AdjParams& a, const AdjFixTables& f, int sms, void* stream) {
+    adjoint_samples_kernel<<<4 * sms, 128, 0, static_cast<cudaStream_t>(stream)>>>(p, a, f);
+    return (int)cudaGetLastError();
 }
 
 int radiality_adjoint_max_ctas_per_sm(const FwdParams& p, int* out) {
