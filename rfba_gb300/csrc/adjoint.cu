@@ -670,7 +670,7 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
     const int* offy = reinterpret_cast<const int*>(tab + p.l_offm);
     const int NIX = p.NIX, NIY = p.NIY, NIZ = p.NIZ, R = p.R;
     const int nin = NIX * NIY * NIZ;
-    const FastDiv div_nu(NU), div_nv(NV), div_ty(TY), div_nix(NIX), div_nixy(NIX * NIY);
+    const FastDiv div_nu(NU), div_nv(NV), div_nix(NIX), div_nixy(NIX * NIY);
     const float* in = static_cast<const float*>(p.in);
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
 
@@ -800,25 +800,38 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                     }
                 }
             };
-            // first pass transposed: dL/dU planes [y][u] into cells [v][u]
-            auto mid_transpose = [&](const float4* src, float4* dst, int planes, bool add) {
-                for (int c = tid; c < planes * gplane; c += nthr) {
-                    const int r = div_nu(c), u = c - r * NU;
-                    const int pw = div_nv(r), v = r - pw * NV;
-                    const float4 o4 = add ? dst[c] : zero4;
-                    float2 lo = lo2(o4), hi = hi2(o4);
+            // first pass transposed: dL/dU planes [y][u] into cells [v][u]. One thread takes
+            // a column of rows; their first tap cell steps by 0 or 1, so a window of four
+            // cells slides along and every cell is written by one thread (testing all rows
+            // for every cell took 15 % of the kernel).
+            auto mid_transpose = [&](const float4* src, float4* dst, int planes) {
+                for (int c = tid; c < planes * NQ * NU; c += nthr) {
+                    const int pw = div_nu(c), u = c - pw * NU;
                     const float4* col = src + pw * TY * NU + u;
-#pragma unroll 4
+                    float4* cell = dst + (pw * NV + s_base[0]) * NU + u;
+                    float2 l0 = make_float2(0.f, 0.f), h0 = l0, l1 = l0, h1 = l0, l2 = l0, h2 = l0, l3 = l0, h3 = l0;
+                    auto flush = [&]() {
+                        const float4 o4 = *cell;
+                        *cell = make_float4(o4.x + l0.x, o4.y + l0.y, o4.z + h0.x, o4.w + h0.y);
+                        cell += NU;
+                        l0 = l1, h0 = h1, l1 = l2, h1 = h2, l2 = l3, h2 = h3;
+                        l3 = h3 = make_float2(0.f, 0.f);
+                    };
+                    int b = s_base[0];
                     for (int y = 0; y < TY; ++y) {
-                        const int k = v - s_base[y];
-                        if ((unsigned)k < 4u) {
-                            const float2 wk = dup(s_weight[y * 4 + k]);
-                            const float4 g = col[y * NU];
-                            lo = fma2(wk, lo2(g), lo);
-                            hi = fma2(wk, hi2(g), hi);
+                        if (s_base[y] != b) {
+                            ++b;
+                            flush();
                         }
+                        const float4 w = *reinterpret_cast<const float4*>(s_weight + y * 4);
+                        const float4 g = col[y * NU];
+                        const float2 gl = lo2(g), gh = hi2(g);
+                        l0 = fma2(dup(w.x), gl, l0), h0 = fma2(dup(w.x), gh, h0);
+                        l1 = fma2(dup(w.y), gl, l1), h1 = fma2(dup(w.y), gh, h1);
+                        l2 = fma2(dup(w.z), gl, l2), h2 = fma2(dup(w.z), gh, h2);
+                        l3 = fma2(dup(w.w), gl, l3), h3 = fma2(dup(w.w), gh, h3);
                     }
-                    dst[c] = make_float4(lo.x, lo.y, hi.x, hi.y);
+                    for (int k = 0; k < 4; ++k) flush();
                 }
             };
             // the tile rows' first tap cell and weights for a ring value of the mid axis
@@ -835,12 +848,22 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                 __syncthreads();  // gt built / the previous group's dL/dU folded into the cells
                 row_table(__float_as_int(grp.x));
                 __syncthreads();
-                for (int c = tid; c < 3 * uplane; c += nthr) {
-                    const int r = div_nu(c), u = c - r * NU;
-                    const int pw = div_ty(r), y = r - pw * TY;
-                    ut4[c] = filter_rows(*reinterpret_cast<const float4*>(s_weight + y * 4),
-                                         gt + (pw * NV + s_base[y]) * NU + u, NU);
-                    gu[c] = zero4;
+                // first pass, a column of rows to a thread as above
+                for (int c = tid; c < 3 * NQ * NU; c += nthr) {
+                    const int pw = div_nu(c), u = c - pw * NU;
+                    int b = s_base[0];
+                    const float4* src = gt + (pw * NV + b) * NU + u;
+                    float4 c0 = src[0], c1 = src[NU], c2 = src[2 * NU], c3 = src[3 * NU];
+                    for (int y = 0; y < TY; ++y) {
+                        if (s_base[y] != b) {
+                            ++b;
+                            src += NU;
+                            c0 = c1, c1 = c2, c2 = c3, c3 = src[3 * NU];
+                        }
+                        const int at = (pw * TY + y) * NU + u;
+                        ut4[at] = filter_cells(*reinterpret_cast<const float4*>(s_weight + y * 4), c0, c1, c2, c3);
+                        gu[at] = zero4;
+                    }
                 }
                 __syncthreads();
                 for (int pi = __float_as_int(grp.y); pi < __float_as_int(grp.z); ++pi) {
@@ -973,7 +996,7 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                     x_transpose(gZ, xv, mask, gu + pc * uplane, true);
                 }
                 __syncthreads();
-                mid_transpose(gu, gg, 3, true);
+                mid_transpose(gu, gg, 3);
             }
             // intensity at the subvoxel centre: the same passes with ring value 0
             {
@@ -996,9 +1019,10 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                 }
                 __syncthreads();  // the last group's dL/dU is folded into the cells
                 row_table(p.zero_m);
+                for (int c = tid; c < gplane; c += nthr) icell[c] = zero4;
                 x_transpose(gW, p.zero_x, p.zero_xoff, gu, false);
                 __syncthreads();
-                mid_transpose(gu, icell, 1, false);
+                mid_transpose(gu, icell, 1);
             }
             __syncthreads();
             // stencil transpose onto the input tile positions, then into dL/dI'. Cells

@@ -145,13 +145,16 @@ __device__ __forceinline__ void filter4(float4 w, const float4* src, float (&r)[
     r[2] = fmaf(w.w, u3.z, fmaf(w.z, u2.z, fmaf(w.y, u1.z, w.x * u0.z)));
     r[3] = fmaf(w.w, u3.w, fmaf(w.z, u2.w, fmaf(w.y, u1.w, w.x * u0.w)));
 }
-// Four taps along the tile's mid axis (rows src, src + stride, ..), four cells at once.
-__device__ __forceinline__ float4 filter_rows(float4 w, const float4* src, int stride) {
-    const float4 c0 = src[0], c1 = src[stride], c2 = src[2 * stride], c3 = src[3 * stride];
+// Four taps, four cells of the innermost axis at once.
+__device__ __forceinline__ float4 filter_cells(float4 w, float4 c0, float4 c1, float4 c2, float4 c3) {
     const float2 w0 = dup(w.x), w1 = dup(w.y), w2 = dup(w.z), w3 = dup(w.w);
     const float2 l = fma2(w3, lo2(c3), fma2(w2, lo2(c2), fma2(w1, lo2(c1), mul2(w0, lo2(c0)))));
     const float2 h = fma2(w3, hi2(c3), fma2(w2, hi2(c2), fma2(w1, hi2(c1), mul2(w0, hi2(c0)))));
     return make_float4(l.x, l.y, h.x, h.y);
+}
+// The same along the tile's mid axis (rows src, src + stride, ..).
+__device__ __forceinline__ float4 filter_rows(float4 w, const float4* src, int stride) {
+    return filter_cells(w, src[0], src[stride], src[2 * stride], src[3 * stride]);
 }
 // Cell w of a column into the packed halves (compile-time w).
 template <int CH, int NH>
