@@ -1549,7 +1549,7 @@ int rfba_ctx_destroy(rfba_ctx* c) {
     cudaSetDevice(c->device);
     for (DevBuf* b : {&c->in, &c->out, &c->rad, &c->inten, &c->blocks, &c->tiles, &c->tables, &c->counter, &c->prefix,
                       &c->shifted, &c->tmp1, &c->tmp2, &c->gS, &c->gI, &c->gin, &c->dshift, &c->ablocks, &c->atiles,
-                      &c->acounter, &c->asamples, &c->errw, &c->tb_val, &c->tb_der, &c->tb_em, &c->tb_res, &c->tb_par, &c->tb_bg,
+                      &c->acounter, &c->asamples, &c->errw, &c->tb_val, &c->tb_der, &c->tb_em, &c->tb_res, &c->tb_bg,
                       &c->tb_pix, &c->tb_pixels, &c->tb_dfd, &c->tb_vdf, &c->seed_w, &c->seed_sums, &c->seed_carry, &c->seed_map, &c->seed_vox,
                       &c->seed_xyz, &c->gb_pix, &c->gb_pixels, &c->gb_par, &c->hs_tab, &c->hs_part, &c->hs_gg, &c->hs_phi,
                       &c->hs_frame, &c->hs_out, &c->tstate})

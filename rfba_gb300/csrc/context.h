@@ -187,7 +187,7 @@ struct rfba_ctx {
     // spot seeding scratch
     rfba::DevBuf seed_w, seed_sums, seed_carry, seed_map, seed_vox, seed_xyz;
     // 3B spot-gradient scratch
-    rfba::DevBuf tb_val, tb_der, tb_em, tb_res, tb_par, tb_bg, tb_pix, tb_pixels, tb_dfd, tb_vdf;
+    rfba::DevBuf tb_val, tb_der, tb_em, tb_res, tb_bg, tb_pix, tb_pixels, tb_dfd, tb_vdf;
     // 3B Gibbs sampler scratch
     rfba::DevBuf gb_pix, gb_pixels, gb_par;
     rfba::GibbsScratch gb[2];  // one set per chain run side by side

@@ -380,10 +380,12 @@ int launch_hessian_parts(const HessParams& h, bool samples_hold_spot, void* stre
 
 // 3B spot gradient (threeb.cu): spot voxel table, emission sums per (sample,
 // frame), forward algorithm per sample; res[s] = (gradient[5], log probability).
-int launch_threeb(const double* bg, const double* pix, const int* pixels, int S, int F, int P, const double* phi_dev,
-                  double zf, double variance, double c0, const double* A_dev, const double* pi_dev,
-                  double* val, double* der, double* em, double* res, const float2* dfd, float2* vdf,
-                  void* stream);
+struct ThreeBPar {
+    double phi[5], A[9], pi[3];  // the spot, the transitions (row-major), the start
+};
+int launch_threeb(const double* bg, const double* pix, const int* pixels, int S, int F, int P, const ThreeBPar& par,
+                  double zf, double variance, double c0, double* val, double* der, double* em, double* res,
+                  const float2* dfd, float2* vdf, void* stream);
 // The samples' residuals (data minus background) as double-floats [S][F][P],
 // for the gradient-only evaluations of launch_threeb (dfd; vdf is [P][6]).
 int launch_threeb_residual(const double* bg, const double* pix, int S, int F, int P, float2* dfd, void* stream);

@@ -7,7 +7,8 @@
 // (RFBA Main/multispot5.cc:616-664). Four kernels:
 //   1. spot_pixels_kernel: the spot's intensity and its parameter derivative
 //      at every mask voxel (spot_shape_diff_position, storm.h:51-84);
-//   2. spot_sums_kernel: the spot's sums over the mask (sum v^2, sum der v);
+//   2. spot_scan_kernel: the spot's sums over the mask (sum v^2, sum der v), and
+//      its support's indices for the double-float path;
 //   3. emission_kernel, one CTA per (sample, frame): the frame's log
 //      probability with the spot on and off and the derivative of the "on" one
 //      (SpotWithBackground, spot_with_background.hh:98-133), reduced over the
@@ -34,7 +35,7 @@
 // 2^-46 relative per operation, four samples of a frame per CTA so the spot's
 // table is read once per four, over the spot's support only (the pixels where
 // its Gaussian factor is at least 2^-60, listed in pixel order by
-// support_compact_kernel); forward_df_kernel runs the recursion in
+// spot_scan_kernel); forward_df_kernel runs the recursion in
 // double-float too. The FP64 pipe, 1/64 of the FP32 one here, would otherwise
 // bound every evaluation. The log-probability path keeps the FP64 sums over
 // every pixel.
@@ -55,9 +56,13 @@ constexpr double kSupportS = -41.58883083359672;  // ln(2^-60)
 
 using namespace dfloat;
 
-constexpr int kPixThreads = 256;
+// One pixel a thread, about 150 FP64 operations each, on a pipe of 2 lanes a cycle
+// and SM: bound by that pipe on the SMs that have work, so the blocks are small
+// enough to reach all of them (24,389 pixels are 382 blocks; as 96 blocks of 256 on
+// 152 SMs they took 14 us). Each warp leaves its share of the spot's sums.
+constexpr int kPixThreads = 64;
 __global__ void __launch_bounds__(kPixThreads) spot_pixels_kernel(const int* __restrict__ pixels, int P,
-                                                                   const double* __restrict__ phi_in, double zf,
+                                                                   const __grid_constant__ ThreeBPar par, double zf,
                                                                    double* __restrict__ val, double* __restrict__ der,
                                                                    float2* __restrict__ vdf,
                                                                    double* __restrict__ partial,
@@ -65,7 +70,7 @@ __global__ void __launch_bounds__(kPixThreads) spot_pixels_kernel(const int* __r
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     double acc[6] = {0, 0, 0, 0, 0, 0};  // this pixel's v^2 and der_n v
     if (p < P) {
-        const double phi0 = phi_in[0], phi1 = phi_in[1], phi2 = phi_in[2], phi3 = phi_in[3], phi4 = phi_in[4];
+        const double phi0 = par.phi[0], phi1 = par.phi[1], phi2 = par.phi[2], phi3 = par.phi[3], phi4 = par.phi[4];
         const double x0 = pixels[3 * p], x1 = pixels[3 * p + 1], x2 = pixels[3 * p + 2];
         const double d0 = x0 - phi2, d1 = x1 - phi3, d2 = (x2 - phi4) / zf;
         const double s = -(d0 * d0 + d1 * d1 + d2 * d2) / (2 * phi1 * phi1);
@@ -92,20 +97,13 @@ __global__ void __launch_bounds__(kPixThreads) spot_pixels_kernel(const int* __r
 #pragma unroll
         for (int n = 0; n < kM; ++n) acc[1 + n] = d[n] * v;
     }
-    // the block's share of the spot's sums, in a fixed order
+    // the warp's share of the spot's sums, in a fixed order
 #pragma unroll
     for (int i = 0; i < 6; ++i)
         for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_down_sync(0xffffffffu, acc[i], o);
-    __shared__ double part[kPixThreads / 32][6];
     if ((threadIdx.x & 31) == 0)
 #pragma unroll
-        for (int i = 0; i < 6; ++i) part[threadIdx.x >> 5][i] = acc[i];
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        double t = 0;
-        for (int w = 0; w < kPixThreads / 32; ++w) t += part[w][threadIdx.x];
-        partial[(size_t)blockIdx.x * 6 + threadIdx.x] = t;
-    }
+        for (int i = 0; i < 6; ++i) partial[(size_t)(p >> 5) * 6 + i] = acc[i];
 }
 
 // The samples' residuals, data minus background, as double-floats [S][F][P].
@@ -117,25 +115,46 @@ __global__ void residual_df_kernel(const double* __restrict__ bg, const double* 
     out[i] = df_from(pix[fp] - bg[i]);
 }
 
-// The spot's own sums over the mask, sum v^2 and sum der_n v, from the
-// blocks' partial sums in block order (one thread per sum): with d = I - G,
-// sum (d - v)^2 = sum d^2 - 2 sum d v + sum v^2 and sum der_n (d - v) =
+// Block 0, the spot's own sums over the mask, sum v^2 and sum der_n v, from the
+// warps' partial sums, eight warps (kSumGroup) in order and then the groups in order:
+// with d = I - G, sum (d - v)^2 = sum d^2 - 2 sum d v + sum v^2 and sum der_n (d - v) =
 // sum der_n d - sum der_n v, so the per-(sample, frame) pass needs 8 FP64
-// operations per voxel instead of 10.
-__global__ void spot_sums_kernel(const double* __restrict__ partial, int nblocks, double* __restrict__ sums) {
-    if (threadIdx.x >= 6) return;
-    double t = 0;
-    for (int b = 0; b < nblocks; ++b) t += partial[(size_t)b * 6 + threadIdx.x];
-    sums[threadIdx.x] = t;
-}
-
-// The support's pixel indices in pixel order (one CTA): each thread counts a
-// contiguous run of flags, a block-wide exclusive scan places the runs, and
-// the indices are written in order; count[0] = the support's size.
+// operations per voxel instead of 10. Block 1, the support's pixel indices in pixel
+// order: each thread counts a contiguous run of flags, a block-wide exclusive scan
+// places the runs, and the indices are written in order; count[0] = the support's
+// size. The two are independent: one after the other as two launches they took 8.5
+// and 6.2 us of an evaluation's 106 at 24,389 pixels.
 constexpr int kScanThreads = 1024;
-__global__ void __launch_bounds__(kScanThreads) support_compact_kernel(const unsigned char* __restrict__ flag, int P,
-                                                                        int* __restrict__ idx,
-                                                                        int* __restrict__ count) {
+constexpr int kSumGroup = 8;
+constexpr int kSumChunk = kScanThreads / 6;  // groups a pass
+__global__ void __launch_bounds__(kScanThreads) spot_scan_kernel(const double* __restrict__ partial, int nwarps,
+                                                                  double* __restrict__ sums,
+                                                                  const unsigned char* __restrict__ flag, int P,
+                                                                  int* __restrict__ idx, int* __restrict__ count) {
+    if (blockIdx.x == 0) {
+        __shared__ double part[kSumChunk * 6];
+        const int ngroups = (nwarps + kSumGroup - 1) / kSumGroup;
+        double total = 0;
+        for (int g0 = 0; g0 < ngroups; g0 += kSumChunk) {
+            const int n = min(kSumChunk, ngroups - g0) * 6;
+            if (threadIdx.x < n) {
+                const int w0 = (g0 + threadIdx.x / 6) * kSumGroup;
+                double v[kSumGroup], t = 0;
+#pragma unroll
+                for (int w = 0; w < kSumGroup; ++w)
+                    v[w] = w0 + w < nwarps ? partial[(size_t)(w0 + w) * 6 + threadIdx.x % 6] : 0.0;
+#pragma unroll
+                for (int w = 0; w < kSumGroup; ++w) t += v[w];
+                part[threadIdx.x] = t;
+            }
+            __syncthreads();
+            if (threadIdx.x < 6)
+                for (int i = threadIdx.x; i < n; i += 6) total += part[i];
+            __syncthreads();
+        }
+        if (threadIdx.x < 6) sums[threadIdx.x] = total;
+        return;
+    }
     const int per = (P + kScanThreads - 1) / kScanThreads;
     const int p0 = min(P, threadIdx.x * per), p1 = min(P, p0 + per);
     int n = 0;
@@ -359,8 +378,9 @@ __device__ __forceinline__ double pow2i(int d) {  // 2^d for -1022 <= d <= 1023
 }
 
 __global__ void __launch_bounds__(32) forward_kernel(const double* __restrict__ em, int S, int F,
-                                                      const double* __restrict__ A9,
-                                                      const double* __restrict__ pi3, double* __restrict__ res) {
+                                                      const __grid_constant__ ThreeBPar par,
+                                                      double* __restrict__ res) {
+    const double *A9 = par.A, *pi3 = par.pi;
     const int s = blockIdx.x;
     const int lane = threadIdx.x;
     const int l = lane % 18;
@@ -460,8 +480,9 @@ __global__ void __launch_bounds__(32) forward_kernel(const double* __restrict__ 
 // largest exponent among the states that reach j, terms more than 2^100 below
 // it dropped (below the format's precision).
 __global__ void __launch_bounds__(32) forward_df_kernel(const EmDf* __restrict__ em, int S, int F,
-                                                         const double* __restrict__ A9, const double* __restrict__ pi3,
+                                                         const __grid_constant__ ThreeBPar par,
                                                          double* __restrict__ res) {
+    const double *A9 = par.A, *pi3 = par.pi;
     const int s = blockIdx.x;
     const int lane = threadIdx.x;
     const int l = lane % 18;
@@ -581,30 +602,29 @@ int launch_threeb_residual(const double* bg, const double* pix, int S, int F, in
     return (int)cudaGetLastError();
 }
 
-int launch_threeb(const double* bg, const double* pix, const int* pixels, int S, int F, int P, const double* phi_dev,
-                  double zf, double variance, double c0, const double* A_dev, const double* pi_dev,
-                  double* val, double* der, double* em, double* res, const float2* dfd, float2* vdf, void* stream) {
+int launch_threeb(const double* bg, const double* pix, const int* pixels, int S, int F, int P, const ThreeBPar& par,
+                  double zf, double variance, double c0, double* val, double* der, double* em, double* res, const float2* dfd, float2* vdf, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nblk = (P + kPixThreads - 1) / kPixThreads;
-    double* sums = res + (size_t)S * 6;  // 6 doubles after the per-sample results, then the blocks' partials
+    double* sums = res + (size_t)S * 6;  // 6 doubles after the per-sample results, then the warps' partials
     // the double-float path's support flags and list share the table's buffer:
     // vdf [P][6] float2, then P flag bytes, then the P indices and the count
     unsigned char* flag = dfd ? reinterpret_cast<unsigned char*>(vdf + (size_t)P * 6) : nullptr;
     int* sup = dfd ? reinterpret_cast<int*>(flag + (((size_t)P + 15) & ~(size_t)15)) : nullptr;
-    spot_pixels_kernel<<<nblk, kPixThreads, 0, st>>>(pixels, P, phi_dev, zf, val, der, dfd ? vdf : nullptr,
+    spot_pixels_kernel<<<nblk, kPixThreads, 0, st>>>(pixels, P, par, zf, val, der, dfd ? vdf : nullptr,
                                                      sums + 6, flag);
-    spot_sums_kernel<<<1, 32, 0, st>>>(sums + 6, nblk, sums);
+    spot_scan_kernel<<<dfd ? 2 : 1, kScanThreads, 0, st>>>(sums + 6, nblk * (kPixThreads / 32), sums, flag, P, sup,
+                                                             sup + P);
     if (dfd) {
-        support_compact_kernel<<<1, kScanThreads, 0, st>>>(flag, P, sup, sup + P);
         EmDf* emd = reinterpret_cast<EmDf*>(em);  // 64 B per (sample, frame), within the FP64 path's 80
         emission_df_kernel<<<dim3((unsigned)F, (unsigned)((S + kDfTile - 1) / kDfTile)), kEmitThreads, 0, st>>>(
             dfd, vdf, sup, sup + P, sums, S, F, P, 2 * variance, variance, emd);
-        forward_df_kernel<<<S, 32, 0, st>>>(emd, S, F, A_dev, pi_dev, res);
+        forward_df_kernel<<<S, 32, 0, st>>>(emd, S, F, par, res);
         return (int)cudaGetLastError();
     }
     emission_kernel<<<(unsigned)((long long)S * F), kEmitThreads, 0, st>>>(bg, pix, val, der, sums, F, P,
                                                                            2 * variance, variance, c0, em);
-    forward_kernel<<<S, 32, 0, st>>>(em, S, F, A_dev, pi_dev, res);
+    forward_kernel<<<S, 32, 0, st>>>(em, S, F, par, res);
     return (int)cudaGetLastError();
 }
 

@@ -59,8 +59,7 @@ static int threeb_stage(rfba_ctx* ctx, const double* sample_bg, const double* pi
     int s;
     const size_t nbg = (size_t)S * F * P, npix = (size_t)F * P;
     if ((s = ctx->tb_val.ensure((size_t)P * 8, "3B spot table")) || (s = ctx->tb_der.ensure((size_t)P * 40, "3B spot table")) ||
-        (s = ctx->tb_em.ensure((size_t)S * F * 80, "3B emissions")) || (s = ctx->tb_res.ensure((size_t)S * 48 + 48 + (size_t)(P / 256 + 1) * 48, "3B results")) ||
-        (s = ctx->tb_par.ensure(17 * 8, "3B parameters")))
+        (s = ctx->tb_em.ensure((size_t)S * F * 80, "3B emissions")) || (s = ctx->tb_res.ensure((size_t)S * 48 + 48 + (size_t)(P / 32 + 2) * 48, "3B results")))
         return s;
     d->bg = sample_bg;
     d->pix = pixel_intensities;
@@ -96,16 +95,13 @@ static int threeb_stage(rfba_ctx* ctx, const double* sample_bg, const double* pi
 static int threeb_eval(rfba_ctx* ctx, const rfba_3b_model* m, const ThreeBData& d, const double* spot, double* out,
                        double* log_prob, cudaStream_t st) {
     const int S = d.S, F = d.F, P = d.P;
-    // parameters: spot, A (row-major), pi
-    double par[17];
-    for (int n = 0; n < 5; ++n) par[n] = spot[n];
-    for (int n = 0; n < 9; ++n) par[5 + n] = m->A[n];
-    for (int n = 0; n < 3; ++n) par[14 + n] = m->pi[n];
-    RFBA_CUDA(cudaMemcpyAsync(ctx->tb_par.p, par, sizeof par, cudaMemcpyHostToDevice, st), "parameter upload");
+    ThreeBPar par;
+    for (int n = 0; n < 5; ++n) par.phi[n] = spot[n];
+    for (int n = 0; n < 9; ++n) par.A[n] = m->A[n];
+    for (int n = 0; n < 3; ++n) par.pi[n] = m->pi[n];
     const unsigned int n_pix = (unsigned int)P;
     const double c0 = n_pix * ::log(2 * M_PI * m->variance) / 2;  // spot_with_background.hh:126-127
-    const double* dpar = static_cast<const double*>(ctx->tb_par.p);
-    int e = launch_threeb(d.bg, d.pix, d.pixels, S, F, P, dpar, m->z_factor, m->variance, c0, dpar + 5, dpar + 14,
+    int e = launch_threeb(d.bg, d.pix, d.pixels, S, F, P, par, m->z_factor, m->variance, c0,
                           static_cast<double*>(ctx->tb_val.p), static_cast<double*>(ctx->tb_der.p),
                           static_cast<double*>(ctx->tb_em.p), static_cast<double*>(ctx->tb_res.p),
                           log_prob ? nullptr : d.dfd, static_cast<float2*>(ctx->tb_vdf.p), st);

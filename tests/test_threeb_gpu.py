@@ -156,3 +156,19 @@ def test_golden_gradient_and_optimiser(ctx):
         x, it, ev = ctx.optimise_spot_3b(_model(1.0, 1.0), c["bg"], c["pix"], c["px"], c["spot"], _limit(),
                                          int(c["iters"]))
         np.testing.assert_allclose(x, c["opt"], rtol=1e-6, atol=1e-8)
+
+
+@pytest.mark.parametrize("n", [1, 32, 33, 255, 256, 257, 8705, 43520, 43521])
+def test_spot_sums_at_the_edges_of_their_groups(ctx, n):
+    """The spot's own sums are left per warp (32 pixels), added eight warps
+    at a time and 170 groups a pass (43,520 pixels), and the support's list is
+    written beside them: masks of one pixel, of whole and broken warps and
+    groups, and of more than one pass, on both paths and to the bounds above."""
+    bg, pix, px, spot = T.synthetic_block(11, 2, 3, (29, 39, 39))
+    near = np.sort(np.argsort(((px - spot[2:]) ** 2).sum(1), kind="stable")[:n])
+    bg, pix, px = (np.ascontiguousarray(a) for a in (bg[..., near], pix[..., near], px[near]))
+    want, lpw = T.spot_neg_prob_diff(bg, pix, px, spot, with_logp=True)
+    got, lp = ctx.spot_gradient_3b(_model(1.0, 1.0), bg, pix, px, spot)
+    _compare(got, lp, want, lpw)
+    got, _ = ctx.spot_gradient_3b(_model(1.0, 1.0), bg, pix, px, spot, want_log_prob=False)
+    assert np.max(np.abs(got - want)) <= 1e-9 * np.max(np.abs(want)), (got, want)
