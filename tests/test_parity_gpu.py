@@ -115,3 +115,17 @@ def test_sub_regions_match_whole(ctx, oracle_mod):
     ref = whole[7:13, 5:17, 3:21]
     assert np.array_equal(np.isnan(sub), np.isnan(ref))
     assert np.array_equal(np.nan_to_num(sub), np.nan_to_num(ref))
+
+
+@pytest.mark.parametrize("order,T", [(2, 1), (2, 2), (2, 7), (2, 8), (2, 9), (3, 3), (3, 4), (3, 28), (4, 4), (4, 5),
+                                     (4, 17), (4, 96), (2, 454), (4, 454), (3, 455)])
+@pytest.mark.parametrize("iw", [0, 1])
+def test_itc_series_lengths(ctx, oracle_mod, order, T, iw):
+    """ITC 1 with each series in a column of shared memory: series at and about
+    the order, about the eight volumes a load batch takes, of the longest column
+    (454 volumes) and one longer, which is binned in place; to the cases' bound."""
+    cfg, oc = _cfg_pair(mag=(2, 2, 1), method=3, itc=1, trac_order=order, intensity_w=iw, gradient_smooth=1, x_range=1,
+                        y_range=1, z_range=1)
+    x = _series(300 + T, T, 6, 7, 6)
+    ref = oracle_mod.srrf_region(x.astype(np.float32), oc)
+    assert_parity(ctx.forward(cfg, x), ref, tol_for(cfg.method), f"order {order}, {T} volumes")
