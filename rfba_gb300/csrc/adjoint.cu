@@ -54,52 +54,69 @@ __device__ __forceinline__ float dcr(float xx) {
 }
 
 // ---------------------------------------------------------------------------
-// Drift operator, one axis: mode 0 resamples, mode 1 resamples with derivative
-// weights, mode 2 applies the transpose (gather over the outputs whose clamped
-// taps hit each input position).
-__global__ void shift_axis_kernel(const float* __restrict__ src, float* __restrict__ dst, int W, int H, int D, int T,
-                                  int axis, const float* __restrict__ shifts, int mode, unsigned long long* err) {
-    const long long n = (long long)W * H * D * T;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % W);
-        const int y = (int)((i / W) % H);
-        const int z = (int)((i / ((long long)W * H)) % D);
-        const int t = (int)(i / ((long long)W * H * D));
-        const int len = axis == 0 ? W : (axis == 1 ? H : D);
-        const long long stride = axis == 0 ? 1 : (axis == 1 ? W : (long long)W * H);
-        const int c = axis == 0 ? x : (axis == 1 ? y : z);
-        const long long line = i - (long long)c * stride;
-        const float d = shifts[3 * t + axis];
-        float acc = 0.f;
-        if (mode != 2) {
-            const float pos = (float)c + d;
-            const int base = (int)floorf(pos);
+// Transpose of the drift operator on one axis: a gather over the outputs whose
+// clamped taps hit each input position. Away from the axis's ends an output xo hits
+// position c with one tap, c - floor(xo + d), so at most eight outputs in a row are
+// looked at and one weight formed for each; at the ends, where clamped taps pile up,
+// every output's four taps are tried. One warp a row (t, z, y) with x across its
+// lanes, so y's and z's weights are formed once a row. 60 volumes of 64^3, per axis:
+// x 0.22, y 0.13, z 0.13 ms against 0.35 when each voxel divided its index in 64 bits
+// and formed the weight of each of the 28 pairs of output and tap; floor 0.02.
+__device__ __forceinline__ float end_weight(int xo, float d, int c, int len) {
+    const float pos = (float)xo + d;
+    const int base = (int)floorf(pos);
+    float w = 0.f;
 #pragma unroll
-            for (int k = -1; k <= 2; ++k) {
-                const int ii = clampi(base + k, 0, len - 1);
-                const float u = pos - (float)(base + k);
-                const long long si = line + ii * stride;
-                if (in_range(si, n, err, 1)) acc = fmaf(mode == 1 ? dcr(u) : cr(u), src[si], acc);
-            }
-        } else {
-            // outputs x whose taps floor(x + d) - 1 .. + 2, clamped, include c
-            int lo = (int)floorf((float)c - d) - 3, hi = (int)ceilf((float)c - d) + 3;
-            if (c == 0) lo = -1000000;
-            if (c == len - 1) hi = 1000000;
-            lo = max(lo, 0);
-            hi = min(hi, len - 1);
-            for (int xo = lo; xo <= hi; ++xo) {
+    for (int k = -1; k <= 2; ++k)
+        if (clampi(base + k, 0, len - 1) == c) w += cr(pos - (float)(base + k));
+    return w;
+}
+template <int AXIS>
+__global__ void __launch_bounds__(256) shift_adjoint_kernel(const float* __restrict__ src, float* __restrict__ dst,
+                                                            int W, int H, int D, int T,
+                                                            const float* __restrict__ shifts) {
+    const int lane = threadIdx.x & 31;
+    const long long rows = (long long)D * H, stride = AXIS == 0 ? 1 : (AXIS == 1 ? W : (long long)W * H);
+    const int len = AXIS == 0 ? W : (AXIS == 1 ? H : D);
+    for (long long r = blockIdx.x * 8LL + (threadIdx.x >> 5); r < rows * T; r += gridDim.x * 8LL) {
+        const int t = (int)(r / rows), zy = (int)(r - t * rows);
+        const int z = zy / H, y = zy - z * H;
+        const float d = shifts[3 * t + AXIS];
+        constexpr int N = 8;
+        float w[N];
+        int first = 0;
+        auto weights = [&](int c) {
+            first = (int)floorf((float)c - d) - 3;
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                const int xo = (int)((unsigned)first + j);
                 const float pos = (float)xo + d;
-                const int base = (int)floorf(pos);
-                float w = 0.f;
-#pragma unroll
-                for (int k = -1; k <= 2; ++k)
-                    if (clampi(base + k, 0, len - 1) == c) w += cr(pos - (float)(base + k));
-                const long long si = line + xo * stride;
-                if (w != 0.f && in_range(si, n, err, 2)) acc = fmaf(w, src[si], acc);
+                const int k = c - (int)floorf(pos);
+                w[j] = xo >= 0 && xo < len && k >= -1 && k <= 2 ? cr(pos - (float)c) : 0.f;
             }
+        };
+        const int c0 = AXIS == 1 ? y : z;
+        if (AXIS != 0) weights(c0);
+        for (int x = lane; x < W; x += 32) {
+            const int c = AXIS == 0 ? x : c0;
+            const long long i = r * W + x;
+            const float* line = src + (i - c * stride);
+            float acc = 0.f;
+            if (c > 0 && c < len - 1) {
+                if (AXIS == 0) weights(c);
+#pragma unroll
+                for (int j = 0; j < N; ++j)
+                    if (w[j] != 0.f) acc = fmaf(w[j], __ldg(line + (first + j) * stride), acc);
+            } else {
+                const int lo = c == 0 ? 0 : max((int)floorf((float)c - d) - 3, 0);
+                const int hi = c == len - 1 ? len - 1 : min((int)ceilf((float)c - d) + 3, len - 1);
+                for (int xo = lo; xo <= hi; ++xo) {
+                    const float we = end_weight(xo, d, c, len);
+                    if (we != 0.f) acc = fmaf(we, __ldg(line + xo * stride), acc);
+                }
+            }
+            dst[i] = acc;
         }
-        dst[i] = acc;
     }
 }
 
@@ -126,77 +143,108 @@ __global__ void drift_dot_kernel(const float* __restrict__ g, const float* __res
 // per-axis index clamping compose to one 4 x 4 x 4 tensor-product stencil with
 // clamped indices. mode 0 writes I'_t; mode 1 adds, per volume, the sums over
 // voxels of g * dI'/dd_a (a = x, y, z: derivative weights on axis a) into
-// out[3 t + a] (FP64, one atomic per block and axis).
+// out[3 t + a] (FP64, one atomic per block and axis). A warp takes 32 columns of x
+// at one y and walks L planes of z, keeping the last four planes' x- and y-passes in
+// registers: a step reads one plane's 16 taps instead of four planes' 64. The
+// passes and their sums are the stencil's. Bound by the taps' load instructions: 60
+// volumes of 64^3 take 0.17 ms (mode 0) and 0.43 (mode 1), 0.56 and 0.82 with all 64
+// taps a voxel.
+constexpr int kDriftThreads = 256;
 template <int MODE>
-__global__ void drift3d_kernel(const float* __restrict__ src, float* __restrict__ dst, const float* __restrict__ g,
-                               int W, int H, int D, const float* __restrict__ shifts, double* __restrict__ out) {
+__global__ void __launch_bounds__(kDriftThreads) drift3d_kernel(const float* __restrict__ src, float* __restrict__ dst,
+                                                                const float* __restrict__ g, int W, int H, int D,
+                                                                int L, const float* __restrict__ shifts,
+                                                                double* __restrict__ out) {
     const int t = blockIdx.y;
     const long long nv = (long long)W * H * D;
     const float* st = src + (long long)t * nv;
     const float dx = shifts[3 * t], dy = shifts[3 * t + 1], dz = shifts[3 * t + 2];
     double acc[3] = {0.0, 0.0, 0.0};
-    // one (z, y) output row per block iteration, x across the threads; every
-    // index is clamped into the volume, so no tap can leave it
-    for (int row = blockIdx.x; row < D * H; row += gridDim.x) {
-        const int z = row / H, y = row - z * H;
-        const float py = (float)y + dy, pz = (float)z + dz;
-        const int by = (int)floorf(py), bz = (int)floorf(pz);
-        float wy[4], wz[4], ey[4], ez[4];
-        const float* rows[4][4];
+    const int nx = (W + 31) / 32, nz = (D + L - 1) / L;
+    // every index is clamped into the volume, so no tap can leave it
+    for (long long i = blockIdx.x * (kDriftThreads / 32LL) + (threadIdx.x >> 5); i < (long long)nx * H * nz;
+         i += gridDim.x * (kDriftThreads / 32LL)) {
+        const long long q = i / nx;
+        const int x = (int)(i - q * nx) * 32 + (threadIdx.x & 31);
+        const int y = (int)(q % H), z0 = (int)(q / H) * L;
+        if (x >= W) continue;
+        const float px = (float)x + dx, py = (float)y + dy;
+        const int bx = (int)floorf(px), by = (int)floorf(py);
+        float wx[4], ex[4], wy[4], ey[4];
+        long long ty[4];  // a tap's row in a plane
+        int ix[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
+            wx[k] = cr(px - (float)(bx + k - 1));
             wy[k] = cr(py - (float)(by + k - 1));
-            wz[k] = cr(pz - (float)(bz + k - 1));
             if (MODE == 1) {
+                ex[k] = dcr(px - (float)(bx + k - 1));
                 ey[k] = dcr(py - (float)(by + k - 1));
-                ez[k] = dcr(pz - (float)(bz + k - 1));
             }
+            ty[k] = (long long)clampi(by + k - 1, 0, H - 1) * W;
+            ix[k] = clampi(bx + k - 1, 0, W - 1);
         }
-#pragma unroll
-        for (int kz = 0; kz < 4; ++kz)
+        // a plane's x pass per row, then its y pass
+        float s[4], s_dx[4], s_dy[4];
+        auto plane = [&](int z, int k) {
+            const float* rp = st + (long long)clampi(z, 0, D - 1) * H * W;
+            float v[4][4];
 #pragma unroll
             for (int ky = 0; ky < 4; ++ky)
-                rows[kz][ky] = st + ((long long)clampi(bz + kz - 1, 0, D - 1) * H + clampi(by + ky - 1, 0, H - 1)) * W;
-        for (int x = threadIdx.x; x < W; x += blockDim.x) {
-            const float px = (float)x + dx;
-            const int bx = (int)floorf(px);
-            float wx[4], ex[4];
-            int ix[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                ix[k] = clampi(bx + k - 1, 0, W - 1);
-                wx[k] = cr(px - (float)(bx + k - 1));
-                if (MODE == 1) ex[k] = dcr(px - (float)(bx + k - 1));
+                for (int kx = 0; kx < 4; ++kx) v[ky][kx] = __ldg(rp + ty[ky] + ix[kx]);
+            float sy = 0.f, sy_dx = 0.f, sy_dy = 0.f;
+#pragma unroll
+            for (int ky = 0; ky < 4; ++ky) {
+                float sx = 0.f, sx_d = 0.f;
+#pragma unroll
+                for (int kx = 0; kx < 4; ++kx) {
+                    sx = fmaf(wx[kx], v[ky][kx], sx);
+                    if (MODE == 1) sx_d = fmaf(ex[kx], v[ky][kx], sx_d);
+                }
+                sy = fmaf(wy[ky], sx, sy);
+                if (MODE == 1) {
+                    sy_dx = fmaf(wy[ky], sx_d, sy_dx);
+                    sy_dy = fmaf(ey[ky], sx, sy_dy);
+                }
             }
-            // x pass per (z, y) row, then y, then z, as the per-axis passes compose
+            s[k] = sy;
+            if (MODE == 1) {
+                s_dx[k] = sy_dx;
+                s_dy[k] = sy_dy;
+            }
+        };
+        int held = 0;
+        for (int z = z0; z < min(z0 + L, D); ++z) {
+            const float pz = (float)z + dz;
+            const int bz = (int)floorf(pz);
+            if (z == z0 || (bz != held && bz != held + 1)) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) plane(bz + k - 1, k);
+            } else if (bz != held) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    s[k] = s[k + 1];
+                    if (MODE == 1) {
+                        s_dx[k] = s_dx[k + 1];
+                        s_dy[k] = s_dy[k + 1];
+                    }
+                }
+                plane(bz + 2, 3);
+            }
+            held = bz;
             float v = 0.f, gx_ = 0.f, gy_ = 0.f, gz_ = 0.f;
 #pragma unroll
-            for (int kz = 0; kz < 4; ++kz) {
-                float sy = 0.f, sy_dx = 0.f, sy_dy = 0.f;
-#pragma unroll
-                for (int ky = 0; ky < 4; ++ky) {
-                    const float* rp = rows[kz][ky];
-                    float sx = 0.f, sx_d = 0.f;
-#pragma unroll
-                    for (int kx = 0; kx < 4; ++kx) {
-                        const float val = __ldg(rp + ix[kx]);
-                        sx = fmaf(wx[kx], val, sx);
-                        if (MODE == 1) sx_d = fmaf(ex[kx], val, sx_d);
-                    }
-                    sy = fmaf(wy[ky], sx, sy);
-                    if (MODE == 1) {
-                        sy_dx = fmaf(wy[ky], sx_d, sy_dx);
-                        sy_dy = fmaf(ey[ky], sx, sy_dy);
-                    }
-                }
-                v = fmaf(wz[kz], sy, v);
+            for (int k = 0; k < 4; ++k) {
+                const float wz = cr(pz - (float)(bz + k - 1));
+                v = fmaf(wz, s[k], v);
                 if (MODE == 1) {
-                    gx_ = fmaf(wz[kz], sy_dx, gx_);
-                    gy_ = fmaf(wz[kz], sy_dy, gy_);
-                    gz_ = fmaf(ez[kz], sy, gz_);
+                    gx_ = fmaf(wz, s_dx[k], gx_);
+                    gy_ = fmaf(wz, s_dy[k], gy_);
+                    gz_ = fmaf(dcr(pz - (float)(bz + k - 1)), s[k], gz_);
                 }
             }
-            const long long o = (long long)t * nv + (long long)row * W + x;
+            const long long o = (long long)t * nv + ((long long)z * H + y) * W + x;
             if (MODE == 0) {
                 dst[o] = v;
             } else {
@@ -208,11 +256,11 @@ __global__ void drift3d_kernel(const float* __restrict__ src, float* __restrict_
         }
     }
     if (MODE == 1) {
-        __shared__ double red[3][256];
+        __shared__ double red[3][kDriftThreads];
 #pragma unroll
         for (int a = 0; a < 3; ++a) red[a][threadIdx.x] = acc[a];
         __syncthreads();
-        for (int s2 = blockDim.x / 2; s2 > 0; s2 >>= 1) {
+        for (int s2 = kDriftThreads / 2; s2 > 0; s2 >>= 1) {
             if (threadIdx.x < s2)
 #pragma unroll
                 for (int a = 0; a < 3; ++a) red[a][threadIdx.x] += red[a][threadIdx.x + s2];
@@ -1112,7 +1160,7 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
 // 4 x 4 x 4 cells its taps reach, interpolated along x, then y, then z, the derivative
 // of the radiality term in the plain rotated frame less the one at the bound, and
 // its transpose onto the input voxels (the taps and the stencil are products over
-// the axes). 8 volumes of 64^3 take 0.1 ms beside the kernel's 4.5.
+// the axes). 60 volumes of 64^3 at mag 2 take 0.9 ms beside the kernel's 29.8.
 __global__ void __launch_bounds__(128) adjoint_samples_kernel(const __grid_constant__ FwdParams p, const AdjParams a,
                                                               const AdjFixTables f) {
     const unsigned int n = min(*a.nsamples, kAdjSamples);
@@ -1315,12 +1363,12 @@ int launch_temporal_adjoint(const BlockDev* blocks, long long vox, const float* 
     return (int)cudaGetLastError();
 }
 
-int launch_shift_axis(const float* src, float* dst, int W, int H, int D, int T, int axis, const float* shifts, int mode,
-                      unsigned long long* err, void* stream) {
-    const long long n = (long long)W * H * D * T;
-    const long long grid = std::min<long long>((n + 255) / 256, 152LL * 16);
-    shift_axis_kernel<<<(unsigned)grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(src, dst, W, H, D, T, axis,
-                                                                                     shifts, mode, err);
+int launch_shift_adjoint(const float* src, float* dst, int W, int H, int D, int T, int axis, const float* shifts,
+                         void* stream) {
+    const long long rows = (long long)D * H * T;
+    const unsigned grid = (unsigned)std::min<long long>((rows + 7) / 8, 152LL * 64);
+    auto k = axis == 0 ? shift_adjoint_kernel<0> : axis == 1 ? shift_adjoint_kernel<1> : shift_adjoint_kernel<2>;
+    k<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(src, dst, W, H, D, T, shifts);
     return (int)cudaGetLastError();
 }
 
@@ -1338,15 +1386,15 @@ int launch_double_to_float(const double* src, float* dst, int n, void* stream) {
 }
 
 int launch_drift3d(const float* src, float* dst, const float* g, int W, int H, int D, int T, const float* shifts,
-                   int mode, double* out, unsigned long long* err, void* stream) {
-    (void)err;  // every tap index is clamped into the volume
-    const int threads = W >= 256 ? 256 : (W >= 128 ? 128 : (W >= 64 ? 64 : 32));
-    dim3 grid((unsigned)std::min<long long>((long long)D * H, std::max(152LL * 16 / std::max(T, 1), 8LL)),
-              (unsigned)T);
-    if (mode == 0)
-        drift3d_kernel<0><<<grid, threads, 0, static_cast<cudaStream_t>(stream)>>>(src, dst, g, W, H, D, shifts, out);
-    else
-        drift3d_kernel<1><<<grid, threads, 0, static_cast<cudaStream_t>(stream)>>>(src, dst, g, W, H, D, shifts, out);
+                   int mode, double* out, void* stream) {
+    // walks of 16 planes (19 planes' taps for 16 of output) where they leave every SM
+    // its warps, else of 4, whose chain of loads is shorter
+    const long long cols = (long long)((W + 31) / 32) * H;
+    const int L = cols * ((D + 15) / 16) * T >= 152 * 16 ? 16 : 4;
+    const long long warps = cols * ((D + L - 1) / L);
+    dim3 grid((unsigned)std::min<long long>((warps + 7) / 8, 152LL * 64), (unsigned)T);
+    auto k = mode == 0 ? drift3d_kernel<0> : drift3d_kernel<1>;
+    k<<<grid, kDriftThreads, 0, static_cast<cudaStream_t>(stream)>>>(src, dst, g, W, H, D, L, shifts, out);
     return (int)cudaGetLastError();
 }
 

@@ -970,8 +970,7 @@ static int apply_drift(rfba_ctx* ctx, const float* in, const float* shifts, cons
         (s = ctx->tmp2.ensure(n * 4, "scratch")))
         return s;
     float* out = static_cast<float*>(ctx->shifted.p);
-    unsigned long long* err = static_cast<unsigned long long*>(ctx->errw.p);
-    const int e = launch_drift3d(in, out, nullptr, dims[0], dims[1], dims[2], dims[3], shifts, 0, nullptr, err, st);
+    const int e = launch_drift3d(in, out, nullptr, dims[0], dims[1], dims[2], dims[3], shifts, 0, nullptr, st);
     if (e) return cuda_fail((cudaError_t)e, "drift resampling");
     ctx->launches += 1;
     *iprime = out;
@@ -1411,20 +1410,19 @@ static int backward_locked(rfba_ctx* ctx, const rfba_srrf_config* cfg, const flo
     }
     // through the drift operator
     float* gin = static_cast<float*>(ctx->gin.p);
-    unsigned long long* err = static_cast<unsigned long long*>(ctx->errw.p);
     int e = 0;
     if (shifts) {
         float* t1 = static_cast<float*>(ctx->tmp1.p);
         float* t2 = static_cast<float*>(ctx->tmp2.p);
-        e = launch_shift_axis(gin, t1, dims[0], dims[1], dims[2], T, 2, shifts, 2, err, st);
-        if (!e) e = launch_shift_axis(t1, t2, dims[0], dims[1], dims[2], T, 1, shifts, 2, err, st);
-        if (!e) e = launch_shift_axis(t2, din, dims[0], dims[1], dims[2], T, 0, shifts, 2, err, st);
+        e = launch_shift_adjoint(gin, t1, dims[0], dims[1], dims[2], T, 2, shifts, st);
+        if (!e) e = launch_shift_adjoint(t1, t2, dims[0], dims[1], dims[2], T, 1, shifts, st);
+        if (!e) e = launch_shift_adjoint(t2, din, dims[0], dims[1], dims[2], T, 0, shifts, st);
         ctx->launches += 3;
         if (!e && dshift) {
             if ((s = ctx->dshift.ensure((size_t)T * 3 * sizeof(double), "drift adjoint"))) return s;
             double* ds = static_cast<double*>(ctx->dshift.p);
             RFBA_CUDA(cudaMemsetAsync(ds, 0, (size_t)T * 3 * sizeof(double), st), "drift adjoint clear");
-            e = launch_drift3d(in, nullptr, gin, dims[0], dims[1], dims[2], T, shifts, 1, ds, err, st);
+            e = launch_drift3d(in, nullptr, gin, dims[0], dims[1], dims[2], T, shifts, 1, ds, st);
             ctx->launches += 1;
             if (!e) e = launch_double_to_float(ds, dshift, 3 * T, st);
             ctx->launches += 1;

@@ -21,7 +21,7 @@ constexpr int kMaxThreads = 256;  // 16 x 16 threads for the 32-row tile (mid ma
 constexpr int kMaxMag = 8;
 constexpr int kMaxGradRange = 3;
 // The forward kernel's register limit for MZ x CZ tiles: MZ CZ for the sums and
-// 6 (CZ / 2 + 4) for the y-filtered columns are live through the point loop.
+// 6 (CZ / 2 + 4) for the x-filtered columns are live through the point loop.
 constexpr int fwd_regs(int mz, int cz) { return mz * cz + 6 * (cz / 2 + 4) <= 88 ? 128 : 168; }
 
 // The adjoint's tile depth (it holds two sets of columns), its register limit (12
@@ -272,12 +272,12 @@ int radiality_adjoint_max_ctas_per_sm(const FwdParams& p, int* out);
 int launch_temporal_adjoint(const BlockDev* blocks, long long vox, const float* rad, const float* inten,
                             const float* gmap, int T, int method, int itc, int order, int iw, int renorm, int poscon,
                             float* gS, float* gI, long long nmap, unsigned long long* err, void* stream);
-int launch_shift_axis(const float* src, float* dst, int W, int H, int D, int T, int axis, const float* shifts, int mode,
-                      unsigned long long* err, void* stream);
+int launch_shift_adjoint(const float* src, float* dst, int W, int H, int D, int T, int axis, const float* shifts,
+                         void* stream);
 // Drift operator, all axes fused: mode 0 resamples src into dst; mode 1 adds
 // sum_voxels g * dI'/dd_a into out[3 t + a] (FP64).
 int launch_drift3d(const float* src, float* dst, const float* g, int W, int H, int D, int T, const float* shifts,
-                   int mode, double* out, unsigned long long* err, void* stream);
+                   int mode, double* out, void* stream);
 int launch_drift_dot(const float* g, const float* dv, long long nv, int T, int axis, double* out,
                      unsigned long long* err, void* stream);
 int launch_double_to_float(const double* src, float* dst, int n, void* stream);

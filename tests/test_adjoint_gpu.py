@@ -280,3 +280,22 @@ def test_adjoint_plan_choice_matches_fp64_adjoint(ctx, oracle_mod, mag, axes, sh
     assert_parity(m, mo, 1e-4, f"{mag} forward")
     _, din_o, dsh_o = O.adjoint(x, O.make_conf(**kw), _gmap(mo), sh)
     assert rel_linf(din, din_o) < 2e-4 and rel_linf(dsh, dsh_o) < 2e-4
+
+
+@pytest.mark.parametrize("mag,shape", [((2, 2, 2), (4, 17, 6, 33)), ((2, 2, 2), (4, 5, 8, 32)), ((2, 2, 2), (4, 8, 17, 7)),
+                                       ((1, 1, 1), (31, 17, 20, 33))])
+def test_drift_operator_strips_match_fp64_adjoint(ctx, oracle_mod, mag, shape):
+    """The drift operator walks strips of 4 planes of z, or 16 where there are
+    enough of them (the last case), 32 columns of x to a warp: broken strips and
+    warps, shifts of 0, whole, half and several voxels either way, so that taps are
+    clamped on every side; to the bounds of the cases above."""
+    from rfba_gb300 import srrf
+    O = oracle_mod
+    kw = dict(mag=mag, method=3, itc=0, trac_order=2, **SHIPPED)
+    x, sh = _case(90, *shape)
+    sh[:4] = [[0, 0, 0], [1, -1, 2], [0.5, -0.5, -1.5], [-2.25, 1.75, 2.5]]
+    m, din, dsh = _gpu(ctx, srrf.Config.make(**kw), x, sh)
+    mo = O.forward_shifted(x, O.make_conf(**kw), sh)
+    assert_parity(m, mo, 1e-4, f"{shape} forward")
+    _, din_o, dsh_o = O.adjoint(x, O.make_conf(**kw), _gmap(mo), sh)
+    assert rel_linf(din, din_o) < 2e-4 and rel_linf(dsh, dsh_o) < 2e-4
