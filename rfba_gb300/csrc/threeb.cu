@@ -311,51 +311,58 @@ __global__ void __launch_bounds__(kEmitThreads) emission_df_kernel(const float2*
     for (int a = 0; a < kDfTile; ++a)
 #pragma unroll
         for (int n = 0; n < 6; ++n) acc[a][n] = df_two_sum(acc[a][n].x, acc[a][n].y);
-    __shared__ float2 part[kEmitThreads / 32][kDfTile][6];
+    // The warp's 24 sums: at each of the first three steps a lane hands half of its
+    // sums to the lane across and keeps the other half, 12 + 6 + 3 adds, then two
+    // steps on the three it is left with, 27 adds where 24 whole trees take 120. The
+    // pairs are the trees' pairs.
+    constexpr int kSums = kDfTile * 6, kKept = kSums / 8;
+    static_assert(kSums % 8 == 0, "three halvings");
+    float2* r = &acc[0][0];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto across = [](float2 v, int o) {
+        return make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+    };
+    int first = 0;
 #pragma unroll
-    for (int a = 0; a < kDfTile; ++a)
+    for (int o = 16, n = kSums / 2; o > 2; o >>= 1, n >>= 1) {
+        const bool up = lane & o;
 #pragma unroll
-        for (int n = 0; n < 6; ++n) {
-            float2 v = acc[a][n];
-            for (int o = 16; o > 0; o >>= 1) {
-                float2 u;
-                u.x = __shfl_down_sync(0xffffffffu, v.x, o);
-                u.y = __shfl_down_sync(0xffffffffu, v.y, o);
-                v = df_add(v, u);
-            }
-            if (lane == 0) part[warp][a][n] = v;
+        for (int i = 0; i < n; ++i) {
+            const float2 give = up ? r[i] : r[n + i], keep = up ? r[n + i] : r[i];
+            r[i] = df_add(keep, across(give, o));
         }
+        first += up ? n : 0;
+    }
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < kKept; ++i) r[i] = df_add(r[i], across(r[i], o));
+    __shared__ float2 part[kEmitThreads / 32][kSums];
+    if ((lane & 3) == 0)
+#pragma unroll
+        for (int i = 0; i < kKept; ++i) part[warp][first + i] = r[i];
     __syncthreads();
-    if (threadIdx.x < ns) {
-        const int a = threadIdx.x;
-        double t[6];
+    // one thread per sum, so the FP64 divisions of a sample run side by side
+    if (threadIdx.x < ns * 6) {
+        const int a = threadIdx.x / 6, n = threadIdx.x % 6;
+        float2 v = part[0][threadIdx.x];
 #pragma unroll
-        for (int n = 0; n < 6; ++n) {
-            float2 v = part[0][a][n];
-            for (int w = 1; w < kEmitThreads / 32; ++w) v = df_add(v, part[w][a][n]);
-            t[n] = df_to(v);
-        }
+        for (int w = 1; w < kEmitThreads / 32; ++w) v = df_add(v, part[w][threadIdx.x]);
+        const double t = df_to(v);
         EmDf* o = out + (size_t)(s0 + a) * F + f;
-        const double gap = (2.0 * t[0] - spot_sums[0]) / twovar;  // log p_on - log p_off
-        double m[2], k[2];
-        if (gap <= 0.0) {
-            exp_split(gap, &m[0], &k[0]);
-            m[1] = 1.0;
-            k[1] = 0.0;
+        // n = 0: log p_on - log p_off; else d(log p_on) / d phi_(n - 1)
+        const double q = ((n == 0 ? 2.0 * t : t) - spot_sums[n]) / (n == 0 ? twovar : var);
+        if (n > 0) {
+            o->q[n - 1] = df_from(q);
         } else {
-            m[0] = 1.0;
-            k[0] = 0.0;
-            exp_split(-gap, &m[1], &k[1]);
+            double m, k;
+            exp_split(-fabs(q), &m, &k);
+            const int low = q <= 0.0 ? 0 : 1;  // the smaller probability
+            o->mant[low] = df_from(m);
+            o->k[low] = (int)k;
+            o->mant[1 - low] = make_float2(1.f, 0.f);
+            o->k[1 - low] = 0;
         }
-        EmDf r;
-        for (int i = 0; i < 2; ++i) {
-            r.mant[i] = df_from(m[i]);
-            r.k[i] = (int)k[i];
-        }
-#pragma unroll
-        for (int n = 0; n < kM; ++n) r.q[n] = df_from((t[1 + n] - spot_sums[1 + n]) / var);
-        *o = r;
     }
 }
 
@@ -558,7 +565,7 @@ __global__ void __launch_bounds__(32) forward_df_kernel(const EmDf* __restrict__
             int Em = kZeroExp;
 #pragma unroll
             for (int i = 0; i < 3; ++i) Em = (nz[i] && E[i] > Em) ? E[i] : Em;
-            float2 y = make_float2(0.f, 0.f);
+            float2 y;
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
                 const float2 xi = shfl2(x, i * 6 + k);
@@ -568,7 +575,7 @@ __global__ void __launch_bounds__(32) forward_df_kernel(const EmDf* __restrict__
                 float2 tm = df_mul(Aj[i], xi);
                 tm.x *= sc;
                 tm.y *= sc;
-                y = df_add(y, tm);
+                y = i == 0 ? tm : df_add(y, tm);
             }
             y = df_mul(y, mant);
             const float2 y05 = shfl2(y, 5);
