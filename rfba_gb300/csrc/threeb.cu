@@ -509,14 +509,13 @@ __global__ void __launch_bounds__(32) forward_df_kernel(const EmDf* __restrict__
         return make_float2(__shfl_sync(full, v.x, src), __shfl_sync(full, v.y, src));
     };
     // normalise the new values y of this lane's state by the exponent of its
-    // probability lane; returns the state's new exponent
+    // probability prob; returns the state's new exponent
     // (branch-free: the lanes of a state whose probability is 0 must not
     // diverge from the others)
-    auto normalise = [&](float2 y, int Ebase, float2* x) {
-        const float2 y5 = shfl2(y, j * 6 + 5);
-        const int ex = (__float_as_int(y5.x) >> 23) & 0xff;
-        const bool zero = y5.x == 0.f || ex == 0 || Ebase == kZeroExp;
-        const int sh = ex - 126;  // y5 = m 2^sh, m in [0.5, 1)
+    auto normalise = [&](float2 y, float prob, int Ebase, float2* x) {
+        const int ex = (__float_as_int(prob) >> 23) & 0xff;
+        const bool zero = prob == 0.f || ex == 0 || Ebase == kZeroExp;
+        const int sh = ex - 126;  // prob = m 2^sh, m in [0.5, 1)
         const float sc = zero ? 1.f : pow2f(-sh);
         *x = make_float2(y.x * sc, y.y * sc);
         return zero ? kZeroExp : Ebase + sh;
@@ -526,7 +525,7 @@ __global__ void __launch_bounds__(32) forward_df_kernel(const EmDf* __restrict__
     {
         const float2 a = df_mul(df_from(pi3[j]), e[0].mant[mi]);
         const float2 y = k == 5 ? a : (has_de ? df_mul(a, e[0].q[k]) : make_float2(0.f, 0.f));
-        const int En = normalise(y, pi3[j] == 0.0 ? kZeroExp : e[0].k[mi], &x);
+        const int En = normalise(y, a.x, pi3[j] == 0.0 ? kZeroExp : e[0].k[mi], &x);
 #pragma unroll
         for (int i = 0; i < 3; ++i) E[i] = __shfl_sync(full, En, i * 6 + 5);
     }
@@ -578,9 +577,13 @@ __global__ void __launch_bounds__(32) forward_df_kernel(const EmDf* __restrict__
                 y = i == 0 ? tm : df_add(y, tm);
             }
             y = df_mul(y, mant);
+            // final here already: the derivative's term below adds to the others only,
+            // and the exponents are formed beside it (behind it they cost an evaluation of
+            // 100 frames 7 us; each lane forming the probability itself, 16)
+            const float prob = __shfl_sync(full, y.x, j * 6 + 5);
             const float2 y05 = shfl2(y, 5);
             y = df_add(y, df_mul(y05, q));
-            const int En = normalise(y, (Em == kZeroExp || ke == kZeroExp) ? kZeroExp : Em + ke, &x);
+            const int En = normalise(y, prob, (Em == kZeroExp || ke == kZeroExp) ? kZeroExp : Em + ke, &x);
 #pragma unroll
             for (int i = 0; i < 3; ++i) E[i] = __shfl_sync(full, En, i * 6 + 5);
         }
