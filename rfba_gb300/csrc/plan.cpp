@@ -686,7 +686,7 @@ int forward_depth(const FwdPlan& fp, const std::vector<FwdRegion>& regions, int 
     }
     // Two deep items or fewer to an SM: a launch lasts as long as one item, and a
     // shallow one ends sooner (5 x 10x12x12 at mag 2, the whole call: 63.6 us with
-    // deep tiles, 57 with shallow ones).
+    // deep tiles, 55.5 with shallow ones).
     if (items <= 2LL * sms) return 4;
     return time[1] < time[0] ? 4 : 8;
 }
