@@ -93,7 +93,7 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
 def _build_locked(force: bool, verbose_ptxas: bool) -> Path:
     cu, cpp = sources()
     srcs = cu + cpp
-    headers = list(CSRC.glob("*.h")) + list((PKG.parent / "include").glob("*.h"))
+    headers = list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + list((PKG.parent / "include").glob("*.h"))
     newest = max(p.stat().st_mtime for p in srcs + headers)
     if LIB.exists() and not force and not verbose_ptxas and LIB.stat().st_mtime >= newest:
         build_cli()
