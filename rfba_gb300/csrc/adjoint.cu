@@ -24,6 +24,7 @@
 #include <cstring>
 
 #include "radiality_common.cuh"
+#include "shared_limit.h"
 #include "srrf_internal.h"
 
 namespace rfba {
@@ -1329,7 +1330,7 @@ int launch_radiality_adjoint(const FwdParams& p, const FwdPlan& plan, const AdjP
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     return with_adj_kernel(p, [&](auto k, auto n) -> int {
         constexpr int UN = decltype(n)::value;
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = allow_shared(k, smem);
         if (e != cudaSuccess) return (int)e;
         UTab<UN> tab;
         std::memset(&tab, 0, sizeof tab);
@@ -1347,7 +1348,7 @@ int launch_adjoint_samples(const FwdParams& p, const AdjParams& a, const AdjFixT
 int radiality_adjoint_max_ctas_per_sm(const FwdParams& p, int* out) {
     const size_t smem = radiality_adjoint_smem_bytes(p);
     return with_adj_kernel(p, [&](auto k, auto) -> int {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = allow_shared(k, smem);
         if (e != cudaSuccess) return (int)e;
         return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k, p.TY * kTileX, smem);
     });

@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "shared_limit.h"
 #include "srrf_internal.h"
 
 namespace rfba {
@@ -223,8 +224,7 @@ int launch_combine(const double* spots, long long n, int zoom, int Xp, int Yp, i
     box_z_mask_kernel<<<grid_for((long long)Xp * Yp, 256), 256, 0, st>>>(S, Xp, Yp, Zp, r, rz, thr, hist);
     compact_kernel<<<grid_for(nvox, 256), 256, 0, st>>>(hist, nvox, idx, val, counters + 1, cap);
     const size_t psf_bytes = (size_t)Kx * Ky * Kz * 2;
-    cudaError_t e = cudaFuncSetAttribute(scatter_conv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)psf_bytes);
+    const cudaError_t e = allow_shared(scatter_conv_kernel, psf_bytes);
     if (e != cudaSuccess) return (int)e;
     // nonzero count is on the device: launch a fixed persistent grid that strides over it
     scatter_conv_kernel<<<4 * 152, 256, psf_bytes, st>>>(idx, val, counters + 1, cap, psf, Kx, Ky, Kz, Xp, Yp, Zp,

@@ -35,6 +35,7 @@
 
 #include "ffbs.cuh"
 #include "philox.h"
+#include "shared_limit.h"
 #include "srrf_internal.h"
 
 namespace rfba {
@@ -320,7 +321,7 @@ size_t gibbs_smem_bytes(int F) {
 
 int gibbs_max_blocks(int F, int* out) {
     const size_t smem = gibbs_smem_bytes(F);
-    cudaError_t e = cudaFuncSetAttribute(gibbs_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared(gibbs_chain_kernel, smem);
     if (e != cudaSuccess) return (int)e;
     int dev = 0, sms = 0, per = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
@@ -334,7 +335,7 @@ int gibbs_max_blocks(int F, int* out) {
 
 int launch_gibbs(const GibbsParams* chains_dev, int nchains, int grid_per_chain, int F, void* stream) {
     const size_t smem = gibbs_smem_bytes(F);
-    cudaError_t e = cudaFuncSetAttribute(gibbs_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared(gibbs_chain_kernel, smem);
     if (e != cudaSuccess) return (int)e;
     const GibbsParams* q = chains_dev;
     int n = nchains;

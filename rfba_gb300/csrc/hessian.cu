@@ -40,6 +40,7 @@
 
 #include "ffbs.cuh"
 #include "philox.h"
+#include "shared_limit.h"
 #include "srrf_internal.h"
 
 namespace rfba {
@@ -306,9 +307,7 @@ int launch_spot_hessian(const HessParams& h, void* stream) {
     for (int n = 0; n < 3; ++n) a.pi[n] = h.pi[n];
     a.seed = h.seed;
     const size_t smem = ffbs_smem(h.F);
-    if ((e = cudaFuncSetAttribute(hess_ffbs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-        cudaSuccess)
-        return (int)e;
+    if ((e = allow_shared(hess_ffbs_kernel, smem)) != cudaSuccess) return (int)e;
     hess_ffbs_kernel<<<h.S, kFfbsThreads, smem, st>>>(a);
     return (int)cudaGetLastError();
 }

@@ -67,6 +67,7 @@
 #include <cudaTypedefs.h>
 
 #include "radiality_common.cuh"
+#include "shared_limit.h"
 #include "srrf_internal.h"
 
 namespace rfba {
@@ -597,7 +598,7 @@ int launch_radiality(const FwdParams& p, const FwdPlan& plan, int grid, size_t s
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     return with_kernel(p, [&](auto k, auto n) -> int {
         constexpr int UN = decltype(n)::value;
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = allow_shared(k, smem);
         if (e != cudaSuccess) return (int)e;
         FwdParams q = p;
         CUtensorMap map;
@@ -618,7 +619,7 @@ int launch_radiality(const FwdParams& p, const FwdPlan& plan, int grid, size_t s
 int radiality_max_ctas_per_sm(const FwdParams& p, int* out) {
     const size_t smem = radiality_smem_bytes(p);
     return with_kernel(p, [&](auto k, auto) -> int {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = allow_shared(k, smem);
         if (e != cudaSuccess) return (int)e;
         return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k, p.TY * kTileX, smem);
     });

@@ -19,6 +19,7 @@
 // is defined as 0.
 #include <cuda_runtime.h>
 
+#include "shared_limit.h"
 #include "srrf_internal.h"
 
 namespace rfba {
@@ -298,8 +299,7 @@ int launch_temporal(const TemporalParams& p, void* stream) {
                                     : p.order == 4 ? trac_itc_kernel<4>
                                                    : trac_itc_kernel<2>;
         if (smem > 48 * 1024) {
-            // the same limit for every T: contexts on other threads share the function
-            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColMaxSmem);
+            const cudaError_t e = allow_shared(k, smem);
             if (e != cudaSuccess) return (int)e;
         }
         const long long grid = (p.total_vox + kColThreads - 1) / kColThreads;
