@@ -645,15 +645,17 @@ __device__ __forceinline__ float4 f4fma(float s, float4 a, float4 c) {
 
 // Ring samples whose gradient nearly vanishes or nearly follows the ring direction
 // amplify the rounding of the interpolated gradient into the derivative, by |g|^2 of
-// the column over |g| |g_perp| of the sample. Below a bound on c2 g2 (this factor
-// times the square of the sum of |g|^2 over four cells of the column) the kernel
-// takes the derivative at the bound, which needs no operation more than the guard
-// against 0 that was there, and lists the sample; adjoint_samples_kernel then adds
-// the difference to the derivative as it comes out in the rounding of passes along x,
-// then y, then z, whatever order this kernel's passes take. About one sample in a
-// million is listed; once kAdjSamplesOpen are, pairs begun later take no bound (the
-// list has room for all that may be under way then). Without that, single voxels of dL/dI differed between the two
-// orders by up to 5e-3 of their size on one of four drift series.
+// the column over |g| |g_perp| of the sample. With the passes in the plan's order single
+// voxels of dL/dI came out up to 5e-3 away from those with passes along x, then y, then
+// z, on one of four drift series: neither is the more accurate (on a crop at 4 x 4 x 2
+// both are 2.1e-5 from 64 bits), but dL/dI is to be the same whatever the plan. So below
+// a bound on c2 g2, this factor times the square of the sum of |g|^2 over four cells of
+// the column, the point loop takes the derivative at the bound, which costs no operation
+// more than the guard against 0 does, and marks the subvoxel; fix_marked then adds what
+// is missing, from the derivative in the fixed order. Samples under the bound are ten in a
+// million on a series of 60 volumes of 64^3 at mag 2 (82 thousand; correcting them takes
+// 0.3 of the pair's 42.2 ms), and two of a subvoxel's 62 where a whole volume is a ramp
+// along a ring direction (12 volumes of 64^3 then take 30 to 47 ms instead of 6).
 constexpr float kSampleBound = 6e-9f;
 
 // The derivative of one sample's sine term with respect to (-P, E, Z), times K.
@@ -669,9 +671,115 @@ __device__ __forceinline__ Derivative sample_derivative(float P, float E, float 
     return Derivative{fmaf(c, m * cp, h * (b * dot)), m * E, fmaf(h, m * cp, -c * (b * dot))};
 }
 
-__device__ __forceinline__ void list_sample(const AdjParams& a, long long index, int point, float bound) {
-    const unsigned int i = atomicAdd(a.nsamples, 1u);
-    if (i < kAdjSamples) a.samples[i] = AdjSample{index, point, bound};
+// What the correction needs of a tile and time point.
+struct FixTile {
+    const FwdParams* p;
+    const float4* gt;  // gradient planes [NQ][nv][nu]
+    float4* gu;        // dL/dU planes [NQ][ty][nu]
+    const float* wx;   // the x values' tap weights
+    const float* wm;   // the tile rows' mid weights and first tap cells
+    const int* base;
+    const float* gS;
+    long long zstride;
+};
+
+// Four taps along x (weights w) at innermost cell c of a row of planes [quad][rows][nu].
+__device__ __forceinline__ float along_x(const float4* row, int quad, int c, const float* w) {
+    const float* g = reinterpret_cast<const float*>(row + (c >> 2) * quad) + (c & 3);
+    return fmaf(w[3], g[12], fmaf(w[2], g[8], fmaf(w[1], g[4], w[0] * g[0])));
+}
+
+// A store that the compiler knows to be to shared memory: through a generic pointer, in a
+// function that is called, it counts as one that may reach the caller's locals.
+__device__ __forceinline__ void store_shared(float* p, float v) {
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "f"(v) : "memory");
+}
+
+// The correction of a pair's samples below the bound, by the whole warp for one subvoxel
+// after another. Of this lane's column, u0, ax, bound and sbase are its first x cell, x
+// weight index, bound and place in the stacks, marked its subvoxels that have such a
+// sample. Adds to dL/dU what the derivative in the fixed order exceeds the one at the bound
+// by: u = |u| (h x' + c z), x' = (ca, sb) in the x-y plane, the gradient interpolated along
+// x, then y, turned by (ca, sb), then along z; lanes 4 o + i take plane o of z and row i of
+// y. The point loop's frame is this one times scale. Nothing here depends on other tiles or
+// launches. A call takes 1.7 us, out of line so that the point loop keeps its registers
+// (60 volumes of 64^3 at mag 2: 1 pair of a warp in 115 comes here).
+template <int MZ, int CZ>
+__device__ __noinline__ void fix_marked(const FixTile& f, int pair, int u0, int ax, float bound, long long sbase,
+                                        unsigned int marked) {
+    constexpr int NQ = CZ / 4 + 1;
+    const unsigned int full = 0xffffffffu;
+    const FwdParams& p = *f.p;
+    const int lane = threadIdx.x & 31, o = (lane >> 2) & 3, i = lane & 3;
+    const bool y_inner = p.ax1 == 2;
+    const float4 r3 = __ldg(p.utab + p.u_pair + 4 * pair + 3);
+    for (unsigned int open = __ballot_sync(full, marked != 0); open; open &= open - 1) {
+        const int src = __ffs(open) - 1;
+        const int su = __shfl_sync(full, u0, src);
+        const float* wx = f.wx + 4 * __shfl_sync(full, ax, src);
+        const float least = __shfl_sync(full, bound, src);
+        const long long at = __shfl_sync(full, sbase, src);
+        const int row = (threadIdx.x >> 5) * 2 + (src >> 4);
+        const float* wm = f.wm + 4 * row;
+        for (unsigned int left = __shfl_sync(full, marked, src); left; left &= left - 1) {
+            const int z = __ffs(left) - 1;
+            const float gS = f.gS[at + z * f.zstride];
+#pragma unroll 1
+            for (int qi = __float_as_int(r3.x); qi < __float_as_int(r3.y); ++qi) {
+                const float4 fr = __ldg(p.fix + 2 * qi), wt = __ldg(p.fix + 2 * qi + 1);
+                const float4 c = __ldg(p.utab + p.u_pt + 3 * qi + 2);
+                // weights along the innermost axis: every second word of their record
+                const float* wi = reinterpret_cast<const float*>(p.utab + p.u_wz + 2 * (__float_as_int(c.x) + z % MZ));
+                const int w0 = z / MZ + ((__float_as_int(c.y) >> (z % MZ)) & 1);
+                float v[3];
+                {
+                    const float4* row0 = f.gt + (f.base[row] + (y_inner ? o : i)) * p.NU + su;
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                        v[d] = along_x(row0 + (d == 0 ? 0 : (d == 1) == y_inner ? 2 : 1) * NQ * p.NV * p.NU, p.NV * p.NU,
+                                       w0 + (y_inner ? i : o), wx);
+                }
+                // the sums over y of each z, then over z
+#pragma unroll 1
+                for (int pass = 0; pass < 2; ++pass) {
+                    float acc[3];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float w = y_inner == (pass == 0) ? __ldg(wi + 2 * k) : wm[k];
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) {
+                            const float u = __shfl_sync(full, v[d], pass == 0 ? 4 * o + k : 4 * k);
+                            acc[d] = k ? fmaf(w, u, acc[d]) : w * u;
+                        }
+                    }
+                    v[0] = pass == 0 ? fmaf(acc[1], fr.y, __fmul_rn(acc[0], fr.x)) : acc[0];
+                    v[1] = pass == 0 ? fmaf(acc[1], fr.x, __fmul_rn(acc[0], -fr.y)) : acc[1];
+                    v[2] = acc[2];
+                }
+                const float P = v[0], E = v[1], Z = v[2], hh = fr.z, cc = fr.w;
+                const float dot = fmaf(cc, Z, __fmul_rn(hh, P)), cp = fmaf(hh, Z, __fmul_rn(-cc, P));
+                const float c2 = fmaf(cp, cp, __fmul_rn(E, E)), xx = c2 * fmaf(dot, dot, c2);
+                const float scale = wt.z, s4 = scale * scale * scale * scale;
+                const Derivative e = sample_derivative(P, E, Z, hh, cc, wt.x, wt.y, gS, rsqrt_approx(fmaxf(xx, kGuard)));
+                const Derivative q = sample_derivative(P, E, Z, hh, cc, wt.x, wt.y, gS,
+                                                       scale * scale * rsqrt_approx(fmaxf(xx * s4, least)));
+                const float dP = q.P - e.P, dE = e.E - q.E;
+                const float dG[3] = {fmaf(dE, -fr.y, dP * fr.x), fmaf(dE, fr.x, dP * fr.y), e.Z - q.Z};
+                if (lane < 16) {
+                    const int w = w0 + o;
+                    const float spread = __ldg(wi + 2 * o) * wx[i];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        const int k = d == 0 ? 0 : (d == 1) == y_inner ? 2 : 1;
+                        float* g = reinterpret_cast<float*>(f.gu + ((k * NQ + (w >> 2)) * p.TY + row) * p.NU + su + i) +
+                                   (w & 3);
+                        store_shared(g, fmaf(dG[d], spread, *g));
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    }
 }
 
 template <int MZ, int CZ, int UN>
@@ -684,6 +792,7 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
     constexpr int NH = CH + 4;
     constexpr int NW = CZ + 4;
     constexpr int NQ = NW / 4;
+    static_assert(FZ <= 32, "a column's marks fit a word");
     extern __shared__ float4 smem4[];
 
     const int NU = p.NU, NV = p.NV, TY = p.TY;
@@ -796,7 +905,8 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                     for (int w = 0; w < 4; ++w) g[k][w] = 0.f;
                 if (cu >= 0 && cu < bw && cv >= 0 && cv < bh && cw + 3 >= 0 && cw < bd) {
                     const float* base = inp + (v + R) * NIX + (u + R);
-                    gradient4(p.grad_mode, p.gr, [&](int k) { return base + (w0 + R + k) * (NIY * NIX); }, NIX, g);
+                    gradient4<true>(p.grad_mode, p.gr, [&](int k) { return base + (w0 + R + k) * (NIY * NIX); }, NIX, g,
+                                    a1 == 2);
 #pragma unroll
                     for (int w = 0; w < 4; ++w)
                         if (cw + w < 0 || cw + w >= bd) g[0][w] = g[1][w] = g[2][w] = 0.f;
@@ -924,7 +1034,6 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                     const float4 wv = *reinterpret_cast<const float4*>(wx + ax * 4);
                     const float4* ubase = ut4 + q * NU + xi - cx0 - 2 + offx[ax];
                     const int pa = __float_as_int(r2.x), pb = __float_as_int(r2.y), pc = __float_as_int(r2.z);
-                    const unsigned int listed = *static_cast<volatile unsigned int*>(a.nsamples);
                     float2 TP[NH], TE[NH], TZ[NH];
 #pragma unroll
                     for (int wq = 0; wq < NQ; ++wq) {
@@ -945,13 +1054,19 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                         TP[w] = fma2(hi2(r0), Bv, mul2(lo2(r0), A));
                         TE[w] = fma2(hi2(r1), Bv, mul2(lo2(r1), A));
                     }
-                    float bound = 1e-30f;
-                    if (listed < kAdjSamplesOpen) {
+                    // the bound, and whether it is above the guard (kGuard, in this frame): with
+                    // gradients of 1e-8 or so every sample is below the guard, and none is fixed
+                    float bound = r3.w;
+                    bool fixing;
+                    {
                         constexpr int w = NH / 2;
                         const float2 lo = fma2(TZ[w - 1], TZ[w - 1], fma2(TE[w - 1], TE[w - 1], mul2(TP[w - 1], TP[w - 1])));
                         const float2 g = fma2(TZ[w], TZ[w], fma2(TE[w], TE[w], fma2(TP[w], TP[w], lo)));
-                        bound = fmaxf((g.x + g.y) * (g.x + g.y) * kSampleBound, 1e-30f);
+                        const float rel = (g.x + g.y) * (g.x + g.y) * kSampleBound;
+                        fixing = rel > bound && rel < 1e38f;
+                        if (fixing) bound = rel;
                     }
+                    unsigned int marked = 0;
                     float2 gP[NH], gE[NH], gZ[NH];  // gP with the sign turned
 #pragma unroll
                     for (int w = 0; w < NH; ++w) gP[w] = gE[w] = gZ[w] = make_float2(0.f, 0.f);
@@ -964,7 +1079,7 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                         asm volatile("" : "+f"(wun));
                         auto zpass = [&](auto OFF, int zr, float2 w0, float2 w1, float2 w2, float2 w3) {
                             constexpr int o = decltype(OFF)::value;
-                            float lowest = 1e30f;  // c2 g2 over these samples
+                            float lowest = 1e38f;  // c2 g2 over these samples
 #pragma unroll
                             for (int zi = 0; zi < CH; ++zi) {
                                 const float2 P = fma2(w3, TP[zi + o + 3], fma2(w2, TP[zi + o + 2], fma2(w1, TP[zi + o + 1], mul2(w0, TP[zi + o]))));
@@ -1003,7 +1118,7 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                                 gE[zi + o + 3] = fma2(w3, dE, gE[zi + o + 3]);
                                 gZ[zi + o + 3] = fma2(w3, dZ, gZ[zi + o + 3]);
                             }
-                            if (lowest < bound) {
+                            if (fixing && lowest < bound) {
 #pragma unroll
                                 for (int zi = 0; zi < CH; ++zi) {
                                     const float2 P = fma2(w3, TP[zi + o + 3], fma2(w2, TP[zi + o + 2], fma2(w1, TP[zi + o + 1], mul2(w0, TP[zi + o]))));
@@ -1014,8 +1129,8 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                                     const float2 c2 = fma2(cp, cp, mul2(E, E));
                                     const float2 xx = mul2(c2, fma2(dot, dot, c2));
                                     const int z = zi * MZ + zr;
-                                    if (xx.x < bound && gS[z].x != 0.f) list_sample(a, sbase + z * zstride, qi, bound);
-                                    if (xx.y < bound && gS[z].y != 0.f) list_sample(a, sbase + (z + HZ) * zstride, qi, bound);
+                                    if (xx.x < bound && gS[z].x != 0.f) marked |= 1u << z;
+                                    if (xx.y < bound && gS[z].y != 0.f) marked |= 1u << (z + HZ);
                                 }
                             }
                         };
@@ -1043,6 +1158,11 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
                     x_transpose(gP, xv, mask, gu + pa * uplane, true);
                     x_transpose(gE, xv, mask, gu + pb * uplane, true);
                     x_transpose(gZ, xv, mask, gu + pc * uplane, true);
+                    if (__any_sync(0xffffffffu, marked != 0)) {
+                        __syncwarp();  // the row's sums above
+                        const FixTile f = {&p, gt, gu, wx, s_weight, s_base, a.gS, zstride};
+                        fix_marked<MZ, CZ>(f, pi, xi - cx0 - 2 + offx[ax], ax, bound, sbase, marked);
+                    }
                 }
                 __syncthreads();
                 mid_transpose(gu, gg, 3);
@@ -1157,138 +1277,6 @@ __global__ void __maxnreg__(adj_regs(MZ, CZ))
     }
 }
 
-// The samples that the kernel above listed, one warp to a sample: the gradient at the
-// 4 x 4 x 4 cells its taps reach, interpolated along x, then y, then z, the derivative
-// of the radiality term in the plain rotated frame less the one at the bound, and
-// its transpose onto the input voxels (the taps and the stencil are products over
-// the axes). 60 volumes of 64^3 at mag 2 take 0.9 ms beside the kernel's 29.8.
-__global__ void __launch_bounds__(128) adjoint_samples_kernel(const __grid_constant__ FwdParams p, const AdjParams a,
-                                                              const AdjFixTables f) {
-    const unsigned int n = min(*a.nsamples, kAdjSamples);
-    const int lane = threadIdx.x & 31;
-    const BlockDev& B = p.blocks[0];
-    const float* in = static_cast<const float*>(p.in);
-    const bool zin = p.ax2 == 2;
-    const int mag[3] = {p.mag[0], zin ? p.mag[1] : p.mag[2], zin ? p.mag[2] : p.mag[1]};
-    const int range[3] = {p.gr[1], zin ? p.gr[2] : p.gr[3], zin ? p.gr[3] : p.gr[2]};
-    const int mR = p.gr[0];
-    for (unsigned int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s < n;
-         s += gridDim.x * (blockDim.x >> 5)) {
-        const AdjSample e = a.samples[s];
-        const long long rel = e.index - B.stack_off, row = rel / B.vox;
-        const int t = p.stack_t0 + (int)row, v0 = (int)(rel - row * B.vox);
-        const int at[3] = {B.lo[0] + v0 % B.nreg[0], B.lo[1] + v0 / B.nreg[0] % B.nreg[1],
-                           B.lo[2] + v0 / B.nreg[0] / B.nreg[1]};
-        const int4 vi = f.idx[e.point];
-        const int val[3] = {vi.x, vi.y, vi.z};
-        float w[3][4];
-        int c0[3];  // first tap cell
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const int xi = floordiv(at[k], mag[k]), i = val[k] * mag[k] + at[k] - xi * mag[k];
-            const float4 v = f.w[k][i];
-            w[k][0] = v.x, w[k][1] = v.y, w[k][2] = v.z, w[k][3] = v.w;
-            c0[k] = xi - 2 + f.off[k][i];
-        }
-        const long long tbase = (long long)t * p.D * p.H * p.W;
-        auto index = [&](int x, int y, int z) -> long long {
-            return tbase + ((long long)(B.origin[2] + clampi(z, 0, B.size[2] - 1)) * p.H +
-                            (B.origin[1] + clampi(y, 0, B.size[1] - 1))) * p.W + (B.origin[0] + clampi(x, 0, B.size[0] - 1));
-        };
-        // cells 4 (j + 4 k) + i: this lane's and the one 32 further on
-        float g[2][3];
-        for (int h = 0; h < 2; ++h) {
-            const int c = lane + 32 * h;
-            const int cx = c0[0] + (c & 3), cy = c0[1] + ((c >> 2) & 3), cz = c0[2] + (c >> 4);
-            float gx = 0.f, gy = 0.f, gz = 0.f;
-            if (cx >= 0 && cx < B.size[0] && cy >= 0 && cy < B.size[1] && cz >= 0 && cz < B.size[2]) {
-                auto I = [&](int dx, int dy, int dz) -> float {
-                    const long long i = index(cx + dx, cy + dy, cz + dz);
-                    return in_range(i, a.n_in, a.err, 11) ? __ldg(in + i) : 0.f;
-                };
-                for (int i = 1; i <= mR; ++i)
-                    for (int j = -range[1]; j <= range[1]; ++j)
-                        for (int k = -range[2]; k <= range[2]; ++k) gx += I(i, j, k) - I(-i, j, k);
-                for (int j = 1; j <= mR; ++j)
-                    for (int i = -range[0]; i <= range[0]; ++i)
-                        for (int k = -range[2]; k <= range[2]; ++k) gy += I(i, j, k) - I(i, -j, k);
-                for (int k = 1; k <= mR; ++k)
-                    for (int i = -range[0]; i <= range[0]; ++i)
-                        for (int j = -range[1]; j <= range[1]; ++j) gz += I(i, j, k) - I(i, j, -k);
-            }
-            g[h][0] = gx, g[h][1] = gy, g[h][2] = gz;
-        }
-        // x: lanes 0 .. 15 hold (j, k) = (lane & 3, lane >> 2); y: lanes 0 .. 3 hold k; z
-        float v[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            float acc = 0.f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float lo = __shfl_sync(0xffffffffu, g[0][d], (4 * lane + i) & 31);
-                const float hi = __shfl_sync(0xffffffffu, g[1][d], (4 * lane + i) & 31);
-                const float u = lane < 8 ? lo : hi;
-                acc = i ? fmaf(w[0][i], u, acc) : w[0][0] * u;
-            }
-            v[d] = acc;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float u = __shfl_sync(0xffffffffu, v[d], (4 * lane + i) & 31);
-                acc = i ? fmaf(w[1][i], u, acc) : w[1][0] * u;
-            }
-            v[d] = acc;
-        }
-        const float4 fr = f.frame[e.point];
-        float pez[3] = {fmaf(v[1], fr.y, __fmul_rn(v[0], fr.x)), fmaf(v[1], fr.x, __fmul_rn(v[0], -fr.y)), v[2]};
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            float acc = 0.f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float u = __shfl_sync(0xffffffffu, pez[d], i);
-                acc = i ? fmaf(w[2][i], u, acc) : w[2][0] * u;
-            }
-            v[d] = acc;
-        }
-        const float P = v[0], E = v[1], Z = v[2], hh = fr.z, cc = fr.w;
-        const float dot = fmaf(cc, Z, __fmul_rn(hh, P)), cp = fmaf(hh, Z, __fmul_rn(-cc, P));
-        const float c2 = fmaf(cp, cp, __fmul_rn(E, E)), xx = c2 * fmaf(dot, dot, c2);
-        // the kernel above scales this frame by 1 / h (by 1 on the z axis of its plan)
-        const float scale = f.scale[e.point], s4 = scale * scale * scale * scale;
-        const float2 wt = f.weight[e.point];
-        const float gS = in_range(e.index, a.n_stack, a.err, 9) ? a.gS[e.index] : 0.f;
-        const Derivative r = sample_derivative(P, E, Z, hh, cc, wt.x, wt.y, gS, rsqrt_approx(fmaxf(xx, 1e-30f)));
-        const Derivative q0 = sample_derivative(P, E, Z, hh, cc, wt.x, wt.y, gS,
-                                                scale * scale * rsqrt_approx(fmaxf(xx * s4, e.bound)));
-        const float dP = q0.P - r.P, dE = r.E - q0.E, dZ = r.Z - q0.Z;
-        const float dG[3] = {fmaf(dE, -fr.y, dP * fr.x), fmaf(dE, fr.x, dP * fr.y), dZ};
-        // transposed: taps, then the stencil, per axis along the gradient's component (der)
-        // and across it (box); cells outside the block hold no gradient
-        const int nx = 4 + 2 * p.R;
-        for (int q = lane; q < nx * nx * nx; q += 32) {
-            const int pos[3] = {q % nx - p.R, q / nx % nx - p.R, q / (nx * nx) - p.R};
-            float der[3], box[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                der[d] = box[d] = 0.f;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (c0[d] + i < 0 || c0[d] + i >= B.size[d]) continue;
-                    const int o = pos[d] - i;
-                    if (o != 0 && abs(o) <= mR) der[d] += o > 0 ? w[d][i] : -w[d][i];
-                    if (abs(o) <= range[d]) box[d] += w[d][i];
-                }
-            }
-            const float acc = dG[0] * der[0] * box[1] * box[2] + dG[1] * box[0] * der[1] * box[2] +
-                              dG[2] * box[0] * box[1] * der[2];
-            if (acc != 0.f) {
-                const long long i = index(c0[0] + pos[0], c0[1] + pos[1], c0[2] + pos[2]);
-                if (in_range(i, a.n_in, a.err, 11)) atomicAdd(a.gin + i, acc);
-            }
-        }
-    }
-}
-
 template <class F>
 int with_adj_kernel(const FwdParams& p, F&& f) {
     auto go = [&](auto mz) -> int {
@@ -1338,11 +1326,6 @@ int launch_radiality_adjoint(const FwdParams& p, const FwdPlan& plan, const AdjP
         k<<<grid, p.TY * kTileX, smem, st>>>(p, a, tab);
         return (int)cudaGetLastError();
     });
-}
-
-int launch_adjoint_samples(const FwdParams& p, const AdjParams& a, const AdjFixTables& f, int sms, void* stream) {
-    adjoint_samples_kernel<<<4 * sms, 128, 0, static_cast<cudaStream_t>(stream)>>>(p, a, f);
-    return (int)cudaGetLastError();
 }
 
 int radiality_adjoint_max_ctas_per_sm(const FwdParams& p, int* out) {

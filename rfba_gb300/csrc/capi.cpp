@@ -1144,7 +1144,6 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
     if ((s = ctx->gS.ensure((size_t)V * TW * 4, "adjoint stack")) || (s = ctx->gI.ensure((size_t)V * TW * 4, "adjoint stack")) ||
         (s = ctx->ablocks.ensure(sizeof(BlockDev), "blocks")) ||
         (s = ctx->atiles.ensure(tiles.size() * sizeof(TileDesc), "tiles")) || (s = ctx->acounter.ensure(256, "counter")) ||
-        (s = ctx->asamples.ensure(kAdjSamples * sizeof(AdjSample), "adjoint samples")) ||
         (s = ctx->errw.ensure(256, "check word")))
         return s;
     RFBA_CUDA(cudaMemcpyAsync(ctx->ablocks.p, &blk, sizeof blk, cudaMemcpyHostToDevice, st), "blocks upload");
@@ -1166,6 +1165,7 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
     FwdParams rp = adjoint_params(fp, *cfg, iprime, dims);
     rp.lane = static_cast<const float*>(ctx->tables.p);
     rp.utab = reinterpret_cast<const float4*>(rp.lane + ctx->plan.adj_utab);
+    rp.fix = reinterpret_cast<const float4*>(rp.lane + ctx->plan.fix);
     rp.blocks = dblk;
     rp.tiles = static_cast<const TileDesc*>(ctx->atiles.p);
     rp.ntiles = (int)tiles.size();
@@ -1197,24 +1197,9 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
                  static_cast<float*>(ctx->gin.p),
                  (long long)nin,
                  (long long)V * TW,
-                 static_cast<AdjSample*>(ctx->asamples.p),
-                 static_cast<unsigned int*>(ctx->acounter.p) + 32,
                  err};
     e = launch_radiality_adjoint(rp, fp, ap, grid, smem, st);
     if (e) return cuda_fail((cudaError_t)e, "radiality adjoint launch");
-    const float* fix = static_cast<const float*>(ctx->tables.p) + ctx->plan.fix;
-    AdjFixTables ft;
-    ft.idx = reinterpret_cast<const int4*>(fix + fp.f_idx);
-    ft.frame = reinterpret_cast<const float4*>(fix + fp.f_frame);
-    ft.weight = reinterpret_cast<const float2*>(fix + fp.f_weight);
-    ft.scale = fix + fp.f_scale;
-    for (int a = 0; a < 3; ++a) {
-        ft.w[a] = reinterpret_cast<const float4*>(fix + fp.f_w[a]);
-        ft.off[a] = reinterpret_cast<const int*>(fix + fp.f_off[a]);
-    }
-    e = launch_adjoint_samples(rp, ap, ft, ctx->sm_count, st);
-    if (e) return cuda_fail((cudaError_t)e, "adjoint samples launch");
-    ctx->launches += 1;
     ctx->launches += window ? 1 : 2;
     return RFBA_OK;
 }
@@ -1550,7 +1535,7 @@ int rfba_ctx_destroy(rfba_ctx* c) {
     cudaSetDevice(c->device);
     for (DevBuf* b : {&c->in, &c->out, &c->rad, &c->inten, &c->blocks, &c->tiles, &c->tables, &c->counter, &c->prefix,
                       &c->shifted, &c->tmp1, &c->tmp2, &c->gS, &c->gI, &c->gin, &c->dshift, &c->ablocks, &c->atiles,
-                      &c->acounter, &c->asamples, &c->errw, &c->tb_val, &c->tb_der, &c->tb_em, &c->tb_res, &c->tb_bg,
+                      &c->acounter, &c->errw, &c->tb_val, &c->tb_der, &c->tb_em, &c->tb_res, &c->tb_bg,
                       &c->tb_pix, &c->tb_pixels, &c->tb_dfd, &c->tb_vdf, &c->seed_w, &c->seed_sums, &c->seed_carry, &c->seed_map, &c->seed_vox,
                       &c->seed_xyz, &c->gb_pix, &c->gb_pixels, &c->gb_par, &c->hs_tab, &c->hs_part, &c->hs_gg, &c->hs_phi,
                       &c->hs_frame, &c->hs_out, &c->tstate})

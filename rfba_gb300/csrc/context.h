@@ -47,7 +47,7 @@ struct PlanCache {
     RingPlan ring;
     FwdPlan fwd;
     std::vector<float> words;  // the uploaded tables: lane tables, uniform tables, the adjoint's uniform
-                               // and exact-order tables
+                               // and per-point tables
     size_t fwd_utab = 0, adj_utab = 0, fix = 0;  // word offsets in them
 };
 
@@ -167,7 +167,7 @@ struct rfba_ctx {
         long long total = 0;
     } trainb;
     // differentiable path: buffers and the forward the backward can reuse
-    rfba::DevBuf shifted, tmp1, tmp2, gS, gI, gin, dshift, ablocks, atiles, acounter, asamples, errw;
+    rfba::DevBuf shifted, tmp1, tmp2, gS, gI, gin, dshift, ablocks, atiles, acounter, errw;
     struct Train {
         bool valid = false;
         rfba_srrf_config cfg;

@@ -504,7 +504,7 @@ bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err
         const int q0 = o.pair0[i], q1 = i + 1 < npairs ? o.pair0[i + 1] : npts;
         const P& f = o.pts[q0];
         const double ux = f.u[0], um = f.u[1];
-        double pa = 1, pb = 0, ea = 0, eb = 1;
+        double pa = 1, pb = 0, ea = 0, eb = 1, scale = 1;
         int plane[3] = {2, 1, 0};
         if (ux == 0 && um == 0) {
             pa = f.u[2] < 0 ? -1 : 1;
@@ -517,7 +517,7 @@ bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err
                 kappa[q] = o.pts[q].u[2] / h;
                 mean += std::fabs(kappa[q]) / (q1 - q0);
             }
-            const double scale = std::sqrt(1 + mean * mean);
+            scale = std::sqrt(1 + mean * mean);
             pa = ux / h;
             pb = um / h;
             ea = -scale * um / h;
@@ -527,6 +527,7 @@ bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err
         put(ea, ea, eb, eb);
         put_bits(plane[0], plane[1], plane[2], f.a);
         put_bits(q0, q1, x_mask[f.a], 0);
+        U.back() = (float)(kGuard * scale * scale * scale * scale);
     }
     w.clear();
     off.clear();
@@ -564,41 +565,17 @@ bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err
     fp->u_wx = (int)(fp->adj_utab.size() / 4);
     for (auto& t : w_x)
         for (int k : {0, 0, 1, 1, 2, 2, 3, 3}) fp->adj_utab.push_back(t[k]);
-    // exact-order tables, on the volume's axes
-    std::vector<float>& X = fp->fix;
-    X.clear();
     int tile_axis[3];  // of x, y, z
     for (int k = 0; k < 3; ++k) tile_axis[ax[k]] = k;
-    fp->f_idx = 0;
-    for (const P& p : o.pts) {
-        const int v[3] = {p.a, p.b, p.c};
-        for (int k = 0; k < 3; ++k) X.push_back(bits(v[tile_axis[k]]));
-        X.push_back(0.f);
-    }
-    fp->f_frame = (int)X.size();
-    std::vector<float> weight;
-    for (const P& p : o.pts) {
+    fp->fix.clear();
+    for (int q = 0; q < npts; ++q) {
+        const P& p = o.pts[q];
         const double ux = p.u[tile_axis[0]], uy = p.u[tile_axis[1]], uz = p.u[tile_axis[2]];
         const double h = std::sqrt(ux * ux + uy * uy), un = std::sqrt(ux * ux + uy * uy + uz * uz);
-        for (double v : {h > 0 ? ux / h : 1.0, h > 0 ? uy / h : 0.0, h / un, uz / un}) X.push_back((float)v);
-        weight.push_back((float)p.m / (float)n * (2.0f * (float)un));
-        weight.push_back((float)un);
-    }
-    fp->f_weight = (int)X.size();
-    X.insert(X.end(), weight.begin(), weight.end());
-    fp->f_scale = (int)X.size();
-    for (int q = 0; q < npts; ++q) X.push_back((float)std::sqrt(1 + kappa[q] * kappa[q]));
-    while (X.size() % 4) X.push_back(0.f);
-    for (int k = 0; k < 3; ++k) {
-        w.clear();
-        off.clear();
-        for (float v : o.val[tile_axis[k]])
-            if (!taps(tile_axis[k], v, &w, &off)) return false;
-        fp->f_w[k] = (int)X.size();
-        for (auto& t : w) X.insert(X.end(), t.begin(), t.end());
-        fp->f_off[k] = (int)X.size();
-        for (int of : off) X.push_back(bits(of));
-        while (X.size() % 4) X.push_back(0.f);
+        for (double v : {h > 0 ? ux / h : 1.0, h > 0 ? uy / h : 0.0, h / un, uz / un}) fp->fix.push_back((float)v);
+        for (float v : {(float)p.m / (float)n * (2.0f * (float)un), (float)un,
+                        (float)std::sqrt(1 + kappa[q] * kappa[q]), 0.f})
+            fp->fix.push_back(v);
     }
     return true;
 }

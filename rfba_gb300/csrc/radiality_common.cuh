@@ -79,9 +79,12 @@ __device__ __forceinline__ float4 uget(const UTab<UN>& ut, const float4* g, int 
 // order. Ranges (1, 1, 1, 1) share their 6 x 9 loads between the four cells;
 // with smoothing off the reference's central difference is the case mR = 1 and
 // all lateral ranges 0. Integer inputs make the sums exact in float whatever
-// the order.
-template <class Row>
-__device__ __forceinline__ void gradient4(int mode, const int gr[4], Row&& row, int sv, float (&g)[3][4]) {
+// the order. ORDERED adds the terms in the reference's order, i outside j outside k in
+// the volume's x, y, z, whichever axis is innermost (y_inner: y is, and mid is z), so
+// that a float input's gradient does not depend on the plan.
+template <bool ORDERED = false, class Row>
+__device__ __forceinline__ void gradient4(int mode, const int gr[4], Row&& row, int sv, float (&g)[3][4],
+                                          bool y_inner = false) {
     if (mode == 1) {
         float v[6][3][3];  // [w - 1 .. w + 4][mid][x]
 #pragma unroll
@@ -99,10 +102,20 @@ __device__ __forceinline__ void gradient4(int mode, const int gr[4], Row&& row, 
             for (int a = 0; a < 3; ++a)
 #pragma unroll
                 for (int b = 0; b < 3; ++b) {
-                    gx += v[w + b][a][2] - v[w + b][a][0];
+                    if (!ORDERED) gx += v[w + b][a][2] - v[w + b][a][0];
                     gm += v[w + b][2][a] - v[w + b][0][a];
-                    gn += v[w + 2][a][b] - v[w][a][b];
+                    gn += ORDERED ? v[w + 2][b][a] - v[w][b][a] : v[w + 2][a][b] - v[w][a][b];
                 }
+            if (ORDERED) {
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) {
+                        const float(&u)[3] = v[w + b][a];
+                        const float(&s)[3] = v[w + a][b];
+                        gx += y_inner ? s[2] - s[0] : u[2] - u[0];
+                    }
+            }
             g[0][w] = gx;
             g[1][w] = gm;
             g[2][w] = gn;
@@ -121,9 +134,12 @@ __device__ __forceinline__ void gradient4(int mode, const int gr[4], Row&& row, 
         for (int w = 0; w < 4; ++w) {
             float gx = 0.f, gm = 0.f, gn = 0.f;
             auto I = [&](int dx, int dm, int dn) { return row(w + dn)[dm * sv + dx]; };
+            const bool swap = ORDERED && y_inner;
+            const int oR = swap ? zR : yR, pR = swap ? yR : zR;
             for (int i = 1; i <= mR; ++i)
-                for (int j = -yR; j <= yR; ++j)
-                    for (int k = -zR; k <= zR; ++k) gx += I(i, j, k) - I(-i, j, k);
+                for (int j = -oR; j <= oR; ++j)
+                    for (int k = -pR; k <= pR; ++k)
+                        gx += swap ? I(i, k, j) - I(-i, k, j) : I(i, j, k) - I(-i, j, k);
             for (int j = 1; j <= mR; ++j)
                 for (int i = -xR; i <= xR; ++i)
                     for (int k = -zR; k <= zR; ++k) gm += I(i, j, k) - I(i, -j, k);

@@ -82,6 +82,9 @@ struct RingPlan {
     std::vector<float> rx, ry, rz;
 };
 
+// The adjoint's least c2 g2 under 1 / sqrt(c2 g2).
+constexpr float kGuard = 1e-30f;
+
 // Largest uniform table (float4s) that travels in the forward kernel's parameters.
 constexpr int kUTabMax = 768;
 // The same for the adjoint's, which holds the x weights too.
@@ -107,7 +110,7 @@ constexpr int kUAdjMax = 1024;
 // utab, records of float4 (words as int bits where marked *):
 //   groups [ngroups]     {mid value*, first pair*, end pair*, 0}
 //   pairs  [npairs][4]   P = r0.x A + r0.z B: {r0.x, r0.x, r0.z, r0.z}, E likewise,
-//                        {plane of A*, B*, Z*, x value*}, {first point*, end point*, offset mask of the x value*, 0}
+//                        {plane of A*, B*, Z*, x value*}, {first point*, end point*, offset mask of the x value*, kGuard x scale^4}
 //   points [npoints][3]  {kappa, kappa, -kappa, -kappa}, {-sqrt(rho)|u| x 2, sqrt(rho) x 2},
 //                        {first record of the n value's weights*, offset mask*, 0, 0}
 //   wz     [nzv][mz][2]  {w0, w0, w1, w1}, {w2, w2, w3, w3}
@@ -124,9 +127,10 @@ struct FwdPlan {
     // points' second record, and wx [nxv][mx][2] {w0, w0, w1, w1}, {w2, w2, w3, w3} at u_wx
     std::vector<float> adj_utab;
     int u_wx = 0;
-    // AdjFixTables' arrays one after another, their word offsets
+    // per point, for the adjoint's samples in a fixed order: {ca, sb, h, c} with u = |u| (h x' +
+    // c z), x' = (ca, sb) along the volume's (x, y), and {2 weight |u|, |u|, scale, 0}, scale
+    // that of the pair's frame
     std::vector<float> fix;
-    int f_idx = 0, f_frame = 0, f_weight = 0, f_scale = 0, f_w[3] = {0, 0, 0}, f_off[3] = {0, 0, 0};
     int u_grp = 0, u_pair = 0, u_pt = 0, u_wz = 0, u_wi = 0;
     int l_wx = 0, l_offx = 0, l_wm = 0, l_offm = 0;
     int ngroups = 0, npairs = 0, npoints = 0, zero_x = 0, zero_xoff = 0, zero_m = 0;
@@ -155,6 +159,7 @@ struct FwdParams {
     const float* lane;    // lane tables
     int lane_words, l_wx, l_offx, l_wm, l_offm;
     const float4* utab;   // uniform tables in global memory (read when they do not fit the parameters)
+    const float4* fix;    // FwdPlan::fix (the adjoint's)
     int u_count, u_grp, u_pair, u_pt, u_wz, u_wi, u_wx;
     int ngroups, zero_x, zero_xoff, zero_m;
     float neg_weight;     // minus the commonest point's weight
@@ -227,28 +232,6 @@ struct StreamAdjParams {
     unsigned long long* err;
 };
 
-// A ring sample that the radiality adjoint kernel leaves to the exact-order kernel:
-// its element of the adjoint stacks, its point of the plan and the bound it was under.
-struct alignas(16) AdjSample {
-    long long index;
-    int point;
-    float bound;
-};
-constexpr unsigned int kAdjSamples = 1u << 22;      // capacity of a launch's list
-constexpr unsigned int kAdjSamplesOpen = 1u << 18;  // pairs begun after this many take no bound
-
-// The exact-order kernel's tables: per point its value index on each axis and {ca, sb,
-// h, c} (u = |u| (h x' + c z), x' = (ca, sb)), {2 weight |u|, |u|}, and per axis, value and
-// phase the four tap weights and their offset.
-struct AdjFixTables {
-    const int4* idx;
-    const float4* frame;
-    const float2* weight;
-    const float* scale;  // of the kernel's frame against the plain one
-    const float4* w[3];
-    const int* off[3];
-};
-
 // Adjoint inputs and output of the radiality adjoint kernel.
 struct AdjParams {
     const float* gS;  // dL/d(radiality before transforms) per subvoxel and time, [t][v]
@@ -256,16 +239,12 @@ struct AdjParams {
     float* gin;       // dL/dI' accumulated, [t][z][y][x] of the full input
     long long n_in;   // elements of the input / gin
     long long n_stack;  // elements of gS / gI
-    AdjSample* samples;  // samples left to the exact-order kernel, and their number
-    unsigned int* nsamples;
     unsigned long long* err;  // first out-of-range global index (site << 56 | index), 0 if none
 };
 
 // Launchers (radiality.cu / temporal.cu / adjoint.cu). Return a cudaError_t as int.
 int launch_radiality_adjoint(const FwdParams& p, const FwdPlan& plan, const AdjParams& a, int grid, size_t smem,
                              void* stream);
-// Corrects the contributions of the samples that launch_radiality_adjoint put on its list.
-int launch_adjoint_samples(const FwdParams& p, const AdjParams& a, const AdjFixTables& f, int sms, void* stream);
 int radiality_adjoint_u_region(const FwdParams& p);
 size_t radiality_adjoint_smem_bytes(const FwdParams& p);
 int radiality_adjoint_max_ctas_per_sm(const FwdParams& p, int* out);
