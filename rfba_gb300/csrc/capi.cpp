@@ -156,9 +156,10 @@ int order_streams(rfba_ctx* ctx, cudaStream_t st) {
 }
 
 // Turn caller blocks into device block descriptors, splitting regions along z
-// so that one pass's radiality + intensity stack fits the scratch budget.
+// so that one pass's radiality + intensity stack fits the scratch budget. cz: the
+// tiles' depth, 0 to choose it.
 static int make_blocks(rfba_ctx* ctx, const rfba_srrf_config& cfg, const int dims[4], const rfba_block* blocks,
-                       int nblocks, std::vector<BlockDev>* outb, int ty = 0, int tb = 0, int fields = 0) {
+                       int nblocks, std::vector<BlockDev>* outb, int ty = 0, int tb = 0, int fields = 0, int cz = 0) {
     const RingPlan& rp = ctx->plan.ring;
     const int T = dims[3];
     // z slabs are whole tiles deep
@@ -172,7 +173,7 @@ static int make_blocks(rfba_ctx* ctx, const rfba_srrf_config& cfg, const int dim
         }
         regions.push_back(r);
     }
-    const int cz = forward_depth(fp, regions, T, ctx->sm_count);
+    if (cz == 0) cz = forward_depth(fp, regions, T, ctx->sm_count);
     const int FZ = fp.ax2 == 2 ? fp.mag[2] * cz : (ty > 0 ? ty : kTileRows);
     outb->clear();
     // bytes per subvoxel: the stacks of the volumes held at once plus the
@@ -461,8 +462,8 @@ static int enqueue_passes(rfba_ctx* ctx, const rfba_srrf_config& cfg, const void
         if (evs) RFBA_CUDA(rec(evs[3 * i + 2]), "event");
         if (verbose())
             std::fprintf(stderr,
-                         "rfba: pass blocks=%zu tiles=%d ty=%d chunk=%d items=%lld grid=%d smem=%zu batches=%d of %d\n",
-                         pp.b1 - pp.b0, rp.ntiles, ps.ty, pp.chunk, pp.nitems, pp.grid, pp.smem, ps.nbatch, tb);
+                         "rfba: pass blocks=%zu tiles=%d ty=%d cz=%d chunk=%d items=%lld grid=%d smem=%zu batches=%d of %d\n",
+                         pp.b1 - pp.b0, rp.ntiles, ps.ty, ps.cz, pp.chunk, pp.nitems, pp.grid, pp.smem, ps.nbatch, tb);
     }
     return RFBA_OK;
 }
@@ -620,10 +621,11 @@ static std::string sched_key(const rfba_srrf_config& cfg, rfba_dtype dtype, cons
 
 // Autotuner: time every candidate schedule (tile rows, and for
 // block lists the two tile orders) on the first few volumes of this call's
-// own input, keep the fastest.
+// own input, keep the fastest. The tiles have the depth of the whole call (cz), which
+// the few volumes alone might not be given.
 static int autotune(rfba_ctx* ctx, const rfba_srrf_config& cfg, const void* in_dev, rfba_dtype dtype,
-                    const int dims[4], const rfba_block* blocks, int nblocks, float* out_dev, cudaStream_t st,
-                    Tuning* best) {
+                    const int dims[4], const rfba_block* blocks, int nblocks, int cz, float* out_dev,
+                    cudaStream_t st, Tuning* best) {
     const std::vector<int> tys = {kTileRows, 2 * kTileRows};
     std::vector<int> orders = {0};
     if (nblocks > 1) orders.push_back(1);
@@ -642,7 +644,7 @@ static int autotune(rfba_ctx* ctx, const rfba_srrf_config& cfg, const void* in_d
             t.ty = ty;
             t.order = order;
             std::vector<BlockDev> all;
-            if ((rc = make_blocks(ctx, cfg, sd, blocks, nblocks, &all, ty))) break;
+            if ((rc = make_blocks(ctx, cfg, sd, blocks, nblocks, &all, ty, 0, 0, cz))) break;
             float ms = 0.f;
             for (int rep = 0; rep < 2 && !rc; ++rep) {
                 if (rep == 1) cudaEventRecord(e0, st);
@@ -750,7 +752,7 @@ static int forward_blocks_locked(rfba_ctx* ctx, const rfba_srrf_config* cfg, con
                 tin = ctx->in.p;
                 tout = static_cast<float*>(ctx->out.p);
             }
-            if ((s = autotune(ctx, *cfg, tin, dtype, dims, blocks, nblocks, tout, st, &tune))) return s;
+            if ((s = autotune(ctx, *cfg, tin, dtype, dims, blocks, nblocks, all.empty() ? 0 : all[0].cz, tout, st, &tune))) return s;
             ctx->tunes[tkey] = std::make_pair(tune.ty, tune.order);
             ctx->last_tuned = 1;
         }
