@@ -157,7 +157,7 @@ int order_streams(rfba_ctx* ctx, cudaStream_t st) {
 
 // Turn caller blocks into device block descriptors, splitting regions along z
 // so that one pass's radiality + intensity stack fits the scratch budget. cz: the
-// tiles' depth, 0 to choose it.
+// tiles' depth, 0 for the one that suits the volumes a launch holds.
 static int make_blocks(rfba_ctx* ctx, const rfba_srrf_config& cfg, const int dims[4], const rfba_block* blocks,
                        int nblocks, std::vector<BlockDev>* outb, int ty = 0, int tb = 0, int fields = 0, int cz = 0) {
     const RingPlan& rp = ctx->plan.ring;
@@ -173,7 +173,7 @@ static int make_blocks(rfba_ctx* ctx, const rfba_srrf_config& cfg, const int dim
         }
         regions.push_back(r);
     }
-    if (cz == 0) cz = forward_depth(fp, regions, T, ctx->sm_count);
+    if (cz == 0) cz = forward_depth(fp, regions, tb > 0 ? std::min(tb, T) : T, ctx->sm_count);
     const int FZ = fp.ax2 == 2 ? fp.mag[2] * cz : (ty > 0 ? ty : kTileRows);
     outb->clear();
     // bytes per subvoxel: the stacks of the volumes held at once plus the

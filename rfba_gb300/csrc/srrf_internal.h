@@ -291,7 +291,7 @@ FwdParams forward_params(const FwdPlan& fp, const rfba_srrf_config& c, const voi
 FwdParams adjoint_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, const int dims[4]);
 // Tiles of a block's region [lo, hi) in the plan's tile axes (b->cz set).
 void forward_tiles(const FwdPlan& fp, int ty, BlockDev* b);
-// Tile depth (innermost cells, 4 or 8) for these regions of T volumes on sms SMs.
+// Tile depth (innermost cells, 4 or 8) for launches of these regions of T volumes on sms SMs.
 struct FwdRegion {
     int lo[3], hi[3];
 };

@@ -41,3 +41,9 @@ def test_schedule_search_times_the_depth_of_the_call(built_lib, T, cz):
     rows = _depths(T, 20, 24, 24, 0)
     assert {r[0] for r in rows} == {8, 16}, rows  # the search ran
     assert {r[1] for r in rows} == {cz}, rows
+
+
+def test_depth_is_for_the_volumes_of_one_launch(built_lib):
+    """The same map in batches of 4 of 64 volumes: each launch has 4 volumes' items."""
+    rows = [r for r in _depths(64, 20, 24, 24, 4) if r[2] > 1]
+    assert rows and {r[1] for r in rows} == {4}, rows
