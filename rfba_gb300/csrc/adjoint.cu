@@ -1282,7 +1282,7 @@ int with_adj_kernel(const FwdParams& p, F&& f) {
     auto go = [&](auto mz) -> int {
         constexpr int MZ = decltype(mz)::value;
         constexpr int CZ = adj_cz(MZ);
-        return p.u_count <= kUAdjMax ? f(radiality_adjoint_kernel<MZ, CZ, kUAdjMax>, IntC<kUAdjMax>{})
+        return p.u_count <= kUTabMax ? f(radiality_adjoint_kernel<MZ, CZ, kUTabMax>, IntC<kUTabMax>{})
                                      : f(radiality_adjoint_kernel<MZ, CZ, 1>, IntC<1>{});
     };
     switch (p.mag[2]) {

@@ -641,11 +641,11 @@ FwdParams adjoint_params(const FwdPlan& fp, const rfba_srrf_config& c, const voi
 }
 
 int forward_depth(const FwdPlan& fp, const std::vector<FwdRegion>& regions, int T, int sms) {
-    // records too many for the kernel parameters run on the shallow kernel only, and
-    // so do depths whose sums would not fit the registers beside the columns
-    if (fp.utab.size() / 4 > (size_t)kUTabMax || fp.mag[2] > 5) return 4;
+    if (fp.mag[2] > kDeepMag) return 4;
     // time per tile column in clocks (one SM, as measured): a point at one subvoxel
-    // 29, a pair's second pass at one cell 22, a group's first pass at one cell 7
+    // 29, a pair's second pass at one cell 22, a group's first pass at one cell 7. The
+    // same holds for tables in global memory: 20 volumes of 32^3 at 2 x 2 x 2 and 16 axes
+    // take 3.82 ms with shallow tiles, 3.13 with deep ones (24^3 at 4 x 4 x 2: 4.65, 4.56)
     double time[2] = {0, 0};
     long long items = 0;  // (tile, volume) pairs of the deep tiles
     for (int i = 0; i < 2; ++i) {

@@ -551,9 +551,13 @@ template <class F>
 int with_kernel(const FwdParams& p, F&& f) {
     auto go = [&](auto mz) -> int {
         constexpr int MZ = decltype(mz)::value;
-        if (p.u_count > kUTabMax) return f(radiality_kernel<MZ, 4, 1>, IntC<1>{});
-        if (p.cz == 8) return f(radiality_kernel<MZ, 8, kUTabMax>, IntC<kUTabMax>{});
-        return f(radiality_kernel<MZ, 4, kUTabMax>, IntC<kUTabMax>{});
+        const bool global = p.u_count > kUTabMax;
+        if constexpr (MZ <= kDeepMag)
+            if (p.cz == 8)
+                return global ? f(radiality_kernel<MZ, 8, 1>, IntC<1>{})
+                              : f(radiality_kernel<MZ, 8, kUTabMax>, IntC<kUTabMax>{});
+        return global ? f(radiality_kernel<MZ, 4, 1>, IntC<1>{})
+                      : f(radiality_kernel<MZ, 4, kUTabMax>, IntC<kUTabMax>{});
     };
     switch (p.mag[2]) {
         case 1: return go(IntC<1>{});

@@ -85,10 +85,16 @@ struct RingPlan {
 // The adjoint's least c2 g2 under 1 / sqrt(c2 g2).
 constexpr float kGuard = 1e-30f;
 
-// Largest uniform table (float4s) that travels in the forward kernel's parameters.
-constexpr int kUTabMax = 768;
-// The same for the adjoint's, which holds the x weights too.
-constexpr int kUAdjMax = 1024;
+// Largest uniform table (float4s) that travels in the parameters of the radiality kernel
+// or its adjoint: parameters hold 32764 bytes. Rings of 12 axes and most of 13 fit (the
+// adjoint's table, which has the x weights too, up to 10 to 12). 20 volumes of 32^3 at 2 x 2
+// x 2, ms with a limit of 768 (1024), whose rings of 9 axes and more read global memory, and
+// now: 9 axes 1.34 and 1.02, 12 axes 2.20 and 1.76; with the adjoint 4.46 and 4.14, 8.79
+// and 6.91. Smaller tables lose nothing (5 x 10x12x12: 55.5 us either way).
+constexpr int kUTabMax = 1984;
+// Deepest innermost magnification with tiles of 8 cells: above it the sums would not fit
+// the registers beside the columns.
+constexpr int kDeepMag = 5;
 
 // The forward kernel's plan of a configuration. Its tiles run over (x, mid,
 // innermost) = (x, y, z) or (x, z, y). The first pass filters along mid, once for

@@ -1,4 +1,5 @@
-"""The cases of the deep-tile tests get deep tiles, their two-volume forms shallow ones."""
+"""The cases of the deep-tile tests get deep tiles, their two-volume forms shallow ones,
+and the rings of tests/test_large_rings_gpu.py lie on both sides of the table limit."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -6,8 +7,10 @@ from pathlib import Path
 import pytest
 
 from tests.test_deep_tiles_gpu import CASES
+from tests.test_large_rings_gpu import RINGS
 
 ROOT = Path(__file__).resolve().parent.parent
+UTAB_MAX = 1984  # kUTabMax
 
 
 @pytest.fixture(scope="module")
@@ -29,6 +32,12 @@ def plans(built_lib, tmp_path_factory):
 
 
 def test_series_of_the_deep_cases_get_deep_tiles(plans):
-    rows = [(mag, axes, shape) for mag, shape, axes, _, _ in CASES]
+    rows = [(mag, axes, shape) for mag, shape, axes, _, _ in CASES] + [tuple(r) for r in RINGS]
     assert [r[0] for r in plans(rows)] == [8] * len(rows)
     assert {r[0] for r in plans([(m, a, (2,) + s[1:]) for m, a, s in rows])} == {4}
+
+
+def test_rings_lie_on_both_sides_of_the_table_limit(plans):
+    sizes = plans(RINGS)
+    assert {s[1] <= UTAB_MAX for s in sizes} == {True, False}
+    assert {s[2] <= UTAB_MAX for s in sizes} == {True, False}
