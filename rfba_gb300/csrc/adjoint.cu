@@ -121,25 +121,6 @@ __global__ void __launch_bounds__(256) shift_adjoint_kernel(const float* __restr
     }
 }
 
-// dL/dd[t][axis] = sum over volume t of g[t] * dv[t] (double accumulation).
-__global__ void drift_dot_kernel(const float* __restrict__ g, const float* __restrict__ dv, long long nv, int axis,
-                                 double* __restrict__ out, unsigned long long* err) {
-    const int t = blockIdx.y;
-    const float* gt = g + (long long)t * nv;
-    const float* dt = dv + (long long)t * nv;
-    double acc = 0.0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x)
-        acc += (double)gt[i] * (double)dt[i];
-    __shared__ double red[256];
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) atomicAdd(out + 3 * t + axis, red[0]);
-}
-
 // Drift operator on all three axes at once: the x-, y- and z-passes with
 // per-axis index clamping compose to one 4 x 4 x 4 tensor-product stencil with
 // clamped indices. mode 0 writes I'_t; mode 1 adds, per volume, the sums over
@@ -783,7 +764,7 @@ __device__ __noinline__ void fix_marked(const FixTile& f, int pair, int u0, int 
 }
 
 template <int MZ, int CZ, int UN>
-__global__ void __maxnreg__(adj_regs(MZ, CZ))
+__global__ void __maxnreg__(kAdjRegs)
     radiality_adjoint_kernel(const __grid_constant__ FwdParams p, const __grid_constant__ AdjParams a,
                              const __grid_constant__ UTab<UN> ut) {
     constexpr int CH = CZ / 2;
@@ -1379,13 +1360,6 @@ int launch_drift3d(const float* src, float* dst, const float* g, int W, int H, i
     dim3 grid((unsigned)std::min<long long>((warps + 7) / 8, 152LL * 64), (unsigned)T);
     auto k = mode == 0 ? drift3d_kernel<0> : drift3d_kernel<1>;
     k<<<grid, kDriftThreads, 0, static_cast<cudaStream_t>(stream)>>>(src, dst, g, W, H, D, L, shifts, out);
-    return (int)cudaGetLastError();
-}
-
-int launch_drift_dot(const float* g, const float* dv, long long nv, int T, int axis, double* out,
-                     unsigned long long* err, void* stream) {
-    dim3 grid((unsigned)std::min<long long>((nv + 255) / 256, 64), (unsigned)T);
-    drift_dot_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(g, dv, nv, axis, out, err);
     return (int)cudaGetLastError();
 }
 

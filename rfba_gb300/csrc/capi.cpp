@@ -215,7 +215,6 @@ static int make_blocks(rfba_ctx* ctx, const rfba_srrf_config& cfg, const int dim
             s.hi[2] = (int)std::min<long long>(b.hi[2], z0 + slab);
             s.out_offset = d.out_offset + (long long)(z0 - b.lo[2]) * d.out_stride[2];
             for (int a = 0; a < 3; ++a) s.nreg[a] = s.hi[a] - s.lo[a];
-            s.zbase = (s.lo[2] / cfg.mag[2]) * cfg.mag[2];
             forward_tiles(fp, ty, &s);
             s.vox = (long long)s.nreg[0] * s.nreg[1] * s.nreg[2];
             outb->push_back(s);

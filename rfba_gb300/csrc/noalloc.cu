@@ -187,7 +187,6 @@ extern "C" int rfba_srrf_forward_static_scratch(const rfba_srrf_config* cfg, con
         window_range(cfg->ring_radius, rc, cfg->mag[a], dims[a], &b.rad_lo[a], &b.rad_hi[a]);
         fine_window_int(cfg->mag[a], dims[a], &b.int_lo[a], &b.int_hi[a]);
     }
-    b.zbase = 0;
     b.cz = forward_depth(plan, {{{0, 0, 0}, {b.hi[0], b.hi[1], b.hi[2]}}}, T, 0);
     forward_tiles(plan, 0, &b);
     b.vox = (long long)b.nreg[0] * b.nreg[1] * b.nreg[2];

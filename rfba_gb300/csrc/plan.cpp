@@ -226,21 +226,10 @@ bool build_ring_plan(const rfba_srrf_config& c, RingPlan* rp, std::string* err) 
     std::sort(yv.begin(), yv.end());
     std::sort(zv.begin(), zv.end());
     struct P {
-        int a, b, c, m;
-        float x, y, z;
+        int a, b, c;
     };
     std::vector<P> pts;
-    for (size_t k = 0; k < reps.size(); ++k) {
-        P p;
-        p.a = value_index(xv, reps[k][0], tol);
-        p.b = value_index(yv, reps[k][1], tol);
-        p.c = value_index(zv, reps[k][2], tol);
-        p.m = mult[k];
-        p.x = reps[k][0];
-        p.y = reps[k][1];
-        p.z = reps[k][2];
-        pts.push_back(p);
-    }
+    for (auto& p : reps) pts.push_back({value_index(xv, p[0], tol), value_index(yv, p[1], tol), value_index(zv, p[2], tol)});
     std::sort(pts.begin(), pts.end(), [](const P& u, const P& v) {
         return std::tie(u.a, u.b, u.c) < std::tie(v.a, v.b, v.c);
     });
@@ -252,8 +241,6 @@ bool build_ring_plan(const rfba_srrf_config& c, RingPlan* rp, std::string* err) 
     rp->pair_yval.clear();
     rp->pair_pt.clear();
     rp->pt_zval.clear();
-    rp->pt_vec.clear();
-    rp->pair_rot.clear();
     rp->zero_x = rp->zero_y = -1;
     for (size_t i = 0; i < xv.size(); ++i)
         if (xv[i] == 0.f) rp->zero_x = (int)i;
@@ -272,21 +259,12 @@ bool build_ring_plan(const rfba_srrf_config& c, RingPlan* rp, std::string* err) 
             last_a = p.a;
             last_b = -1;
         }
-        const double ux = (double)p.x / r, uy = (double)p.y / r, uz = (double)p.z / r;
-        const double hxy = std::sqrt(ux * ux + uy * uy);
-        const double un = std::sqrt(ux * ux + uy * uy + uz * uz);
         if (p.b != last_b) {
             rp->pair_yval.push_back(p.b);
             rp->pair_pt.push_back((int)k);
             last_b = p.b;
-            rp->pair_rot.push_back(hxy > 0 ? (float)(ux / hxy) : 1.f);
-            rp->pair_rot.push_back(hxy > 0 ? (float)(uy / hxy) : 0.f);
         }
         rp->pt_zval.push_back(p.c);
-        rp->pt_vec.push_back((float)(hxy / un));
-        rp->pt_vec.push_back((float)(uz / un));
-        rp->pt_vec.push_back((float)p.m / (float)n);  // kernel.cu:244 divides by n, not n^2
-        rp->pt_vec.push_back((float)(-un));
     }
     rp->grp.push_back((int)rp->pair_yval.size());
     rp->pair_pt.push_back((int)pts.size());

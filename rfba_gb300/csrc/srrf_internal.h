@@ -17,7 +17,7 @@ namespace rfba {
 // TY = kTileRows unless tuned) and FZ = MZ * CZ subvoxels deep along its innermost axis, held in registers.
 constexpr int kTileX = 16;
 constexpr int kTileRows = 8;
-constexpr int kMaxThreads = 256;  // 16 x 16 threads for the 32-row tile (mid magnification 8)
+constexpr int kMaxThreads = 256;  // 16 x 16, the taller tile of the schedule search
 constexpr int kMaxMag = 8;
 constexpr int kMaxGradRange = 3;
 // The forward kernel's register limit for MZ x CZ tiles: MZ CZ for the sums and
@@ -25,10 +25,10 @@ constexpr int kMaxGradRange = 3;
 constexpr int fwd_regs(int mz, int cz) { return mz * cz + 6 * (cz / 2 + 4) <= 88 ? 128 : 168; }
 
 // The adjoint's tile depth (it holds two sets of columns), its register limit (12
-// (CZ / 2 + 4) for the columns, MZ CZ for dL/dS) and the width of an exchange row
-// per x phase (the tile's coarse cells and four zeros).
+// (CZ / 2 + 4) for the columns and MZ CZ for dL/dS leave no instance below 128) and the
+// width of an exchange row per x phase (the tile's coarse cells and four zeros).
 constexpr int adj_cz(int mz) { return mz <= 4 ? 8 : 4; }
-constexpr int adj_regs(int mz, int cz) { return mz * cz + 12 * (cz / 2 + 4) <= 88 ? 128 : 168; }
+constexpr int kAdjRegs = 168;
 #ifdef __CUDACC__
 __host__ __device__
 #endif
@@ -44,7 +44,6 @@ struct BlockDev {
     int rad_hi[3];
     int int_lo[3];   // fine indices whose centre passes the window (inclusive)
     int int_hi[3];
-    int zbase;       // first fine z of the tile grid (multiple of mz, <= lo[2])
     int ntile[3];    // tiles along x, y, z
     int nreg[3];     // region extent hi - lo
     int cz;          // coarse cells per forward tile along its innermost axis (4 or 8)
@@ -73,9 +72,6 @@ struct RingPlan {
     std::vector<int> pair_yval;    // per pair: y value index
     std::vector<int> pair_pt;      // npairs + 1
     std::vector<int> pt_zval;      // per point: z value index
-    std::vector<float> pt_vec;     // per point: h, c, multiplicity/n, -|u| (u = (x, y, z)/radius
-                                   // = |u| (h x' + c z) in the pair's rotated frame)
-    std::vector<float> pair_rot;   // per pair: x' = (ux, uy)/|(ux, uy)|, (1, 0) on the z axis
     int zero_x = -1, zero_y = -1;  // value index of 0 on x and y
     int npoints_raw = 0;
     // Raw float ring (n*n points) exactly as the reference builds it.
@@ -263,8 +259,6 @@ int launch_shift_adjoint(const float* src, float* dst, int W, int H, int D, int 
 // sum_voxels g * dI'/dd_a into out[3 t + a] (FP64).
 int launch_drift3d(const float* src, float* dst, const float* g, int W, int H, int D, int T, const float* shifts,
                    int mode, double* out, void* stream);
-int launch_drift_dot(const float* g, const float* dv, long long nv, int T, int axis, double* out,
-                     unsigned long long* err, void* stream);
 int launch_double_to_float(const double* src, float* dst, int n, void* stream);
 int launch_radiality(const FwdParams& p, const FwdPlan& plan, int grid, size_t smem, void* stream);
 // Box width (elements) of the TMA input staging for this tile, 0 when the input
