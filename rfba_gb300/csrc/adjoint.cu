@@ -1329,9 +1329,9 @@ int launch_temporal_adjoint(const BlockDev* blocks, long long vox, const float* 
 }
 
 int launch_shift_adjoint(const float* src, float* dst, int W, int H, int D, int T, int axis, const float* shifts,
-                         void* stream) {
+                         int sms, void* stream) {
     const long long rows = (long long)D * H * T;
-    const unsigned grid = (unsigned)std::min<long long>((rows + 7) / 8, 152LL * 64);
+    const unsigned grid = (unsigned)std::min<long long>((rows + 7) / 8, 64LL * sms);
     auto k = axis == 0 ? shift_adjoint_kernel<0> : axis == 1 ? shift_adjoint_kernel<1> : shift_adjoint_kernel<2>;
     k<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(src, dst, W, H, D, T, shifts);
     return (int)cudaGetLastError();
@@ -1351,13 +1351,13 @@ int launch_double_to_float(const double* src, float* dst, int n, void* stream) {
 }
 
 int launch_drift3d(const float* src, float* dst, const float* g, int W, int H, int D, int T, const float* shifts,
-                   int mode, double* out, void* stream) {
+                   int mode, double* out, int sms, void* stream) {
     // walks of 16 planes (19 planes' taps for 16 of output) where they leave every SM
     // its warps, else of 4, whose chain of loads is shorter
     const long long cols = (long long)((W + 31) / 32) * H;
-    const int L = cols * ((D + 15) / 16) * T >= 152 * 16 ? 16 : 4;
+    const int L = cols * ((D + 15) / 16) * T >= 16LL * sms ? 16 : 4;
     const long long warps = cols * ((D + L - 1) / L);
-    dim3 grid((unsigned)std::min<long long>((warps + 7) / 8, 152LL * 64), (unsigned)T);
+    dim3 grid((unsigned)std::min<long long>((warps + 7) / 8, 64LL * sms), (unsigned)T);
     auto k = mode == 0 ? drift3d_kernel<0> : drift3d_kernel<1>;
     k<<<grid, kDriftThreads, 0, static_cast<cudaStream_t>(stream)>>>(src, dst, g, W, H, D, L, shifts, out);
     return (int)cudaGetLastError();

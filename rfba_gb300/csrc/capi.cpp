@@ -974,7 +974,7 @@ static int apply_drift(rfba_ctx* ctx, const float* in, const float* shifts, cons
         (s = ctx->tmp2.ensure(n * 4, "scratch")))
         return s;
     float* out = static_cast<float*>(ctx->shifted.p);
-    const int e = launch_drift3d(in, out, nullptr, dims[0], dims[1], dims[2], dims[3], shifts, 0, nullptr, st);
+    const int e = launch_drift3d(in, out, nullptr, dims[0], dims[1], dims[2], dims[3], shifts, 0, nullptr, ctx->sm_count, st);
     if (e) return cuda_fail((cudaError_t)e, "drift resampling");
     ctx->launches += 1;
     *iprime = out;
@@ -1403,15 +1403,15 @@ static int backward_locked(rfba_ctx* ctx, const rfba_srrf_config* cfg, const flo
     if (shifts) {
         float* t1 = static_cast<float*>(ctx->tmp1.p);
         float* t2 = static_cast<float*>(ctx->tmp2.p);
-        e = launch_shift_adjoint(gin, t1, dims[0], dims[1], dims[2], T, 2, shifts, st);
-        if (!e) e = launch_shift_adjoint(t1, t2, dims[0], dims[1], dims[2], T, 1, shifts, st);
-        if (!e) e = launch_shift_adjoint(t2, din, dims[0], dims[1], dims[2], T, 0, shifts, st);
+        e = launch_shift_adjoint(gin, t1, dims[0], dims[1], dims[2], T, 2, shifts, ctx->sm_count, st);
+        if (!e) e = launch_shift_adjoint(t1, t2, dims[0], dims[1], dims[2], T, 1, shifts, ctx->sm_count, st);
+        if (!e) e = launch_shift_adjoint(t2, din, dims[0], dims[1], dims[2], T, 0, shifts, ctx->sm_count, st);
         ctx->launches += 3;
         if (!e && dshift) {
             if ((s = ctx->dshift.ensure((size_t)T * 3 * sizeof(double), "drift adjoint"))) return s;
             double* ds = static_cast<double*>(ctx->dshift.p);
             RFBA_CUDA(cudaMemsetAsync(ds, 0, (size_t)T * 3 * sizeof(double), st), "drift adjoint clear");
-            e = launch_drift3d(in, nullptr, gin, dims[0], dims[1], dims[2], T, shifts, 1, ds, st);
+            e = launch_drift3d(in, nullptr, gin, dims[0], dims[1], dims[2], T, shifts, 1, ds, ctx->sm_count, st);
             ctx->launches += 1;
             if (!e) e = launch_double_to_float(ds, dshift, 3 * T, st);
             ctx->launches += 1;

@@ -254,11 +254,11 @@ int launch_temporal_adjoint(const BlockDev* blocks, long long vox, const float* 
                             const float* gmap, int T, int method, int itc, int order, int iw, int renorm, int poscon,
                             float* gS, float* gI, long long nmap, unsigned long long* err, void* stream);
 int launch_shift_adjoint(const float* src, float* dst, int W, int H, int D, int T, int axis, const float* shifts,
-                         void* stream);
+                         int sms, void* stream);
 // Drift operator, all axes fused: mode 0 resamples src into dst; mode 1 adds
 // sum_voxels g * dI'/dd_a into out[3 t + a] (FP64).
 int launch_drift3d(const float* src, float* dst, const float* g, int W, int H, int D, int T, const float* shifts,
-                   int mode, double* out, void* stream);
+                   int mode, double* out, int sms, void* stream);
 int launch_double_to_float(const double* src, float* dst, int n, void* stream);
 int launch_radiality(const FwdParams& p, const FwdPlan& plan, int grid, size_t smem, void* stream);
 // Box width (elements) of the TMA input staging for this tile, 0 when the input
