@@ -323,9 +323,10 @@ static int plan_passes(rfba_ctx* ctx, const rfba_srrf_config& cfg, rfba_dtype dt
         pp.vox = vox;
         ps->max_vox = std::max(ps->max_vox, vox);
         const long long nt = (long long)(pp.t1 - pp.t0);
-        // time chunk: enough work items for 64 per CTA slot, so that the last round
-        // of items leaves the chip idle for at most 1 / 64 of the launch (an item
-        // costs a few microseconds beyond its volumes' 100 and more each)
+        // time chunk: 64 work items per CTA slot where there are that many (tile, volume)
+        // pairs, so that the last round of items leaves the chip idle for at most 1 / 64 of
+        // the launch, else an item for each pair (an item costs a few microseconds beyond
+        // its volumes' 100 and more each)
         int chunk = ctx->chunk_override;
         if (chunk <= 0) {
             const long long want = 64LL * slots;
@@ -1101,8 +1102,9 @@ static int forward_shifted_locked(rfba_ctx* ctx, const rfba_srrf_config* cfg, co
         return s;
     // the backward can reuse this forward's stacks when they are all resident
     // (one spatial pass over the whole series at once: a forward in time batches
-    // keeps only its last batch) and the temporal reduction left them intact
-    // (ITC 1 bins the series in place)
+    // keeps only its last batch) and the temporal reduction leaves them intact at
+    // any length (ITC 1 bins a series in place that is too long for its column of
+    // shared memory)
     if (!rlo && ctx->last_passes == 1 && ctx->last_time_batch == 0 && !(cfg->method == 3 && cfg->itc == 1)) {
         std::vector<BlockDev> all;
         if ((s = make_blocks(ctx, *cfg, dims, &b, 1, &all))) return s;
@@ -1385,7 +1387,7 @@ static int backward_locked(rfba_ctx* ctx, const rfba_srrf_config* cfg, const flo
         std::vector<BlockDev> all;
         if (btb == 0 && (s = make_blocks(ctx, *cfg, dims, &b, 1, &all))) return s;
         // the recomputed stacks must stay as the radiality kernel wrote them: TRAC
-        // with ITC 1 would bin them in place, so its map (unused here) is formed
+        // with ITC 1 bins a long series in place, so its map (unused here) is formed
         // with ITC 0, which only reads them
         rfba_srrf_config fcfg = *cfg;
         if (fcfg.method == 3) fcfg.itc = 0;
