@@ -655,6 +655,7 @@ __device__ __forceinline__ Derivative sample_derivative(float P, float E, float 
 // What the correction needs of a tile and time point.
 struct FixTile {
     const FwdParams* p;
+    const float4* fix;
     const float4* gt;  // gradient planes [NQ][nv][nu]
     float4* gu;        // dL/dU planes [NQ][ty][nu]
     const float* wx;   // the x values' tap weights
@@ -707,7 +708,7 @@ __device__ __noinline__ void fix_marked(const FixTile& f, int pair, int u0, int 
             const float gS = f.gS[at + z * f.zstride];
 #pragma unroll 1
             for (int qi = __float_as_int(r3.x); qi < __float_as_int(r3.y); ++qi) {
-                const float4 fr = __ldg(p.fix + 2 * qi), wt = __ldg(p.fix + 2 * qi + 1);
+                const float4 fr = __ldg(f.fix + 2 * qi), wt = __ldg(f.fix + 2 * qi + 1);
                 const float4 c = __ldg(p.utab + p.u_pt + 3 * qi + 2);
                 // weights along the innermost axis: every second word of their record
                 const float* wi = reinterpret_cast<const float*>(p.utab + p.u_wz + 2 * (__float_as_int(c.x) + z % MZ));
@@ -1141,7 +1142,7 @@ __global__ void __maxnreg__(kAdjRegs)
                     x_transpose(gZ, xv, mask, gu + pc * uplane, true);
                     if (__any_sync(0xffffffffu, marked != 0)) {
                         __syncwarp();  // the row's sums above
-                        const FixTile f = {&p, gt, gu, wx, s_weight, s_base, a.gS, zstride};
+                        const FixTile f = {&p, a.fix, gt, gu, wx, s_weight, s_base, a.gS, zstride};
                         fix_marked<MZ, CZ>(f, pi, xi - cx0 - 2 + offx[ax], ax, bound, sbase, marked);
                     }
                 }
@@ -1299,7 +1300,7 @@ int launch_radiality_adjoint(const FwdParams& p, const FwdPlan& plan, const AdjP
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     return with_adj_kernel(p, [&](auto k, auto n) -> int {
         constexpr int UN = decltype(n)::value;
-        const cudaError_t e = allow_shared(k, smem);
+        const cudaError_t e = allow_shared(k, smem, kStaticShared);
         if (e != cudaSuccess) return (int)e;
         UTab<UN> tab;
         std::memset(&tab, 0, sizeof tab);
@@ -1312,7 +1313,7 @@ int launch_radiality_adjoint(const FwdParams& p, const FwdPlan& plan, const AdjP
 int radiality_adjoint_max_ctas_per_sm(const FwdParams& p, int* out) {
     const size_t smem = radiality_adjoint_smem_bytes(p);
     return with_adj_kernel(p, [&](auto k, auto) -> int {
-        const cudaError_t e = allow_shared(k, smem);
+        const cudaError_t e = allow_shared(k, smem, kStaticShared);
         if (e != cudaSuccess) return (int)e;
         return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k, p.TY * kTileX, smem);
     });

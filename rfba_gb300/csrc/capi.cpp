@@ -1168,7 +1168,6 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
     FwdParams rp = adjoint_params(fp, *cfg, iprime, dims);
     rp.lane = static_cast<const float*>(ctx->tables.p);
     rp.utab = reinterpret_cast<const float4*>(rp.lane + ctx->plan.adj_utab);
-    rp.fix = reinterpret_cast<const float4*>(rp.lane + ctx->plan.fix);
     rp.blocks = dblk;
     rp.tiles = static_cast<const TileDesc*>(ctx->atiles.p);
     rp.ntiles = (int)tiles.size();
@@ -1198,6 +1197,7 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
     AdjParams ap{gS,
                  gI,
                  static_cast<float*>(ctx->gin.p),
+                 reinterpret_cast<const float4*>(rp.lane + ctx->plan.fix),
                  (long long)nin,
                  (long long)V * TW,
                  err};

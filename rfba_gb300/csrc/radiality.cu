@@ -551,13 +551,15 @@ template <class F>
 int with_kernel(const FwdParams& p, F&& f) {
     auto go = [&](auto mz) -> int {
         constexpr int MZ = decltype(mz)::value;
-        const bool global = p.u_count > kUTabMax;
+        auto depth = [&](auto cz) -> int {
+            constexpr int CZ = decltype(cz)::value;
+            if (p.u_count > kUTabMax) return f(radiality_kernel<MZ, CZ, 1>, IntC<1>{});
+            if (p.u_count > kUTabSmall) return f(radiality_kernel<MZ, CZ, kUTabMax>, IntC<kUTabMax>{});
+            return f(radiality_kernel<MZ, CZ, kUTabSmall>, IntC<kUTabSmall>{});
+        };
         if constexpr (MZ <= kDeepMag)
-            if (p.cz == 8)
-                return global ? f(radiality_kernel<MZ, 8, 1>, IntC<1>{})
-                              : f(radiality_kernel<MZ, 8, kUTabMax>, IntC<kUTabMax>{});
-        return global ? f(radiality_kernel<MZ, 4, 1>, IntC<1>{})
-                      : f(radiality_kernel<MZ, 4, kUTabMax>, IntC<kUTabMax>{});
+            if (p.cz == 8) return depth(IntC<8>{});
+        return depth(IntC<4>{});
     };
     switch (p.mag[2]) {
         case 1: return go(IntC<1>{});
@@ -602,7 +604,7 @@ int launch_radiality(const FwdParams& p, const FwdPlan& plan, int grid, size_t s
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     return with_kernel(p, [&](auto k, auto n) -> int {
         constexpr int UN = decltype(n)::value;
-        const cudaError_t e = allow_shared(k, smem);
+        const cudaError_t e = allow_shared(k, smem, kStaticShared);
         if (e != cudaSuccess) return (int)e;
         FwdParams q = p;
         CUtensorMap map;
@@ -623,7 +625,7 @@ int launch_radiality(const FwdParams& p, const FwdPlan& plan, int grid, size_t s
 int radiality_max_ctas_per_sm(const FwdParams& p, int* out) {
     const size_t smem = radiality_smem_bytes(p);
     return with_kernel(p, [&](auto k, auto) -> int {
-        const cudaError_t e = allow_shared(k, smem);
+        const cudaError_t e = allow_shared(k, smem, kStaticShared);
         if (e != cudaSuccess) return (int)e;
         return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k, p.TY * kTileX, smem);
     });

@@ -20,6 +20,9 @@ constexpr int kTileRows = 8;
 constexpr int kMaxThreads = 256;  // 16 x 16, the taller tile of the schedule search
 constexpr int kMaxMag = 8;
 constexpr int kMaxGradRange = 3;
+// Bound on the static shared memory of the radiality kernel and its adjoint; no configuration
+// needs more dynamic shared memory than it leaves of a block's.
+constexpr size_t kStaticShared = 1024;
 // The forward kernel's register limit for MZ x CZ tiles: MZ CZ for the sums and
 // 6 (CZ / 2 + 4) for the x-filtered columns are live through the point loop.
 constexpr int fwd_regs(int mz, int cz) { return mz * cz + 6 * (cz / 2 + 4) <= 88 ? 128 : 168; }
@@ -86,8 +89,11 @@ constexpr float kGuard = 1e-30f;
 // adjoint's table, which has the x weights too, up to 10 to 12). 20 volumes of 32^3 at 2 x 2
 // x 2, ms with a limit of 768 (1024), whose rings of 9 axes and more read global memory, and
 // now: 9 axes 1.34 and 1.02, 12 axes 2.20 and 1.76; with the adjoint 4.46 and 4.14, 8.79
-// and 6.91. Smaller tables lose nothing (5 x 10x12x12: 55.5 us either way).
+// and 6.91.
 constexpr int kUTabMax = 1984;
+// Largest table in the smaller parameters: every launch copies all of them, and a call on a
+// host buffer of 5 x 10x12x12 takes 102 us with 1984 records, 98 with 768.
+constexpr int kUTabSmall = 768;
 // Deepest innermost magnification with tiles of 8 cells: above it the sums would not fit
 // the registers beside the columns.
 constexpr int kDeepMag = 5;
@@ -161,7 +167,6 @@ struct FwdParams {
     const float* lane;    // lane tables
     int lane_words, l_wx, l_offx, l_wm, l_offm;
     const float4* utab;   // uniform tables in global memory (read when they do not fit the parameters)
-    const float4* fix;    // FwdPlan::fix (the adjoint's)
     int u_count, u_grp, u_pair, u_pt, u_wz, u_wi, u_wx;
     int ngroups, zero_x, zero_xoff, zero_m;
     float neg_weight;     // minus the commonest point's weight
@@ -239,6 +244,7 @@ struct AdjParams {
     const float* gS;  // dL/d(radiality before transforms) per subvoxel and time, [t][v]
     const float* gI;  // dL/d(interpolated intensity), [t][v]
     float* gin;       // dL/dI' accumulated, [t][z][y][x] of the full input
+    const float4* fix;  // FwdPlan::fix
     long long n_in;   // elements of the input / gin
     long long n_stack;  // elements of gS / gI
     unsigned long long* err;  // first out-of-range global index (site << 56 | index), 0 if none

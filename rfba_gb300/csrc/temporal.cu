@@ -299,7 +299,7 @@ int launch_temporal(const TemporalParams& p, void* stream) {
                                     : p.order == 4 ? trac_itc_kernel<4>
                                                    : trac_itc_kernel<2>;
         if (smem > 48 * 1024) {
-            const cudaError_t e = allow_shared(k, smem);
+            const cudaError_t e = allow_shared(k, smem, 0);
             if (e != cudaSuccess) return (int)e;
         }
         const long long grid = (p.total_vox + kColThreads - 1) / kColThreads;
