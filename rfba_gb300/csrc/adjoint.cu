@@ -689,7 +689,7 @@ __device__ __forceinline__ void store_shared(float* p, float v) {
 template <int MZ, int CZ>
 __device__ __noinline__ void fix_marked(const FixTile& f, int pair, int u0, int ax, float bound, long long sbase,
                                         unsigned int marked) {
-    constexpr int NQ = CZ / 4 + 1;
+    constexpr int NQ = tile_quads(CZ);
     const unsigned int full = 0xffffffffu;
     const FwdParams& p = *f.p;
     const int lane = threadIdx.x & 31, o = (lane >> 2) & 3, i = lane & 3;
@@ -773,7 +773,7 @@ __global__ void __maxnreg__(kAdjRegs)
     constexpr int FZ = MZ * CZ;
     constexpr int NH = CH + 4;
     constexpr int NW = CZ + 4;
-    constexpr int NQ = NW / 4;
+    constexpr int NQ = tile_quads(CZ);
     static_assert(FZ <= 32, "a column's marks fit a word");
     extern __shared__ float4 smem4[];
 
@@ -1264,8 +1264,9 @@ int with_adj_kernel(const FwdParams& p, F&& f) {
     auto go = [&](auto mz) -> int {
         constexpr int MZ = decltype(mz)::value;
         constexpr int CZ = adj_cz(MZ);
-        return p.u_count <= kUTabMax ? f(radiality_adjoint_kernel<MZ, CZ, kUTabMax>, IntC<kUTabMax>{})
-                                     : f(radiality_adjoint_kernel<MZ, CZ, 1>, IntC<1>{});
+        if (p.u_count > kUTabMax) return f(radiality_adjoint_kernel<MZ, CZ, 1>, IntC<1>{});
+        if (p.cz < CZ) return f(radiality_adjoint_kernel<MZ, CZ / 2, kUTabMax>, IntC<kUTabMax>{});
+        return f(radiality_adjoint_kernel<MZ, CZ, kUTabMax>, IntC<kUTabMax>{});
     };
     switch (p.mag[2]) {
         case 1: return go(IntC<1>{});
@@ -1284,12 +1285,12 @@ int with_adj_kernel(const FwdParams& p, F&& f) {
 
 // float4s of the place that U, the input tile and the intensity's cells share
 int radiality_adjoint_u_region(const FwdParams& p) {
-    const int nq = p.cz / 4 + 1;
+    const int nq = tile_quads(p.cz);
     return std::max(std::max(3 * nq * p.TY * p.NU, (p.NIX * p.NIY * p.NIZ + 3) / 4), nq * p.NV * p.NU);
 }
 
 size_t radiality_adjoint_smem_bytes(const FwdParams& p) {
-    const int nq = p.cz / 4 + 1, warps = p.TY * kTileX / 32;
+    const int nq = tile_quads(p.cz), warps = p.TY * kTileX / 32;
     const size_t f4 = (size_t)6 * nq * p.NV * p.NU + p.u_region + (size_t)3 * nq * p.TY * p.NU +
                       (size_t)warps * 2 * nq * (4 + p.mag[0] * adj_cells(p.mag[0]));
     return (f4 * sizeof(float4) + (size_t)p.lane_words * sizeof(float) + 15) & ~(size_t)15;

@@ -1138,7 +1138,7 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
     const long long V = blk.vox;
     blk.stack_off = 0;
     const FwdPlan& fp = ctx->plan.fwd;
-    blk.cz = adj_cz(fp.mag[2]);
+    blk.cz = adjoint_depth(fp, {{blk.lo[0], blk.lo[1], blk.lo[2]}, {blk.hi[0], blk.hi[1], blk.hi[2]}}, TW, ctx->sm_count);
     forward_tiles(fp, 0, &blk);
     std::vector<TileDesc> tiles;
     for (int tz = 0; tz < blk.ntile[2]; ++tz)
@@ -1165,7 +1165,7 @@ static int adjoint_slab(rfba_ctx* ctx, const rfba_srrf_config* cfg, const float*
                                     gS, gI, ngmap, err, st);
         if (e) return cuda_fail((cudaError_t)e, "temporal adjoint launch");
     }
-    FwdParams rp = adjoint_params(fp, *cfg, iprime, dims);
+    FwdParams rp = adjoint_params(fp, *cfg, iprime, dims, blk.cz);
     rp.lane = static_cast<const float*>(ctx->tables.p);
     rp.utab = reinterpret_cast<const float4*>(rp.lane + ctx->plan.adj_utab);
     rp.blocks = dblk;

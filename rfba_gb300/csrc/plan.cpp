@@ -585,7 +585,7 @@ FwdParams forward_params(const FwdPlan& fp, const rfba_srrf_config& c, const voi
     p.NV = (p.TY - 1) / fp.mag[1] + 2 + 4;
     p.NIX = p.NU + 2 * p.R;
     p.NIY = p.NV + 2 * p.R;
-    p.NIZ = cz + 4 + 2 * p.R;
+    p.NIZ = 4 * tile_quads(cz) + 2 * p.R;
     p.u_region = radiality_u_region(p);
     p.renorm = c.renormalize == 1;
     p.poscon = c.remove_con == 1;
@@ -610,40 +610,58 @@ FwdParams forward_params(const FwdPlan& fp, const rfba_srrf_config& c, const voi
     return p;
 }
 
-FwdParams adjoint_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, const int dims[4]) {
-    FwdParams p = forward_params(fp, c, in, 0, dims, 0, adj_cz(fp.mag[2]));
+FwdParams adjoint_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, const int dims[4], int cz) {
+    FwdParams p = forward_params(fp, c, in, 0, dims, 0, cz);
     p.tma_bx = 0;
     p.u_region = radiality_adjoint_u_region(p);
     p.u_count = (int)(fp.adj_utab.size() / 4);
     return p;
 }
 
+// (tile, volume) pairs of tiles of cz cells and kTileRows rows; tiles: their number along
+// the innermost axis, over the regions
+static long long tile_items(const FwdPlan& fp, const std::vector<FwdRegion>& regions, int T, int cz, double* tiles) {
+    const int mz = fp.mag[2], fz = mz * cz;
+    long long items = 0;
+    for (auto& r : regions) {
+        const int lo = r.lo[fp.ax2], hi = r.hi[fp.ax2];
+        const int n = (hi - (lo / mz) * mz + fz - 1) / fz;
+        if (tiles) *tiles += n;
+        items += (long long)n * ((r.hi[0] - r.lo[0] + kTileX - 1) / kTileX) *
+                 ((r.hi[fp.ax1] - r.lo[fp.ax1] + kTileRows - 1) / kTileRows) * T;
+    }
+    return items;
+}
+
 int forward_depth(const FwdPlan& fp, const std::vector<FwdRegion>& regions, int T, int sms) {
-    if (fp.mag[2] > kDeepMag) return 4;
+    // Two items or fewer to an SM: a launch lasts as long as one item, and a shallower one
+    // ends sooner. 5 x 10x12x12 at mag 2, the whole call: 63.6 us with 8 cells, 55.5 with
+    // 4. At innermost magnifications from kFlatMag on 4 cells are 20 to 32 subvoxels deep
+    // already, and 2 are left: 5x6x8 at mag 6 and 5 axes 86 us with 4 cells, 71 with 2, 8
+    // such volumes (192 items) 97 and 82, 12 of them (288) 110 and 112.
+    const auto few = [&](int cz) { return tile_items(fp, regions, T, cz, nullptr) <= 2LL * sms; };
+    const int shallow = fp.mag[2] >= kFlatMag && few(4) ? 2 : 4;
+    if (fp.mag[2] > kDeepMag || few(8)) return shallow;
     // time per tile column in clocks (one SM, as measured): a point at one subvoxel
     // 29, a pair's second pass at one cell 22, a group's first pass at one cell 7. The
     // same holds for tables in global memory: 20 volumes of 32^3 at 2 x 2 x 2 and 16 axes
     // take 3.82 ms with shallow tiles, 3.13 with deep ones (24^3 at 4 x 4 x 2: 4.65, 4.56)
-    double time[2] = {0, 0};
-    long long items = 0;  // (tile, volume) pairs of the deep tiles
-    for (int i = 0; i < 2; ++i) {
-        const int mz = fp.mag[2], cz = i ? 4 : 8, fz = mz * cz;
+    const auto time = [&](int cz) {
         double tiles = 0;
-        for (auto& r : regions) {
-            const int lo = r.lo[fp.ax2], hi = r.hi[fp.ax2];
-            const int n = (hi - (lo / mz) * mz + fz - 1) / fz;
-            tiles += n;
-            if (i == 0)
-                items += (long long)n * ((r.hi[0] - r.lo[0] + kTileX - 1) / kTileX) *
-                         ((r.hi[fp.ax1] - r.lo[fp.ax1] + kTileRows - 1) / kTileRows) * T;
-        }
-        time[i] = tiles * (fz * 29.0 * fp.npoints + (cz + 4) * (22.0 * fp.npairs + 7.0 * fp.ngroups));
-    }
-    // Two deep items or fewer to an SM: a launch lasts as long as one item, and a
-    // shallow one ends sooner (5 x 10x12x12 at mag 2, the whole call: 63.6 us with
-    // deep tiles, 55.5 with shallow ones).
-    if (items <= 2LL * sms) return 4;
-    return time[1] < time[0] ? 4 : 8;
+        tile_items(fp, regions, T, cz, &tiles);
+        return tiles * (fp.mag[2] * cz * 29.0 * fp.npoints + (cz + 4) * (22.0 * fp.npairs + 7.0 * fp.ngroups));
+    };
+    return time(4) < time(8) ? shallow : 8;
+}
+
+int adjoint_depth(const FwdPlan& fp, const FwdRegion& region, int T, int sms) {
+    // Half the depth for one item or fewer to an SM. Map and derivative of 9x16x16 at mag
+    // 2: one volume (12 items) 263 us with 8 cells, 223 with 4, 12 of them 279 and 251, 24
+    // 338 and 389; 4x4x6 at mag 8: 417 us with 4 cells, 343 with 2. Not built for tables in
+    // global memory, which are no small calls.
+    const int cz = adj_cz(fp.mag[2]);
+    if (fp.adj_utab.size() / 4 > (size_t)kUTabMax) return cz;
+    return tile_items(fp, {region}, T, cz, nullptr) <= sms ? cz / 2 : cz;
 }
 
 void forward_tiles(const FwdPlan& fp, int ty, BlockDev* b) {

@@ -137,9 +137,7 @@ __global__ void __maxnreg__(fwd_regs(MZ, CZ))
     constexpr int HZ = MZ * CH;
     constexpr int FZ = MZ * CZ;
     constexpr int NH = CH + 4;
-    constexpr int NW = CZ + 4;
-    constexpr int NQ = NW / 4;
-    static_assert(CZ % 4 == 0, "whole quads");
+    constexpr int NQ = tile_quads(CZ);
     extern __shared__ float4 smem4[];
 
     // Shared layout: [G planes][U planes, the input tile from plane 1 on][lane tables][TMA staging, 128-byte aligned].
@@ -542,7 +540,7 @@ bool encode_input_map(const FwdParams& p, CUtensorMap* map) {
 }
 
 size_t g4_words(const FwdParams& p) {  // float4s of the G planes
-    const int nq = p.cz / 4 + 1;
+    const int nq = tile_quads(p.cz);
     return (size_t)3 * nq * p.NV * p.NU;
 }
 
@@ -559,6 +557,8 @@ int with_kernel(const FwdParams& p, F&& f) {
         };
         if constexpr (MZ <= kDeepMag)
             if (p.cz == 8) return depth(IntC<8>{});
+        if constexpr (MZ >= kFlatMag)
+            if (p.cz == 2) return depth(IntC<2>{});
         return depth(IntC<4>{});
     };
     switch (p.mag[2]) {
@@ -579,7 +579,7 @@ int with_kernel(const FwdParams& p, F&& f) {
 // float4s of the U planes, which also hold the input tile (from plane 1 on)
 // while the gradient is formed
 int radiality_u_region(const FwdParams& p) {
-    const int nq = p.cz / 4 + 1;
+    const int nq = tile_quads(p.cz);
     const int plane = nq * p.TY * p.NU;
     return std::max(3 * plane, plane + (p.NIX * p.NIY * p.NIZ + 3) / 4);
 }

@@ -176,13 +176,13 @@ __device__ __forceinline__ float4 filter_rows(float4 w, const float4* src, int s
 template <int CH, int NH>
 __device__ __forceinline__ void put_half(float2 (&T)[NH], int w, float v) {
     if (w < NH) T[w].x = v;
-    if (w >= CH) T[w - CH].y = v;
+    if (w >= CH && w - CH < NH) T[w - CH].y = v;
 }
 
 // Sum of what the packed halves hold for cell w (compile-time w).
 template <int CH, int NH>
 __device__ __forceinline__ float get_halves(const float2 (&T)[NH], int w) {
-    return w >= NH ? T[w - CH].y : w < CH ? T[w].x : T[w].x + T[w - CH].y;
+    return w >= NH + CH ? 0.f : w >= NH ? T[w - CH].y : w < CH ? T[w].x : T[w].x + T[w - CH].y;
 }
 
 }  // namespace

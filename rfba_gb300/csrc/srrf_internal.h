@@ -30,7 +30,7 @@ constexpr int fwd_regs(int mz, int cz) { return mz * cz + 6 * (cz / 2 + 4) <= 88
 // The adjoint's tile depth (it holds two sets of columns), its register limit (12
 // (CZ / 2 + 4) for the columns and MZ CZ for dL/dS leave no instance below 128) and the
 // width of an exchange row per x phase (the tile's coarse cells and four zeros).
-constexpr int adj_cz(int mz) { return mz <= 4 ? 8 : 4; }
+constexpr int adj_cz(int mz) { return mz <= 4 ? 8 : 4; }  // half of it for launches of few items
 constexpr int kAdjRegs = 168;
 #ifdef __CUDACC__
 __host__ __device__
@@ -49,7 +49,7 @@ struct BlockDev {
     int int_hi[3];
     int ntile[3];    // tiles along x, y, z
     int nreg[3];     // region extent hi - lo
-    int cz;          // coarse cells per forward tile along its innermost axis (4 or 8)
+    int cz;          // coarse cells per tile along its innermost axis
     long long vox;        // region voxels
     long long stack_off;  // element offset of this block's [t][v] stack slice
     long long out_offset;
@@ -97,6 +97,13 @@ constexpr int kUTabSmall = 768;
 // Deepest innermost magnification with tiles of 8 cells: above it the sums would not fit
 // the registers beside the columns.
 constexpr int kDeepMag = 5;
+// Innermost magnifications from this on have tiles of 2 cells too, for launches of few items.
+constexpr int kFlatMag = 5;
+// Quads of innermost cells that a tile of cz cells and its taps take.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr int tile_quads(int cz) { return (cz + 7) / 4; }
 
 // The forward kernel's plan of a configuration. Its tiles run over (x, mid,
 // innermost) = (x, y, z) or (x, z, y). The first pass filters along mid, once for
@@ -294,14 +301,16 @@ bool build_forward_plan(const rfba_srrf_config& c, FwdPlan* fp, std::string* err
 FwdParams forward_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, int in_u16, const int dims[4],
                          int ty, int cz);
 // The same for the adjoint kernel.
-FwdParams adjoint_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, const int dims[4]);
+FwdParams adjoint_params(const FwdPlan& fp, const rfba_srrf_config& c, const void* in, const int dims[4], int cz);
 // Tiles of a block's region [lo, hi) in the plan's tile axes (b->cz set).
 void forward_tiles(const FwdPlan& fp, int ty, BlockDev* b);
-// Tile depth (innermost cells, 4 or 8) for launches of these regions of T volumes on sms SMs.
+// Tile depth (innermost cells: 2, 4 or 8) for launches of these regions of T volumes on sms SMs,
+// and that of the adjoint for one region.
 struct FwdRegion {
     int lo[3], hi[3];
 };
 int forward_depth(const FwdPlan& fp, const std::vector<FwdRegion>& regions, int T, int sms);
+int adjoint_depth(const FwdPlan& fp, const FwdRegion& region, int T, int sms);
 bool window_range(float ring_radius_dummy, const std::vector<float>& rcoord, int mag, int dim, int* lo, int* hi);
 int fine_window_int(int mag, int dim, int* lo, int* hi);
 

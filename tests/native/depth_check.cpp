@@ -1,6 +1,6 @@
 // Prints, for each line "magx magy magz axes T D H W" of standard input, the tile depth
-// that the library chooses for that whole series on a GPU of 152 SMs, and the sizes of the
-// forward's and the adjoint's uniform tables.
+// that the library chooses for that whole series on a GPU of 152 SMs, the adjoint's, and the
+// sizes of the forward's and the adjoint's uniform tables.
 #include <cstdio>
 #include <string>
 
@@ -19,7 +19,8 @@ int main() {
             std::printf("%s\n", err.c_str());
             return 1;
         }
-        const int cz = rfba::forward_depth(plan, {{{0, 0, 0}, {W * m[0], H * m[1], D * m[2]}}}, T, 152);
-        std::printf("%d %zu %zu\n", cz, plan.utab.size() / 4, plan.adj_utab.size() / 4);
+        const rfba::FwdRegion map = {{0, 0, 0}, {W * m[0], H * m[1], D * m[2]}};
+        std::printf("%d %d %zu %zu\n", rfba::forward_depth(plan, {map}, T, 152),
+                    rfba::adjoint_depth(plan, map, T, 152), plan.utab.size() / 4, plan.adj_utab.size() / 4);
     }
 }
