@@ -636,7 +636,7 @@ __device__ __forceinline__ float4 f4fma(float s, float4 a, float4 c) {
 // is missing, from the derivative in the fixed order. Samples under the bound are ten in a
 // million on a series of 60 volumes of 64^3 at mag 2 (82 thousand; correcting them takes
 // 0.3 of the pair's 42.2 ms), and two of a subvoxel's 62 where a whole volume is a ramp
-// along a ring direction (12 volumes of 64^3 then take 30 to 47 ms instead of 6).
+// along a ring direction (12 volumes of 64^3 then take 20 to 29 ms instead of 6).
 constexpr float kSampleBound = 6e-9f;
 
 // The derivative of one sample's sine term with respect to (-P, E, Z), times K.
@@ -677,14 +677,14 @@ __device__ __forceinline__ void store_shared(float* p, float v) {
     asm volatile("st.shared.f32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "f"(v) : "memory");
 }
 
-// The correction of a pair's samples below the bound, by the whole warp for one subvoxel
-// after another. Of this lane's column, u0, ax, bound and sbase are its first x cell, x
+// The correction of a pair's samples below the bound: each half of the warp takes its own
+// row's columns, one subvoxel after another. Of this lane's column, u0, ax, bound and sbase are its first x cell, x
 // weight index, bound and place in the stacks, marked its subvoxels that have such a
 // sample. Adds to dL/dU what the derivative in the fixed order exceeds the one at the bound
 // by: u = |u| (h x' + c z), x' = (ca, sb) in the x-y plane, the gradient interpolated along
-// x, then y, turned by (ca, sb), then along z; lanes 4 o + i take plane o of z and row i of
-// y. The point loop's frame is this one times scale. Nothing here depends on other tiles or
-// launches. A call takes 1.7 us, out of line so that the point loop keeps its registers
+// x, then y, turned by (ca, sb), then along z; a half's lanes 4 o + i take plane o of z and
+// row i of y. The point loop's frame is this one times scale. Nothing here depends on other tiles or
+// launches. A call takes 1.9 us, out of line so that the point loop keeps its registers
 // (60 volumes of 64^3 at mag 2: 1 pair of a warp in 115 comes here).
 template <int MZ, int CZ>
 __device__ __noinline__ void fix_marked(const FixTile& f, int pair, int u0, int ax, float bound, long long sbase,
@@ -695,17 +695,20 @@ __device__ __noinline__ void fix_marked(const FixTile& f, int pair, int u0, int 
     const int lane = threadIdx.x & 31, o = (lane >> 2) & 3, i = lane & 3;
     const bool y_inner = p.ax1 == 2;
     const float4 r3 = __ldg(p.utab + p.u_pair + 4 * pair + 3);
-    for (unsigned int open = __ballot_sync(full, marked != 0); open; open &= open - 1) {
-        const int src = __ffs(open) - 1;
+    const int half = lane & 16, row = threadIdx.x / kTileX;
+    const float* wm = f.wm + 4 * row;
+    // a half that has no column or subvoxel left goes along with the other's, its own kept out
+    for (unsigned int open = (__ballot_sync(full, marked != 0) >> half) & 0xffff; __any_sync(full, open != 0);
+         open &= open - 1) {
+        const int src = open ? half + __ffs(open) - 1 : lane;
         const int su = __shfl_sync(full, u0, src);
         const float* wx = f.wx + 4 * __shfl_sync(full, ax, src);
         const float least = __shfl_sync(full, bound, src);
         const long long at = __shfl_sync(full, sbase, src);
-        const int row = (threadIdx.x >> 5) * 2 + (src >> 4);
-        const float* wm = f.wm + 4 * row;
-        for (unsigned int left = __shfl_sync(full, marked, src); left; left &= left - 1) {
-            const int z = __ffs(left) - 1;
-            const float gS = f.gS[at + z * f.zstride];
+        const unsigned int subvoxels = __shfl_sync(full, marked, src);
+        for (unsigned int left = open ? subvoxels : 0; __any_sync(full, left != 0); left &= left - 1) {
+            const int z = left ? __ffs(left) - 1 : 0;
+            const float gS = left ? f.gS[at + z * f.zstride] : 0.f;
 #pragma unroll 1
             for (int qi = __float_as_int(r3.x); qi < __float_as_int(r3.y); ++qi) {
                 const float4 fr = __ldg(f.fix + 2 * qi), wt = __ldg(f.fix + 2 * qi + 1);
@@ -730,7 +733,7 @@ __device__ __noinline__ void fix_marked(const FixTile& f, int pair, int u0, int 
                         const float w = y_inner == (pass == 0) ? __ldg(wi + 2 * k) : wm[k];
 #pragma unroll
                         for (int d = 0; d < 3; ++d) {
-                            const float u = __shfl_sync(full, v[d], pass == 0 ? 4 * o + k : 4 * k);
+                            const float u = __shfl_sync(full, v[d], half + (pass == 0 ? 4 * o + k : 4 * k));
                             acc[d] = k ? fmaf(w, u, acc[d]) : w * u;
                         }
                     }
@@ -747,7 +750,7 @@ __device__ __noinline__ void fix_marked(const FixTile& f, int pair, int u0, int 
                                                        scale * scale * rsqrt_approx(fmaxf(xx * s4, least)));
                 const float dP = q.P - e.P, dE = e.E - q.E;
                 const float dG[3] = {fmaf(dE, -fr.y, dP * fr.x), fmaf(dE, fr.x, dP * fr.y), e.Z - q.Z};
-                if (lane < 16) {
+                if (left) {
                     const int w = w0 + o;
                     const float spread = __ldg(wi + 2 * o) * wx[i];
 #pragma unroll
